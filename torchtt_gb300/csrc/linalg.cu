@@ -1,5 +1,5 @@
 // FP64 dense linear algebra: shifted CholeskyQR3 with a Householder fallback, one-sided Jacobi
-// thin SVD, LU solve with partial pivoting.
+// thin SVD.
 //
 // GB300 note: FP64 runs at ~1.9 FMA/clock/SM (measured), so every O(m n^2) step is expressed as a
 // GEMM on the contraction engine (spread over all SMs); only O(n^3) steps on the small n x n
@@ -867,81 +867,6 @@ __global__ void __launch_bounds__(1024) svd_sort_kernel(const double* __restrict
   }
 }
 
-// ---------------------------------------------------------------------------------------------
-// LU with partial pivoting on an n x n row-major copy, solving for one right-hand side.
-// ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) lu_solve_kernel(double* LU, double* x, int n, int* status) {
-  __shared__ double shv[32];
-  __shared__ double piv_inv;
-  __shared__ int shi[32];
-  __shared__ int piv;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  for (int j = 0; j < n; ++j) {
-    // pivot search
-    double best = -1.0;
-    int bi = j;
-    for (int i = j + tid; i < n; i += nt) {
-      const double v = fabs(LU[(int64_t)i * n + j]);
-      if (v > best) { best = v; bi = i; }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ov = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
-    if (lane == 0) { shv[warp] = best; shi[warp] = bi; }
-    __syncthreads();
-    if (tid == 0) {
-      double b = -1.0; int ib = j;
-      for (int w = 0; w < (nt >> 5); ++w)
-        if (shv[w] > b || (shv[w] == b && shi[w] < ib)) { b = shv[w]; ib = shi[w]; }
-      piv = ib;
-      if (!(b > 0.0)) *status = 1;
-    }
-    __syncthreads();
-    const int p = piv;
-    if (p != j) {
-      for (int c = tid; c < n; c += nt) {
-        const double t = LU[(int64_t)j * n + c];
-        LU[(int64_t)j * n + c] = LU[(int64_t)p * n + c];
-        LU[(int64_t)p * n + c] = t;
-      }
-      if (tid == 0) { const double t = x[j]; x[j] = x[p]; x[p] = t; }
-    }
-    __syncthreads();
-    if (tid == 0) piv_inv = 1.0 / LU[(int64_t)j * n + j];   // one FP64 division per step
-    __syncthreads();
-    const double inv = piv_inv;
-    const int w = n - j - 1;
-    // multipliers
-    for (int i = j + 1 + tid; i < n; i += nt) LU[(int64_t)i * n + j] *= inv;
-    __syncthreads();
-    for (int i = j + 1 + tid; i < n; i += nt) x[i] = fma(-LU[(int64_t)i * n + j], x[j], x[i]);
-    for (int64_t t = tid; t < (int64_t)w * w; t += nt) {
-      const int i = j + 1 + (int)(t / w), c = j + 1 + (int)(t % w);
-      LU[(int64_t)i * n + c] = fma(-LU[(int64_t)i * n + j], LU[(int64_t)j * n + c], LU[(int64_t)i * n + c]);
-    }
-    __syncthreads();
-  }
-  // back substitution
-  __shared__ double shs[32];
-  for (int i = n - 1; i >= 0; --i) {
-    double s = 0.0;
-    for (int c = i + 1 + tid; c < n; c += nt) s = fma(LU[(int64_t)i * n + c], x[c], s);
-    s = warp_sum_d(s);
-    if (lane == 0) shs[warp] = s;
-    __syncthreads();
-    if (tid == 0) {
-      double t = 0.0;
-      for (int w2 = 0; w2 < (nt >> 5); ++w2) t += shs[w2];
-      x[i] = (x[i] - t) / LU[(int64_t)i * n + i];
-    }
-    __syncthreads();
-  }
-}
-
 __global__ void gemv_rm_kernel(const double* __restrict__ B, int64_t n, const double* __restrict__ x,
                                double* y) {
   const int lane = threadIdx.x & 31;
@@ -1198,15 +1123,6 @@ void svd(const double* A, int64_t lda, int64_t m, int64_t n, double* U, double* 
   gemm_cm(Qb.p, m, Vw, n, U, m, m, n, n, 1.0, 0.0, s);
   // Vh (n x n col-major) = U'^T
   transpose(Up.p, n, Vh, n, n, n, s);
-}
-
-void lu_solve(const double* B, int64_t n, const double* rhs, double* x, LinalgWS& ws,
-              cudaStream_t s) {
-  ws.e.ensure(n * n + 16, s);
-  copy(B, ws.e.p, n * n, s);
-  copy(rhs, x, n, s);
-  lu_solve_kernel<<<1, 1024, 0, s>>>(ws.e.p, x, (int)n, ws.status);
-  TTGB_CHECK_LAUNCH();
 }
 
 void gemv(const double* B, int64_t n, const double* x, double* y, cudaStream_t s) {
