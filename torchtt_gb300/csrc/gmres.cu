@@ -62,7 +62,6 @@ namespace {
 
 using red::RT;
 using red::block_sum;
-constexpr int KC = 8;          // vectors per chunk of the projection's multi-dot
 constexpr int kMaxVec = 128;   // basis vectors a cycle may hold (RedWS::cap_vec + 1)
 
 // scalar slots after the Hessenberg data in GmresWS::small
@@ -72,24 +71,19 @@ enum ScalSlot : int {
   kWNorm2,        // ||w||^2 of the operator output, before orthogonalisation
   kHn,            // H[k+1, k]
   kErr,           // |beta[k+1]| / ||rhs||
-  kWpNorm2,       // ||w'||^2 after the first projection
-  kHp,            // the norm the finishing pass divides by
-  kInv,           // its reciprocal
-  kMode,          // 0: one projection kept, 1: second projection, 2: second projection, norm taken directly
   kNumScal = 12
 };
 
 struct Layout {   // GmresWS::small
   int iters;
-  int64_t H, cs, sn, beta, h1, h2, scal, total;
+  int64_t H, cs, sn, beta, h1, scal, total;
   explicit Layout(int it) : iters(it) {
     H = 0;
     cs = H + (int64_t)(it + 1) * it;
     sn = cs + it;
     beta = sn + it;
     h1 = beta + it + 1;
-    h2 = h1 + it + 1;
-    scal = h2 + it + 1;
+    scal = h1 + it + 1;
     total = scal + kNumScal;
   }
 };
@@ -155,190 +149,348 @@ __global__ void scale_by_kernel(const double* x, double* y, int64_t n, const dou
   }
 }
 
-// Arnoldi pass 1: h1 = V^T w over the kv basis vectors, and ||w||^2.
+// ---------------------------------------------------------------------------------------------
+// The Arnoldi step in three launches over the basis V (kv vectors of n doubles).
+//
+// On GB300 a warp-wide FP64 instruction holds the SM's FP64 pipe for 16 cycles, so at these sizes
+// the multiply-adds (kv n per pass) weigh less than the adds of the reductions: a butterfly per
+// vector and warp costs 5 instructions for every multiply-add of a 32-element slice. The passes
+// therefore deal the vectors, not the elements, to the warps of a block (warp w takes the vectors
+// w, w + 8, ...; a lane accumulates E elements of each before any reduction), reduce the vectors of
+// a warp together (a step halves the number of values as it halves the lanes: 9 adds for 8 vectors
+// instead of 40), and leave the sum over the blocks to the blocks of the next launch, each of which
+// adds the G x nv partial sums for itself, so that no pass ends in one block's serial tail.
+// Measured per launch (n = 4 k to 32 k, kv up to 41): project 2.3-7 us, update 4-16 us, finish 8-17 us;
+// with the elements dealt to the warps and the last block adding the partial sums 18, 31 and 13.5 us.
+// ---------------------------------------------------------------------------------------------
+constexpr int kWarps = RT / 32;
+
+// Sums of NV per-lane values over the warp's 32 lanes (NV a power of two). On return the lane holds
+// the sum of value j = lane / (32 / NV).
+template <int NV>
+__device__ __forceinline__ double warp_sums(double (&v)[NV]) {
+  const int lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int m = NV; m > 1; m >>= 1, o >>= 1) {
+    const bool upper = (lane & o) != 0;
+#pragma unroll
+    for (int j = 0; j < m / 2; ++j) {   // keep one half of the values, send the other
+      const double send = upper ? v[j] : v[j + m / 2];
+      const double keep = upper ? v[j + m / 2] : v[j];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  double s = v[0];
+#pragma unroll
+  for (int q = 16 / NV; q > 0; q >>= 1) s += __shfl_xor_sync(0xffffffffu, s, q);
+  return s;
+}
+
+// Partial sums of the warp's vectors (acc[i]: vector warp + 8 i, nv vectors in all) into row
+// blockIdx.x of part.
+template <int VP>
+__device__ __forceinline__ void store_partials(const double (&acc)[VP], int nv, double* part) {
+  constexpr int N = VP <= 1 ? 1 : VP <= 2 ? 2 : VP <= 4 ? 4 : 8;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* row = part + (int64_t)blockIdx.x * nv;
+#pragma unroll
+  for (int g = 0; g < VP; g += N) {
+    if (warp + kWarps * g >= nv) break;   // uniform in the warp
+    double v[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] = g + j < VP ? acc[g + j < VP ? g + j : 0] : 0.0;
+    const double s = warp_sums<N>(v);
+    const int vec = warp + kWarps * (g + lane / (32 / N));
+    if (lane % (32 / N) == 0 && vec < nv) row[vec] = s;
+  }
+}
+
+// out[v] (shared, v < nv <= 128) = sum over the G rows of part of its column v, in a fixed order;
+// sh holds RT doubles. Every thread of the block calls it.
+__device__ __forceinline__ void reduce_partials(const double* part, int G, int nv, double* out,
+                                                double* sh) {
+  int width = 8;
+  while (width < nv) width <<= 1;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int col = tid & (width - 1), first = tid / width, step = RT / width;
+  double s = 0.0;
+  if (col < nv) {
+#pragma unroll 8
+    for (int g = first; g < G; g += step) s += __ldcg(part + (int64_t)g * nv + col);
+  }
+  int rows = step;
+  if (width < 32) {
+    for (int o = width; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane < width) sh[(tid >> 5) * width + lane] = s;
+    rows = kWarps;
+  } else {
+    sh[tid] = s;
+  }
+  __syncthreads();
+  if (tid < nv) {
+    double t = 0.0;
+    for (int q = 0; q < rows; ++q) t += sh[q * width + tid];
+    out[tid] = t;
+  }
+  __syncthreads();
+}
+
+// Pass 1: part[block] = partial sums of h1 = V^T w (kv values) and ||w||^2.
+template <int E, int VP>
 __global__ void __launch_bounds__(RT) arnoldi_project_kernel(const double* __restrict__ Q,
                                                               int64_t ldq, int kv,
                                                               const double* __restrict__ w,
-                                                              int64_t n, int64_t chunk,
-                                                              double* partial, unsigned* counter,
-                                                              double* h1, double* scal,
+                                                              int64_t n, int64_t chunk, double* part,
                                                               const int* gate) {
-  __shared__ double sh[32];
-  __shared__ double shv[(RT / 32) * KC];
   if (*gate != 0) return;   // an iteration queued past the cycle's stopping point
-  const int G = gridDim.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t beg = blockIdx.x * chunk, end = min(n, beg + chunk);
-  double ww = 0.0;
-  for (int c0 = 0; c0 < kv; c0 += KC) {
-    double acc[KC];
+  double acc[VP];
 #pragma unroll
-    for (int j = 0; j < KC; ++j) acc[j] = 0.0;
-    const int nc = min(KC, kv - c0);
-    for (int64_t i = beg + threadIdx.x; i < end; i += blockDim.x) {
-      const double qv = w[i];
-      if (c0 == 0) ww = fma(qv, qv, ww);
+  for (int i = 0; i < VP; ++i) acc[i] = 0.0;
+  for (int64_t c = beg; c < end; c += 32 * E) {
+    double x[E];
 #pragma unroll
-      for (int j = 0; j < KC; ++j)
-        if (j < nc) acc[j] = fma(Q[(int64_t)(c0 + j) * ldq + i], qv, acc[j]);
+    for (int e = 0; e < E; ++e) {
+      const int64_t i = c + e * 32 + lane;
+      x[e] = i < end ? w[i] : 0.0;
     }
-    red::block_sums_to_partials<KC>(acc, nc, shv, partial, c0, G);
+#pragma unroll
+    for (int i = 0; i < VP; ++i) {
+      const int v = warp + kWarps * i;
+      if (v > kv) break;
+      const double* q = v < kv ? Q + (int64_t)v * ldq : w;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int64_t t = c + e * 32 + lane;
+        acc[i] = fma(t < end ? q[t] : 0.0, x[e], acc[i]);
+      }
+    }
   }
-  ww = block_sum(ww, sh);
-  if (threadIdx.x == 0) partial[(int64_t)kv * G + blockIdx.x] = ww;
-  if (!red::take_last_ticket(counter)) return;
-  red::reduce_vectors(partial, kv + 1, G, [&](int v, double t) {
-    if (v < kv) h1[v] = t;
-    else scal[kWNorm2] = t;
-  });
-  red::reset_ticket(counter);
+  store_partials<VP>(acc, kv + 1, part);
 }
 
-// Arnoldi pass 2: w' = w - V h1 and, in the same pass over V, h2 = V^T w' and ||w'||^2. With
-// KB > 0 (kv <= KB) each thread keeps its element's kv basis entries and the kv partial dots in
-// registers, so V is read once; KB = 0 re-reads the block's slice of V for the dots. The last block chooses
-// the finishing pass (classical Gram-Schmidt with the reorthogonalisation criterion of Daniel,
-// Gragg, Kaufman and Stewart, Math. Comp. 30 (1976), with eta = 1/sqrt(2)):
-//   mode 0: ||w'||^2 >= ||w||^2 / 2, the first projection is kept, hp = ||w'||;
+// t = the block's slice of V h (h in shared memory): the warps' shares through sh (8 x 32 E doubles);
+// element c of the slice is returned to thread c (0 past the slice).
+template <int E, int VP>
+__device__ __forceinline__ double slice_combination(const double* __restrict__ Q, int64_t ldq, int kv,
+                                                    const double* h, int64_t c, int64_t end,
+                                                    double* sh) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double t[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) t[e] = 0.0;
+#pragma unroll
+  for (int i = 0; i < VP; ++i) {
+    const int v = warp + kWarps * i;
+    if (v >= kv) break;
+    const double hv = h[v];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int64_t j = c + e * 32 + lane;
+      t[e] = fma(hv, j < end ? Q[(int64_t)v * ldq + j] : 0.0, t[e]);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e) sh[warp * 32 * E + e * 32 + lane] = t[e];
+  __syncthreads();
+  double s = 0.0;
+  const int used = min(kv, kWarps);   // the other warps hold zeros
+  if (threadIdx.x < 32 * E)
+    for (int q = 0; q < used; ++q) s += sh[q * 32 * E + threadIdx.x];
+  return s;
+}
+
+// Pass 2: w' = w - V h1, and the partial sums of h2 = V^T w' and ||w'||^2 (V's slice is read again from
+// the L1 cache). Block 0 keeps h1 and ||w||^2 for the finishing pass.
+template <int E, int VP>
+__global__ void __launch_bounds__(RT) arnoldi_reorth_kernel(const double* __restrict__ Q,
+                                                             int64_t ldq, int kv, double* w, int64_t n,
+                                                             int64_t chunk, const double* part_in,
+                                                             double* part_out, double* h1, double* scal,
+                                                             const int* gate) {
+  __shared__ double sums[kMaxVec];
+  __shared__ double sh[kWarps * 32 * E];
+  __shared__ double wn[32 * E];
+  if (*gate != 0) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  reduce_partials(part_in, gridDim.x, kv + 1, sums, sh);
+  if (blockIdx.x == 0 && tid <= kv) {
+    if (tid < kv) h1[tid] = sums[tid];
+    else scal[kWNorm2] = sums[kv];
+  }
+  const int64_t beg = blockIdx.x * chunk, end = min(n, beg + chunk);
+  double acc[VP];
+#pragma unroll
+  for (int i = 0; i < VP; ++i) acc[i] = 0.0;
+  for (int64_t c = beg; c < end; c += 32 * E) {
+    const double s = slice_combination<E, VP>(Q, ldq, kv, sums, c, end, sh);
+    if (tid < 32 * E) {
+      double v = 0.0;
+      if (c + tid < end) {
+        v = w[c + tid] - s;
+        w[c + tid] = v;
+      }
+      wn[tid] = v;
+    }
+    __syncthreads();
+    double x[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) x[e] = wn[e * 32 + lane];
+#pragma unroll
+    for (int i = 0; i < VP; ++i) {
+      const int v = warp + kWarps * i;
+      if (v > kv) break;
+      const double* q = Q + (int64_t)v * ldq;   // row kv is w itself, whose slice is in x
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int64_t t = c + e * 32 + lane;
+        acc[i] = fma(v < kv ? (t < end ? q[t] : 0.0) : x[e], x[e], acc[i]);
+      }
+    }
+  }
+  store_partials<VP>(acc, kv + 1, part_out);
+}
+
+// The Givens rotations of the cycle applied to the new Hessenberg column h (k + 2 values, shared
+// memory), the new rotation, the residual estimate and the stop flag (apply_givens_rotation_cpu and
+// the convergence test, cpp/gmres.h:20-31,105-129). One warp; cs and sn are read in parallel first.
+__device__ __forceinline__ void givens_step(double* h, double* rot, int k, int iters, double hn,
+                                            double* H, double* cs, double* sn, double* beta,
+                                            double threshold, double* scal, int* flag, int reorth_vecs) {
+  const int lane = threadIdx.x & 31;
+  for (int i = lane; i < k; i += 32) {
+    rot[2 * i] = cs[i];
+    rot[2 * i + 1] = sn[i];
+  }
+  __syncwarp();
+  double* hc = H + (int64_t)k * (iters + 1);
+  if (lane == 0) {
+    double cur = h[0];
+    for (int i = 0; i < k; ++i) {
+      const double c = rot[2 * i], s = rot[2 * i + 1], nx = h[i + 1];
+      h[i] = c * cur + s * nx;
+      cur = c * nx - s * cur;
+    }
+    const double den = sqrt(cur * cur + hn * hn);
+    double c = 1.0, s = 0.0;
+    if (den > 0.0) { c = cur / den; s = hn / den; }
+    h[k] = c * cur + s * hn;
+    h[k + 1] = 0.0;
+    cs[k] = c;
+    sn[k] = s;
+    const double bk = beta[k], b1 = -s * bk;
+    beta[k + 1] = b1;
+    beta[k] = c * bk;
+    const double err = fabs(b1) / scal[kRhsNorm];
+    scal[kErr] = err;
+    scal[kHn] = hn;
+    const bool breakdown = !(hn > 0.0) || !isfinite(hn);
+    int state = (err <= threshold || breakdown) ? 1 : 0;
+    if (!isfinite(err)) state = 3;
+    flag[kGmresBreakdown] = breakdown ? 1 : 0;
+    if (state != 0) flag[kGmresAtIter] = k;
+    if (reorth_vecs > 0) {
+      flag[kGmresReorth] += 1;
+      flag[kGmresReorthVecs] += reorth_vecs;
+    }
+    flag[kGmresState] = state;
+  }
+  __syncwarp();
+  for (int i = lane; i < k + 2; i += 32) hc[i] = h[i];
+}
+
+// Pass 3. Every block adds the partial sums of pass 2 and takes the same decision (classical
+// Gram-Schmidt with the reorthogonalisation criterion of Daniel, Gragg, Kaufman and Stewart, Math.
+// Comp. 30 (1976), with eta = 1/sqrt(2)):
+//   mode 0: ||w'||^2 >= ||w||^2 / 2, the first projection is kept, q = w' / ||w'||;
 //   mode 1: w'' = w' - V h2 with ||w''||^2 = ||w'||^2 - ||h2||^2 (V orthonormal), used while the
 //           difference keeps at least half of ||w'||^2 (no cancellation to speak of);
 //   mode 2: w'' = w' - V h2 with its norm taken from the finished vector (near breakdown).
-template <int KB>
-__global__ void __launch_bounds__(RT, KB <= 8 ? 2 : 1) arnoldi_reorth_kernel(const double* __restrict__ Q,
-                                                             int64_t ldq, int kv,
-                                                             const double* __restrict__ h1,
-                                                             double* w, int64_t n, int64_t chunk,
-                                                             double* partial, unsigned* counter,
-                                                             double* h2, double* scal,
-                                                             const int* gate, double orth_tol2) {
-  __shared__ double sh[32];
-  __shared__ double hs[kMaxVec];
-  __shared__ double sums[kMaxVec + 1];
-  __shared__ double shv[(RT / 32) * (KB > KC ? KB : KC)];
-  if (*gate != 0) return;
-  const int G = gridDim.x;
-  const int64_t beg = blockIdx.x * chunk, end = min(n, beg + chunk);
-  for (int j = threadIdx.x; j < kv; j += blockDim.x) hs[j] = h1[j];
-  __syncthreads();
-  double ss = 0.0;
-  if constexpr (KB > 0) {
-    double acc[KB];
-#pragma unroll
-    for (int j = 0; j < KB; ++j) acc[j] = 0.0;
-    for (int64_t i = beg + threadIdx.x; i < end; i += blockDim.x) {
-      double q[KB];
-      double v = w[i];
-#pragma unroll
-      for (int j = 0; j < KB; ++j) {
-        if (j < kv) {
-          q[j] = Q[(int64_t)j * ldq + i];
-          v = fma(-hs[j], q[j], v);
-        }
-      }
-      w[i] = v;
-      ss = fma(v, v, ss);
-#pragma unroll
-      for (int j = 0; j < KB; ++j)
-        if (j < kv) acc[j] = fma(q[j], v, acc[j]);
-    }
-    red::block_sums_to_partials<(KB > 0 ? KB : 1)>(acc, kv, shv, partial, 0, G);
-  } else {
-    for (int64_t i = beg + threadIdx.x; i < end; i += blockDim.x) {
-      double v = w[i];
-      for (int j = 0; j < kv; ++j) v = fma(-hs[j], Q[(int64_t)j * ldq + i], v);
-      w[i] = v;
-      ss = fma(v, v, ss);
-    }
-    for (int c0 = 0; c0 < kv; c0 += KC) {   // each thread re-reads only the elements it wrote
-      double acc[KC];
-#pragma unroll
-      for (int j = 0; j < KC; ++j) acc[j] = 0.0;
-      const int nc = min(KC, kv - c0);
-      for (int64_t i = beg + threadIdx.x; i < end; i += blockDim.x) {
-        const double qv = w[i];
-#pragma unroll
-        for (int j = 0; j < KC; ++j)
-          if (j < nc) acc[j] = fma(Q[(int64_t)(c0 + j) * ldq + i], qv, acc[j]);
-      }
-      red::block_sums_to_partials<KC>(acc, nc, shv, partial, c0, G);
-    }
-  }
-  ss = block_sum(ss, sh);
-  if (threadIdx.x == 0) partial[(int64_t)kv * G + blockIdx.x] = ss;
-  if (!red::take_last_ticket(counter)) return;
-  red::reduce_vectors(partial, kv + 1, G, [&](int v, double t) {
-    sums[v] = t;
-    if (v < kv) h2[v] = t;
-  });
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const double a = sums[kv], ww = scal[kWNorm2];
-    double b = 0.0;
-    for (int j = 0; j < kv; ++j) b = fma(sums[j], sums[j], b);
-    double mode, hp, inv;
-    // b <= orth_tol^2 a: the new vector's component along the basis, |V^T w'| / |w'|, is already
-    // below the tolerated loss of orthogonality, so the second projection is not needed either
-    if (!(a < 0.5 * ww) || (a > 0.0 && b <= orth_tol2 * a)) {   // NaN: the finishing pass reports it
-      mode = 0.0;
-      hp = sqrt(a);
-      inv = (hp > 0.0) ? 1.0 / hp : 1.0;
-    } else if (a > 0.0 && a - b >= 0.5 * a) {
-      mode = 1.0;
-      hp = sqrt(a - b);
-      inv = 1.0 / hp;
-    } else {
-      mode = 2.0;
-      hp = 1.0;
-      inv = 1.0;
-    }
-    scal[kWpNorm2] = a;
-    scal[kHp] = hp;
-    scal[kInv] = inv;
-    scal[kMode] = mode;
-  }
-  red::reset_ticket(counter);
-}
-
-// Arnoldi pass 3: q_{k+1} = (w' - V h2) / hp (mode 1, 2) or w' / hp (mode 0), and its norm nu;
-// with a split target, q_{k+1} is also written as the tcgen05 engine's TF32 operand, so the next
-// operator application starts from it without a split launch.
-// The last block corrects the scale when nu is not 1 to rounding (mode 2, or a cancelled norm),
-// then applies the Givens rotations to the new Hessenberg column, takes the new one, and updates
-// the residual estimate and the stop flag (apply_givens_rotation_cpu and the convergence test,
-// cpp/gmres.h:20-31,105-129). Once the flag is set, later iterations leave H, beta and the flag
+// b <= orth_tol^2 a (the new vector's component along the basis, |V^T w'| / |w'|, is already below the
+// tolerated loss of orthogonality) also takes mode 0. With a split target, q is also written as
+// the tcgen05 engine's TF32 operand, so the next operator application starts from it without a
+// split launch. In mode 0 the norm is known and block 0 takes the Givens step while the others write; in
+// modes 1 and 2 the last block takes it, after it has corrected the scale where the finished vector's
+// norm is not 1 to rounding. Once the flag is set, later iterations leave H, beta and the flag
 // alone, so iterations queued past the stopping point change nothing the solution uses.
+template <int E, int VP>
 __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
     const double* __restrict__ Q, int64_t ldq, int kv, const double* __restrict__ h1,
-    const double* __restrict__ h2, double* w, int64_t n, int64_t chunk, double* partial,
-    unsigned* counter, double* scal, int k, int iters, double* H, double* cs, double* sn,
-    double* beta, double threshold, int* flag, SplitOut so) {
-  __shared__ double sh[32];
-  __shared__ double hs[kMaxVec];
+    const double* part_in, double* w, int64_t n, int64_t chunk, double* part_out, unsigned* counter,
+    double* scal, int iters, double* H, double* cs, double* sn, double* beta, double threshold,
+    int* flag, SplitOut so, double orth_tol2) {
+  __shared__ double sums[kMaxVec];          // h2 and ||w'||^2
+  __shared__ double sh[kWarps * 32 * E];
+  __shared__ double hcol[kMaxVec + 1], rot[2 * kMaxVec];
+  __shared__ double dec[3];                 // mode, norm, 1 / norm
   __shared__ double fac;
   if (flag[kGmresState] != 0) return;   // queued past the stopping point: nothing changes
-  const int mode = (int)scal[kMode];
-  const double inv = scal[kInv];
-  if (mode != 0)
-    for (int j = threadIdx.x; j < kv; j += blockDim.x) hs[j] = h2[j];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  reduce_partials(part_in, gridDim.x, kv + 1, sums, sh);
+  if (warp == 0) {
+    double b = 0.0;
+    for (int j = lane; j < kv; j += 32) b = fma(sums[j], sums[j], b);
+    b = red::warp_sum(b);
+    if (lane == 0) {
+      const double a = sums[kv], ww = scal[kWNorm2];
+      double mode, hp, inv;
+      if (!(a < 0.5 * ww) || (a > 0.0 && b <= orth_tol2 * a)) {   // NaN: the Givens step reports it
+        mode = 0.0;
+        hp = sqrt(a);
+        inv = (hp > 0.0) ? 1.0 / hp : 1.0;
+      } else if (a > 0.0 && a - b >= 0.5 * a) {
+        mode = 1.0;
+        hp = sqrt(a - b);
+        inv = 1.0 / hp;
+      } else {
+        mode = 2.0;
+        hp = 1.0;
+        inv = 1.0;
+      }
+      dec[0] = mode;
+      dec[1] = hp;
+      dec[2] = inv;
+    }
+  }
   __syncthreads();
+  const int mode = (int)dec[0], k = kv - 1;
+  const double hp = dec[1], inv = dec[2];
   const int64_t beg = blockIdx.x * chunk, end = min(n, beg + chunk);
+  if (mode == 0) {
+    for (int64_t i = beg + tid; i < end; i += RT) {
+      const double v = w[i] * inv;
+      w[i] = v;
+      if (so.hi) put_split(so, i, v);
+    }
+    if (blockIdx.x != 0 || warp != 0) return;
+    for (int i = lane; i <= k; i += 32) hcol[i] = h1[i];
+    __syncwarp();
+    // a block that starts after this has set the flag leaves its slice of q unscaled: the cycle has
+    // ended then, and its solution does not use q
+    givens_step(hcol, rot, k, iters, hp, H, cs, sn, beta, threshold, scal, flag, 0);
+    return;
+  }
   double ss = 0.0;
-  for (int64_t i = beg + threadIdx.x; i < end; i += blockDim.x) {
-    double v = w[i];
-    if (mode != 0)
-      for (int j = 0; j < kv; ++j) v = fma(-hs[j], Q[(int64_t)j * ldq + i], v);
-    v *= inv;
-    w[i] = v;
-    if (so.hi) put_split(so, i, v);
-    ss = fma(v, v, ss);
+  for (int64_t c = beg; c < end; c += 32 * E) {
+    const double s = slice_combination<E, VP>(Q, ldq, kv, sums, c, end, sh);
+    if (tid < 32 * E && c + tid < end) {
+      const double v = (w[c + tid] - s) * inv;
+      w[c + tid] = v;
+      if (so.hi) put_split(so, c + tid, v);
+      ss = fma(v, v, ss);
+    }
+    __syncthreads();
   }
   ss = block_sum(ss, sh);
-  if (threadIdx.x == 0) partial[blockIdx.x] = ss;
+  if (tid == 0) part_out[blockIdx.x] = ss;
   if (!red::take_last_ticket(counter)) return;
   double tot = 0.0;
-  if (threadIdx.x < 32) tot = red::warp_sum_partials(partial, 0, gridDim.x);
-  if (threadIdx.x == 0) {
+  if (warp == 0) tot = red::warp_sum_partials(part_out, 0, gridDim.x);
+  if (tid == 0) {
     const double nu = sqrt(tot);
-    double hn = scal[kHp], f = 1.0;
+    double hn = hp, f = 1.0;
     if (mode == 2) {
       hn = nu;
       if (nu > 0.0) f = 1.0 / nu;
@@ -347,42 +499,16 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
       hn *= nu;
     }
     fac = f;
-    scal[kHn] = hn;
-    if (flag[kGmresState] == 0) {
-      double* hc = H + (int64_t)k * (iters + 1);
-      for (int i = 0; i <= k; ++i) hc[i] = (mode != 0) ? h1[i] + h2[i] : h1[i];
-      hc[k + 1] = hn;
-      for (int i = 0; i < k; ++i) {   // apply_givens_rotation_cpu, gmres.h:20-31
-        const double t = cs[i] * hc[i] + sn[i] * hc[i + 1];
-        hc[i + 1] = -sn[i] * hc[i] + cs[i] * hc[i + 1];
-        hc[i] = t;
-      }
-      const double den = sqrt(hc[k] * hc[k] + hc[k + 1] * hc[k + 1]);
-      double c = 1.0, s = 0.0;
-      if (den > 0.0) { c = hc[k] / den; s = hc[k + 1] / den; }
-      hc[k] = c * hc[k] + s * hc[k + 1];
-      hc[k + 1] = 0.0;
-      cs[k] = c;
-      sn[k] = s;
-      beta[k + 1] = -s * beta[k];
-      beta[k] = c * beta[k];
-      const double err = fabs(beta[k + 1]) / scal[kRhsNorm];
-      scal[kErr] = err;
-      const bool breakdown = !(hn > 0.0) || !isfinite(hn);
-      int state = (err <= threshold || breakdown) ? 1 : 0;
-      if (!isfinite(err)) state = 3;
-      flag[kGmresState] = state;
-      flag[kGmresBreakdown] = breakdown ? 1 : 0;
-      if (state != 0) flag[kGmresAtIter] = k;
-      if (mode != 0) {
-        flag[kGmresReorth] += 1;
-        flag[kGmresReorthVecs] += kv;
-      }
-    }
+    dec[1] = hn;
   }
   __syncthreads();
+  if (warp == 0) {
+    for (int i = lane; i <= k; i += 32) hcol[i] = h1[i] + sums[i];
+    __syncwarp();
+    givens_step(hcol, rot, k, iters, dec[1], H, cs, sn, beta, threshold, scal, flag, kv);
+  }
   if (fac != 1.0) {   // rare: only when the direct norm differs from the divisor used above
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+    for (int64_t i = tid; i < n; i += RT) {
       const double v = w[i] * fac;
       w[i] = v;
       if (so.hi) put_split(so, i, v);
@@ -393,8 +519,10 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
 
 // sol += V[:, 0..kk] y (sol = V y when `first`, the start x0 = 0) with
 // y = H[0..kk, 0..kk]^{-1} beta[0..kk] (upper triangular after the rotations; gmres.h:131-139).
-// Every block solves the small triangular system itself (warp 0, the inner sums across the
-// warp), then adds its slice of the combination.
+// Every block solves the small triangular system itself, then adds its slice of the combination.
+// The solve runs by columns in one warp: the divisions are taken at once before it, and a step is
+// one broadcast and one multiply-add per 32 rows (by rows, with a sum over the warp and a division
+// per step, the launch took 28-43 us; now 10-13).
 __global__ void __launch_bounds__(RT) cycle_update_kernel(int kk, int iters, const double* H,
                                                            const double* beta,
                                                            const double* __restrict__ Q,
@@ -403,15 +531,26 @@ __global__ void __launch_bounds__(RT) cycle_update_kernel(int kk, int iters, con
   __shared__ double ys[kMaxVec];
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
-    for (int i = kk; i >= 0; --i) {
-      double t = 0.0;
-      for (int j = i + 1 + lane; j <= kk; j += 32) t = fma(H[(int64_t)j * (iters + 1) + i], ys[j], t);
-      t = red::warp_sum(t);
-      if (lane == 0) {
-        const double d = H[(int64_t)i * (iters + 1) + i];
-        ys[i] = (d != 0.0) ? (beta[i] - t) / d : 0.0;
+    double b[kMaxVec / 32], r[kMaxVec / 32];
+#pragma unroll
+    for (int q = 0; q < kMaxVec / 32; ++q) {
+      const int i = q * 32 + lane;
+      const double d = i <= kk ? H[(int64_t)i * (iters + 1) + i] : 0.0;
+      b[q] = i <= kk ? beta[i] : 0.0;
+      r[q] = d != 0.0 ? 1.0 / d : 0.0;
+    }
+#pragma unroll
+    for (int q = kMaxVec / 32 - 1; q >= 0; --q) {
+      for (int i = min(kk, q * 32 + 31); i >= q * 32; --i) {
+        const double* col = H + (int64_t)i * (iters + 1);
+        const double y = __shfl_sync(0xffffffffu, b[q] * r[q], i & 31);
+        if (lane == 0) ys[i] = y;
+#pragma unroll
+        for (int t = 0; t <= q; ++t) {
+          const int row = t * 32 + lane;
+          if (row < i) b[t] = fma(-y, col[row], b[t]);
+        }
       }
-      __syncwarp();
     }
   }
   __syncthreads();
@@ -431,18 +570,56 @@ unsigned elem_grid(int64_t n) {
   return g;
 }
 
-void launch_reorth(int kv, dim3 g, const double* Q, int64_t ldq, const double* h1, double* w,
-                   int64_t n, int64_t chunk, const RedWS& red, double* h2, double* scal,
-                   const int* gate, double orth_tol2, cudaStream_t s) {
-  if (kv <= 4)
-    arnoldi_reorth_kernel<4><<<g, RT, 0, s>>>(Q, ldq, kv, h1, w, n, chunk, red.partial, red.counter, h2, scal, gate, orth_tol2);
-  else if (kv <= 8)
-    arnoldi_reorth_kernel<8><<<g, RT, 0, s>>>(Q, ldq, kv, h1, w, n, chunk, red.partial, red.counter, h2, scal, gate, orth_tol2);
-  else if (kv <= 16)
-    arnoldi_reorth_kernel<16><<<g, RT, 0, s>>>(Q, ldq, kv, h1, w, n, chunk, red.partial, red.counter, h2, scal, gate, orth_tol2);
-  else
-    arnoldi_reorth_kernel<0><<<g, RT, 0, s>>>(Q, ldq, kv, h1, w, n, chunk, red.partial, red.counter, h2, scal, gate, orth_tol2);
+// Slices of the Arnoldi passes: one block per SM at most. Blocks of 64 elements up to 64 per SM,
+// then 128 and 256 (longer slices run in steps of 256): every pass adds G partial sums per vector in
+// every block, so more and shorter slices would only move the work there.
+struct ArnoldiGrid {
+  int G, E;
+  int64_t chunk;
+  explicit ArnoldiGrid(int64_t n) {
+    const int64_t sms = num_sms();
+    E = n <= 64 * sms ? 2 : n <= 128 * sms ? 4 : 8;
+    const int64_t step = 32 * E;
+    chunk = step * ((n + step * sms - 1) / (step * sms));
+    G = (int)((n + chunk - 1) / chunk);
+  }
+};
+
+struct ArnoldiStep {
+  const double* Q;
+  int64_t n;
+  int kv;
+  double* w;
+  double *part1, *part2, *h1, *scal, *H, *cs, *sn, *beta;
+  unsigned* counter;
+  int iters;
+  double threshold, orth_tol2;
+  int* flag;
+  SplitOut so;
+};
+
+template <int E, int VP>
+void launch_arnoldi(const ArnoldiStep& a, const ArnoldiGrid& g, cudaStream_t s) {
+  int* gate = a.flag + kGmresState;
+  arnoldi_project_kernel<E, VP><<<g.G, RT, 0, s>>>(a.Q, a.n, a.kv, a.w, a.n, g.chunk, a.part1, gate);
   TTGB_CHECK_LAUNCH();
+  arnoldi_reorth_kernel<E, VP><<<g.G, RT, 0, s>>>(a.Q, a.n, a.kv, a.w, a.n, g.chunk, a.part1, a.part2,
+                                                  a.h1, a.scal, gate);
+  TTGB_CHECK_LAUNCH();
+  arnoldi_finish_kernel<E, VP><<<g.G, RT, 0, s>>>(a.Q, a.n, a.kv, a.h1, a.part2, a.w, a.n, g.chunk,
+                                                  a.part1, a.counter, a.scal, a.iters, a.H, a.cs, a.sn,
+                                                  a.beta, a.threshold, a.flag, a.so, a.orth_tol2);
+  TTGB_CHECK_LAUNCH();
+}
+
+template <int E>
+void launch_arnoldi(const ArnoldiStep& a, const ArnoldiGrid& g, cudaStream_t s) {
+  const int nv = a.kv + 1;   // vectors per warp: the basis and w
+  if (nv <= kWarps) launch_arnoldi<E, 1>(a, g, s);
+  else if (nv <= 2 * kWarps) launch_arnoldi<E, 2>(a, g, s);
+  else if (nv <= 4 * kWarps) launch_arnoldi<E, 4>(a, g, s);
+  else if (nv <= 6 * kWarps) launch_arnoldi<E, 6>(a, g, s);
+  else launch_arnoldi<E, kMaxVec / kWarps>(a, g, s);
 }
 
 }  // namespace
@@ -478,12 +655,23 @@ GmresResult gmres(const LocalOperator& op, const double* rhs, double* sol, int i
   double* sn = sm + L.sn;
   double* beta = sm + L.beta;
   double* h1 = sm + L.h1;
-  double* h2 = sm + L.h2;
   double* scal = sm + L.scal;
   int G1; int64_t ch1;
   red_launch_dims(red, n, 1, G1, ch1);
   // the kernels that write the operator's next input also write its tcgen05 operand split
   const SplitOut so = op.input_split();
+
+  const ArnoldiGrid grid(n);
+  TTGB_REQUIRE(2 * (int64_t)grid.G * kMaxVec <= (int64_t)red.cap_blocks * red.cap_vec,
+               "gmres: reduction workspace too small");
+  ArnoldiStep st;
+  st.Q = Q; st.n = n;
+  st.part1 = red.partial;
+  st.part2 = red.partial + (int64_t)grid.G * kMaxVec;
+  st.counter = red.counter;
+  st.h1 = h1; st.scal = scal; st.H = H; st.cs = cs; st.sn = sn; st.beta = beta;
+  st.iters = iters; st.threshold = threshold; st.orth_tol2 = orth_tol * orth_tol;
+  st.flag = ws.d_flag; st.so = so;
 
   // x0 = 0: the first cycle's update writes sol, so it is not cleared beforehand
   for (int cycle = 0; cycle < resets; ++cycle) {
@@ -509,17 +697,11 @@ GmresResult gmres(const LocalOperator& op, const double* rhs, double* sol, int i
       // q_k's split was written with q_k; past the stopping point the product does nothing
       op.apply(qk, w, true, s, so.hi != nullptr, ws.d_flag + kGmresState);
       if (op.prof_krylov) op.prof_krylov->begin();
-      int G; int64_t chunk;
-      red_launch_dims(red, n, kv + 1, G, chunk);
-      arnoldi_project_kernel<<<G, RT, 0, s>>>(Q, n, kv, w, n, chunk, red.partial, red.counter, h1, scal,
-                                              ws.d_flag + kGmresState);
-      TTGB_CHECK_LAUNCH();
-      launch_reorth(kv, dim3(G), Q, n, h1, w, n, chunk, red, h2, scal, ws.d_flag + kGmresState,
-                    orth_tol * orth_tol, s);
-      arnoldi_finish_kernel<<<G, RT, 0, s>>>(Q, n, kv, h1, h2, w, n, chunk, red.partial, red.counter,
-                                             scal, k, iters, H, cs, sn, beta, threshold, ws.d_flag,
-                                             so);
-      TTGB_CHECK_LAUNCH();
+      st.kv = kv;
+      st.w = w;
+      if (grid.E == 2) launch_arnoldi<2>(st, grid, s);
+      else if (grid.E == 4) launch_arnoldi<4>(st, grid, s);
+      else launch_arnoldi<8>(st, grid, s);
       // bytes of the reference's MGS iteration, 8 N (2k + 3), and of the three passes here
       // without the second projection, 8 N (2k + 7); the second projection's kv reads are added
       // per cycle from the device's count

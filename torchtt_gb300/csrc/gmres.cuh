@@ -95,7 +95,7 @@ enum GmresFlag : int {
 
 struct GmresWS {
   DBuf Q;        // (iters + 1) x n Krylov basis
-  DBuf small;    // H, cs, sn, beta, h1, h2, scalars
+  DBuf small;    // H, cs, sn, beta, h1, scalars
   int* h_flag = nullptr;   // pinned, >= kGmresFlagWords ints
   int* d_flag = nullptr;   // device, >= kGmresFlagWords ints
   double log_rate = 0.0;   // log(threshold) / iterations of the last converged cycle (0: unknown)
