@@ -1,13 +1,12 @@
 // FP64 contraction engine and the AMEn contraction recipes built on it.
 //
-// The kernel is a shared-memory-tiled FP64 GEMM (BMxBN output tile, BK=16, 256 threads, each
-// thread a (BM/16)x(BN/16) register tile). Every operand index may be a pair of tensor indices with
-// their own strides (struct Ax), so the reference's tensordot permutes (cpp/amen_solve.h:17-98)
-// cost no copies. FP64 FMA throughput is the bound on this path. The tile shape and split-K
-// (atomic FP64 adds) of a launch come from the tile autotuner's record for its shape class, or
-// from an occupancy heuristic: the largest tile whose grid covers the SMs, split-K when even the
-// smallest tile leaves SMs idle. The same engine runs in double-float arithmetic on the FP32 pipe
-// (contract_df_kernel) and in FP32.
+// Every operand index of the GEMM kernels here may be a pair of tensor indices with their own strides
+// (struct Ax), so the reference's tensordot permutes (cpp/amen_solve.h:17-98) cost no copies.
+// contract_kernel multiplies shared-memory tiles in the operand type (BK = 16, 256 threads, each thread
+// a (BM/16) x (BN/16) register tile); contract_emu_kernel takes the large FP64 products on the tensor
+// cores; contract_df_kernel runs in double-float arithmetic on the FP32 pipe where the caller takes
+// that accuracy. Which kernel, tile shape and split-K (atomic FP64 adds) a launch gets comes from the
+// tile autotuner's record for its shape class, or from an occupancy heuristic.
 #include <climits>
 
 #include <atomic>
@@ -18,6 +17,8 @@
 #include <shared_mutex>
 #include <type_traits>
 #include <unordered_map>
+
+#include <cuda_bf16.h>
 
 #include "contract.cuh"
 #include "df.cuh"
@@ -304,6 +305,8 @@ __global__ void __launch_bounds__(NT) contract_df_kernel(KParams<double> p) {
   }
 }
 
+#include "contract_emu.cuh"
+
 // C <- beta * C over the (batched, strided) output index space
 template <typename T>
 __global__ void scale_output_kernel(T* C, int M, int N, int batch, AxD cm, AxD cn, int64_t c_bs,
@@ -344,12 +347,41 @@ thread_local int t_fp64_engine = kFp64Native;
 // use the record. Launches that cannot be tuned (beta != 0, aliasing, a capturing stream, a
 // deterministic request) and classes being tuned by another thread use the occupancy heuristic.
 // ---------------------------------------------------------------------------------------------
+enum TileKind : int {
+  kFma = 0,   // multiply-adds in the operand type
+  kEmu = 1,   // FP64 from BF16 digits on the tensor cores (contract_emu.cuh)
+  kDf = 2     // double-float on the FP32 pipe
+};
 struct TileCfg {
   int bm, bn, split;   // split: 0 no split-K, 1 split-K sized to fill the GPU
+  TileKind kind = kFma;
 };
-constexpr TileCfg kCandidates[] = {{64, 64, 0}, {64, 32, 0}, {32, 64, 0}, {32, 32, 0},
-                                   {64, 64, 1}, {64, 32, 1}, {32, 64, 1}, {32, 32, 1}};
-constexpr int kNumCandidates = (int)(sizeof(kCandidates) / sizeof(kCandidates[0]));
+// FP64: on the FP64 pipe the work per SM sets the time, so the smallest tiles win below about 4 M
+// multiply-adds (32 x 32 tiles took 11 us where 16 x 16 take 4-5) and the tensor-core kernel above.
+constexpr TileCfg kCandidates64[] = {
+    {16, 16, 0}, {16, 32, 0}, {32, 16, 0}, {32, 32, 0}, {16, 16, 1}, {32, 32, 1},
+    {64, 32, 0, kEmu}, {32, 64, 0, kEmu}, {64, 16, 0, kEmu}, {16, 64, 0, kEmu},
+    {64, 32, 1, kEmu}, {32, 64, 1, kEmu}, {64, 16, 1, kEmu}, {16, 64, 1, kEmu}};
+// where the caller takes double-float accuracy
+constexpr TileCfg kCandidatesDf[] = {
+    {16, 16, 0}, {16, 16, 1}, {32, 32, 0, kDf}, {64, 32, 0, kDf}, {32, 64, 0, kDf},
+    {32, 32, 1, kDf}, {64, 32, 1, kDf}, {32, 64, 1, kDf},
+    {64, 32, 0, kEmu}, {32, 64, 0, kEmu}, {64, 32, 1, kEmu}, {32, 64, 1, kEmu}};
+constexpr TileCfg kCandidates32[] = {{64, 64, 0}, {64, 32, 0}, {32, 64, 0}, {32, 32, 0},
+                                     {64, 64, 1}, {64, 32, 1}, {32, 64, 1}, {32, 32, 1}};
+struct CandidateList {
+  const TileCfg* t;
+  int n;
+};
+// the calling thread's candidates for a contraction of type T
+template <typename T>
+CandidateList candidates() {
+  if (!std::is_same<T, double>::value)
+    return {kCandidates32, (int)(sizeof(kCandidates32) / sizeof(TileCfg))};
+  if (t_fp64_engine == kFp64DoubleFloat)
+    return {kCandidatesDf, (int)(sizeof(kCandidatesDf) / sizeof(TileCfg))};
+  return {kCandidates64, (int)(sizeof(kCandidates64) / sizeof(TileCfg))};
+}
 
 std::atomic<int> g_autotune{-1};   // -1: not read yet from TTGB_AUTOTUNE
 std::shared_mutex g_tune_mu;   // readers: every launch of a recorded class; writers: tuning
@@ -369,7 +401,7 @@ void load_table() {
   unsigned long long k = 0;
   int c = 0;
   while (std::fscanf(f, "%llx %d", &k, &c) == 2)
-    if (c >= 0 && c < kNumCandidates) g_tune_table[(uint64_t)k] = c;
+    if (c >= 0) g_tune_table[(uint64_t)k] = c;
   std::fclose(f);
 }
 
@@ -432,12 +464,30 @@ int heuristic_split(const ContractDescT<T>& d, int bm, int bn, int sms, bool for
   return splitk < 1 ? 1 : splitk;
 }
 
+// A triangular right factor is an inverse R factor: its columns are graded, and the product has to be
+// accurate relative to each element's own terms (the tensor-core kernel's bound is per row and
+// column: with it a CholeskyQR of a matrix of condition 1e12 left a residual of 2e-13, not 7e-16).
 template <typename T>
-void launch_tiles(const ContractDescT<T>& d, KParams<T> p, int bm, int bn, int splitk,
+bool componentwise(const ContractDescT<T>& d) {
+  return (d.tri & kTriUpperB) != 0;
+}
+
+template <int BM, int BN>
+void launch_emu(const KParams<double>& p, dim3 grid, cudaStream_t stream) {
+  using Tile = EmuTile<BM, BN>;
+  smem_optin((const void*)contract_emu_kernel<BM, BN>, (int)Tile::kSmem);
+  contract_emu_kernel<BM, BN><<<grid, Tile::kThreads, Tile::kSmem, stream>>>(p);
+  TTGB_CHECK_LAUNCH();
+}
+
+template <typename T>
+void launch_tiles(const ContractDescT<T>& d, KParams<T> p, const TileCfg& t, int splitk,
                   cudaStream_t stream) {
+  const int bm = t.bm, bn = t.bn;
   int kchunk = d.K;
   if (splitk > 1) {
-    kchunk = (int)cdiv(cdiv(d.K, splitk), BK) * BK;
+    const int unit = t.kind == kEmu ? kEmuK : BK;
+    kchunk = (int)cdiv(cdiv(d.K, splitk), unit) * unit;
     splitk = (int)cdiv(d.K, kchunk);
   }
   p.splitk = splitk;
@@ -452,25 +502,33 @@ void launch_tiles(const ContractDescT<T>& d, KParams<T> p, int bm, int bn, int s
   dim3 grid(cdiv(d.N, bn), cdiv(d.M, bm), (unsigned)(d.batch * splitk));
   TTGB_REQUIRE(grid.y < 65536 && grid.z < 65536, "contraction grid too large");
   if constexpr (std::is_same<T, double>::value) {
-    if (t_fp64_engine == kFp64DoubleFloat) {
-      if (bm == 64 && bn == 64) contract_df_kernel<64, 64><<<grid, NT, 0, stream>>>(p);
-      else if (bm == 64 && bn == 32) contract_df_kernel<64, 32><<<grid, NT, 0, stream>>>(p);
-      else if (bm == 32 && bn == 64) contract_df_kernel<32, 64><<<grid, NT, 0, stream>>>(p);
-      else contract_df_kernel<32, 32><<<grid, NT, 0, stream>>>(p);
-      TTGB_CHECK_LAUNCH();
+    if (t.kind == kEmu) {
+      if (bm == 64 && bn == 32) launch_emu<64, 32>(p, grid, stream);
+      else if (bm == 32 && bn == 64) launch_emu<32, 64>(p, grid, stream);
+      else if (bm == 64 && bn == 16) launch_emu<64, 16>(p, grid, stream);
+      else launch_emu<16, 64>(p, grid, stream);
       return;
     }
+    if (t.kind == kDf) {
+      if (bm == 64 && bn == 32) contract_df_kernel<64, 32><<<grid, NT, 0, stream>>>(p);
+      else if (bm == 32 && bn == 64) contract_df_kernel<32, 64><<<grid, NT, 0, stream>>>(p);
+      else contract_df_kernel<32, 32><<<grid, NT, 0, stream>>>(p);
+    } else if (bm == 16 && bn == 16) contract_kernel<T, 16, 16><<<grid, NT, 0, stream>>>(p);
+    else if (bm == 16 && bn == 32) contract_kernel<T, 16, 32><<<grid, NT, 0, stream>>>(p);
+    else if (bm == 32 && bn == 16) contract_kernel<T, 32, 16><<<grid, NT, 0, stream>>>(p);
+    else contract_kernel<T, 32, 32><<<grid, NT, 0, stream>>>(p);
+  } else {
+    if (bm == 64 && bn == 64) contract_kernel<T, 64, 64><<<grid, NT, 0, stream>>>(p);
+    else if (bm == 64 && bn == 32) contract_kernel<T, 64, 32><<<grid, NT, 0, stream>>>(p);
+    else if (bm == 32 && bn == 64) contract_kernel<T, 32, 64><<<grid, NT, 0, stream>>>(p);
+    else contract_kernel<T, 32, 32><<<grid, NT, 0, stream>>>(p);
   }
-  if (bm == 64 && bn == 64) contract_kernel<T, 64, 64><<<grid, NT, 0, stream>>>(p);
-  else if (bm == 64 && bn == 32) contract_kernel<T, 64, 32><<<grid, NT, 0, stream>>>(p);
-  else if (bm == 32 && bn == 64) contract_kernel<T, 32, 64><<<grid, NT, 0, stream>>>(p);
-  else contract_kernel<T, 32, 32><<<grid, NT, 0, stream>>>(p);
   TTGB_CHECK_LAUNCH();
 }
 
 template <typename T>
 uint64_t tune_key(const ContractDescT<T>& d) {
-  const int eng = std::is_same<T, float>::value ? 2 : (t_fp64_engine == kFp64DoubleFloat ? 1 : 0);
+  const int eng = std::is_same<T, float>::value ? 2 : (t_fp64_engine == kFp64DoubleFloat ? 4 : 3);
   const int units = (d.am.s0 == 1) | ((d.ak.s0 == 1) << 1) | ((d.bk.s0 == 1) << 2) |
                     ((d.bn.s0 == 1) << 3) | ((d.cm.s0 == 1) << 4);
   uint64_t k = (uint64_t)eng;
@@ -496,16 +554,17 @@ int tuned_choice(const ContractDescT<T>& d, const KParams<T>& p, cudaStream_t st
   const int64_t sc = (d.batch - 1) * d.c_bs + ax_span(d.cm, d.M) + ax_span(d.cn, d.N);
   if (overlaps<T>(d.C, sc, d.A, sa) || overlaps<T>(d.C, sc, d.B, sb)) return -1;
   std::call_once(g_table_once, load_table);
+  const CandidateList cand = candidates<T>();
   const uint64_t key = tune_key(d);
   {
     std::shared_lock<std::shared_mutex> g(g_tune_mu);
     auto it = g_tune_table.find(key);
-    if (it != g_tune_table.end()) return it->second;
+    if (it != g_tune_table.end()) return it->second < cand.n ? it->second : -1;
   }
   {
     std::unique_lock<std::shared_mutex> g(g_tune_mu);
     auto it = g_tune_table.find(key);
-    if (it != g_tune_table.end()) return it->second;
+    if (it != g_tune_table.end()) return it->second < cand.n ? it->second : -1;
     if (t_no_tuning_runs) return -1;   // a caller that must not block: heuristic tile
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
@@ -526,12 +585,13 @@ int tuned_choice(const ContractDescT<T>& d, const KParams<T>& p, cudaStream_t st
   int best = -1;
   float best_ms = 0.f;
   for (int rep = 0; rep < 2; ++rep) {
-    for (int c = 0; c < kNumCandidates; ++c) {
-      const TileCfg& t = kCandidates[c];
+    for (int c = 0; c < cand.n; ++c) {
+      const TileCfg& t = cand.t[c];
+      if (t.kind == kEmu && componentwise(d)) continue;
       const int split = t.split ? heuristic_split(d, t.bm, t.bn, sms, true) : 1;
       if (t.split && split == 1) continue;   // the same launch as the unsplit candidate
       TTGB_CUDA(cudaEventRecord(ev[0], stream));
-      launch_tiles(d, p, t.bm, t.bn, split, stream);
+      launch_tiles(d, p, t, split, stream);
       TTGB_CUDA(cudaEventRecord(ev[1], stream));
       TTGB_CUDA(cudaEventSynchronize(ev[1]));
       float ms = 0.f;
@@ -575,22 +635,35 @@ void launch_contract(const ContractDescT<T>& d, cudaStream_t stream, bool determ
     // after tuning, C holds the last candidate's result: the chosen tile runs once more, so the
     // first launch of a class gives what every later launch of the class computes
     if (c >= 0) {
-      const TileCfg& t = kCandidates[c];
-      launch_tiles(tuned ? dz : d, p, t.bm, t.bn,
+      const TileCfg& t = candidates<T>().t[c];
+      launch_tiles(tuned ? dz : d, p, t,
                    t.split ? heuristic_split(d, t.bm, t.bn, sms, true) : 1, stream);
       return;
     }
   }
   // occupancy heuristic: the largest tile whose grid still gives two CTAs per SM, split-K when
-  // even 32 x 32 tiles leave SMs idle
+  // even the smallest tiles leave SMs idle
   auto tiles = [&](int bm, int bn) { return (int64_t)cdiv(d.M, bm) * cdiv(d.N, bn) * d.batch; };
-  int bm = 64, bn = 64;
   const int64_t target = 2 * (int64_t)sms;
-  if (tiles(64, 64) < target) {
-    if (d.M >= d.N) { bm = 64; bn = 32; } else { bm = 32; bn = 64; }
-    if (tiles(bm, bn) < target) { bm = 32; bn = 32; }
+  TileCfg t{64, 64, 0};
+  if (std::is_same<T, double>::value) {
+    const double work = (double)d.M * d.N * d.K * d.batch;
+    if (componentwise(d) ? t_fp64_engine == kFp64DoubleFloat : work > 4e6)
+      t.kind = componentwise(d) ? kDf : kEmu;
+    t.bm = t.bn = 32;
+    if (t.kind == kEmu) {
+      if (d.N <= 16) { t.bm = 64; t.bn = 16; }
+      else if (d.M <= 16) { t.bm = 16; t.bn = 64; }
+      else if (d.M >= d.N) t.bm = 64;
+      else t.bn = 64;
+    } else if (t.kind == kFma && tiles(32, 32) < target) {
+      t.bm = t.bn = 16;
+    }
+  } else if (tiles(64, 64) < target) {
+    if (d.M >= d.N) { t.bm = 64; t.bn = 32; } else { t.bm = 32; t.bn = 64; }
+    if (tiles(t.bm, t.bn) < target) { t.bm = 32; t.bn = 32; }
   }
-  launch_tiles(d, p, bm, bn, deterministic ? 1 : heuristic_split(d, bm, bn, sms, false), stream);
+  launch_tiles(d, p, t, deterministic ? 1 : heuristic_split(d, t.bm, t.bn, sms, false), stream);
 }
 
 }  // namespace

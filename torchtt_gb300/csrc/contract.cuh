@@ -45,9 +45,10 @@ constexpr int kTriUpperB = 2;
 using ContractDesc = ContractDescT<double>;
 using ContractDescF = ContractDescT<float>;
 
-// Arithmetic of the FP64 contractions issued by the calling thread: kFp64Native runs them on the
-// FP64 pipe; kFp64DoubleFloat in double-float arithmetic on the FP32 pipe (~1e-13 relative, for
-// operands within the FP32 exponent range). Set for a scope with Fp64EngineScope.
+// Accuracy of the FP64 contractions issued by the calling thread: kFp64Native computes them at least as
+// accurately as FP64 multiply-adds; kFp64DoubleFloat also admits double-float arithmetic on the FP32
+// pipe (~1e-13 relative, for operands within the FP32 exponent range) where it is the faster.
+// Set for a scope with Fp64EngineScope.
 constexpr int kFp64Native = 0;
 constexpr int kFp64DoubleFloat = 1;
 struct Fp64EngineScope {

@@ -1,0 +1,374 @@
+// FP64 contraction on the tensor cores: C = alpha A B + beta C for FP64 operands, computed from exact
+// products of 8-bit slices (the error-free splitting of Ozaki, Ogita, Oishi and Rump, Numer.
+// Algorithms 59 (2012)). Included by contract.cu inside its anonymous namespace.
+//
+// Why: GB300's FP64 pipe does 1.9 multiply-adds per clock and SM, mma.sync with BF16 operands about a
+// thousand, and 36 slice products replace one FP64 product.
+//
+// A tile's K chunk of 64 is brought to a common fixed point: column j of B by its largest exponent
+// Fj; then row k of B by the largest exponent kb(k) that this leaves in it, which is folded into A's
+// column k (their product does not change); then row i of A by Ei = max_k exponent(a_ik) + kb(k), and
+// column j of B once more by Ec = max_k exponent(b_kj) - Fj - kb(k). An element becomes a signed 62-bit integer, cut into 8 balanced 8-bit digits, which BF16 holds
+// exactly. The products of digits p and q with p + q = d (0 is the leading digit) share one FP32
+// accumulator: at most 8 x 64 products of at most 2^14, below 2^24, so every sum is exact. The digits
+// with p + q <= 7 are used; what is left out is below 2^-60 of the largest |a_ik| |b_kj| of a term, and
+// with the two scales folded together that bound holds for rows and columns of any grading. The
+// eight sums are put together as a 64-bit integer and rounded once to FP64 by integer operations;
+// several chunks (and splits) are added in FP64.
+//
+// Relative error (2-norm) of random products with K = 30 to 130: 4e-17 to 1e-16, FP64 multiply-adds
+// 1.9e-16 to 3.7e-16; graded rows, columns and opposite gradings of both alike. A chunk with an
+// infinity, a NaN or a subnormal number is computed with FP64 multiply-adds, so these go through as
+// before.
+//
+// Measured (M = 322, N = 5024, K = 161): 130 us against 513 us for FP64 multiply-adds in 32 x 32 tiles, which
+// ran at 80% of the FP64 pipe. The tensor pipe is 25% busy; what bounds the kernel is the integer work of
+// making digits (each element once per tile that reads it) and of putting the sums together.
+
+constexpr int kEmuK = 64;                    // K chunk
+constexpr int kEmuPitch = kEmuK + 8;         // BF16 per shared-memory row: conflict-free ldmatrix
+constexpr int kEmuSlices = 8;
+constexpr int kEmuZero = -20000;             // exponent of a zero: far below any other
+
+// exponent field of x, kEmuZero for a zero (subnormal numbers take the FP64 path)
+__device__ __forceinline__ int emu_exponent(double x) {
+  const int e = (__double2hiint(x) >> 20) & 0x7ff;
+  return e == 0 ? kEmuZero : e;
+}
+
+// whether x is an infinity, a NaN or subnormal
+__device__ __forceinline__ bool emu_special(double x) {
+  const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  return h >= 0x7ff00000u || (h < 0x00100000u && (h | (unsigned)__double2loint(x)) != 0u);
+}
+
+// x in fixed point, 2^(E - e) below the leading position of a 62-bit integer, plus the 0x80 of every
+// byte that makes the bytes of the sum the balanced digits + 128
+__device__ __forceinline__ uint2 fixed_digits(double x, int e, int E) {
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+  unsigned hi = ((h & 0xfffffu) | 0x100000u) << 9 | l >> 23, lo = l << 9;   // 53 bits at 2^61
+  int sh = E - e;
+  if (sh >= 32) { lo = hi; hi = 0u; sh -= 32; }
+  sh = min(sh, 32);   // a zero, whose exponent is far below E, leaves no bits
+  lo = __funnelshift_rc(lo, hi, sh);
+  hi = sh < 32 ? hi >> sh : 0u;
+  const unsigned neg = (unsigned)((int)h >> 31);
+  const unsigned long long y = ((unsigned long long)(hi ^ neg) << 32 | (lo ^ neg)) +
+                               (0x8080808080808080ull - (unsigned long long)(long long)(int)neg);
+  return make_uint2((unsigned)y, (unsigned)(y >> 32));
+}
+
+// 4 consecutive k of one row, all slices, into s[slice][row][k]. With a byte b the digit is b - 128, the
+// difference of the BF16 values 128 + (b mod 128) and 256 - 128 (b div 128), whose bits are b's own.
+__device__ __forceinline__ void store_digits(const uint2 (&y)[4], __nv_bfloat16* s, int rows) {
+#pragma unroll
+  for (int p = 0; p < kEmuSlices; ++p) {
+    const int byte = 7 - p;
+    const unsigned sel = (unsigned)(byte & 3) | (unsigned)(4 + (byte & 3)) << 8;
+    unsigned v[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const unsigned w = byte >= 4 ? __byte_perm(y[2 * i].y, y[2 * i + 1].y, sel | sel << 4)
+                                   : __byte_perm(y[2 * i].x, y[2 * i + 1].x, sel | sel << 4);
+      const unsigned a = (w & 0x007f007fu) | 0x43004300u, b = (w & 0x00800080u) ^ 0x43804380u;
+      asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(v[i]) : "r"(a), "r"(b));
+    }
+    *reinterpret_cast<uint2*>(s + (size_t)p * rows * kEmuPitch) = make_uint2(v[0], v[1]);
+  }
+}
+
+__device__ __forceinline__ void ldmatrix_x4(unsigned (&r)[4], const __nv_bfloat16* p) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a));
+}
+
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const unsigned (&a)[4], unsigned b0,
+                                         unsigned b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, "
+               "{%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// The value of the eight exact sums D (weight 2^(8 (14 - d)) each) at scale exponents E, rounded to
+// nearest. Neighbouring sums fit one 32-bit integer: |D[d]| < 2^22.9, 2^18 for d = 0.
+__device__ __forceinline__ double emu_value(const float (&D)[8], int E) {
+  int w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) w[i] = __float2int_rn(D[2 * i]) * 256 + __float2int_rn(D[2 * i + 1]);
+  const long long H = (long long)w[0] * 65536 + w[1], L = (long long)w[2] * 65536 + w[3];
+  // |H| < 2^42.1: 20 bits up leave the sign; the lower half is rounded to that unit
+  const long long T = (H << 20) + ((L + (1 << 11)) >> 12);
+  if (T == 0 || E < -15000) return 0.0;   // E: of a row or column of zeros, whose digits mean nothing
+  unsigned long long m = (unsigned long long)(T < 0 ? -T : T);
+  const int lz = __clzll((long long)m);
+  // the value is T 2^(56 + 32 - 20) 2^(E - 2168)
+  int ef = 63 - lz + E - 2100 + 1023;
+  m <<= lz;
+  const unsigned long long r = m + 0x3ffull + ((m >> 11) & 1ull);   // to 53 bits, ties to even
+  ef += r < m ? 1 : 0;                                              // carried out of the top bit
+  const unsigned long long frac = r < m ? 0ull : (r >> 11) & 0xfffffffffffffull;
+  const unsigned long long sign = T < 0 ? 1ull << 63 : 0ull;
+  if (ef >= 1 && ef <= 2046)
+    return __longlong_as_double((long long)(sign | ((unsigned long long)ef << 52) | frac));
+  const double v = scalbn(__longlong_as_double((long long)((1023ull << 52) | frac)), ef - 1023);
+  return T < 0 ? -v : v;   // subnormal or infinite
+}
+
+// One operand's share of a thread: row `row` of the tile, quads of 4 consecutive k.
+template <int ROWS, int NTH>
+struct EmuLoader {
+  static constexpr int kPer = NTH / ROWS;                 // threads per row
+  static constexpr int kQuads = kEmuK / 4 / kPer;         // quads per thread
+  static_assert(kPer * ROWS == NTH && kQuads >= 1, "tile and block sizes");
+  double v[kQuads][4];
+  int row, part;
+  bool ok;
+  int64_t off;
+  __device__ __forceinline__ void init(int tid, int r0, int extent, const AxD& ax) {
+    row = tid % ROWS;
+    part = tid / ROWS;
+    ok = r0 + row < extent;
+    off = ok ? ax_off(ax, r0 + row) : 0;
+  }
+  __device__ __forceinline__ int k(int q) const { return (part + q * kPer) * 4; }
+  // Loads the chunk of len elements at k0; true when an element is special.
+  __device__ __forceinline__ bool load(const double* base, const AxD& ak, int k0, int len) {
+    bool special = false;
+#pragma unroll
+    for (int q = 0; q < kQuads; ++q) {
+      const int kk = k(q);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[q][i] = 0.0;
+      if (ok && kk < len) {
+        if (ak.e0 == INT_MAX) {
+          const double* p = base + off + (int64_t)(k0 + kk) * ak.s0;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (kk + i < len) v[q][i] = __ldg(p + i * ak.s0);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (kk + i < len) v[q][i] = __ldg(base + off + ax_off(ak, k0 + kk + i));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) special |= emu_special(v[q][i]);
+    }
+    return special;
+  }
+};
+
+// BM x BN tile, one warp per 16 x 16 of it. MINB: blocks per SM that the registers have to leave room
+// for (as many as the shared memory does).
+template <int BM, int BN>
+struct EmuTile {
+  static constexpr int kWarpsN = BN / 16;
+  static constexpr int kThreads = 32 * (BM / 16) * kWarpsN;
+  static constexpr size_t kSmem = (size_t)kEmuSlices * (BM + BN) * kEmuPitch * sizeof(__nv_bfloat16);
+  static constexpr int kMinBlocks = (int)(220 * 1024 / kSmem);
+};
+
+template <int BM, int BN>
+__global__ void __launch_bounds__(EmuTile<BM, BN>::kThreads, EmuTile<BM, BN>::kMinBlocks)
+    contract_emu_kernel(KParams<double> p) {
+  using Tile = EmuTile<BM, BN>;
+  constexpr int NTH = Tile::kThreads;
+  extern __shared__ __align__(16) unsigned char emu_sm[];
+  __nv_bfloat16* As = reinterpret_cast<__nv_bfloat16*>(emu_sm);
+  __nv_bfloat16* Bs = As + (size_t)kEmuSlices * BM * kEmuPitch;
+  // scales of a chunk, by the parity of the chunk: kb(k), Ei, Fj, Ec
+  __shared__ __align__(16) int kmax[2][kEmuK];
+  __shared__ int emax_a[2][BM], fmax_b[2][BN], emax_b[2][BN];
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int bz = blockIdx.z;
+  const int bidx = bz / p.splitk;
+  const int ks = bz - bidx * p.splitk;
+  const int kbeg = ks * p.kchunk;
+  int kend = min(p.K, kbeg + p.kchunk);
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  if ((p.tri & kTriLowerC) && m0 + BM <= n0) return;   // tile strictly above the diagonal
+  if (p.tri & kTriUpperB) kend = min(kend, n0 + BN);   // B(k, n) = 0 for k > n
+  const double* A = p.A + (int64_t)bidx * p.a_bs;
+  const double* B = p.B + (int64_t)bidx * p.b_bs;
+
+  EmuLoader<BM, NTH> la;
+  EmuLoader<BN, NTH> lb;
+  la.init(tid, m0, p.M, p.am);
+  lb.init(tid, n0, p.N, p.bn);
+  const int wm = (warp / Tile::kWarpsN) * 16, wn = (warp % Tile::kWarpsN) * 16;
+  const int g = lane >> 2, t2 = (lane & 3) * 2;   // fragment row and column of the accumulators
+  const bool work = m0 + wm < p.M && n0 + wn < p.N;   // the warp's part of the tile is not empty
+
+  double acc[2][4];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) acc[j][r] = 0.0;
+
+  int par = 0;
+  for (int k0 = kbeg; k0 < kend; k0 += kEmuK, par ^= 1) {
+    const int len = min(kend - k0, kEmuK);
+    const int steps = (len + 15) / 16, len16 = steps * 16;   // digits are made up to len16
+    const bool special = la.load(A, p.ak, k0, len) | lb.load(B, p.bk, k0, len);
+    for (int i = tid; i < kEmuK; i += NTH) kmax[par][i] = kEmuZero;
+    for (int i = tid; i < BM; i += NTH) emax_a[par][i] = kEmuZero;
+    for (int i = tid; i < BN; i += NTH) { fmax_b[par][i] = kEmuZero; emax_b[par][i] = kEmuZero; }
+    // the previous chunk's digits have been read, this chunk's scales are cleared
+    if (__syncthreads_or(special ? 1 : 0)) {   // rare: infinities, NaN or subnormals in the chunk
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const int m = m0 + wm + g + 8 * (r >> 1), n = n0 + wn + 8 * j + t2 + (r & 1);
+          if (m >= p.M || n >= p.N) continue;
+          const int64_t mo = ax_off(p.am, m), no = ax_off(p.bn, n);
+          double s = acc[j][r];
+          for (int k = k0; k < k0 + len; ++k)
+            s = fma(A[mo + ax_off(p.ak, k)], B[no + ax_off(p.bk, k)], s);
+          acc[j][r] = s;
+        }
+      continue;
+    }
+    int mb = kEmuZero;
+#pragma unroll
+    for (int q = 0; q < lb.kQuads; ++q)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) mb = max(mb, emu_exponent(lb.v[q][i]));
+    atomicMax(&fmax_b[par][lb.row], mb);
+    __syncthreads();
+    const int F = fmax_b[par][lb.row];
+#pragma unroll
+    for (int q = 0; q < lb.kQuads; ++q) {
+      if (q * lb.kPer * 4 >= len) break;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        constexpr bool kHalf = BN < 32;   // lanes of a half warp share k
+        const int e = emu_exponent(lb.v[q][i]);
+        const int m = __reduce_max_sync(kHalf ? 0xffffu << (lane & 16) : 0xffffffffu,
+                                        e == kEmuZero ? kEmuZero : e - F);
+        if ((lane & (kHalf ? 15 : 31)) == 0) atomicMax(&kmax[par][lb.k(q) + i], m);
+      }
+    }
+    __syncthreads();
+    auto kb = [&](int k, int (&out)[4]) {
+      const int4 m = *reinterpret_cast<const int4*>(&kmax[par][k]);
+      out[0] = m.x; out[1] = m.y; out[2] = m.z; out[3] = m.w;
+    };
+    // a row k of B that is zero (kb = kEmuZero) takes column k of A out of the scale; a zero of A or
+    // B stays more than 2^11 below any other exponent
+    int ma = 2 * kEmuZero;
+    mb = kEmuZero;
+#pragma unroll
+    for (int q = 0; q < la.kQuads; ++q) {
+      if (q * la.kPer * 4 >= len) break;
+      int b[4];
+      kb(la.k(q), b);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ma = max(ma, emu_exponent(la.v[q][i]) + b[i]);
+    }
+#pragma unroll
+    for (int q = 0; q < lb.kQuads; ++q) {
+      if (q * lb.kPer * 4 >= len) break;
+      int b[4];
+      kb(lb.k(q), b);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int e = emu_exponent(lb.v[q][i]);
+        mb = max(mb, e == kEmuZero ? kEmuZero : e - F - b[i]);
+      }
+    }
+    atomicMax(&emax_a[par][la.row], ma);
+    atomicMax(&emax_b[par][lb.row], mb);
+    __syncthreads();
+    {
+      const int E = emax_a[par][la.row];
+#pragma unroll
+      for (int q = 0; q < la.kQuads; ++q) {
+        if (q * la.kPer * 4 >= len16) break;
+        int b[4];
+        uint2 y[4];
+        kb(la.k(q), b);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          y[i] = fixed_digits(la.v[q][i], emu_exponent(la.v[q][i]) + b[i], E);
+        store_digits(y, As + (size_t)la.row * kEmuPitch + la.k(q), BM);
+      }
+      const int G = emax_b[par][lb.row];
+#pragma unroll
+      for (int q = 0; q < lb.kQuads; ++q) {
+        if (q * lb.kPer * 4 >= len16) break;
+        int b[4];
+        uint2 y[4];
+        kb(lb.k(q), b);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int e = emu_exponent(lb.v[q][i]);
+          y[i] = fixed_digits(lb.v[q][i], e == kEmuZero ? kEmuZero : e - F - b[i], G);
+        }
+        store_digits(y, Bs + (size_t)lb.row * kEmuPitch + lb.k(q), BN);
+      }
+    }
+    __syncthreads();
+    if (!work) continue;
+    // one n8 half of the warp's tile at a time: its eight accumulators and B digits stay in registers
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      float d[kEmuSlices][4];
+#pragma unroll
+      for (int s = 0; s < kEmuSlices; ++s)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) d[s][r] = 0.f;
+      for (int kk = 0; kk < steps; ++kk) {
+        // four slices' digits of n8 x k16 per two loads (lanes 0-15: slice s, 16-31: slice s + 1)
+        unsigned b[kEmuSlices / 2][4];
+        const __nv_bfloat16* bp = Bs + (size_t)((lane >> 4) * BN + wn + 8 * j + (lane & 7)) * kEmuPitch +
+                                  kk * 16 + (((lane >> 3) & 1) << 3);
+#pragma unroll
+        for (int q = 0; q < kEmuSlices / 2; ++q) ldmatrix_x4(b[q], bp + (size_t)(2 * q) * BN * kEmuPitch);
+        const __nv_bfloat16* ap = As + (size_t)(wm + (lane & 15)) * kEmuPitch + kk * 16 +
+                                  ((lane >> 4) << 3);
+#pragma unroll
+        for (int s = 0; s < kEmuSlices; ++s) {
+          unsigned a[4];
+          ldmatrix_x4(a, ap + (size_t)s * BM * kEmuPitch);
+#pragma unroll
+          for (int q = 0; q < kEmuSlices - s; ++q)
+            mma_bf16(d[s + q], a, b[q / 2][2 * (q & 1)], b[q / 2][2 * (q & 1) + 1]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        float D[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) D[s] = d[s][r];
+        const int n = wn + 8 * j + t2 + (r & 1);
+        const double v =
+            emu_value(D, emax_a[par][wm + g + 8 * (r >> 1)] + fmax_b[par][n] + emax_b[par][n]);
+        acc[j][r] = k0 == kbeg ? v : acc[j][r] + v;
+      }
+    }
+  }
+
+  double* C = p.C + (int64_t)bidx * p.c_bs;
+#pragma unroll
+  for (int r = 0; r < 4; r += 2) {
+    const int m = m0 + wm + g + 8 * (r >> 1);
+    if (m >= p.M) continue;
+    const int64_t cmo = ax_off(p.cm, m);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int n = n0 + wn + 8 * j + t2 + h;
+        if (n >= p.N) continue;
+        double* c = C + cmo + ax_off(p.cn, n);
+        const double v = p.alpha == 1.0 ? acc[j][r + h] : p.alpha * acc[j][r + h];
+        if (p.splitk > 1) atomicAdd(c, v);
+        else *c = (p.beta == 0.0) ? v : fma(p.beta, *c, v);
+      }
+  }
+}
