@@ -332,7 +332,7 @@ int ttgb_local_product(int64_t rl, int64_t s, int64_t r, int64_t m, int64_t n, i
     LocalOpDims d{rl, s, r, m, n, S, RL, R};
     DBuf w1(local_product_w1(d), st), w2(local_product_w2(d), st);
     SparseCore sp;   // the solver's structured A stage when A is sparse enough
-    sp.build(A, s, m, n, S, st);
+    sp.build(A, s, m, n, S, st, SparseCore::kLp);
     for (int32_t i = 0; i < nrhs; ++i)
       local_product(d, phi_l, A, phi_r, x + (int64_t)i * r * n * R, y + (int64_t)i * rl * m * RL,
                     w1.p, w2.p, st, 1.0, 0.0, &sp);
@@ -355,7 +355,7 @@ int ttgb_local_product_lowp(int64_t rl, int64_t s, int64_t r, int64_t m, int64_t
       Fp64EngineScope eng(kFp64DoubleFloat);
       DBuf w1(local_product_w1(d), st), w2(local_product_w2(d), st);
       SparseCore sp;
-      sp.build(A, s, m, n, S, st);
+      sp.build(A, s, m, n, S, st, SparseCore::kLp);
       local_product(d, phi_l, A, phi_r, x, y, w1.p, w2.p, st, 1.0, 0.0, &sp);
     } else if (engine == TTGB_ENGINE_TC) {
       TTGB_REQUIRE(tc_available(), "tcgen05 engine needs an sm_100-family GPU");
@@ -364,7 +364,7 @@ int ttgb_local_product_lowp(int64_t rl, int64_t s, int64_t r, int64_t m, int64_t
       TTGB_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
       {
         SparseCore sp;
-        sp.build(A, s, m, n, S, st);
+        sp.build(A, s, m, n, S, st, SparseCore::kLp);
         TcCore core;
         if (!sp.use) core.build(A, s, m, n, S, st);
         TcLocal tl;
@@ -385,7 +385,7 @@ int ttgb_local_product_lowp(int64_t rl, int64_t s, int64_t r, int64_t m, int64_t
       cast(phi_r, pr.p, RL * S * R, st);
       cast(x, xf.p, (int64_t)nx, st);
       SparseCore sp;
-      sp.build(A, s, m, n, S, st);
+      sp.build(A, s, m, n, S, st, SparseCore::kLp);
       local_product(d, pl.p, a32.p, pr.p, xf.p, yf.p, w1.p, w2.p, st, 1.0f, 0.0f, &sp);
       cast(yf.p, y, (int64_t)ny, st);
     }
@@ -403,7 +403,7 @@ static int phi_A_entry(bool fwd, int64_t l, int64_t L, int64_t s, int64_t S, int
     PhiDims d{l, L, s, S, r, R, M, N};
     DBuf w(phi_A_workspace(d), st);
     SparseCore sp;
-    sp.build(A, s, M, N, S, st);
+    sp.build(A, s, M, N, S, st, fwd ? SparseCore::kFw : SparseCore::kBk);
     if (fwd) phi_fwd_A(d, phi, left, A, right, out, w.p, st, &sp);
     else phi_bck_A(d, phi, left, A, right, out, w.p, st, &sp);
   });

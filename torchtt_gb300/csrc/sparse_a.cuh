@@ -15,25 +15,33 @@ namespace ttgb {
 // Nonzeros of one A core grouped by an output key (CSR): for each key, the nonzeros with their
 // two remaining indices (a, b) and value.
 struct SparseCsr {
-  int64_t keys = 0, nnz = 0;
-  int max_row = 0;
-  DevBuf<int> rp;      // keys + 1 row pointers
-  DevBuf<int> a, b;    // nnz
-  DBuf val;            // nnz, FP64
-  FBuf val32;          // nnz, FP32 (low-precision engines)
+  int64_t keys = 0;
+  const int* rp = nullptr;          // keys + 1 row pointers
+  const int* a = nullptr;           // per nonzero
+  const int* b = nullptr;
+  const double* val = nullptr;      // FP64
+  const float* val32 = nullptr;     // FP32 (low-precision engines)
 };
 
-struct SparseCore {
+class SparseCore {
+ public:
+  static constexpr int kGroupings = 4;
+  static constexpr unsigned kLp = 1, kFw = 2, kBk = 4, kRh = 8, kAll = 15;
+  static constexpr int kMaxRow = 64;
   bool use = false;
   int64_t s = 0, M = 0, N = 0, S = 0;
   SparseCsr lp;   // key (m, S) = m*S + S, pairs (s, n): local product stage
   SparseCsr fw;   // key (N, S) = N*S + S, pairs (s, M): forward interface stage
   SparseCsr bk;   // key (s, N) = s*N + N, pairs (M, S): backward interface stage
   SparseCsr rh;   // key (s, M) = s*M + M, pairs (N, S): right half of a two-site product
-  // Reads the core (device, FP64, s x M x N x S) once and sets `use` when fewer than a quarter of
-  // its entries are nonzero and no key has more than kMaxRow nonzeros.
-  void build(const double* A, int64_t s, int64_t M, int64_t N, int64_t S, cudaStream_t st);
-  static constexpr int kMaxRow = 64;
+  // Counts the nonzeros of the core (device, FP64, s x M x N x S), waits for the count, and sets `use`
+  // when fewer than a quarter of its entries are nonzero and no key has more than kMaxRow of them;
+  // the groupings in `which` are then built on the stream.
+  void build(const double* A, int64_t s, int64_t M, int64_t N, int64_t S, cudaStream_t st,
+             unsigned which = kAll);
+
+ private:
+  DevBuf<unsigned char> head_, entries_;
 };
 
 // out[koff(key) + o1*so1 + o2] = sum_{j in row key} val[j] * in[o1*si1 + o2 + a[j]*pa + b[j]*pb]
