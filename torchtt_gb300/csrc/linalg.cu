@@ -113,125 +113,241 @@ __global__ void __launch_bounds__(512) chol_kernel(double* G, int n, int64_t shi
   }
 }
 
-// Fused, shared-memory resident Cholesky + triangular inverse for n <= kCholSmemMax:
-// G (row-major, global) -> R (upper, G = R^T R) written to Rout, Ri = R^{-1} written to Riout.
-// Same shift / identity check semantics as chol_kernel. One block; both n x n factors live in
-// shared memory, so every step is a shared-memory FP64 update plus one barrier.
-constexpr int kCholSmemMax = 112;
+// Fused, shared-memory resident Cholesky + triangular inverse for n <= kCholSmemMax, one block:
+// G (row-major, global) -> R (upper, G = R^T R) to Rout, R^{-1} to Riout; one n x n array holds R in
+// its upper and L^{-1} = R^{-T} in its strictly lower triangle.
+//
+// A column at a time, every step waits for a square root and a division and for three barriers, and
+// that chain, not the n^3 / 3 multiply-adds, set the time (133 us at n = 77). By panels of 16 the chain
+// runs over a 16 x 32 block [G_JJ | I] with one element per thread: row j is scaled by its warp (the
+// reciprocal square root from FP32 with a correction of third order) and published, one barrier per
+// step, which gives R_JJ and L_JJ^{-1}; the other columns of the panel's rows and the rows below are
+// then two plain products.
+//
+// pass 0 factors without a shift first (condition of A up to ~1e5: the next pass then sees a matrix
+// near the identity); a pivot below kPivotTol of the largest diagonal entry starts over with the shift
+// of sCholQR3. pass 1 sets *done when its G is near enough to the identity that Q needs no third
+// pass. pass 2 sets *status = 2 when max |G - I| > 0.1. Gin is cleared (the next Gram product
+// accumulates into it); Rout and Riout must not overlap it.
+constexpr int kCholSmemMax = 160;
+constexpr int kCholNb = 16;
 constexpr double kNearIdentity = 1e-9;   // max |G - I| below which the first-order factor is used
+constexpr double kPivotTol = 1e-11;
 
-// Gin is cleared after it is read (the next Gram product accumulates into it); Rout and Riout
-// must not overlap it.
+// 1 / sqrt(d) for d in the FP32 range: y from FP32, y (1 + e / 2 + 3 e^2 / 8) with e = 1 - d y^2
+__device__ __forceinline__ double rsqrt_refined(double d) {
+  const double y = (double)rsqrtf((float)d);
+  const double e = fma(-d * y, y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// Largest |G - I| and largest diagonal entry of an upper triangle by their high words (upper bounds
+// within 2^-20; 1e300 for an infinity or a NaN), and the trace. FP64 comparisons and block-wide FP64
+// reductions would hold the FP64 pipe for microseconds; these are integer maxima.
+struct GramStats {
+  unsigned mx, dmax;
+  double tr;
+};
+
+__device__ __forceinline__ double from_high_word(unsigned hi) {
+  return hi >= 0x7ff00000u ? 1e300 : __hiloint2double((int)hi + 1, 0);
+}
+
+// All threads; st is cleared by the caller before a barrier, valid after the next one.
+__device__ __forceinline__ void gram_stats(const double* g, int n, int pitch, bool identity, GramStats* st) {
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
+  unsigned mx = 0u, dmax = 0u;
+  for (int t = tid; t < n * n; t += nt) {
+    const int i = t / n, k = t - i * n;
+    if (k < i) continue;
+    const double v = g[i * pitch + k];
+    if (i == k) dmax = max(dmax, (unsigned)__double2hiint(v));
+    if (identity) mx = max(mx, (unsigned)__double2hiint(i == k ? v - 1.0 : v) & 0x7fffffffu);
+  }
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  dmax = __reduce_max_sync(0xffffffffu, dmax);   // a negative diagonal entry counts as infinite
+  if (lane == 0) {
+    atomicMax(&st->mx, mx);
+    atomicMax(&st->dmax, dmax);
+  }
+  if (tid < 32) {
+    double tr = 0.0;
+    for (int i = lane; i < n; i += 32) tr += g[i * pitch + i];
+    tr = warp_sum_d(tr);
+    if (lane == 0) st->tr = tr;
+  }
+}
+
+// 2^-e, 2^(e/2) and 2^(-e/2) for the even e with 2^e <= d < 2^(e+2) (1 when d is not a normal number)
+__device__ __forceinline__ void even_scale(double d, double& sc, double& root, double& inv_root) {
+  int e = ((__double2hiint(d) >> 20) & 0x7ff) - 1023;
+  if (!(d > 0.0) || d >= 1e300 || e < -1000) e = 0;
+  e &= ~1;
+  sc = __hiloint2double((1023 - e) << 20, 0);
+  root = __hiloint2double((1023 + e / 2) << 20, 0);
+  inv_root = __hiloint2double((1023 - e / 2) << 20, 0);
+}
+
+// Shared memory of chol_panels.
+struct CholShared {
+  double rowbuf[2][2 * kCholNb];
+  double Ls[kCholNb][kCholNb + 1];   // L_JJ^{-1} of the panel
+  double xd[kCholSmemMax];           // diagonal of L^{-1}
+  int bad;                           // a pivot not above floor_d (cleared by the caller)
+};
+
+// The factorisation described at chol_inv_smem_kernel, by the 512 threads of a block: A (shared, pitch
+// n + 1) holds G in its upper triangle and zeros below; on return R and, below the diagonal, L^{-1}.
+__device__ void chol_panels(double* A, int n, double floor_d, CholShared& ch) {
+  const int ld = n + 1;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+      for (int j0 = 0; j0 < n; j0 += kCholNb) {
+        const int w = min(kCholNb, n - j0);
+        {   // [R_JJ | L_JJ^{-1}] of the diagonal block: element (i, c) = (warp, lane)
+          const int i = warp, c = lane;
+          double v = (i == (c & 15)) ? 1.0 : 0.0;   // also the padding of the last panel
+          if (c < w && i < w) v = c >= i ? A[(j0 + i) * ld + j0 + c] : A[(j0 + c) * ld + j0 + i];
+  #pragma unroll 1
+          for (int j = 0; j < kCholNb; ++j) {
+            if (i == j) {
+              const double d = __shfl_sync(0xffffffffu, v, j);
+              if (!(d > floor_d) || !isfinite(d)) ch.bad = 1;   // the same in every lane
+              v *= rsqrt_refined(d);
+              ch.rowbuf[j & 1][c] = v;
+            }
+            __syncthreads();
+            if (i > j) v = fma(-ch.rowbuf[j & 1][i], ch.rowbuf[j & 1][c], v);
+          }
+          if (i < w) {
+            if (c < w && c >= i) A[(j0 + i) * ld + j0 + c] = v;
+            if (c >= kCholNb) {
+              const int q = c - kCholNb;
+              ch.Ls[i][q] = v;   // zero above the diagonal
+              if (q < i) A[(j0 + i) * ld + j0 + q] = v;
+              if (q == i) ch.xd[j0 + i] = v;
+            }
+          }
+        }
+        __syncthreads();
+        if (ch.bad) return;
+        {   // the panel's rows of the other columns: L_JJ^{-1} [X | G]
+          const int cols = n - w;
+          constexpr int kPer = kCholNb * kCholSmemMax / 512;
+          double y[kPer];
+  #pragma unroll
+          for (int u = 0; u < kPer; ++u) {
+            const int t = tid + u * 512;
+            double sum = 0.0;
+            if (t < w * cols) {
+              const int i = t / cols, q = t - i * cols;
+              const double* col = A + j0 * ld + (q < j0 ? q : q + w);
+              for (int k = 0; k <= i; ++k) sum = fma(ch.Ls[i][k], col[k * ld], sum);
+            }
+            y[u] = sum;
+          }
+          __syncthreads();
+  #pragma unroll
+          for (int u = 0; u < kPer; ++u) {
+            const int t = tid + u * 512;
+            if (t < w * cols) {
+              const int i = t / cols, q = t - i * cols;
+              A[(j0 + i) * ld + (q < j0 ? q : q + w)] = y[u];
+            }
+          }
+        }
+        __syncthreads();
+        // rows below: columns left of the panel and the panel's own (L^{-1}), and from the diagonal on (G)
+        const int r0 = j0 + w;
+        for (int i = r0 + warp; i < n; i += 16) {
+          double f[kCholNb];
+  #pragma unroll
+          for (int k = 0; k < kCholNb; ++k) f[k] = k < w ? A[(j0 + k) * ld + i] : 0.0;
+          for (int q = lane; q < r0 + (n - i); q += 32) {
+            const int c = q < r0 ? q : q - r0 + i;
+            double v = A[i * ld + c];
+            if (c >= j0 && c < r0) {
+  #pragma unroll
+              for (int k = 0; k < kCholNb; ++k)
+                if (k < w) v = fma(-f[k], ch.Ls[k][c - j0], v);
+            } else {
+  #pragma unroll
+              for (int k = 0; k < kCholNb; ++k)
+                if (k < w) v = fma(-f[k], A[(j0 + k) * ld + c], v);
+            }
+            A[i * ld + c] = v;
+          }
+        }
+        __syncthreads();
+      }
+}
+
 __global__ void __launch_bounds__(512) chol_inv_smem_kernel(double* __restrict__ Gin, int n,
-                                                            int64_t shift_rows, int check_identity,
-                                                            double* Rout, double* Riout, int* status) {
-  extern __shared__ double sm[];
-  const int ld = n + 1;   // padded rows
-  double* G = sm;                 // becomes R (upper)
-  double* X = sm + n * ld;        // becomes R^{-1} (upper)
-  __shared__ double sh[32];
-  __shared__ int bad;
+                                                            int64_t shift_rows, int pass, double* Rout,
+                                                            double* Riout, int* status, int* done) {
+  extern __shared__ double A[];
+  const int ld = n + 1;
+  __shared__ CholShared ch;
+  __shared__ GramStats st;
   const int tid = threadIdx.x, nt = blockDim.x;
-  for (int t = tid; t < n * n; t += nt) G[(t / n) * ld + (t % n)] = Gin[t];
-  if (tid == 0) bad = 0;
+  if (tid == 0) { st.mx = 0u; st.dmax = 0u; }
+  for (int t = tid; t < n * n; t += nt) {
+    const int i = t / n, k = t - i * n;
+    A[i * ld + k] = k < i ? 0.0 : Gin[t];   // the Gram matrix is formed in its upper triangle only
+  }
   __syncthreads();
-  for (int t = tid; t < n * n; t += nt) Gin[t] = 0.0;   // ready for the next Gram product
-  if (shift_rows == 0) {   // the second and third passes: G = I + E with E small
-    double mx = 0.0;
-    for (int t = tid; t < n * n; t += nt) {
-      const int i = t / n, k = t % n;
-      if (k < i) continue;   // the Gram matrix is formed (and read) in its upper triangle only
-      const double v = G[i * ld + k] - (i == k ? 1.0 : 0.0);
-      mx = fmax(mx, isfinite(v) ? fabs(v) : 1e300);
+  gram_stats(A, n, ld, pass > 0, &st);
+  __syncthreads();
+  const double mx = from_high_word(st.mx), dmax = from_high_word(st.dmax), tr = st.tr;
+  if (pass > 0) {
+    if (tid == 0) {
+      if (pass == 2 && !(mx <= 0.1)) *status = 2;
+      if (pass == 1) *done = (n * mx <= 0.5) ? 1 : 0;
     }
-    mx = block_max_d(mx, sh);   // the same value in every thread: the branches below are uniform
-    if (check_identity && tid == 0 && !(mx <= 0.1)) *status = 2;
     if (mx <= kNearIdentity) {
       // First-order factor: R = I + U with U the strict upper triangle of E plus half its
-      // diagonal (U + U^T = E), and R^{-1} = I - U. Both are exact to O(n max|E|^2) <= 1.2e-16
-      // for max|E| <= 1e-9 and n <= 112, so the pass costs O(n^2) instead of the factorisation's
-      // n^3 / 3 serial FP64 multiply-adds.
+      // diagonal (U + U^T = E), and R^{-1} = I - U. Both are exact to O(n max|E|^2) <= 1.6e-16
+      // for max|E| <= 1e-9, so the pass costs O(n^2).
       for (int t = tid; t < n * n; t += nt) {
-        const int i = t / n, k = t % n;
-        const double e = (k >= i) ? G[i * ld + k] - (i == k ? 1.0 : 0.0) : 0.0;
+        const int i = t / n, k = t - i * n;
+        const double e = (k >= i) ? A[i * ld + k] - (i == k ? 1.0 : 0.0) : 0.0;
         const double u = (k > i) ? e : (k == i ? 0.5 * e : 0.0);
         const double id = (i == k) ? 1.0 : 0.0;
         Rout[t] = id + u;
         Riout[t] = id - u;
+        Gin[t] = 0.0;
       }
       return;
     }
   }
-  if (shift_rows > 0) {
-    double tr = 0.0;
-    for (int i = tid; i < n; i += nt) tr += G[i * ld + i];
-    tr = block_sum_d(tr, sh);
-    const double sft = 11.0 * ((double)shift_rows * n + (double)n * (n + 1)) * kEps * tr;
-    for (int i = tid; i < n; i += nt) G[i * ld + i] += sft;
-  }
-  __syncthreads();
-  // right-looking Cholesky, upper triangle only. The pivot's square root and reciprocal are
-  // computed once per step by one thread: FP64 sqrt and division expand to several DFMA, and 16
-  // warps computing them redundantly would occupy the SM's FP64 pipe for thousands of cycles.
-  __shared__ double piv_inv;
-  for (int j = 0; j < n; ++j) {
-    if (tid == 0) {
-      const double d = G[j * ld + j];
-      if (!(d > 0.0) || !isfinite(d)) { bad = 1; *status = 1; }
-      else { const double rd = sqrt(d); G[j * ld + j] = rd; piv_inv = 1.0 / rd; }
+  double sc, rsc, irsc;   // a power of four takes the diagonal into the FP32 range
+  even_scale(dmax, sc, rsc, irsc);
+  bool shifted = false;
+  while (true) {
+    if (tid == 0) ch.bad = 0;
+    const double sft =
+        shifted ? 11.0 * ((double)shift_rows * n + (double)n * (n + 1)) * kEps * tr : 0.0;
+    for (int t = tid; t < n * n; t += nt) {
+      const int i = t / n, k = t - i * n;
+      A[i * ld + k] = (k < i) ? 0.0 : (Gin[t] + (i == k ? sft : 0.0)) * sc;
     }
+    const double floor_d = (pass == 0 && !shifted) ? kPivotTol * dmax * sc : 0.0;
     __syncthreads();
-    if (bad) break;
-    const double inv = piv_inv;
-    for (int k = j + 1 + tid; k < n; k += nt) G[j * ld + k] *= inv;
-    __syncthreads();
-    {   // trailing update of the upper triangle: one warp per row, lanes over columns
-      const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-      for (int i = j + 1 + warp; i < n; i += nw) {
-        const double gji = G[j * ld + i];
-        double* gi = G + i * ld;
-        const double* gj = G + j * ld;
-        for (int k = i + lane; k < n; k += 32) gi[k] = fma(-gji, gj[k], gi[k]);
-      }
-    }
-    __syncthreads();
+    chol_panels(A, n, floor_d, ch);
+    if (!ch.bad) break;
+    __syncthreads();   // every thread has read `bad`
+    if (pass > 0 || shifted) break;
+    shifted = true;
   }
-  if (bad) return;
-  {
-    const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-    for (int i = warp; i < n; i += nw)
-      for (int k = lane; k < n; k += 32) {
-        if (k < i) G[i * ld + k] = 0.0;
-        X[i * ld + k] = (k == i) ? 1.0 : 0.0;
-      }
+  if (ch.bad) {
+    if (tid == 0) *status = 1;
+    for (int t = tid; t < n * n; t += nt) Gin[t] = 0.0;
+    return;
   }
-  __syncthreads();
-  // X = R^{-1} by column-oriented back substitution on the identity: for j = n-1..0 the row j of
-  // X is final after scaling, then its multiples are removed from the rows above (one warp per row).
-  {
-    const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-    for (int j = n - 1; j >= 0; --j) {
-      if (tid == 0) piv_inv = 1.0 / G[j * ld + j];
-      __syncthreads();
-      const double inv = piv_inv;
-      for (int k = j + tid; k < n; k += nt) X[j * ld + k] *= inv;
-      __syncthreads();
-      for (int i = warp; i < j; i += nw) {
-        const double gij = G[i * ld + j];
-        double* xi = X + i * ld;
-        const double* xj = X + j * ld;
-        for (int k = j + lane; k < n; k += 32) xi[k] = fma(-gij, xj[k], xi[k]);
-      }
-      __syncthreads();
-    }
-  }
-  {
-    const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-    for (int i = warp; i < n; i += nw)
-      for (int k = lane; k < n; k += 32) {
-        Rout[i * n + k] = G[i * ld + k];
-        Riout[i * n + k] = X[i * ld + k];
-      }
+  for (int t = tid; t < n * n; t += nt) {
+    const int i = t / n, k = t - i * n;
+    Rout[t] = k >= i ? A[i * ld + k] * rsc : 0.0;
+    Riout[t] = k > i ? A[k * ld + i] * irsc : (k == i ? ch.xd[i] * irsc : 0.0);
+    Gin[t] = 0.0;   // ready for the next Gram product
   }
 }
 
@@ -351,6 +467,153 @@ __global__ void __launch_bounds__(512, 1) householder_smem_kernel(const double* 
   householder_body(W, m, n, Q, R, tau);
   __syncthreads();
   for (int64_t t = tid; t < (int64_t)m * k; t += nt) Qout[t] = Q[t];
+}
+
+// ---------------------------------------------------------------------------------------------
+// CholeskyQR of a small matrix in one launch (512 threads, everything in shared memory): the passes of
+// qr() below without their launches and host wait, and the Householder factorisation in the same
+// launch when they break down. A Householder sweep pays two reductions over the block and a chain of
+// square root and divisions per column, twice (once more to form Q): 27 us for 48 x 4, 131 us for
+// 128 x 16. Here a pass is one Gram product, whose sums run over the lanes of a few threads each, the
+// n steps of the 16 x 16 block factorisation, and one triangular product.
+// ---------------------------------------------------------------------------------------------
+constexpr int kCholQrSmallN = 32;
+
+__global__ void __launch_bounds__(512, 1) cholqr_small_kernel(const double* __restrict__ A, int64_t lda,
+                                                              int m, int n, double* Qout, double* Rout) {
+  extern __shared__ double hs[];
+  const int ldq = m | 1;   // odd pitch of the columns
+  double* X = hs;                            // m x n, this pass's input
+  double* Y = X + (int64_t)ldq * n;          // its output
+  double* G = Y + (int64_t)ldq * n;          // n x (n + 1)
+  double* R = G + n * (n + 1);               // product of the R factors, upper, row-major pitch n
+  double* S = R + n * n;
+  __shared__ CholShared ch;
+  __shared__ GramStats st;
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
+  const int ld = n + 1;
+  for (int t = tid; t < m * n; t += nt) {
+    const int j = t / m, i = t - j * m;
+    X[j * ldq + i] = A[(int64_t)j * lda + i];
+  }
+  for (int t = tid; t < n * n; t += nt) R[t] = (t / n == t % n) ? 1.0 : 0.0;
+  __syncthreads();
+  const int pairs = n * (n + 1) / 2;
+  const int lpe = pairs <= 16 ? 32 : pairs <= 64 ? 8 : pairs <= 256 ? 4 : 2;   // lanes per Gram entry
+  bool ok = true;
+  for (int pass = 0; pass < 3; ++pass) {
+    if (tid == 0) { st.mx = 0u; st.dmax = 0u; }
+    // G = X^T X, upper triangle: lpe lanes share an entry's rows
+    for (int e0 = warp * (32 / lpe); e0 < pairs; e0 += (nt / 32) * (32 / lpe)) {
+      const int e = min(e0 + lane / lpe, pairs - 1);
+      int k = (int)((sqrtf(8.0f * (float)e + 1.0f) - 1.0f) * 0.5f);   // column of entry e = k (k + 1) / 2 + i
+      while (k * (k + 1) / 2 > e) --k;
+      while ((k + 1) * (k + 2) / 2 <= e) ++k;
+      const int i = e - k * (k + 1) / 2;
+      const double* x = X + i * ldq;
+      const double* y = X + k * ldq;
+      double s0 = 0.0, s1 = 0.0;
+      int r = lane % lpe;
+      for (; r + lpe < m; r += 2 * lpe) {
+        s0 = fma(x[r], y[r], s0);
+        s1 = fma(x[r + lpe], y[r + lpe], s1);
+      }
+      if (r < m) s0 = fma(x[r], y[r], s0);
+      s0 += s1;
+      for (int o = lpe >> 1; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+      if (lane % lpe == 0 && e0 + lane / lpe < pairs) {
+        S[i * n + k] = s0;
+      }
+    }
+    __syncthreads();
+    gram_stats(S, n, n, pass > 0, &st);
+    __syncthreads();
+    const double mx = from_high_word(st.mx), dmax = from_high_word(st.dmax), tr = st.tr;
+    if (pass == 2 && !(mx <= 0.1)) { ok = false; break; }
+    double rsc = 1.0, irsc = 1.0;
+    if (pass > 0 && mx <= kNearIdentity) {   // first-order factor, see chol_inv_smem_kernel
+      for (int t = tid; t < n * n; t += nt) {
+        const int i = t / n, k = t - i * n;
+        const double e = S[i <= k ? i * n + k : k * n + i] - (i == k ? 1.0 : 0.0);
+        G[i * ld + k] = i == k ? 1.0 + 0.5 * e : (k > i ? e : -e);   // R above, L^{-1} = R^{-T} below
+        if (i == k) ch.xd[i] = 1.0 - 0.5 * e;
+      }
+      __syncthreads();
+    } else {
+      double sc;
+      even_scale(dmax, sc, rsc, irsc);
+      for (int shifted = 0; shifted < 2; ++shifted) {
+        const double sft = shifted ? 11.0 * ((double)m * n + (double)n * (n + 1)) * kEps * tr : 0.0;
+        __syncthreads();
+        if (tid == 0) ch.bad = 0;
+        for (int t = tid; t < n * n; t += nt) {
+          const int i = t / n, k = t - i * n;
+          G[i * ld + k] = (k < i) ? 0.0 : (S[t] + (i == k ? sft : 0.0)) * sc;
+        }
+        __syncthreads();
+        chol_panels(G, n, (pass == 0 && !shifted) ? kPivotTol * dmax * sc : 0.0, ch);
+        __syncthreads();
+        if (!ch.bad || pass > 0) break;
+      }
+      if (ch.bad) { ok = false; break; }
+    }
+    // Y = X R^{-1}, columns k and n - 1 - k by one thread (n + 1 terms)
+    const int half = (n + 1) / 2;
+    for (int t = tid; t < m * half; t += nt) {
+      const int p = t / m, r = t - p * m;
+#pragma unroll 1
+      for (int side = 0; side < 2; ++side) {
+        const int k = side ? n - 1 - p : p;
+        if (side && k == p) break;
+        double s0 = X[k * ldq + r] * ch.xd[k], s1 = 0.0;
+        int i = 0;
+        for (; i + 1 < k; i += 2) {
+          s0 = fma(X[i * ldq + r], G[k * ld + i], s0);
+          s1 = fma(X[(i + 1) * ldq + r], G[k * ld + i + 1], s1);
+        }
+        if (i < k) s0 = fma(X[i * ldq + r], G[k * ld + i], s0);
+        Y[k * ldq + r] = (s0 + s1) * irsc;
+      }
+    }
+    // R <- R_pass R (through S)
+    for (int t = tid; t < n * n; t += nt) {
+      const int i = t / n, k = t - i * n;
+      double v = 0.0;
+      for (int l = i; l <= k; ++l) v = fma(G[i * ld + l], R[l * n + k], v);
+      S[t] = v * rsc;
+    }
+    __syncthreads();
+    for (int t = tid; t < n * n; t += nt) R[t] = S[t];
+    double* tmp = X; X = Y; Y = tmp;
+    __syncthreads();
+    if (pass == 1 && n * mx <= 0.5) break;   // near enough to the identity: X is orthonormal
+  }
+  if (ok) {
+    for (int t = tid; t < m * n; t += nt) {
+      const int j = t / m, i = t - j * m;
+      Qout[t] = X[j * ldq + i];
+    }
+    for (int t = tid; t < n * n; t += nt) {   // column-major
+      const int k = t / n, i = t - k * n;
+      Rout[t] = R[i * n + k];
+    }
+    return;
+  }
+  __syncthreads();
+  double* W = hs;
+  double* Q = W + (int64_t)m * n;
+  for (int t = tid; t < m * n; t += nt) {
+    const int j = t / m, i = t - j * m;
+    W[t] = A[(int64_t)j * lda + i];
+  }
+  __syncthreads();
+  householder_body(W, m, n, Q, Rout, Q + (int64_t)m * n);
+  __syncthreads();
+  for (int t = tid; t < m * n; t += nt) Qout[t] = Q[t];
+}
+
+size_t cholqr_small_smem(int64_t m, int64_t n) {
+  return (size_t)(2 * (m | 1) * n + n * (n + 1) + 2 * n * n) * sizeof(double);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -888,12 +1151,6 @@ __global__ void copy_cm_kernel(const double* __restrict__ A, int64_t lda, double
   }
 }
 
-void read_status(LinalgWS& ws, cudaStream_t s, int* out) {
-  TTGB_CUDA(cudaMemcpyAsync(ws.h_status, ws.status, sizeof(int), cudaMemcpyDeviceToHost, s));
-  TTGB_CUDA(cudaStreamSynchronize(s));
-  *out = *ws.h_status;
-}
-
 void householder(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, double* R,
                  LinalgWS& ws, cudaStream_t s) {
   const int64_t k = m < n ? m : n;
@@ -975,15 +1232,19 @@ QRResult qr(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, doubl
   QRResult res;
   res.k = m < n ? m : n;
   if (m <= 0 || n <= 0) return res;
-  // small or wide: single-block Householder (robust, cheap at these sizes). A tall matrix with
-  // few columns (m >= 1024, e.g. the kickrank-wide z blocks of 5120 rows) is not small: one
-  // block's serial column sweep over m rows costs more than the GEMM passes of CholeskyQR3.
-  const bool small = (double)m * n * n < 4.0e5 && m < 1024;
-  if (m < n || small || n > 1024) {
+  if (m < n || n > 1024) {   // wide, or beyond CholeskyQR's factor: single-block Householder
     householder(A, lda, m, n, Q, R, ws, s);
     return res;
   }
-  // shifted CholeskyQR3
+  // One block's FP64 pipe does a pass of m n^2 multiply-adds while the launches of the grid-wide passes
+  // cost about 30 us a pass, so the line lies where one pass fills that.
+  if (n <= kCholQrSmallN && (double)m * n * n <= 3.5e4 && cholqr_small_smem(m, n) <= kHouseholderSmemBytes) {
+    smem_optin((const void*)cholqr_small_kernel, kHouseholderSmemBytes);
+    cholqr_small_kernel<<<1, 512, cholqr_small_smem(m, n), s>>>(A, lda, (int)m, (int)n, Q, R);
+    TTGB_CHECK_LAUNCH();
+    return res;
+  }
+  // CholeskyQR2, or shifted CholeskyQR3
   ws.a.ensure(5 * n * n + 16, s);
   double* Rp[3] = {ws.a.p, ws.a.p + n * n, ws.a.p + 2 * n * n};   // R of each pass (row-major)
   double* Ri = ws.a.p + 3 * n * n;   // inverse of the current factor
@@ -996,22 +1257,25 @@ QRResult qr(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, doubl
   double* G = ws.gram.p;             // n x n Gram matrix (row-major upper triangle)
   ws.b.ensure(m * n + 16, s);
   double* Qt = ws.b.p;
-  TTGB_CUDA(cudaMemsetAsync(ws.status, 0, sizeof(int), s));
+  // words of ws.status: 0 the failure, 2 whether two passes were enough
+  TTGB_CUDA(cudaMemsetAsync(ws.status, 0, 3 * sizeof(int), s));
   const double* Ain = A;
   int64_t ldin = lda;
-  double* outs[3] = {Q, Qt, Q};
+  double* outs[3] = {Qt, Q, Qt};
   const bool smem_chol = n <= kCholSmemMax;
-  for (int pass = 0; pass < 3; ++pass) {
+  int passes = 0;
+  while (passes < 3) {
+    const int pass = passes++;
     // Gram matrix: only its lower (column-major) = upper (row-major) triangle is formed and read;
     // with the shared-memory Cholesky the buffer is already zero (cleared by the previous one)
     gemm_cm(Ain, ldin, Ain, ldin, G, n, n, n, m, 1.0, 0.0, s, true, false, kTriLowerC,
             smem_chol && ws.gram_zero >= n * n);
     if (smem_chol) {
-      const size_t smem = (size_t)2 * n * (n + 1) * sizeof(double);
+      const size_t smem = (size_t)n * (n + 1) * sizeof(double);
       smem_optin((const void*)chol_inv_smem_kernel,
-                 (int)(2 * kCholSmemMax * (kCholSmemMax + 1) * sizeof(double)));
-      chol_inv_smem_kernel<<<1, 512, smem, s>>>(G, (int)n, pass == 0 ? m : 0, pass == 2 ? 1 : 0,
-                                                Rp[pass], Ri, ws.status);
+                 (int)(kCholSmemMax * (kCholSmemMax + 1) * sizeof(double)));
+      chol_inv_smem_kernel<<<1, 512, smem, s>>>(G, (int)n, m, pass, Rp[pass], Ri, ws.status,
+                                                ws.status + 2);
       TTGB_CHECK_LAUNCH();
       if (ws.gram_zero < n * n) ws.gram_zero = n * n;   // the kernel cleared [0, n^2)
     } else {
@@ -1026,17 +1290,27 @@ QRResult qr(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, doubl
     gemm_cm(Ain, ldin, Ri, n, outs[pass], m, m, n, n, 1.0, 0.0, s, false, true, kTriUpperB);
     Ain = outs[pass];
     ldin = m;
+    // After an unshifted first pass the second one's Gram matrix is near the identity, and its Q is
+    // orthonormal to rounding; the third pass is for a shifted start.
+    if (pass > 0 && (smem_chol || pass == 2)) {
+      TTGB_CUDA(cudaMemcpyAsync(ws.h_status, ws.status, 3 * sizeof(int), cudaMemcpyDeviceToHost, s));
+      TTGB_CUDA(cudaStreamSynchronize(s));
+      if (ws.h_status[0] != 0) {
+        householder(A, lda, m, n, Q, R, ws, s);
+        return res;
+      }
+      if (pass == 1 && ws.h_status[2] != 0) break;
+    }
   }
-  int st = 0;
-  read_status(ws, s, &st);
-  if (st != 0) {
-    householder(A, lda, m, n, Q, R, ws, s);
-    return res;
+  // R of the passes multiplied (row-major factors; a row-major X is the column-major X^T), the last
+  // product written column-major
+  if (passes == 2) {
+    gemm_cm(Rp[1], n, Rp[0], n, R, n, n, n, n, 1.0, 0.0, s, true, true);
+  } else {
+    copy(Qt, Q, m * n, s);
+    gemm_cm(Rp[0], n, Rp[1], n, T1, n, n, n, n, 1.0, 0.0, s, false, false);   // T1 = R_1 R_0, row-major
+    gemm_cm(Rp[2], n, T1, n, R, n, n, n, n, 1.0, 0.0, s, true, true);
   }
-  // R = R_2 R_1 R_0 (row-major factors; a row-major X is the column-major X^T):
-  // T1 (row-major) = R_1 R_0, and R (column-major, ld n) = R_2 T1 written directly
-  gemm_cm(Rp[0], n, Rp[1], n, T1, n, n, n, n, 1.0, 0.0, s, false, false);
-  gemm_cm(Rp[2], n, T1, n, R, n, n, n, n, 1.0, 0.0, s, true, true);
   return res;
 }
 
