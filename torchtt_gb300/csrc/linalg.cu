@@ -1,11 +1,11 @@
-// FP64 dense linear algebra: shifted CholeskyQR3 with a Householder fallback, one-sided Jacobi
-// thin SVD.
+// FP64 dense linear algebra: CholeskyQR with a Householder fallback, one-sided Jacobi thin SVD.
 //
 // GB300 note: FP64 runs at ~1.9 FMA/clock/SM (measured), so every O(m n^2) step is expressed as a
 // GEMM on the contraction engine (spread over all SMs); only O(n^3) steps on the small n x n
-// factors run on few SMs: Cholesky + triangular inverse and the Jacobi of n < 16 in one thread
-// block, the block Jacobi of 16 <= n <= 160 on an 8-CTA cluster, larger ones one grid-wide round
-// per launch. Small QRs (the kickrank-wide blocks) run a shared-memory Householder in one block.
+// factors run on few SMs: Cholesky + triangular inverse in one block, the Jacobi of n < 16 in one
+// warp, the block Jacobi of 16 <= n <= 160 on an 8-CTA cluster, larger ones one grid-wide round per
+// launch, all from 16 on after FP32 sweeps in one block that leave them two or three sweeps. Small
+// QRs (the kickrank-wide blocks) run all their passes in one block.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -699,25 +699,18 @@ __global__ void tsqr_stack_kernel(const double* __restrict__ R, int n, int nin, 
   }
 }
 
-// ---------------------------------------------------------------------------------------------
-// One-sided (Hestenes) Jacobi SVD of the n x n column-major matrix W in one thread block, with
-// the round-robin parallel ordering; rotation formulas of Demmel & Veselic (SIAM J. Matrix Anal.
-// Appl. 13, 1992). On exit U (n x n) holds W_j / sigma_j, V the accumulated rotations, both with
-// columns sorted by descending sigma, S the sorted singular values.
-// ---------------------------------------------------------------------------------------------
 // Rotation (c, s) of one-sided Jacobi for a column pair with squared norms a, b and inner product
-// g (Demmel-Veselic formulas): false when the pair is orthogonal to `tol`. The tangent t of the
-// angle comes from FP32 arithmetic (relative error ~1e-7: the pair is left orthogonal to ~1e-7 and
-// a later sweep finishes it), and c = 1/sqrt(1 + t^2) is refined from the FP32 rsqrt to full FP64
-// accuracy by two Newton steps, so (c, s) is orthogonal to rounding. On GB300 an FP64 sqrt or
-// division is a sequence of DFMA on a pipe that issues one warp instruction per 16 cycles; the
-// exact formula costs ~4 sqrt + 3 divisions per rotation, this one ~8 DFMA.
+// g (Demmel-Veselic formulas): false when the pair is orthogonal to `tol`. The angle comes from FP32
+// arithmetic (relative error ~1e-7: the pair is left orthogonal to ~1e-7 and a later sweep finishes
+// it); its cosine and sine, taken to FP64, are divided by their norm to FP64 accuracy with the series
+// of 1 / sqrt(1 - d) for d = 1 - c^2 - s^2 ~ 1e-7, so (c, s) is orthogonal to rounding. An FP64 square
+// root or division is a sequence of DFMA, and each dependent FP64 operation costs some 80 cycles of
+// latency here: five of them follow the FP32 angle.
 __device__ __forceinline__ bool jacobi_rotation(double a, double b, double g, double tol, double& c,
                                                 double& s) {
   if (a == 0.0 || b == 0.0) return false;
   if (!(g * g > tol * tol * a * b)) return false;
-  const double bma = b - a, g2 = 2.0 * g;
-  const float fb = (float)bma, fg = (float)g2;
+  const float fb = (float)(b - a), fg = 2.0f * (float)g;
   float tf;
   if (fabsf(fb) >= fabsf(fg)) {   // r = 2g / (b - a), |r| <= 1: t = r / (1 + sqrt(1 + r^2))
     const float r = __fdividef(fg, fb);
@@ -726,128 +719,26 @@ __device__ __forceinline__ bool jacobi_rotation(double a, double b, double g, do
     const float z = __fdividef(fb, fg);
     tf = __fdividef(copysignf(1.0f, z), fabsf(z) + sqrtf(fmaf(z, z, 1.0f)));
   }
-  double t;
-  if (tf != 0.0f && isfinite(tf)) {
-    t = (double)tf;
-  } else {   // operands outside the FP32 range: the exact FP64 formula
-    const double zeta = bma / g2;
-    t = (fabs(zeta) > 1e150) ? 0.5 / zeta
-                             : copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+  if (tf == 0.0f || !isfinite(tf)) {   // operands outside the FP32 range: the exact FP64 formula
+    const double zeta = (b - a) / (2.0 * g);
+    const double t = (fabs(zeta) > 1e150) ? 0.5 / zeta
+                                          : copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
+    c = 1.0 / sqrt(1.0 + t * t);
+    s = c * t;
+    return true;
   }
-  const double x = fma(t, t, 1.0);
-  double y = (double)rsqrtf((float)x);
-  y = y * fma(-0.5 * x, y * y, 1.5);
-  y = y * fma(-0.5 * x, y * y, 1.5);
-  c = y;
-  s = y * t;
+  const float cf = rsqrtf(fmaf(tf, tf, 1.0f));
+  c = (double)cf;
+  s = (double)(cf * tf);
+  const double d = fma(-s, s, fma(-c, c, 1.0));
+  const double f = fma(d, fma(d, 0.375, 0.5), 1.0);
+  c *= f;
+  s *= f;
   return true;
 }
 
-__device__ __forceinline__ double warp_sum_t(double v) { return warp_sum_d(v); }
-
 __device__ __forceinline__ int rr_index(int p, int r, int nn) {
   return p == 0 ? 0 : ((p - 1 + r) % (nn - 1)) + 1;
-}
-
-__global__ void __launch_bounds__(512) jacobi_svd_kernel(double* Wg, double* Vg, int n, double* U,
-                                                         double* S, int use_smem, int max_sweeps,
-                                                         int* status, const double* Vinit) {
-  extern __shared__ double smem[];
-  __shared__ int nrot;
-  double* W = use_smem ? smem : Wg;
-  double* V = use_smem ? smem + (int64_t)n * n : Vg;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  if (use_smem) {
-    for (int64_t t = tid; t < (int64_t)n * n; t += nt) W[t] = Wg[t];
-  }
-  for (int64_t t = tid; t < (int64_t)n * n; t += nt)
-    V[t] = Vinit ? Vinit[t] : (((t % n) == (t / n)) ? 1.0 : 0.0);
-  __syncthreads();
-  const int nn = n + (n & 1);
-  const double tol = fmax((double)n, 1.0) * kEps;
-  int sweep = 0;
-  for (; sweep < max_sweeps; ++sweep) {
-    if (tid == 0) nrot = 0;
-    __syncthreads();
-    for (int r = 0; r < nn - 1; ++r) {
-      for (int pi = warp; pi < nn / 2; pi += nw) {
-        int p = rr_index(pi, r, nn), q = rr_index(nn - 1 - pi, r, nn);
-        if (p > q) { const int t = p; p = q; q = t; }
-        if (q >= n) continue;
-        double* wp = W + (int64_t)p * n;
-        double* wq = W + (int64_t)q * n;
-        double a = 0.0, b = 0.0, g = 0.0;
-        for (int i = lane; i < n; i += 32) {
-          const double x = wp[i], y = wq[i];
-          a = fma(x, x, a); b = fma(y, y, b); g = fma(x, y, g);
-        }
-        a = warp_sum_d(a); b = warp_sum_d(b); g = warp_sum_d(g);
-        double c, s;
-        if (!jacobi_rotation(a, b, g, tol, c, s)) continue;
-        for (int i = lane; i < n; i += 32) {
-          const double x = wp[i], y = wq[i];
-          wp[i] = c * x - s * y;
-          wq[i] = s * x + c * y;
-        }
-        double* vp = V + (int64_t)p * n;
-        double* vq = V + (int64_t)q * n;
-        for (int i = lane; i < n; i += 32) {
-          const double x = vp[i], y = vq[i];
-          vp[i] = c * x - s * y;
-          vq[i] = s * x + c * y;
-        }
-        if (lane == 0) atomicAdd(&nrot, 1);
-      }
-      __syncthreads();
-    }
-    __syncthreads();
-    if (nrot == 0) break;
-    __syncthreads();
-  }
-  if (tid == 0 && sweep >= max_sweeps) *status = 3;
-  // singular values, ranks by descending value (ties by index)
-  double* sig = S;  // temporary: write unsorted to S via registers below
-  for (int j = warp; j < n; j += nw) {
-    const double* wj = W + (int64_t)j * n;
-    double a = 0.0;
-    for (int i = lane; i < n; i += 32) a = fma(wj[i], wj[i], a);
-    a = warp_sum_d(a);
-    if (lane == 0) U[(int64_t)j] = sqrt(a);   // stash sigma_j in U's first column temporarily
-  }
-  __syncthreads();
-  // rank computation, then write sorted S (U column 0 is rewritten afterwards)
-  __shared__ int rank_sh[1024];
-  for (int j = tid; j < n; j += nt) {
-    const double sj = U[j];
-    int rk = 0;
-    for (int i = 0; i < n; ++i) {
-      const double si = U[i];
-      rk += (si > sj) || (si == sj && i < j);
-    }
-    if (j < 1024) rank_sh[j] = rk;
-  }
-  __syncthreads();
-  for (int j = tid; j < n; j += nt) sig[rank_sh[j]] = U[j];
-  __syncthreads();
-  // U[:, rank_j] = W_j / sigma_j ; V columns permuted into Wg (scratch) then copied back
-  for (int j = warp; j < n; j += nw) {
-    const int rk = rank_sh[j];
-    const double sj = sig[rk];
-    const double inv = sj > 0.0 ? 1.0 / sj : 0.0;
-    const double* wj = W + (int64_t)j * n;
-    for (int i = lane; i < n; i += 32) Vg[(int64_t)n * n + (int64_t)rk * n + i] = wj[i] * inv;
-  }
-  __syncthreads();
-  for (int64_t t = tid; t < (int64_t)n * n; t += nt) U[t] = Vg[(int64_t)n * n + t];
-  __syncthreads();
-  for (int j = warp; j < n; j += nw) {
-    const int rk = rank_sh[j];
-    const double* vj = V + (int64_t)j * n;
-    for (int i = lane; i < n; i += 32) Vg[(int64_t)n * n + (int64_t)rk * n + i] = vj[i];
-  }
-  __syncthreads();
-  for (int64_t t = tid; t < (int64_t)n * n; t += nt) Vg[t] = Vg[(int64_t)n * n + t];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -859,48 +750,179 @@ __global__ void __launch_bounds__(512) jacobi_svd_kernel(double* Wg, double* Vg,
 // pulls the two blocks of its next pair from their holders over DSMEM into its second buffer. Every
 // pair of columns is visited once per sweep, as in the scalar cyclic order, with one cluster
 // barrier per round (P - 1 per sweep), and every dot product reads local memory. The sweep's
-// rotation count is summed in CTA 0 after a barrier and read by every CTA, so all CTAs leave the
-// loop together. The value type T is the arithmetic of the sweeps; Vin (optional) gives starting
-// rotations (identity when null), Vout the accumulated ones.
+// largest cosine and sine are collected in CTA 0 after a barrier and read by every CTA, so all CTAs leave the
+// loop together. Vout: the accumulated rotations.
 // ---------------------------------------------------------------------------------------------
 constexpr int kJacobiCluster = 8;
 constexpr int kJacobiBlockMaxN = 160;
 
-// One rotation of a column pair with tracked squared column norms (*na, *nb): only the inner product is
-// reduced; the norms follow the rotation exactly (a' = c^2 a - 2cs g + s^2 b, b' = s^2 a + 2cs g +
-// c^2 b) and are recomputed from the columns once per sweep, which bounds their drift.
-template <typename T>
-__device__ __forceinline__ int jacobi_rotate_tracked(T* wp, T* wq, T* vp, T* vq, T* na, T* nb, int n,
-                                                     T tol, int lane) {
-  T g = T(0);
-  for (int i = lane; i < n; i += 32) g = fma(wp[i], wq[i], g);
-  g = warp_sum_t(g);
-  const T a = *na, b = *nb;
-  T c, s;
-  if (!jacobi_rotation(a, b, g, tol, c, s)) return 0;
-  for (int i = lane; i < n; i += 32) {
-    const T x = wp[i], y = wq[i];
-    wp[i] = c * x - s * y;
-    wq[i] = s * x + c * y;
-    const T u = vp[i], v = vq[i];
-    vp[i] = c * u - s * v;
-    vq[i] = s * u + c * v;
+// One rotation of a column pair by a group of L lanes, with tracked squared column norms (*na, *nb): only
+// the inner product is reduced; the norms follow the rotation exactly (a' = c^2 a - 2cs g + s^2 b, b' =
+// s^2 a + 2cs g + c^2 b) and are recomputed from the columns once per sweep, which bounds their drift.
+// The lanes' EPL elements of the four columns are loaded before anything is stored, so the loads do not
+// wait for the stores. The rotation is recorded in `worst`.
+//
+// A sweep whose rotations had cosines up to c and sines up to t leaves cosines of about n c t: where that
+// is below the tolerance of n 2^-52 the sweep that would only confirm it is not run. (The cosines alone do
+// not tell: within a cluster of equal norms the angles stay large however small the cosines are.)
+constexpr int kNoRotation = -4096;
+
+struct JacobiWorst {
+  int cosine = kNoRotation, sine = kNoRotation;   // exponents of the largest squares
+  __device__ __forceinline__ bool converged() const { return cosine + sine <= -114; }
+};
+
+template <int L, int EPL>
+__device__ __forceinline__ void jacobi_rotate_tracked(double* wp, double* wq, double* vp, double* vq,
+                                                      double* na, double* nb, int n, double tol, int gl,
+                                                      unsigned mask, JacobiWorst& worst) {
+  double x[EPL], y[EPL], u[EPL], v[EPL];
+  double g = 0.0;
+#pragma unroll
+  for (int k = 0; k < EPL; ++k) {
+    const int i = gl + k * L;
+    x[k] = i < n ? wp[i] : 0.0;
+    y[k] = i < n ? wq[i] : 0.0;
+    u[k] = i < n ? vp[i] : 0.0;
+    v[k] = i < n ? vq[i] : 0.0;
+    g = fma(x[k], y[k], g);
   }
-  if (lane == 0) {
-    const T cc = c * c, ss = s * s, cs2 = T(2) * c * s * g;
-    const T a2 = cc * a - cs2 + ss * b, b2 = ss * a + cs2 + cc * b;
-    *na = a2 > T(0) ? a2 : T(0);
-    *nb = b2 > T(0) ? b2 : T(0);
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) g += __shfl_xor_sync(mask, g, o);
+  const double a = *na, b = *nb;
+  double c, s;
+  if (!jacobi_rotation(a, b, g, tol, c, s)) return;
+#pragma unroll
+  for (int k = 0; k < EPL; ++k) {
+    const int i = gl + k * L;
+    if (i < n) {
+      wp[i] = c * x[k] - s * y[k];
+      wq[i] = s * x[k] + c * y[k];
+      vp[i] = c * u[k] - s * v[k];
+      vq[i] = s * u[k] + c * v[k];
+    }
   }
-  return 1;
+  __syncwarp(mask);   // every lane has read the norms
+  if (gl == 0) {
+    const double cc = c * c, ss = s * s, cs2 = 2.0 * c * s * g;
+    const double a2 = cc * a - cs2 + ss * b, b2 = ss * a + cs2 + cc * b;
+    *na = a2 > 0.0 ? a2 : 0.0;
+    *nb = b2 > 0.0 ? b2 : 0.0;
+  }
+  const auto expo = [](double t) { return (__double2hiint(t) >> 20) & 0x7ff; };
+  worst.cosine = max(worst.cosine, 2 * expo(g) - expo(a) - expo(b));
+  worst.sine = max(worst.sine, 2 * (expo(s) - 1023));
 }
 
-template <typename T>
+// Powers of two that take a matrix whose largest entry has the high word `top` to about 1 and back: the
+// products of squared norms in the rotations stay in range. 1 for a matrix that is zero, not finite or
+// beyond 2^+-959.
+__device__ __forceinline__ void jacobi_scale(unsigned top, double& down, double& up) {
+  int e = (int)((top & 0x7fffffffu) >> 20);
+  if (e < 64 || e > 1982) e = 1023;
+  down = __hiloint2double((2046 - e) << 20, 0);
+  up = __hiloint2double(e << 20, 0);
+}
+
+// W = R^T scaled by jacobi_scale, *up the factor back. One block.
+__global__ void __launch_bounds__(1024) scaled_transpose_kernel(const double* __restrict__ R, int n, double* W,
+                                                                double* up) {
+  __shared__ unsigned top;
+  if (threadIdx.x == 0) top = 0u;
+  __syncthreads();
+  unsigned m = 0u;
+  for (int64_t t = threadIdx.x; t < (int64_t)n * n; t += blockDim.x)
+    m = max(m, (unsigned)__double2hiint(R[t]) & 0x7fffffffu);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(&top, m);
+  __syncthreads();
+  double d, u;
+  jacobi_scale(top, d, u);
+  if (threadIdx.x == 0) *up = u;
+  for (int64_t t = threadIdx.x; t < (int64_t)n * n; t += blockDim.x) {
+    const int64_t j = t / n, i = t - j * n;
+    W[t] = R[i * n + j] * d;
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+// One-sided (Hestenes) Jacobi of R^T (R column-major n x n, n < 16) in one warp: four lanes share a
+// column pair, so a round of the round-robin tournament is one rotation step of the whole warp without
+// a block barrier, and the scalars of all its rotations are computed at once (a warp per pair took 222
+// us at n = 12). Un: the normalised rotated columns, Vs: the rotations, both by descending S.
+// ---------------------------------------------------------------------------------------------
+constexpr int kJacobiWarpMaxN = 16;
+
+__global__ void __launch_bounds__(32) jacobi_warp_kernel(const double* __restrict__ R, int n, double* Un,
+                                                         double* S, double* Vs, int* status) {
+  constexpr int N = kJacobiWarpMaxN, ld = N + 1;
+  __shared__ double W[N * ld], V[N * ld], nrm[N];
+  const int lane = threadIdx.x, gid = lane / 4, gl = lane % 4;
+  const unsigned mask = 0xfu << (lane & 28);
+  unsigned top = 0u;
+  for (int t = lane; t < n * n; t += 32) top = max(top, (unsigned)__double2hiint(R[t]) & 0x7fffffffu);
+  double down, up;
+  jacobi_scale(__reduce_max_sync(0xffffffffu, top), down, up);
+  for (int t = lane; t < N * N; t += 32) {
+    const int j = t / N, i = t % N;
+    W[j * ld + i] = (i < n && j < n) ? R[(int64_t)i * n + j] * down : 0.0;
+    V[j * ld + i] = i == j ? 1.0 : 0.0;
+  }
+  __syncwarp();
+  const int nn = n + (n & 1);
+  const double tol = (double)n * kEps;
+  auto norms = [&]() {   // squared norms: two lanes per column
+    const int c = lane / 2;
+    double a = 0.0;
+#pragma unroll
+    for (int k = 0; k < N / 2; ++k) {
+      const double w = W[c * ld + 2 * k + (lane & 1)];
+      a = fma(w, w, a);
+    }
+    a += __shfl_xor_sync(0xffffffffu, a, 1);
+    if ((lane & 1) == 0) nrm[c] = a;
+    __syncwarp();
+  };
+  bool converged = false;
+  for (int sweep = 0; sweep < 60 && !converged; ++sweep) {
+    norms();
+    JacobiWorst worst;
+    int u = gid, v = nn - 1 - gid;   // the pair's places in the tournament
+    for (int r = 0; r < nn - 1; ++r) {
+      const int p = min(u, v), q = max(u, v);
+      if (gid < nn / 2 && q < n)
+        jacobi_rotate_tracked<4, N / 4>(W + p * ld, W + q * ld, V + p * ld, V + q * ld, nrm + p, nrm + q, n,
+                                        tol, gl, mask, worst);
+      if (u != 0 && ++u == nn) u = 1;
+      if (++v == nn) v = 1;
+      __syncwarp();
+    }
+    worst.cosine = __reduce_max_sync(0xffffffffu, worst.cosine);
+    worst.sine = __reduce_max_sync(0xffffffffu, worst.sine);
+    converged = worst.converged();
+  }
+  if (!converged && lane == 0) *status = 3;
+  norms();
+  if (lane < n) nrm[lane] = sqrt(nrm[lane]);
+  __syncwarp();
+  for (int j = 0; j < n; ++j) {
+    const double sj = nrm[j];
+    const double si = lane < n ? nrm[lane] : -1.0;
+    const int rk = __popc(__ballot_sync(0xffffffffu, lane < n && (si > sj || (si == sj && lane < j))));
+    if (lane == 0) S[rk] = sj * up;
+    if (lane < n) {
+      Un[(int64_t)rk * n + lane] = sj > 0.0 ? W[j * ld + lane] / sj : 0.0;
+      Vs[(int64_t)rk * n + lane] = V[j * ld + lane];
+    }
+  }
+}
+
+template <int EPL>
 __global__ void __cluster_dims__(kJacobiCluster, 1, 1) __launch_bounds__(256)
-    jacobi_block_kernel(const T* __restrict__ Win, int n, T* Wout, T* Vout, int max_sweeps,
-                        int* status, const T* __restrict__ Vin) {
+    jacobi_block_kernel(const double* __restrict__ Win, int n, double* Wout, double* Vout, int max_sweeps,
+                        int* status) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
-  T* sm = reinterpret_cast<T*>(sm_raw);
+  double* sm = reinterpret_cast<double*>(sm_raw);
   cg::cluster_group cluster = cg::this_cluster();
   constexpr int C = kJacobiCluster, P = 2 * kJacobiCluster;
   const int rank = (int)cluster.block_rank();
@@ -908,41 +930,43 @@ __global__ void __cluster_dims__(kJacobiCluster, 1, 1) __launch_bounds__(256)
   const int64_t blk = (int64_t)nb * n;   // elements of one block of W (or of V)
   const int64_t unit = 2 * blk + nb + (nb & 1);   // W block, V block, squared column norms
   // buffer x (0/1), slot s (0/1): W block, V block, norms
-  auto Wb = [&](T* base, int x, int sl) { return base + (int64_t)(x * 2 + sl) * unit; };
-  auto Vb = [&](T* base, int x, int sl) { return base + (int64_t)(x * 2 + sl) * unit + blk; };
-  auto Nb = [&](T* base, int x, int sl) { return base + (int64_t)(x * 2 + sl) * unit + 2 * blk; };
-  __shared__ int counts[kJacobiCluster];
-  __shared__ int local_cnt;
+  auto Wb = [&](double* base, int x, int sl) { return base + (int64_t)(x * 2 + sl) * unit; };
+  auto Vb = [&](double* base, int x, int sl) { return base + (int64_t)(x * 2 + sl) * unit + blk; };
+  auto Nb = [&](double* base, int x, int sl) { return base + (int64_t)(x * 2 + sl) * unit + 2 * blk; };
+  __shared__ int counts[2 * kJacobiCluster];   // in CTA 0: every CTA's largest cosine and sine of a sweep
+  __shared__ int local_cnt[2];
   const int tid = threadIdx.x, nt = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-  const T tol = T(n > 1 ? n : 1) * (sizeof(T) == 8 ? T(kEps) : T(1.1920929e-7f));
+  const double tol = (double)(n > 1 ? n : 1) * kEps;
+
   // round 0 of sweep 0: slot 0 holds block rank, slot 1 block P-1-rank
   for (int sl = 0; sl < 2; ++sl) {
     const int b = sl == 0 ? rank : P - 1 - rank;
-    T* W = Wb(sm, 0, sl);
-    T* V = Vb(sm, 0, sl);
+    double* W = Wb(sm, 0, sl);
+    double* V = Vb(sm, 0, sl);
     for (int64_t t = tid; t < blk; t += nt) {
       const int j = (int)(t / n), i = (int)(t - (int64_t)j * n);
       const int c = b * nb + j;
-      W[t] = (c < n) ? Win[(int64_t)c * n + i] : T(0);
-      V[t] = (c < n) ? (Vin ? Vin[(int64_t)c * n + i] : (i == c ? T(1) : T(0))) : T(0);
+      W[t] = (c < n) ? Win[(int64_t)c * n + i] : 0.0;
+      V[t] = (c < n) ? (i == c ? 1.0 : 0.0) : 0.0;
     }
   }
   int* counts0 = cluster.map_shared_rank(counts, 0);
-  int x = 0, r = 0, sweep = 0, mine = 0;
+  int x = 0, r = 0, sweep = 0;
+  JacobiWorst mine;
   bool converged = false;
-  if (tid == 0) local_cnt = 0;
+  if (tid < 2) local_cnt[tid] = kNoRotation;
   __syncthreads();
   while (true) {
     const int bA = rr_index(rank, r, P), bB = rr_index(P - 1 - rank, r, P);
-    T* WA = Wb(sm, x, 0); T* VA = Vb(sm, x, 0); T* NA = Nb(sm, x, 0);
-    T* WB = Wb(sm, x, 1); T* VB = Vb(sm, x, 1); T* NB = Nb(sm, x, 1);
+    double* WA = Wb(sm, x, 0); double* VA = Vb(sm, x, 0); double* NA = Nb(sm, x, 0);
+    double* WB = Wb(sm, x, 1); double* VB = Vb(sm, x, 1); double* NB = Nb(sm, x, 1);
     if (r == 0) {   // fresh column norms, then the pairs inside each block, once per sweep
       for (int c = warp; c < 2 * nb; c += nw) {
-        const T* w = (c < nb ? WA : WB) + (int64_t)(c % nb) * n;
-        T a = T(0);
+        const double* w = (c < nb ? WA : WB) + (int64_t)(c % nb) * n;
+        double a = 0.0;
         for (int i = lane; i < n; i += 32) a = fma(w[i], w[i], a);
-        a = warp_sum_t(a);
+        a = warp_sum_d(a);
         if (lane == 0) (c < nb ? NA : NB)[c % nb] = a;
       }
       __syncthreads();
@@ -953,11 +977,12 @@ __global__ void __cluster_dims__(kJacobiCluster, 1, 1) __launch_bounds__(256)
           int p = rr_index(pi, t, m2), q = rr_index(m2 - 1 - pi, t, m2);
           if (p > q) { const int u = p; p = q; q = u; }
           if (q >= nb) continue;
-          T* W = sl ? WB : WA;
-          T* V = sl ? VB : VA;
-          T* Nm = sl ? NB : NA;
-          mine += jacobi_rotate_tracked(W + (int64_t)p * n, W + (int64_t)q * n, V + (int64_t)p * n,
-                                        V + (int64_t)q * n, Nm + p, Nm + q, n, tol, lane);
+          double* W = sl ? WB : WA;
+          double* V = sl ? VB : VA;
+          double* Nm = sl ? NB : NA;
+          jacobi_rotate_tracked<32, EPL>(W + (int64_t)p * n, W + (int64_t)q * n, V + (int64_t)p * n,
+                                         V + (int64_t)q * n, Nm + p, Nm + q, n, tol, lane, 0xffffffffu,
+                                         mine);
         }
         __syncthreads();
       }
@@ -966,29 +991,35 @@ __global__ void __cluster_dims__(kJacobiCluster, 1, 1) __launch_bounds__(256)
       for (int j = warp; j < nb; j += nw) {
         const int k = (j + t) % nb;
         const int ga = bA * nb + j, gb = bB * nb + k;
-        T *wp = WA + (int64_t)j * n, *wq = WB + (int64_t)k * n;
-        T *vp = VA + (int64_t)j * n, *vq = VB + (int64_t)k * n;
-        T *np = NA + j, *nq = NB + k;
+        double *wp = WA + (int64_t)j * n, *wq = WB + (int64_t)k * n;
+        double *vp = VA + (int64_t)j * n, *vq = VB + (int64_t)k * n;
+        double *np = NA + j, *nq = NB + k;
         if (ga > gb) {
-          T* u = wp; wp = wq; wq = u; u = vp; vp = vq; vq = u; u = np; np = nq; nq = u;
+          double* u = wp; wp = wq; wq = u; u = vp; vp = vq; vq = u; u = np; np = nq; nq = u;
         }
-        mine += jacobi_rotate_tracked(wp, wq, vp, vq, np, nq, n, tol, lane);
+        jacobi_rotate_tracked<32, EPL>(wp, wq, vp, vq, np, nq, n, tol, lane, 0xffffffffu, mine);
       }
       __syncthreads();
     }
     const bool sweep_end = (r == P - 2);
     if (sweep_end) {
-      if (lane == 0 && mine) atomicAdd(&local_cnt, mine);
-      mine = 0;
+      if (lane == 0) {
+        atomicMax(&local_cnt[0], mine.cosine);
+        atomicMax(&local_cnt[1], mine.sine);
+      }
+      mine = JacobiWorst();
       __syncthreads();
-      if (tid == 0) { counts0[rank] = local_cnt; local_cnt = 0; }
+      if (tid < 2) { counts0[2 * rank + tid] = local_cnt[tid]; local_cnt[tid] = kNoRotation; }
     }
     cluster.sync();   // every CTA finished round r (and published its count at a sweep end)
     if (sweep_end) {
-      int total = 0;
-      for (int c = 0; c < C; ++c) total += counts0[c];
+      JacobiWorst all;
+      for (int c = 0; c < C; ++c) {
+        all.cosine = max(all.cosine, counts0[2 * c]);
+        all.sine = max(all.sine, counts0[2 * c + 1]);
+      }
       ++sweep;
-      if (total == 0) { converged = true; break; }
+      if (all.converged()) { converged = true; break; }
       if (sweep >= max_sweeps) break;
     }
     // pull the blocks of round r+1 into buffer 1-x from their holders' buffer x
@@ -1000,12 +1031,12 @@ __global__ void __cluster_dims__(kJacobiCluster, 1, 1) __launch_bounds__(256)
         if (rr_index(c, r, P) == b) { owner = c; oslot = 0; }
         if (rr_index(P - 1 - c, r, P) == b) { owner = c; oslot = 1; }
       }
-      const T* srcW = cluster.map_shared_rank(Wb(sm, x, oslot), owner);
-      const T* srcV = cluster.map_shared_rank(Vb(sm, x, oslot), owner);
-      const T* srcN = cluster.map_shared_rank(Nb(sm, x, oslot), owner);
-      T* dW = Wb(sm, 1 - x, sl);
-      T* dV = Vb(sm, 1 - x, sl);
-      T* dN = Nb(sm, 1 - x, sl);
+      const double* srcW = cluster.map_shared_rank(Wb(sm, x, oslot), owner);
+      const double* srcV = cluster.map_shared_rank(Vb(sm, x, oslot), owner);
+      const double* srcN = cluster.map_shared_rank(Nb(sm, x, oslot), owner);
+      double* dW = Wb(sm, 1 - x, sl);
+      double* dV = Vb(sm, 1 - x, sl);
+      double* dN = Nb(sm, 1 - x, sl);
       for (int64_t t = tid; t < blk; t += nt) { dW[t] = srcW[t]; dV[t] = srcV[t]; }
       for (int t = tid; t < nb; t += nt) dN[t] = srcN[t];
     }
@@ -1017,8 +1048,8 @@ __global__ void __cluster_dims__(kJacobiCluster, 1, 1) __launch_bounds__(256)
   // buffer x holds the blocks of round r
   for (int sl = 0; sl < 2; ++sl) {
     const int b = rr_index(sl == 0 ? rank : P - 1 - rank, r, P);
-    const T* W = Wb(sm, x, sl);
-    const T* V = Vb(sm, x, sl);
+    const double* W = Wb(sm, x, sl);
+    const double* V = Vb(sm, x, sl);
     for (int64_t t = tid; t < blk; t += nt) {
       const int j = (int)(t / n), i = (int)(t - (int64_t)j * n);
       const int c = b * nb + j;
@@ -1029,6 +1060,181 @@ __global__ void __cluster_dims__(kJacobiCluster, 1, 1) __launch_bounds__(256)
     }
   }
   cluster.sync();   // no CTA leaves while another may still read its shared memory
+}
+
+// ---------------------------------------------------------------------------------------------
+// FP32 one-sided Jacobi on R^T (R column-major n x n) in one block, for a starting basis: X (column-major)
+// gets the normalised columns of the rotated R^T by descending norm, i.e. R's right singular vectors to
+// FP32 accuracy, sig their norms for the matrix scaled to largest entry 1, *scale the factor back,
+// inv_sig the reciprocals of the unscaled norms; *bad = 1 when a norm is zero or not finite.
+// The whole matrix is in shared memory and a round of the tournament one batch of pairs. The block is
+// bound by its instruction issue, so 8 lanes share a pair: the scalars of a rotation are then computed
+// for four pairs at once (with a warp per pair a round took 1600 cycles at n = 77). The column pitch is 8
+// modulo 32, which puts the four column pairs of a warp, neighbours in the tournament, on different
+// banks. A sweep stops the iteration when no cosine in it was above 1e-4: its own rotations leave about
+// n times the square (*bad = 1 when 16 sweeps do not get there).
+// ---------------------------------------------------------------------------------------------
+constexpr int kJacobiF32MaxN = 224;
+
+// pitch of the columns, which hold 8 EPL elements (zeros past n)
+__host__ __device__ constexpr int jacobi_f32_pitch(int epl) { return (8 * epl + 23) / 32 * 32 + 8; }
+
+template <int EPL>
+__global__ void __launch_bounds__(32 * EPL) jacobi_f32_kernel(const double* __restrict__ R, int n, double* X,
+                                                          double* sig, double* inv_sig, double* scale,
+                                                          int* bad) {
+  constexpr int L = 8, ld = jacobi_f32_pitch(EPL);
+  extern __shared__ float wf[];
+  __shared__ unsigned top, cmax;
+  __shared__ float nrm[kJacobiF32MaxN];
+  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
+  if (tid == 0) { top = 0u; cmax = 0u; }
+  __syncthreads();
+  unsigned mx = 0u;
+  for (int t = tid; t < n * n; t += nt) mx = max(mx, (unsigned)__double2hiint(R[t]) & 0x7fffffffu);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (lane == 0) atomicMax(&top, mx);
+  __syncthreads();
+  const int e = (int)(top >> 20);   // exponent field of the largest entry
+  if (e < 64 || e > 1982) {         // zero, not finite, or outside the scale's range
+    if (tid == 0) *bad = 1;
+    return;
+  }
+  double down, up;
+  jacobi_scale(top, down, up);
+  for (int t = tid; t < n * ld; t += nt) wf[t] = 0.f;
+  __syncthreads();
+  for (int t = tid; t < n * n; t += nt) {
+    const int i = t / n, j = t - i * n;   // R[j, i] = R^T[i, j]
+    wf[j * ld + i] = (float)(R[t] * down);
+  }
+  __syncthreads();
+  const int nn = n + (n & 1), gid = tid / L, gl = tid % L;
+  const unsigned mask = 0xffu << (lane & 24);
+  const bool pair = gid < nn / 2;
+  for (int sweep = 0; sweep < 16; ++sweep) {
+    float worst = 0.f;
+    // positions gid and nn - 1 - gid of the tournament: each column but 0 moves on by one per round
+    int u = gid == 0 ? 0 : gid, v = nn - 1 - gid;
+    for (int r = 0; r < nn - 1; ++r) {
+      const int p = min(u, v), q = max(u, v);
+      if (pair && q < n) {
+        float* wp = wf + p * ld + gl;
+        float* wq = wf + q * ld + gl;
+        float x[EPL], y[EPL];
+        float a = 0.f, b = 0.f, g = 0.f;
+#pragma unroll
+        for (int k = 0; k < EPL; ++k) {
+          x[k] = wp[k * L];
+          y[k] = wq[k * L];
+          a = fmaf(x[k], x[k], a);
+          b = fmaf(y[k], y[k], b);
+          g = fmaf(x[k], y[k], g);
+        }
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) {
+          a += __shfl_xor_sync(mask, a, o);
+          b += __shfl_xor_sync(mask, b, o);
+          g += __shfl_xor_sync(mask, g, o);
+        }
+        // the cosine, without the square of a small column's square
+        const float cosine = fabsf(g) * rsqrtf(a) * rsqrtf(b);
+        if (cosine > 3e-7f && a > 0.f && b > 0.f) {
+          worst = fmaxf(worst, cosine);
+          // t = tan of the angle = h / (d + sign(d) sqrt(d^2 + h^2)) with d = b - a, h = 2 g, scaled
+          const float d = b - a, h = 2.0f * g, m = __fdividef(1.0f, fmaxf(fabsf(d), fabsf(h)));
+          const float ds = d * m, hs = h * m, w = fmaf(ds, ds, hs * hs);
+          const float t = __fdividef(hs, ds + copysignf(w * rsqrtf(w), ds));
+          const float c = rsqrtf(fmaf(t, t, 1.0f)), s = c * t;
+#pragma unroll
+          for (int k = 0; k < EPL; ++k) {
+            wp[k * L] = c * x[k] - s * y[k];
+            wq[k * L] = s * x[k] + c * y[k];
+          }
+        }
+      }
+      if (u != 0 && ++u == nn) u = 1;
+      if (++v == nn) v = 1;
+      __syncthreads();
+    }
+    const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(worst));
+    if (lane == 0) atomicMax(&cmax, w);
+    __syncthreads();
+    const float left = __uint_as_float(cmax);
+    __syncthreads();
+    if (tid == 0) {
+      cmax = 0u;
+      if (sweep == 15 && left > 1e-4f) *bad = 1;
+    }
+    if (!(left > 1e-4f)) break;
+  }
+  __syncthreads();
+  for (int j = gid; j < n; j += nt / L) {
+    float a = 0.f;
+    for (int i = gl; i < n; i += L) a = fmaf(wf[j * ld + i], wf[j * ld + i], a);
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) a += __shfl_xor_sync(mask, a, o);
+    if (gl == 0) nrm[j] = sqrtf(a);
+  }
+  __syncthreads();
+  for (int j = gid; j < n; j += nt / L) {
+    const float sj = nrm[j];
+    int rk = 0;
+    for (int i = gl; i < n; i += L) {
+      const float si = nrm[i];
+      rk += (si > sj) || (si == sj && i < j) ? 1 : 0;
+    }
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) rk += __shfl_xor_sync(mask, rk, o);
+    const float inv = 1.0f / sj;
+    if (gl == 0) {
+      if (!(sj > 1e-18f) || !(sj < 1e18f)) *bad = 1;
+      sig[rk] = (double)sj;
+      inv_sig[rk] = 1.0 / ((double)sj * up);
+      if (j == 0) *scale = up;
+    }
+    for (int i = gl; i < n; i += L) X[(int64_t)rk * n + i] = (double)(wf[j * ld + i] * inv);
+  }
+}
+
+// E = G - I into G, both triangles, from the lower (column-major) triangle of G. One block. *bad = 1
+// when ||E||_F > 2e-4 (the polar factor below is then not orthonormal to rounding).
+__global__ void __launch_bounds__(1024) polar_error_kernel(double* G, int n, int* bad) {
+  __shared__ float sums[32];
+  float s = 0.f;
+  for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
+    const int j = t / n, i = t - j * n;
+    if (i < j) continue;
+    const double e = G[t] - (i == j ? 1.0 : 0.0);
+    G[t] = e;
+    if (i != j) G[(int64_t)i * n + j] = e;
+    const float f = (float)e;
+    s = fmaf(f, i == j ? f : 2.0f * f, s);
+  }
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 32; ++w) s += sums[w];
+    if (!(s <= 4e-8f)) *bad = 1;
+  }
+}
+
+// P = I - E / 2 + 3/8 F (column-major n x n)
+__global__ void polar_start_kernel(const double* __restrict__ E, const double* __restrict__ F, double* P,
+                                   int n) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n * n; t += gridDim.x * blockDim.x)
+    P[t] = (t / n == t % n ? 1.0 : 0.0) + fma(0.375, F[t], -0.5 * E[t]);
+}
+
+// X[:, j] *= d[j] (column-major n x n); with T: T[i, j] = X[j, i] d[i] instead
+__global__ void scale_cols_kernel(double* X, const double* __restrict__ d, int n, double* T) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n * n; t += gridDim.x * blockDim.x) {
+    const int j = t / n, i = t - j * n;
+    const double v = X[t] * d[j];
+    if (T) T[i * n + j] = v;
+    else X[t] = v;
+  }
 }
 
 // Grid-wide block Jacobi for larger n (W, V column-major n x n in global memory, L2-resident):
@@ -1094,11 +1300,11 @@ __global__ void identity_kernel(double* V, int n) {
 }
 
 // From the rotated W (column-major n x n) and the rotations V: sigma_j = ||W_j||, descending order;
-// Un[:, rank_j] = W_j / sigma_j, Vs[:, rank_j] = V_j, S[rank_j] = sigma_j. One block.
+// Un[:, rank_j] = W_j / sigma_j, Vs[:, rank_j] = V_j, S[rank_j] = sigma_j *scale. One block.
 __global__ void __launch_bounds__(1024) svd_sort_kernel(const double* __restrict__ W,
                                                         const double* __restrict__ V, int n,
                                                         double* Un, double* S, double* Vs,
-                                                        double* sig) {
+                                                        double* sig, const double* scale) {
   __shared__ int rank_sh[1024];
   const int tid = threadIdx.x, nt = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
@@ -1119,7 +1325,8 @@ __global__ void __launch_bounds__(1024) svd_sort_kernel(const double* __restrict
     rank_sh[j] = rk;
   }
   __syncthreads();
-  for (int j = tid; j < n; j += nt) S[rank_sh[j]] = sig[j];
+  const double up = *scale;
+  for (int j = tid; j < n; j += nt) S[rank_sh[j]] = sig[j] * up;
   for (int j = warp; j < n; j += nw) {
     const int rk = rank_sh[j];
     const double inv = sig[j] > 0.0 ? 1.0 / sig[j] : 0.0;
@@ -1314,6 +1521,109 @@ QRResult qr(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, doubl
   return res;
 }
 
+namespace {
+
+template <int EPL>
+void launch_jacobi_block(double* W, double* V, int n, size_t smem, int* status, cudaStream_t s) {
+  smem_optin((const void*)jacobi_block_kernel<EPL>, (int)smem);
+  jacobi_block_kernel<EPL><<<kJacobiCluster, 256, smem, s>>>(W, n, W, V, 60, status);
+  TTGB_CHECK_LAUNCH();
+}
+
+// FP64 one-sided Jacobi of the columns of W (n x n column-major, n >= 2 kJacobiCluster, rotated in
+// place; V: n x n scratch): W V = Un diag(S) / *scale, S descending, the rotations in Vs.
+void jacobi_columns(double* W, double* V, int64_t n, const double* scale, double* Un, double* S, double* Vs,
+                    LinalgWS& ws, cudaStream_t s) {
+  if (n <= kJacobiBlockMaxN) {
+    const int nb = (int)((n + 2 * kJacobiCluster - 1) / (2 * kJacobiCluster));
+    const int64_t unit = 2 * nb * n + nb + (nb & 1);
+    const size_t smem = (size_t)4 * unit * sizeof(double);
+    if (n <= 32) launch_jacobi_block<1>(W, V, (int)n, smem, ws.status, s);
+    else if (n <= 64) launch_jacobi_block<2>(W, V, (int)n, smem, ws.status, s);
+    else if (n <= 96) launch_jacobi_block<3>(W, V, (int)n, smem, ws.status, s);
+    else launch_jacobi_block<5>(W, V, (int)n, smem, ws.status, s);
+  } else {   // grid-wide block Jacobi, one launch per round
+    const int sms = num_sms();
+    const int nb = (int)std::max<int64_t>(1, (n + 2 * sms - 1) / (2 * sms));
+    int P = (int)((n + nb - 1) / nb);
+    P += P & 1;
+    identity_kernel<<<cdiv((int64_t)n * n, 256), 256, 0, s>>>(V, (int)n);
+    TTGB_CHECK_LAUNCH();
+    DevBuf<unsigned> cnt(1, s);
+    unsigned hcnt = 0;
+    const double tol = std::max((double)n, 1.0) * kEps;
+    int sweep = 0;
+    for (; sweep < 60; ++sweep) {
+      TTGB_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(unsigned), s));
+      for (int r = 0; r < P - 1; ++r) {
+        jacobi_grid_round_kernel<<<P / 2, 256, 0, s>>>(W, V, (int)n, nb, P, r, tol, cnt.p);
+        TTGB_CHECK_LAUNCH();
+      }
+      TTGB_CUDA(cudaMemcpyAsync(&hcnt, cnt.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+      TTGB_CUDA(cudaStreamSynchronize(s));
+      if (hcnt == 0) break;
+    }
+    if (sweep >= 60) TTGB_CUDA(cudaMemsetAsync(ws.status, 0x03, 1, s));
+  }
+  DBuf sig((size_t)n, s);
+  svd_sort_kernel<<<1, 1024, 0, s>>>(W, V, (int)n, Un, S, Vs, sig.p, scale);
+  TTGB_CHECK_LAUNCH();
+}
+
+template <int EPL>
+void launch_jacobi_f32(const double* R, int n, double* X, double* sig, int* bad, cudaStream_t s) {
+  const int smem = 8 * EPL * jacobi_f32_pitch(EPL) * (int)sizeof(float);
+  smem_optin((const void*)jacobi_f32_kernel<EPL>, smem);
+  jacobi_f32_kernel<EPL><<<1, cdiv((n + 1) / 2 * 8, 32) * 32, smem, s>>>(R, n, X, sig, sig + n, sig + 2 * n,
+                                                                           bad);
+  TTGB_CHECK_LAUNCH();
+}
+
+// From here on the preconditioned route is the faster one (n = 16: 256 against 460 us).
+constexpr int64_t kPreconditionMinN = 16;
+
+// A start for the FP64 Jacobi from FP32: X (n x n, orthonormal to FP64 rounding, followed by n
+// estimates of the singular values of the scaled R, the n reciprocals for R itself, and the scale) holds R's right singular vectors to FP32
+// accuracy, and B = R X diag(1 / sigma), whose columns are nearly orthonormal. The QR factor L of R X is
+// then so near to diagonal, whatever the grading, that Jacobi on L^T takes two or three sweeps where
+// it takes nine on R^T (FP32 rotations alone leave six to ten sweeps for a graded R, whose small
+// columns drown in the FP32 rounding of the large ones; the QR step removes that). Returns false
+// when the FP32 sweeps cannot be used (R zero, not finite or numerically singular beyond FP32).
+bool precondition(const double* R, int64_t n, DBuf& X, DBuf& B, LinalgWS& ws, const RedWS& red,
+                  cudaStream_t s) {
+  (void)red;
+  X.reset((size_t)(n * n + 2 * n + 1), s);
+  B.reset((size_t)(n * n), s);
+  DBuf X0((size_t)(n * n), s), G((size_t)(n * n), s), P((size_t)(n * n), s);
+  double* sig = X.p + n * n;
+  double* inv = sig + n;
+  int* bad = ws.status + 3;
+  TTGB_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
+  if (n <= 32) launch_jacobi_f32<4>(R, (int)n, X0.p, sig, bad, s);
+  else if (n <= 64) launch_jacobi_f32<8>(R, (int)n, X0.p, sig, bad, s);
+  else if (n <= 80) launch_jacobi_f32<10>(R, (int)n, X0.p, sig, bad, s);
+  else if (n <= 112) launch_jacobi_f32<14>(R, (int)n, X0.p, sig, bad, s);
+  else if (n <= 160) launch_jacobi_f32<20>(R, (int)n, X0.p, sig, bad, s);
+  else launch_jacobi_f32<28>(R, (int)n, X0.p, sig, bad, s);
+  // X = X0 (I - E/2 + 3/8 E^2 - 5/16 E^3) with E = X0^T X0 - I: the polar factor to fourth order
+  gemm_cm(X0.p, n, X0.p, n, G.p, n, n, n, n, 1.0, 0.0, s, true, false, kTriLowerC);
+  polar_error_kernel<<<1, 1024, 0, s>>>(G.p, (int)n, bad);
+  TTGB_CHECK_LAUNCH();
+  gemm_cm(G.p, n, G.p, n, B.p, n, n, n, n, 1.0, 0.0, s);
+  polar_start_kernel<<<cdiv(n * n, 256), 256, 0, s>>>(G.p, B.p, P.p, (int)n);
+  TTGB_CHECK_LAUNCH();
+  gemm_cm(B.p, n, G.p, n, P.p, n, n, n, n, -0.3125, 1.0, s);
+  gemm_cm(X0.p, n, P.p, n, X.p, n, n, n, n, 1.0, 0.0, s);
+  gemm_cm(R, n, X.p, n, B.p, n, n, n, n, 1.0, 0.0, s);
+  scale_cols_kernel<<<cdiv(n * n, 256), 256, 0, s>>>(B.p, inv, (int)n, nullptr);
+  TTGB_CHECK_LAUNCH();
+  TTGB_CUDA(cudaMemcpyAsync(ws.h_status, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
+  TTGB_CUDA(cudaStreamSynchronize(s));
+  return *ws.h_status == 0;
+}
+
+}  // namespace
+
 void svd(const double* A, int64_t lda, int64_t m, int64_t n, double* U, double* S, double* Vh,
          LinalgWS& ws, const RedWS& red, cudaStream_t s) {
   if (m <= 0 || n <= 0) return;
@@ -1335,68 +1645,39 @@ void svd(const double* A, int64_t lda, int64_t m, int64_t n, double* U, double* 
   DBuf Qb((size_t)(m * n), s), Rb((size_t)(n * n), s);
   qr(A, lda, m, n, Qb.p, Rb.p, ws, red, s);
   TTGB_REQUIRE(n <= 1024, "SVD: too many columns");
-  ws.c.ensure(3 * n * n + 16, s);
-  double* W = ws.c.p;        // n x n: R^T, rotated in place
-  double* Vw = W + n * n;    // 2 n x n: accumulated rotations V' (sorted) and scratch
-  transpose(Rb.p, n, W, n, n, n, s);
-  DBuf Up((size_t)(n * n), s);   // U' (normalised columns of the rotated R^T, sorted)
-  if (n <= kJacobiBlockMaxN && n >= 2 * kJacobiCluster) {
-    const int nb = (int)((n + 2 * kJacobiCluster - 1) / (2 * kJacobiCluster));
-    const int64_t unit = 2 * nb * n + nb + (nb & 1);
-    const size_t smem = (size_t)4 * unit * sizeof(double);
-    smem_optin((const void*)jacobi_block_kernel<double>, (int)smem);
-    jacobi_block_kernel<double><<<kJacobiCluster, 256, smem, s>>>(W, (int)n, W, Vw, 60, ws.status,
-                                                                  nullptr);
-    TTGB_CHECK_LAUNCH();
-    DBuf sig((size_t)n, s);
-    svd_sort_kernel<<<1, 1024, 0, s>>>(W, Vw, (int)n, Up.p, S, Vw + n * n, sig.p);
-    TTGB_CHECK_LAUNCH();
-    gemm_cm(Qb.p, m, Vw + n * n, n, U, m, m, n, n, 1.0, 0.0, s);   // U = Q V'
-    transpose(Up.p, n, Vh, n, n, n, s);                            // Vh = U'^T
-    return;
-  }
-  if (n > kJacobiBlockMaxN) {   // grid-wide block Jacobi, one launch per round
-    const int sms = num_sms();
-    const int nb = (int)std::max<int64_t>(1, (n + 2 * sms - 1) / (2 * sms));
-    int P = (int)((n + nb - 1) / nb);
-    P += P & 1;
-    identity_kernel<<<cdiv((int64_t)n * n, 256), 256, 0, s>>>(Vw, (int)n);
-    TTGB_CHECK_LAUNCH();
-    DevBuf<unsigned> cnt(1, s);
-    unsigned hcnt = 0;
-    const double tol = std::max((double)n, 1.0) * kEps;
-    int sweep = 0;
-    for (; sweep < 60; ++sweep) {
-      TTGB_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(unsigned), s));
-      for (int r = 0; r < P - 1; ++r) {
-        jacobi_grid_round_kernel<<<P / 2, 256, 0, s>>>(W, Vw, (int)n, nb, P, r, tol, cnt.p);
-        TTGB_CHECK_LAUNCH();
-      }
-      TTGB_CUDA(cudaMemcpyAsync(&hcnt, cnt.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-      TTGB_CUDA(cudaStreamSynchronize(s));
-      if (hcnt == 0) break;
+  if (n >= kPreconditionMinN && n <= kJacobiF32MaxN) {
+    DBuf X, B;
+    if (precondition(Rb.p, n, X, B, ws, red, s)) {
+      // R X = Q2 L with L^T = U'' S V''^T:  A = (Q Q2 V'') S (X U'')^T
+      DBuf Q2((size_t)(n * n), s), T((size_t)(n * n), s), Un((size_t)(n * n), s);
+      DBuf Vs((size_t)(n * n), s);
+      const double* sig = X.p + n * n;
+      qr(B.p, n, n, n, Q2.p, T.p, ws, red, s);
+      ws.c.ensure(3 * n * n + 16, s);
+      scale_cols_kernel<<<cdiv(n * n, 256), 256, 0, s>>>(T.p, sig, (int)n, ws.c.p);
+      TTGB_CHECK_LAUNCH();
+      jacobi_columns(ws.c.p, ws.c.p + n * n, n, sig + 2 * n, Un.p, S, Vs.p, ws, s);
+      gemm_cm(Q2.p, n, Vs.p, n, T.p, n, n, n, n, 1.0, 0.0, s);
+      gemm_cm(Qb.p, m, T.p, n, U, m, m, n, n, 1.0, 0.0, s);
+      gemm_cm(Un.p, n, X.p, n, Vh, n, n, n, n, 1.0, 0.0, s, true, true);
+      return;
     }
-    if (sweep >= 60) TTGB_CUDA(cudaMemsetAsync(ws.status, 0x03, 1, s));
-    DBuf sig((size_t)n, s);
-    svd_sort_kernel<<<1, 1024, 0, s>>>(W, Vw, (int)n, Up.p, S, Vw + n * n, sig.p);
-    TTGB_CHECK_LAUNCH();
-    gemm_cm(Qb.p, m, Vw + n * n, n, U, m, m, n, n, 1.0, 0.0, s);   // U = Q V'
-    transpose(Up.p, n, Vh, n, n, n, s);                            // Vh = U'^T
-    return;
   }
-  const size_t smem = (size_t)2 * n * n * sizeof(double);
-  const int use_smem = smem <= 200 * 1024 ? 1 : 0;
-  if (use_smem) smem_optin((const void*)jacobi_svd_kernel, (int)smem);
-  // one warp per column pair of a round (n < 2 * kJacobiCluster here): idle warps would only
-  // lengthen every block barrier of the round-robin sweep
-  const int threads = (int)std::min<int64_t>(512, 32 * std::max<int64_t>(1, (n + 1) / 2));
-  jacobi_svd_kernel<<<1, threads, use_smem ? smem : 0, s>>>(W, Vw, (int)n, Up.p, S, use_smem, 60,
-                                                             ws.status, nullptr);
-  TTGB_CHECK_LAUNCH();
-  // U = Q V'
-  gemm_cm(Qb.p, m, Vw, n, U, m, m, n, n, 1.0, 0.0, s);
-  // Vh (n x n col-major) = U'^T
-  transpose(Up.p, n, Vh, n, n, n, s);
+  ws.c.ensure(3 * n * n + 16, s);
+  double* Vs = ws.c.p;           // V'
+  DBuf Up((size_t)(n * n), s);   // U' (normalised columns of the rotated R^T, sorted)
+  if (n < kJacobiWarpMaxN) {
+    jacobi_warp_kernel<<<1, 32, 0, s>>>(Rb.p, (int)n, Up.p, S, Vs, ws.status);
+    TTGB_CHECK_LAUNCH();
+  } else {
+    double* W = Vs + n * n;      // R^T, rotated in place
+    double* scale = W + 2 * n * n;
+    scaled_transpose_kernel<<<1, 1024, 0, s>>>(Rb.p, (int)n, W, scale);
+    TTGB_CHECK_LAUNCH();
+    jacobi_columns(W, W + n * n, n, scale, Up.p, S, Vs, ws, s);
+  }
+  gemm_cm(Qb.p, m, Vs, n, U, m, m, n, n, 1.0, 0.0, s);   // U = Q V'
+  transpose(Up.p, n, Vh, n, n, n, s);                    // Vh = U'^T
 }
 
 void gemv(const double* B, int64_t n, const double* x, double* y, cudaStream_t s) {
