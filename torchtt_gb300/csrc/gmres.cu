@@ -12,7 +12,7 @@ namespace ttgb {
 
 SplitOut LocalOperator::input_split() const {
   SplitOut o;
-  if (lowp && tc && prec == kNoPrec) {
+  if (lowp && tc && prec == kNoPrec && size() < (int64_t(1) << 31)) {
     o.hi = tc->xh.p;
     o.lo = tc->xl.p;
     o.nR = dims.n * dims.R;
@@ -62,6 +62,7 @@ namespace {
 
 using red::RT;
 using red::block_sum;
+using red::rsqrt_full;
 constexpr int kMaxVec = 128;   // basis vectors a cycle may hold (RedWS::cap_vec + 1)
 
 // scalar slots after the Hessenberg data in GmresWS::small
@@ -71,6 +72,7 @@ enum ScalSlot : int {
   kWNorm2,        // ||w||^2 of the operator output, before orthogonalisation
   kHn,            // H[k+1, k]
   kErr,           // |beta[k+1]| / ||rhs||
+  kRhsInv,        // 1 / ||rhs||
   kNumScal = 12
 };
 
@@ -115,7 +117,10 @@ __global__ void __launch_bounds__(RT) cycle_start_kernel(const double* __restric
   if (tid < 32) tot = red::warp_sum_partials(partial, 0, gridDim.x);
   if (tid == 0) {
     const double nr = sqrt(tot);
-    if (first) scal[kRhsNorm] = nr;
+    if (first) {
+      scal[kRhsNorm] = nr;
+      scal[kRhsInv] = 1.0 / nr;
+    }
     scal[kResNorm] = nr;
     beta[0] = nr;
     flag[kGmresState] = (nr > 0.0) ? 0 : 2;   // 2: r == 0, nothing to do (gmres.h:56-65)
@@ -131,7 +136,9 @@ __global__ void __launch_bounds__(RT) cycle_start_kernel(const double* __restric
 __device__ __forceinline__ void put_split(const SplitOut& o, int64_t i, double v) {
   const float f = (float)v;
   const float h = to_tf32(f);
-  const int64_t off = (i % o.nR) * o.ld + i / o.nR;
+  // 32-bit: input_split() offers a target only for vectors below 2^31 elements
+  const unsigned col = (unsigned)i / (unsigned)o.nR, row = (unsigned)i - col * (unsigned)o.nR;
+  const int64_t off = (int64_t)row * o.ld + col;
   o.hi[off] = h;
   o.lo[off] = to_tf32(f - h);
 }
@@ -215,9 +222,15 @@ __device__ __forceinline__ void reduce_partials(const double* part, int G, int n
   const int tid = threadIdx.x, lane = tid & 31;
   const int col = tid & (width - 1), first = tid / width, step = RT / width;
   double s = 0.0;
-  if (col < nv) {
-#pragma unroll 8
-    for (int g = first; g < G; g += step) s += __ldcg(part + (int64_t)g * nv + col);
+  if (col < nv) {   // four sums at once: a chain of dependent FP64 adds would take longer than the loads
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+    for (int g = first; g < G; g += 4 * step) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (g + q * step < G) a[q] += __ldcg(part + (int64_t)(g + q * step) * nv + col);
+    }
+    s = (a[0] + a[1]) + (a[2] + a[3]);
   }
   int rows = step;
   if (width < 32) {
@@ -228,10 +241,13 @@ __device__ __forceinline__ void reduce_partials(const double* part, int G, int n
     sh[tid] = s;
   }
   __syncthreads();
-  if (tid < nv) {
-    double t = 0.0;
-    for (int q = 0; q < rows; ++q) t += sh[q * width + tid];
-    out[tid] = t;
+  if (tid < nv) {   // rows is a power of two, 2 to 8
+    double a = 0.0, b = 0.0;
+    for (int q = 0; q < rows; q += 2) {
+      a += sh[q * width + tid];
+      b += sh[(q + 1) * width + tid];
+    }
+    out[tid] = a + b;
   }
   __syncthreads();
 }
@@ -296,9 +312,11 @@ __device__ __forceinline__ double slice_combination(const double* __restrict__ Q
   for (int e = 0; e < E; ++e) sh[warp * 32 * E + e * 32 + lane] = t[e];
   __syncthreads();
   double s = 0.0;
-  const int used = min(kv, kWarps);   // the other warps hold zeros
-  if (threadIdx.x < 32 * E)
-    for (int q = 0; q < used; ++q) s += sh[q * 32 * E + threadIdx.x];
+  if (threadIdx.x < 32 * E) {   // the warps without a vector hold zeros
+    const double* p = sh + threadIdx.x;
+    constexpr int o = 32 * E;
+    s = ((p[0] + p[o]) + (p[2 * o] + p[3 * o])) + ((p[4 * o] + p[5 * o]) + (p[6 * o] + p[7 * o]));
+  }
   return s;
 }
 
@@ -353,18 +371,23 @@ __global__ void __launch_bounds__(RT) arnoldi_reorth_kernel(const double* __rest
   store_partials<VP>(acc, kv + 1, part_out);
 }
 
-// The Givens rotations of the cycle applied to the new Hessenberg column h (k + 2 values, shared
-// memory), the new rotation, the residual estimate and the stop flag (apply_givens_rotation_cpu and
-// the convergence test, cpp/gmres.h:20-31,105-129). One warp; cs and sn are read in parallel first.
-__device__ __forceinline__ void givens_step(double* h, double* rot, int k, int iters, double hn,
-                                            double* H, double* cs, double* sn, double* beta,
-                                            double threshold, double* scal, int* flag, int reorth_vecs) {
-  const int lane = threadIdx.x & 31;
-  for (int i = lane; i < k; i += 32) {
+// The new Hessenberg column (h1 + h2, h2 may be null) and the cycle's rotations into shared memory.
+__device__ __forceinline__ void givens_load(double* h, double* rot, const double* h1, const double* h2,
+                                            int k, const double* cs, const double* sn, int tid, int nt) {
+  for (int i = tid; i <= k; i += nt) h[i] = h2 ? h1[i] + h2[i] : h1[i];
+  for (int i = tid; i < k; i += nt) {
     rot[2 * i] = cs[i];
     rot[2 * i + 1] = sn[i];
   }
-  __syncwarp();
+}
+
+// The Givens rotations of the cycle applied to the new Hessenberg column h (k + 2 values, shared
+// memory), the new rotation, the residual estimate and the stop flag (apply_givens_rotation_cpu and
+// the convergence test, cpp/gmres.h:20-31,105-129). One warp, after givens_load.
+__device__ __forceinline__ void givens_step(double* h, const double* rot, int k, int iters, double hn,
+                                            double* H, double* cs, double* sn, double* beta,
+                                            double threshold, double* scal, int* flag, int reorth_vecs) {
+  const int lane = threadIdx.x & 31;
   double* hc = H + (int64_t)k * (iters + 1);
   if (lane == 0) {
     double cur = h[0];
@@ -373,9 +396,13 @@ __device__ __forceinline__ void givens_step(double* h, double* rot, int k, int i
       h[i] = c * cur + s * nx;
       cur = c * nx - s * cur;
     }
-    const double den = sqrt(cur * cur + hn * hn);
+    const double den2 = fma(cur, cur, hn * hn);
     double c = 1.0, s = 0.0;
-    if (den > 0.0) { c = cur / den; s = hn / den; }
+    if (den2 > 0.0) {
+      const double inv = rsqrt_full(den2);
+      c = cur * inv;
+      s = hn * inv;
+    }
     h[k] = c * cur + s * hn;
     h[k + 1] = 0.0;
     cs[k] = c;
@@ -383,7 +410,7 @@ __device__ __forceinline__ void givens_step(double* h, double* rot, int k, int i
     const double bk = beta[k], b1 = -s * bk;
     beta[k + 1] = b1;
     beta[k] = c * bk;
-    const double err = fabs(b1) / scal[kRhsNorm];
+    const double err = fabs(b1) * scal[kRhsInv];
     scal[kErr] = err;
     scal[kHn] = hn;
     const bool breakdown = !(hn > 0.0) || !isfinite(hn);
@@ -411,7 +438,7 @@ __device__ __forceinline__ void givens_step(double* h, double* rot, int k, int i
 // b <= orth_tol^2 a (the new vector's component along the basis, |V^T w'| / |w'|, is already below the
 // tolerated loss of orthogonality) also takes mode 0. With a split target, q is also written as
 // the tcgen05 engine's TF32 operand, so the next operator application starts from it without a
-// split launch. In mode 0 the norm is known and block 0 takes the Givens step while the others write; in
+// split launch. In mode 0 the norm is known and an extra block takes the Givens step while the others write; in
 // modes 1 and 2 the last block takes it, after it has corrected the scale where the finished vector's
 // norm is not 1 to rounding. Once the flag is set, later iterations leave H, beta and the flag
 // alone, so iterations queued past the stopping point change nothing the solution uses.
@@ -427,8 +454,11 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
   __shared__ double dec[3];                 // mode, norm, 1 / norm
   __shared__ double fac;
   if (flag[kGmresState] != 0) return;   // queued past the stopping point: nothing changes
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  reduce_partials(part_in, gridDim.x, kv + 1, sums, sh);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, k = kv - 1;
+  const int G = (int)gridDim.x - 1;   // slices; the block after them takes the Givens step in mode 0
+  const bool extra = (int)blockIdx.x == G;
+  if (extra) givens_load(hcol, rot, h1, nullptr, k, cs, sn, tid, RT);
+  reduce_partials(part_in, G, kv + 1, sums, sh);
   if (warp == 0) {
     double b = 0.0;
     for (int j = lane; j < kv; j += 32) b = fma(sums[j], sums[j], b);
@@ -438,12 +468,12 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
       double mode, hp, inv;
       if (!(a < 0.5 * ww) || (a > 0.0 && b <= orth_tol2 * a)) {   // NaN: the Givens step reports it
         mode = 0.0;
-        hp = sqrt(a);
-        inv = (hp > 0.0) ? 1.0 / hp : 1.0;
+        inv = a > 0.0 ? rsqrt_full(a) : 1.0;
+        hp = a > 0.0 ? a * inv : sqrt(a);   // sqrt: 0 or NaN
       } else if (a > 0.0 && a - b >= 0.5 * a) {
         mode = 1.0;
-        hp = sqrt(a - b);
-        inv = 1.0 / hp;
+        inv = rsqrt_full(a - b);
+        hp = (a - b) * inv;
       } else {
         mode = 2.0;
         hp = 1.0;
@@ -455,7 +485,7 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
     }
   }
   __syncthreads();
-  const int mode = (int)dec[0], k = kv - 1;
+  const int mode = (int)dec[0];
   const double hp = dec[1], inv = dec[2];
   const int64_t beg = blockIdx.x * chunk, end = min(n, beg + chunk);
   if (mode == 0) {
@@ -464,12 +494,10 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
       w[i] = v;
       if (so.hi) put_split(so, i, v);
     }
-    if (blockIdx.x != 0 || warp != 0) return;
-    for (int i = lane; i <= k; i += 32) hcol[i] = h1[i];
-    __syncwarp();
-    // a block that starts after this has set the flag leaves its slice of q unscaled: the cycle has
-    // ended then, and its solution does not use q
-    givens_step(hcol, rot, k, iters, hp, H, cs, sn, beta, threshold, scal, flag, 0);
+    // a block that starts after the flag is set leaves its slice of q unscaled: the cycle has ended
+    // then, and its solution does not use q
+    if (extra && warp == 0)
+      givens_step(hcol, rot, k, iters, hp, H, cs, sn, beta, threshold, scal, flag, 0);
     return;
   }
   double ss = 0.0;
@@ -503,7 +531,7 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
   }
   __syncthreads();
   if (warp == 0) {
-    for (int i = lane; i <= k; i += 32) hcol[i] = h1[i] + sums[i];
+    givens_load(hcol, rot, h1, sums, k, cs, sn, lane, 32);
     __syncwarp();
     givens_step(hcol, rot, k, iters, dec[1], H, cs, sn, beta, threshold, scal, flag, kv);
   }
@@ -606,7 +634,7 @@ void launch_arnoldi(const ArnoldiStep& a, const ArnoldiGrid& g, cudaStream_t s) 
   arnoldi_reorth_kernel<E, VP><<<g.G, RT, 0, s>>>(a.Q, a.n, a.kv, a.w, a.n, g.chunk, a.part1, a.part2,
                                                   a.h1, a.scal, gate);
   TTGB_CHECK_LAUNCH();
-  arnoldi_finish_kernel<E, VP><<<g.G, RT, 0, s>>>(a.Q, a.n, a.kv, a.h1, a.part2, a.w, a.n, g.chunk,
+  arnoldi_finish_kernel<E, VP><<<g.G + 1, RT, 0, s>>>(a.Q, a.n, a.kv, a.h1, a.part2, a.w, a.n, g.chunk,
                                                   a.part1, a.counter, a.scal, a.iters, a.H, a.cs, a.sn,
                                                   a.beta, a.threshold, a.flag, a.so, a.orth_tol2);
   TTGB_CHECK_LAUNCH();
