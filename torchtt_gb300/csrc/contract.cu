@@ -9,6 +9,7 @@
 // tile autotuner's record for its shape class, or from an occupancy heuristic.
 #include <climits>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -18,10 +19,10 @@
 #include <type_traits>
 #include <unordered_map>
 
-#include <cuda_bf16.h>
-
 #include "contract.cuh"
 #include "df.cuh"
+#include "emu_digits.cuh"
+#include "oz_gemm.cuh"
 
 namespace ttgb {
 
@@ -350,7 +351,8 @@ thread_local int t_fp64_engine = kFp64Native;
 enum TileKind : int {
   kFma = 0,   // multiply-adds in the operand type
   kEmu = 1,   // FP64 from BF16 digits on the tensor cores (contract_emu.cuh)
-  kDf = 2     // double-float on the FP32 pipe
+  kDf = 2,    // double-float on the FP32 pipe
+  kOz = 3     // FP64 from digits made beforehand, on tcgen05 (oz_gemm.cu); allocates a workspace
 };
 struct TileCfg {
   int bm, bn, split;   // split: 0 no split-K, 1 split-K sized to fill the GPU
@@ -361,12 +363,14 @@ struct TileCfg {
 constexpr TileCfg kCandidates64[] = {
     {16, 16, 0}, {16, 32, 0}, {32, 16, 0}, {32, 32, 0}, {16, 16, 1}, {32, 32, 1},
     {64, 32, 0, kEmu}, {32, 64, 0, kEmu}, {64, 16, 0, kEmu}, {16, 64, 0, kEmu},
-    {64, 32, 1, kEmu}, {32, 64, 1, kEmu}, {64, 16, 1, kEmu}, {16, 64, 1, kEmu}};
+    {64, 32, 1, kEmu}, {32, 64, 1, kEmu}, {64, 16, 1, kEmu}, {16, 64, 1, kEmu},
+    {128, 32, 0, kOz}, {128, 32, 1, kOz}};
 // where the caller takes double-float accuracy
 constexpr TileCfg kCandidatesDf[] = {
     {16, 16, 0}, {16, 16, 1}, {32, 32, 0, kDf}, {64, 32, 0, kDf}, {32, 64, 0, kDf},
     {32, 32, 1, kDf}, {64, 32, 1, kDf}, {32, 64, 1, kDf},
-    {64, 32, 0, kEmu}, {32, 64, 0, kEmu}, {64, 32, 1, kEmu}, {32, 64, 1, kEmu}};
+    {64, 32, 0, kEmu}, {32, 64, 0, kEmu}, {64, 32, 1, kEmu}, {32, 64, 1, kEmu},
+    {128, 32, 0, kOz}, {128, 32, 1, kOz}};
 constexpr TileCfg kCandidates32[] = {{64, 64, 0}, {64, 32, 0}, {32, 64, 0}, {32, 32, 0},
                                      {64, 64, 1}, {64, 32, 1}, {32, 64, 1}, {32, 32, 1}};
 struct CandidateList {
@@ -472,6 +476,36 @@ bool componentwise(const ContractDescT<T>& d) {
   return (d.tri & kTriUpperB) != 0;
 }
 
+// Whether candidate t may run d: no digit products for componentwise(d), and no workspace for a caller
+// that must not allocate or whose stream is being captured.
+template <typename T>
+bool usable(const TileCfg& t, const ContractDescT<T>& d, cudaStream_t stream) {
+  if (t.kind == kEmu || t.kind == kOz) {
+    if (componentwise(d)) return false;
+  }
+  if constexpr (std::is_same<T, double>::value) {
+    if (t.kind == kOz) {
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+      return !t_no_tuning_runs && oz_takes(d) && cudaStreamIsCapturing(stream, &cap) == cudaSuccess &&
+             cap == cudaStreamCaptureStatusNone;
+    }
+  }
+  return true;
+}
+
+// split-K of candidate t
+template <typename T>
+int tile_split(const TileCfg& t, const ContractDescT<T>& d, int sms) {
+  if constexpr (std::is_same<T, double>::value) {
+    if (t.kind == kOz) {   // one tile per SM at most: a tile takes the SM's tensor memory
+      const int64_t tiles = oz_tiles(d);
+      const int s = (int)std::min<int64_t>(sms / std::max<int64_t>(1, tiles), d.K / kOzChunk);
+      return s < 1 ? 1 : s;
+    }
+  }
+  return heuristic_split(d, t.bm, t.bn, sms, true);
+}
+
 template <int BM, int BN>
 void launch_emu(const KParams<double>& p, dim3 grid, cudaStream_t stream) {
   using Tile = EmuTile<BM, BN>;
@@ -486,7 +520,7 @@ void launch_tiles(const ContractDescT<T>& d, KParams<T> p, const TileCfg& t, int
   const int bm = t.bm, bn = t.bn;
   int kchunk = d.K;
   if (splitk > 1) {
-    const int unit = t.kind == kEmu ? kEmuK : BK;
+    const int unit = t.kind == kOz ? kOzChunk : t.kind == kEmu ? kEmuK : BK;
     kchunk = (int)cdiv(cdiv(d.K, splitk), unit) * unit;
     splitk = (int)cdiv(d.K, kchunk);
   }
@@ -498,6 +532,12 @@ void launch_tiles(const ContractDescT<T>& d, KParams<T> p, const TileCfg& t, int
     if (g > 8192) g = 8192;
     scale_output_kernel<<<g, 256, 0, stream>>>(p.C, p.M, p.N, p.batch, p.cm, p.cn, p.c_bs, p.beta);
     TTGB_CHECK_LAUNCH();
+  }
+  if constexpr (std::is_same<T, double>::value) {
+    if (t.kind == kOz) {
+      oz_contract(d, splitk, kchunk, stream);
+      return;
+    }
   }
   dim3 grid(cdiv(d.N, bn), cdiv(d.M, bm), (unsigned)(d.batch * splitk));
   TTGB_REQUIRE(grid.y < 65536 && grid.z < 65536, "contraction grid too large");
@@ -587,8 +627,8 @@ int tuned_choice(const ContractDescT<T>& d, const KParams<T>& p, cudaStream_t st
   for (int rep = 0; rep < 2; ++rep) {
     for (int c = 0; c < cand.n; ++c) {
       const TileCfg& t = cand.t[c];
-      if (t.kind == kEmu && componentwise(d)) continue;
-      const int split = t.split ? heuristic_split(d, t.bm, t.bn, sms, true) : 1;
+      if (!usable(t, d, stream)) continue;
+      const int split = t.split ? tile_split(t, d, sms) : 1;
       if (t.split && split == 1) continue;   // the same launch as the unsplit candidate
       TTGB_CUDA(cudaEventRecord(ev[0], stream));
       launch_tiles(d, p, t, split, stream);
@@ -634,10 +674,10 @@ void launch_contract(const ContractDescT<T>& d, cudaStream_t stream, bool determ
     const int c = tuned_choice(dz, p, stream, tuned);
     // after tuning, C holds the last candidate's result: the chosen tile runs once more, so the
     // first launch of a class gives what every later launch of the class computes
-    if (c >= 0) {
+    if (c >= 0 && usable(candidates<T>().t[c], d, stream)) {
       const TileCfg& t = candidates<T>().t[c];
       launch_tiles(tuned ? dz : d, p, t,
-                   t.split ? heuristic_split(d, t.bm, t.bn, sms, true) : 1, stream);
+                   t.split ? tile_split(t, d, sms) : 1, stream);
       return;
     }
   }
@@ -651,6 +691,13 @@ void launch_contract(const ContractDescT<T>& d, cudaStream_t stream, bool determ
     if (componentwise(d) ? t_fp64_engine == kFp64DoubleFloat : work > 4e6)
       t.kind = componentwise(d) ? kDf : kEmu;
     t.bm = t.bn = 32;
+    // 200 x 300 x 100 (6 M): 22 us either way; 60 x 13440 x 60 (48 M): 40 us with digits made per tile, 29 us
+    // with digits made beforehand; 176 x 5632 x 88 (87 M): 60 and 31 us
+    const TileCfg oz{128, 32, 1, kOz};
+    if (t.kind == kEmu && work > 3e7 && usable(oz, d, stream)) {
+      launch_tiles(d, p, oz, deterministic ? 1 : tile_split(oz, d, sms), stream);
+      return;
+    }
     if (t.kind == kEmu) {
       if (d.N <= 16) { t.bm = 64; t.bn = 16; }
       else if (d.M <= 16) { t.bm = 16; t.bn = 64; }

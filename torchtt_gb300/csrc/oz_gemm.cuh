@@ -1,0 +1,23 @@
+// Large FP64 contractions on the tcgen05 tensor cores: the digit products of contract_emu.cuh with the
+// digits made once per operand element, in a launch of their own, and multiplied by tcgen05.mma from
+// shared memory that bulk copies fill (see oz_gemm.cu).
+#pragma once
+
+#include "contract.cuh"
+
+namespace ttgb {
+
+// Whether oz_contract takes the contraction.
+bool oz_takes(const ContractDesc& d);
+
+// K units of its split (a split's range is a multiple of this).
+constexpr int kOzChunk = 128;
+
+// Output tiles of a launch (for the split-K choice).
+int64_t oz_tiles(const ContractDesc& d);
+
+// C (+)= alpha A B as launch_tiles' other kernels: splitk ranges of kchunk are added atomically into C
+// (which already holds beta C), one range writes alpha A B + beta C.
+void oz_contract(const ContractDesc& d, int splitk, int kchunk, cudaStream_t s);
+
+}  // namespace ttgb
