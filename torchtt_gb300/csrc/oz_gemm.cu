@@ -25,8 +25,8 @@
 //
 // Measured (digits of Q, digits of P, product; against the kernel of contract_emu.cuh): M = 322, N = 5024, K = 161:
 // 8.7 + 8.0 + 31 us against 130; 176 x 5632 x 88: 7 + 6 + 17 against 60; 60 x 13440 x 60: 7 + 7 + 16 against
-// 40; 161 x 300 x 10000 in splits: 51 + 17 + 50 against 254. One tile per CTA with 64 columns and one set of accumulators took 46 us
-// for the first. What bounds the product is the tensor pipe (a stage 32 columns wide is 770 clocks of
+// 40; 161 x 300 x 10000 in splits: 51 + 18 + 55 against 254. One tile per CTA, 48 columns wide with one set
+// of accumulators, took 46 us for the first. What bounds the product is the tensor pipe (a stage 32 columns wide is 770 clocks of
 // MMAs) and what waits and commits add to it, some 250 clocks per stage; the digit kernels are latency.
 //
 // Every wait is bounded: a CTA whose wait gives up drains its copies and MMAs, frees its tensor memory
