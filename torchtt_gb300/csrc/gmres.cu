@@ -652,17 +652,14 @@ void launch_arnoldi(const ArnoldiStep& a, const ArnoldiGrid& g, cudaStream_t s) 
 
 }  // namespace
 
-// Iterations of a cycle before its first flag read: the convergence rate of the last converged
-// cycle, log(threshold) / iterations, predicts how many this threshold needs; the first read comes
-// one iteration before that, and later reads follow every iteration. A stop earlier than predicted
-// leaves the iterations queued after it, whose kernels read the flag and return at once; a later
-// stop costs one more read per extra iteration.
-static int first_read(const GmresWS& ws, double threshold, int iters) {
-  if (!(ws.log_rate < 0.0) || !(threshold > 0.0) || !(threshold < 1.0)) return 1;
+// Iterations that the convergence rate of the last converged cycle, log(threshold) / iterations, predicts
+// for this threshold; 0: unknown. The flag is read from one iteration before that on. A stop earlier
+// than predicted leaves the iterations queued after it, whose kernels read the flag and return at
+// once; a later stop costs one more read per extra iteration.
+static int predicted_iterations(const GmresWS& ws, double threshold, int iters) {
+  if (!(ws.log_rate < 0.0) || !(threshold > 0.0) || !(threshold < 1.0)) return 0;
   const double need = std::log(threshold) / ws.log_rate;
-  if (!(need < (double)iters)) return iters;
-  int p = (int)std::ceil(need) - 1;
-  return p < 1 ? 1 : p;
+  return need < (double)iters ? (int)std::ceil(need) : iters + 1;
 }
 
 GmresResult gmres(const LocalOperator& op, const double* rhs, double* sol, int iters,
@@ -673,6 +670,8 @@ GmresResult gmres(const LocalOperator& op, const double* rhs, double* sol, int i
   TTGB_REQUIRE(iters >= 1, "gmres: local_iterations must be >= 1");
   TTGB_REQUIRE(iters + 1 <= red.cap_vec && iters + 1 <= kMaxVec,
                "gmres: local_iterations exceeds the Krylov workspace (at most 126)");
+  for (cudaEvent_t& e : ws.read_done)
+    if (!e) TTGB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   ws.Q.ensure((size_t)(iters + 1) * n, s);
   Layout L(iters);
   ws.small.ensure((size_t)L.total, s);
@@ -715,9 +714,21 @@ GmresResult gmres(const LocalOperator& op, const double* rhs, double* sol, int i
     TTGB_CHECK_LAUNCH();
     scale_by_kernel<<<elem_grid(n), 256, 0, s>>>(r, Q, n, &scal[kResNorm], so);
     TTGB_CHECK_LAUNCH();
-    const int first = first_read(ws, threshold, iters);
+    const int predicted = predicted_iterations(ws, threshold, iters);
+    const int first = predicted > 1 ? predicted - 1 : 1;
     int k = 0;
     int state = 0;
+    // A read leaves the GPU without work until the host has seen the flag and launched again, some
+    // 10 us. So the host first launches the next iteration (its kernels return at once when the
+    // flag says stop), except where it expects the stop.
+    int pending = -1;            // iteration whose flag is on its way
+    const int* flag = ws.h_flag;
+    const auto read = [&](int it) {
+      TTGB_CUDA(cudaEventSynchronize(ws.read_done[it & 1]));
+      ++res.syncs;
+      flag = ws.h_flag + (it & 1) * kGmresFlagWords;
+      return flag[kGmresState];
+    };
     for (k = 0; k < iters; ++k) {
       const int kv = k + 1;
       double* qk = Q + (int64_t)k * n;
@@ -736,12 +747,20 @@ GmresResult gmres(const LocalOperator& op, const double* rhs, double* sol, int i
       if (op.prof_krylov)
         op.prof_krylov->end(8.0 * (double)n * (2 * k + 3), 3, 8.0 * (double)n * (2 * k + 7));
       if (k + 1 >= first || k == iters - 1) {
-        TTGB_CUDA(cudaMemcpyAsync(ws.h_flag, ws.d_flag, kGmresFlagWords * sizeof(int),
-                                  cudaMemcpyDeviceToHost, s));
-        TTGB_CUDA(cudaStreamSynchronize(s));
-        ++res.syncs;
-        state = ws.h_flag[kGmresState];
-        if (state != 0) break;
+        if (pending >= 0) {
+          state = read(pending);
+          pending = -1;
+          if (state != 0) break;
+        }
+        TTGB_CUDA(cudaMemcpyAsync(ws.h_flag + (k & 1) * kGmresFlagWords, ws.d_flag,
+                                  kGmresFlagWords * sizeof(int), cudaMemcpyDeviceToHost, s));
+        TTGB_CUDA(cudaEventRecord(ws.read_done[k & 1], s));
+        if (k + 1 == predicted || k == iters - 1) {
+          state = read(k);
+          if (state != 0) break;
+        } else {
+          pending = k;
+        }
       }
     }
     if (state == 2) {          // nothing to do in this cycle (gmres.h:56-65)
@@ -751,10 +770,10 @@ GmresResult gmres(const LocalOperator& op, const double* rhs, double* sol, int i
       break;
     }
     if (state == 3) throw Error(kNumericalError, "GMRES: non-finite residual");
-    const int kk = (state == 1) ? ws.h_flag[kGmresAtIter] : iters - 1;   // gmres.h:131
+    const int kk = (state == 1) ? flag[kGmresAtIter] : iters - 1;   // gmres.h:131
     res.overrun += (k < iters ? k : iters - 1) - kk;
-    res.reorth += ws.h_flag[kGmresReorth];
-    if (op.prof_krylov) op.prof_krylov->aux += 8.0 * (double)n * ws.h_flag[kGmresReorthVecs];
+    res.reorth += flag[kGmresReorth];
+    if (op.prof_krylov) op.prof_krylov->aux += 8.0 * (double)n * flag[kGmresReorthVecs];
     cycle_update_kernel<<<elem_grid(n), RT, 0, s>>>(kk, iters, H, beta, Q, n, sol, n,
                                                     cycle == 0 ? 1 : 0);
     TTGB_CHECK_LAUNCH();

@@ -96,9 +96,17 @@ enum GmresFlag : int {
 struct GmresWS {
   DBuf Q;        // (iters + 1) x n Krylov basis
   DBuf small;    // H, cs, sn, beta, h1, scalars
-  int* h_flag = nullptr;   // pinned, >= kGmresFlagWords ints
+  int* h_flag = nullptr;   // pinned, >= 2 kGmresFlagWords ints: the reads of two iterations in flight
   int* d_flag = nullptr;   // device, >= kGmresFlagWords ints
   double log_rate = 0.0;   // log(threshold) / iterations of the last converged cycle (0: unknown)
+  cudaEvent_t read_done[2] = {nullptr, nullptr};   // the copies into h_flag; made by the first gmres()
+  GmresWS() = default;
+  GmresWS(const GmresWS&) = delete;
+  GmresWS& operator=(const GmresWS&) = delete;
+  ~GmresWS() {
+    for (cudaEvent_t e : read_done)
+      if (e) cudaEventDestroy(e);
+  }
 };
 
 struct GmresResult {
@@ -117,7 +125,8 @@ struct GmresResult {
 // Gram-Schmidt with the DGKS reorthogonalisation criterion, as stable as the reference's modified
 // Gram-Schmidt), normalises, and runs the Givens rotations and the convergence test on the
 // device. The host reads the stop flag only from the iteration where the convergence rate of the
-// previous cycle predicts the stop; iterations queued past the stop leave the solution unchanged.
+// previous cycle predicts the stop, and waits for a flag behind the launches of the next iteration except
+// where the stop is expected; iterations queued past the stop leave the solution unchanged.
 // orth_tol > 0 also skips the second projection when the first leaves |V^T w'| <= orth_tol |w'|
 // (measured in the same pass), i.e. it keeps the basis orthogonal to orth_tol instead of to
 // rounding: for GMRES runs whose own tolerance is far above orth_tol.
