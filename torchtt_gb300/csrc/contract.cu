@@ -71,7 +71,10 @@ __global__ void __launch_bounds__(NT) contract_kernel(KParams<T> p) {
   const int kbeg = ks * p.kchunk;
   int kend = min(p.K, kbeg + p.kchunk);
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  if ((p.tri & kTriLowerC) && m0 + BM <= n0) return;   // tile strictly above the diagonal
+  if ((p.tri & kTriLowerC) && m0 + BM <= n0) {   // tile strictly above the diagonal
+    stream_wait();
+    return;
+  }
   if (p.tri & kTriUpperB) kend = min(kend, n0 + BN);   // B(k, n) = 0 for k > n
 
   const T* A = p.A + (int64_t)bidx * p.a_bs;
@@ -107,6 +110,7 @@ __global__ void __launch_bounds__(NT) contract_kernel(KParams<T> p) {
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = T(0);
 
+  stream_wait();
   // next K tile's operands in registers while the current one is multiplied (same sum order)
   T ra[BM / A_ROWS_PER_PASS], rb[BN / B_COLS_PER_PASS];
   auto load_tile = [&](int k0) {
@@ -116,10 +120,10 @@ __global__ void __launch_bounds__(NT) contract_kernel(KParams<T> p) {
     const int64_t b_koff = kok ? ax_off(p.bk, k) : 0;
 #pragma unroll
     for (int i = 0; i < BM / A_ROWS_PER_PASS; ++i)
-      ra[i] = (kok && a_mok[i]) ? __ldg(A + a_moff[i] + a_koff) : T(0);
+      ra[i] = (kok && a_mok[i]) ? A[a_moff[i] + a_koff] : T(0);
 #pragma unroll
     for (int i = 0; i < BN / B_COLS_PER_PASS; ++i)
-      rb[i] = (kok && b_nok[i]) ? __ldg(B + b_noff[i] + b_koff) : T(0);
+      rb[i] = (kok && b_nok[i]) ? B[b_noff[i] + b_koff] : T(0);
   };
   if (kbeg < kend) load_tile(kbeg);
   for (int k0 = kbeg; k0 < kend; k0 += BK) {
@@ -553,15 +557,15 @@ void launch_tiles(const ContractDescT<T>& d, KParams<T> p, const TileCfg& t, int
       if (bm == 64 && bn == 32) contract_df_kernel<64, 32><<<grid, NT, 0, stream>>>(p);
       else if (bm == 32 && bn == 64) contract_df_kernel<32, 64><<<grid, NT, 0, stream>>>(p);
       else contract_df_kernel<32, 32><<<grid, NT, 0, stream>>>(p);
-    } else if (bm == 16 && bn == 16) contract_kernel<T, 16, 16><<<grid, NT, 0, stream>>>(p);
-    else if (bm == 16 && bn == 32) contract_kernel<T, 16, 32><<<grid, NT, 0, stream>>>(p);
-    else if (bm == 32 && bn == 16) contract_kernel<T, 32, 16><<<grid, NT, 0, stream>>>(p);
-    else contract_kernel<T, 32, 32><<<grid, NT, 0, stream>>>(p);
+    } else if (bm == 16 && bn == 16) launch_early(contract_kernel<T, 16, 16>, grid, NT, 0, stream, p);
+    else if (bm == 16 && bn == 32) launch_early(contract_kernel<T, 16, 32>, grid, NT, 0, stream, p);
+    else if (bm == 32 && bn == 16) launch_early(contract_kernel<T, 32, 16>, grid, NT, 0, stream, p);
+    else launch_early(contract_kernel<T, 32, 32>, grid, NT, 0, stream, p);
   } else {
-    if (bm == 64 && bn == 64) contract_kernel<T, 64, 64><<<grid, NT, 0, stream>>>(p);
-    else if (bm == 64 && bn == 32) contract_kernel<T, 64, 32><<<grid, NT, 0, stream>>>(p);
-    else if (bm == 32 && bn == 64) contract_kernel<T, 32, 64><<<grid, NT, 0, stream>>>(p);
-    else contract_kernel<T, 32, 32><<<grid, NT, 0, stream>>>(p);
+    if (bm == 64 && bn == 64) launch_early(contract_kernel<T, 64, 64>, grid, NT, 0, stream, p);
+    else if (bm == 64 && bn == 32) launch_early(contract_kernel<T, 64, 32>, grid, NT, 0, stream, p);
+    else if (bm == 32 && bn == 64) launch_early(contract_kernel<T, 32, 64>, grid, NT, 0, stream, p);
+    else launch_early(contract_kernel<T, 32, 32>, grid, NT, 0, stream, p);
   }
   TTGB_CHECK_LAUNCH();
 }

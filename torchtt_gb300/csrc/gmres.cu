@@ -254,11 +254,12 @@ __device__ __forceinline__ void reduce_partials(const double* part, int G, int n
 
 // Pass 1: part[block] = partial sums of h1 = V^T w (kv values) and ||w||^2.
 template <int E, int VP>
-__global__ void __launch_bounds__(RT) arnoldi_project_kernel(const double* __restrict__ Q,
+__global__ void __launch_bounds__(RT) arnoldi_project_kernel(const double* Q,
                                                               int64_t ldq, int kv,
-                                                              const double* __restrict__ w,
+                                                              const double* w,
                                                               int64_t n, int64_t chunk, double* part,
                                                               const int* gate) {
+  stream_wait();
   if (*gate != 0) return;   // an iteration queued past the cycle's stopping point
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t beg = blockIdx.x * chunk, end = min(n, beg + chunk);
@@ -290,7 +291,7 @@ __global__ void __launch_bounds__(RT) arnoldi_project_kernel(const double* __res
 // t = the block's slice of V h (h in shared memory): the warps' shares through sh (8 x 32 E doubles);
 // element c of the slice is returned to thread c (0 past the slice).
 template <int E, int VP>
-__device__ __forceinline__ double slice_combination(const double* __restrict__ Q, int64_t ldq, int kv,
+__device__ __forceinline__ double slice_combination(const double* Q, int64_t ldq, int kv,
                                                     const double* h, int64_t c, int64_t end,
                                                     double* sh) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -323,7 +324,7 @@ __device__ __forceinline__ double slice_combination(const double* __restrict__ Q
 // Pass 2: w' = w - V h1, and the partial sums of h2 = V^T w' and ||w'||^2 (V's slice is read again from
 // the L1 cache). Block 0 keeps h1 and ||w||^2 for the finishing pass.
 template <int E, int VP>
-__global__ void __launch_bounds__(RT) arnoldi_reorth_kernel(const double* __restrict__ Q,
+__global__ void __launch_bounds__(RT) arnoldi_reorth_kernel(const double* Q,
                                                              int64_t ldq, int kv, double* w, int64_t n,
                                                              int64_t chunk, const double* part_in,
                                                              double* part_out, double* h1, double* scal,
@@ -331,6 +332,7 @@ __global__ void __launch_bounds__(RT) arnoldi_reorth_kernel(const double* __rest
   __shared__ double sums[kMaxVec];
   __shared__ double sh[kWarps * 32 * E];
   __shared__ double wn[32 * E];
+  stream_wait();
   if (*gate != 0) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   reduce_partials(part_in, gridDim.x, kv + 1, sums, sh);
@@ -444,7 +446,7 @@ __device__ __forceinline__ void givens_step(double* h, const double* rot, int k,
 // alone, so iterations queued past the stopping point change nothing the solution uses.
 template <int E, int VP>
 __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
-    const double* __restrict__ Q, int64_t ldq, int kv, const double* __restrict__ h1,
+    const double* Q, int64_t ldq, int kv, const double* h1,
     const double* part_in, double* w, int64_t n, int64_t chunk, double* part_out, unsigned* counter,
     double* scal, int iters, double* H, double* cs, double* sn, double* beta, double threshold,
     int* flag, SplitOut so, double orth_tol2) {
@@ -453,6 +455,7 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
   __shared__ double hcol[kMaxVec + 1], rot[2 * kMaxVec];
   __shared__ double dec[3];                 // mode, norm, 1 / norm
   __shared__ double fac;
+  stream_wait();
   if (flag[kGmresState] != 0) return;   // queued past the stopping point: nothing changes
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, k = kv - 1;
   const int G = (int)gridDim.x - 1;   // slices; the block after them takes the Givens step in mode 0
@@ -629,14 +632,14 @@ struct ArnoldiStep {
 template <int E, int VP>
 void launch_arnoldi(const ArnoldiStep& a, const ArnoldiGrid& g, cudaStream_t s) {
   int* gate = a.flag + kGmresState;
-  arnoldi_project_kernel<E, VP><<<g.G, RT, 0, s>>>(a.Q, a.n, a.kv, a.w, a.n, g.chunk, a.part1, gate);
+  launch_early(arnoldi_project_kernel<E, VP>, g.G, RT, 0, s, a.Q, a.n, a.kv, a.w, a.n, g.chunk, a.part1, gate);
   TTGB_CHECK_LAUNCH();
-  arnoldi_reorth_kernel<E, VP><<<g.G, RT, 0, s>>>(a.Q, a.n, a.kv, a.w, a.n, g.chunk, a.part1, a.part2,
-                                                  a.h1, a.scal, gate);
+  launch_early(arnoldi_reorth_kernel<E, VP>, g.G, RT, 0, s, a.Q, a.n, a.kv, a.w, a.n, g.chunk, a.part1,
+               a.part2, a.h1, a.scal, gate);
   TTGB_CHECK_LAUNCH();
-  arnoldi_finish_kernel<E, VP><<<g.G + 1, RT, 0, s>>>(a.Q, a.n, a.kv, a.h1, a.part2, a.w, a.n, g.chunk,
-                                                  a.part1, a.counter, a.scal, a.iters, a.H, a.cs, a.sn,
-                                                  a.beta, a.threshold, a.flag, a.so, a.orth_tol2);
+  launch_early(arnoldi_finish_kernel<E, VP>, g.G + 1, RT, 0, s, a.Q, a.n, a.kv, a.h1, a.part2, a.w, a.n,
+               g.chunk, a.part1, a.counter, a.scal, a.iters, a.H, a.cs, a.sn, a.beta, a.threshold, a.flag,
+               a.so, a.orth_tol2);
   TTGB_CHECK_LAUNCH();
 }
 

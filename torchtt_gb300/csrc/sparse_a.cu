@@ -13,11 +13,11 @@ constexpr int kThreads = 256;
 
 template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(kThreads)
-sparse_stage_kernel(const int* __restrict__ rp, const int* __restrict__ ja,
-                    const int* __restrict__ jb, const T* __restrict__ val,
-                    const T* __restrict__ in, T* out, float* out_lo, StageDims g) {
+sparse_stage_kernel(const int* rp, const int* ja, const int* jb, const T* val, const T* in, T* out,
+                    float* out_lo, StageDims g) {
   __shared__ T sv[SparseCore::kMaxRow];
   __shared__ int64_t soff[SparseCore::kMaxRow];
+  stream_wait();
   if (g.gate != nullptr && *g.gate != 0) return;
   const int key = blockIdx.x;
   const int beg = rp[key];
@@ -57,7 +57,7 @@ void launch_stage(const SparseCsr& c, const T* val, const T* in, T* out, float* 
   const int64_t want = std::max<int64_t>(1, (int64_t)8 * num_sms() / c.keys);
   gy = std::max<int64_t>(1, std::min<int64_t>({gy, want, 65535}));
   dim3 grid((unsigned)c.keys, (unsigned)gy);
-  sparse_stage_kernel<T, SPLIT><<<grid, kThreads, 0, s>>>(c.rp, c.a, c.b, val, in, out, lo, g);
+  launch_early(sparse_stage_kernel<T, SPLIT>, grid, kThreads, 0, s, c.rp, c.a, c.b, val, in, out, lo, g);
   TTGB_CHECK_LAUNCH();
 }
 

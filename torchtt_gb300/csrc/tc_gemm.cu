@@ -14,7 +14,7 @@
 //           32 (w % 4) .. +31, the rows its lanes own, and one half of the columns) and write the tile
 //           with arbitrary output strides as FP32, FP64 or a new TF32 split.
 // The local products' GEMMs have K chunks to the number of 2 to 10, so a launch is a chain of latencies: set-up, one
-// copy, the MMAs, the stores. Hence the stop flag and the tensor maps are fetched during the set-up, the
+// copy, the MMAs, the stores. Hence the set-up, tensor maps included, runs beside the kernel before, the
 // issuer asks for a stage before it issues the previous one, and the epilogue has eight warps that
 // walk their columns with one division and store whole rows where C's neighbours lie along N.
 // Averages over the mixed d = 4, n = 32 solve: 6.5 -> 5.75 us (BN = 32), 9.4 -> 6.8 (64), 13.1 -> 9.6 (128).
@@ -153,7 +153,6 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_tma_kernel(const __grid_c
   extern __shared__ uint8_t smraw[];
   // a gated launch (a GMRES iteration queued past its stopping point) leaves before any copy; the flag is
   // set by an earlier kernel on this stream, so every thread of every CTA reads the same value
-  const int gate = P.gate != nullptr ? *P.gate : 0;   // on its way during the set-up
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~uintptr_t(1023));
   constexpr int kABytes = kBM * 128;   // one 128-row operand tile of a chunk (hi or lo)
   constexpr int kBBytes = BN * 128;
@@ -188,6 +187,8 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_tma_kernel(const __grid_c
     const CUtensorMap* map = lane == 0 ? &P.a_hi : lane == 1 ? &P.a_lo : lane == 2 ? &P.b_hi : &P.b_lo;
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
   }
+  stream_wait();
+  const int gate = P.gate != nullptr ? *P.gate : 0;
   asm volatile("tcgen05.fence::before_thread_sync;");
   const int gated = __syncthreads_or(gate);
   asm volatile("tcgen05.fence::after_thread_sync;");
@@ -418,7 +419,7 @@ void launch(const TcGemm& g, int* err, cudaStream_t s) {
   dim3 grid(cdiv(g.N, BN), cdiv(g.M, kBM), (unsigned)g.batch);
   TTGB_REQUIRE(grid.y < 65536 && grid.z < 65536, "tc_gemm grid too large");
   smem_optin((const void*)tc_gemm_tma_kernel<BN>, (int)smem);
-  tc_gemm_tma_kernel<BN><<<grid, kThreads, smem, s>>>(P, err);
+  launch_early(tc_gemm_tma_kernel<BN>, grid, kThreads, smem, s, P, err);
   TTGB_CHECK_LAUNCH();
 }
 
