@@ -30,6 +30,7 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
 
 // Box-Muller on two 53-bit uniforms from a counter-based hash (splitmix64)
 __global__ void randn_kernel(double* out, int64_t n, uint64_t seed, uint64_t offset) {
+  stream_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const uint64_t h1 = splitmix64(seed ^ splitmix64(offset + (uint64_t)i));
@@ -41,9 +42,10 @@ __global__ void randn_kernel(double* out, int64_t n, uint64_t seed, uint64_t off
 }
 
 // B[(l,m,L),(r,n,R)] = sum_{s,S} Phi_l[l,s,r] A[s,m,n,S] Phi_r[L,S,R]  (amen_solve.h:322-324)
-__global__ void assemble_dense_kernel(const double* __restrict__ phil, const double* __restrict__ A,
-                                      const double* __restrict__ phir, int r, int s, int n, int S,
+__global__ void assemble_dense_kernel(const double* phil, const double* A,
+                                      const double* phir, int r, int s, int n, int S,
                                       int R, double* B) {
+  stream_wait();
   const int64_t nl = (int64_t)r * n * R;
   const int64_t total = nl * nl;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
@@ -535,7 +537,7 @@ void AmenRun::forward_step(int k, int swp, bool last, double& max_res) {
   if (use_full) {   // amen_solve.h:319-330
     st_.direct_solves++;
     Bmat.reset((size_t)(nl * nl), s_);
-    assemble_dense_kernel<<<grid_of(nl * nl), 256, 0, s_>>>(
+    launch_early(assemble_dense_kernel, grid_of(nl * nl), 256, 0, s_, 
         Phis_[k].data(), Acore(k), Phis_[k + 1].data(), (int)rk, (int)rA_[k], (int)n,
         (int)rA_[k + 1], (int)rk1, Bmat.p);
     TTGB_CHECK_LAUNCH();
@@ -1035,7 +1037,7 @@ size_t footprint_bound(const TTView& A, const TTView& b, const TTView& x0, const
 
 void randn(double* out, int64_t n, uint64_t seed, uint64_t offset, cudaStream_t s) {
   if (n <= 0) return;
-  randn_kernel<<<grid_of(n), 256, 0, s>>>(out, n, seed, offset);
+  launch_early(randn_kernel, grid_of(n), 256, 0, s, out, n, seed, offset);
   TTGB_CHECK_LAUNCH();
 }
 

@@ -278,7 +278,7 @@ std::vector<DTensor> AmenMv::run(const TTView& x0, std::vector<int64_t>& ranks, 
         transpose(Vh.p, kf, u.p, p, r, p, s_);          // left singular vectors
         v.reset((size_t)(q * r), s_);
         copy(U.p, v.p, q * r, s_);                      // right singular vectors, scaled by S
-        scale_cols_kernel<<<cdiv(q * r, 256), 256, 0, s_>>>(v.p, q, q, r, S.p);
+        launch_early(scale_cols_kernel, cdiv(q * r, 256), 256, 0, s_, v.p, q, q, r, S.p);
         TTGB_CHECK_LAUNCH();
       } else {
         // last core (q = 1): the projection itself

@@ -40,9 +40,10 @@ __device__ void last_block_reduce(double* partial, unsigned* counter, int G, int
   red::reset_ticket(counter);
 }
 
-__global__ void __launch_bounds__(RT) nrm2_kernel(const double* __restrict__ x, int64_t n,
+__global__ void __launch_bounds__(RT) nrm2_kernel(const double* x, int64_t n,
                                                    int64_t chunk, double* partial, unsigned* counter,
                                                    double* out, int post) {
+  stream_wait();
   __shared__ double sh[32];
   const int64_t beg = blockIdx.x * chunk, end = min(n, beg + chunk);
   double s = 0.0;
@@ -68,6 +69,7 @@ struct SegParams {
 
 __global__ void __launch_bounds__(RT) nrm2_multi_kernel(SegParams p, double* partial,
                                                          unsigned* counter) {
+  stream_wait();
   __shared__ double sh[32];
   int seg = 0;
   while (seg + 1 < p.count && (int)blockIdx.x >= p.first_block[seg + 1]) ++seg;
@@ -96,6 +98,7 @@ __global__ void __launch_bounds__(RT) nrm2_multi_kernel(SegParams p, double* par
 }
 
 __global__ void scale_multi_kernel(SegParams p, int64_t total) {
+  stream_wait();
   __shared__ double f[VecSegs::kMax];
   if ((int)threadIdx.x < p.count) {
     const double d = *p.den[threadIdx.x];
@@ -111,14 +114,16 @@ __global__ void scale_multi_kernel(SegParams p, int64_t total) {
   }
 }
 
-__global__ void axpby_kernel(double a, const double* __restrict__ x, double b, double* y, int64_t n) {
+__global__ void axpby_kernel(double a, const double* x, double b, double* y, int64_t n) {
+  stream_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     y[i] = (b == 0.0) ? a * x[i] : fma(a, x[i], b * y[i]);
 }
 
-__global__ void sub_kernel(const double* __restrict__ x, const double* __restrict__ y, double* z,
+__global__ void sub_kernel(const double* x, const double* y, double* z,
                            int64_t n) {
+  stream_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     z[i] = x[i] - y[i];
@@ -127,6 +132,7 @@ __global__ void sub_kernel(const double* __restrict__ x, const double* __restric
 __global__ void __launch_bounds__(RT) sub_nrm2_kernel(const double* x, const double* y, double* z,
                                                        int64_t n, int64_t chunk, double* partial,
                                                        unsigned* counter, double* out) {
+  stream_wait();
   __shared__ double sh[32];
   const int64_t beg = blockIdx.x * chunk, end = min(n, beg + chunk);
   double s = 0.0;
@@ -141,6 +147,7 @@ __global__ void __launch_bounds__(RT) sub_nrm2_kernel(const double* x, const dou
 }
 
 __global__ void scale_dev_kernel(double* x, int64_t n, const double* num, const double* den) {
+  stream_wait();
   const double d = *den;
   if (!(d > 0.0)) return;
   const double f = (num ? *num : 1.0) / d;
@@ -149,27 +156,31 @@ __global__ void scale_dev_kernel(double* x, int64_t n, const double* num, const 
     x[i] *= f;
 }
 
-__global__ void scale_copy_kernel(const double* __restrict__ x, double a, double* y, int64_t n) {
+__global__ void scale_copy_kernel(const double* x, double a, double* y, int64_t n) {
+  stream_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     y[i] = a * x[i];
 }
 
 __global__ void fill_kernel(double* x, double v, int64_t n) {
+  stream_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     x[i] = v;
 }
 
 template <typename S, typename D>
-__global__ void cast_kernel(const S* __restrict__ x, D* y, int64_t n) {
+__global__ void cast_kernel(const S* x, D* y, int64_t n) {
+  stream_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     y[i] = (D)x[i];
 }
 
-__global__ void copy2d_kernel(const double* __restrict__ src, int64_t sld, double* dst, int64_t dld,
+__global__ void copy2d_kernel(const double* src, int64_t sld, double* dst, int64_t dld,
                               int64_t rows, int64_t cols) {
+  stream_wait();
   const int64_t total = rows * cols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -178,8 +189,9 @@ __global__ void copy2d_kernel(const double* __restrict__ src, int64_t sld, doubl
   }
 }
 
-__global__ void transpose_kernel(const double* __restrict__ src, int64_t sld, double* dst,
+__global__ void transpose_kernel(const double* src, int64_t sld, double* dst,
                                  int64_t dld, int64_t rows, int64_t cols) {
+  stream_wait();
   __shared__ double tile[32][33];
   const int64_t r0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32;
   // src is cols x rows: src[c * sld + r]
@@ -226,7 +238,7 @@ void red_launch_dims(const RedWS& ws, int64_t n, int nvec, int& G, int64_t& chun
 void nrm2(const RedWS& ws, const double* x, int64_t n, double* out, cudaStream_t s) {
   int G; int64_t chunk;
   red_launch_dims(ws, n, 1, G, chunk);
-  nrm2_kernel<<<G, RT, 0, s>>>(x, n, chunk, ws.partial, ws.counter, out, 1);
+  launch_early(nrm2_kernel, G, RT, 0, s, x, n, chunk, ws.partial, ws.counter, out, 1);
   TTGB_CHECK_LAUNCH();
 }
 
@@ -251,7 +263,7 @@ void nrm2_multi(const RedWS& ws, const VecSegs& v, cudaStream_t s) {
     G += g;
   }
   p.first_block[v.count] = G;
-  nrm2_multi_kernel<<<G, RT, 0, s>>>(p, ws.partial, ws.counter);
+  launch_early(nrm2_multi_kernel, G, RT, 0, s, p, ws.partial, ws.counter);
   TTGB_CHECK_LAUNCH();
 }
 
@@ -267,19 +279,19 @@ void scale_multi(const VecSegs& v, cudaStream_t s) {
     total += v.n[i];
   }
   if (total <= 0) return;
-  scale_multi_kernel<<<ew_grid(total), 256, 0, s>>>(p, total);
+  launch_early(scale_multi_kernel, ew_grid(total), 256, 0, s, p, total);
   TTGB_CHECK_LAUNCH();
 }
 
 void axpby(double a, const double* x, double b, double* y, int64_t n, cudaStream_t s) {
   if (n <= 0) return;
-  axpby_kernel<<<ew_grid(n), 256, 0, s>>>(a, x, b, y, n);
+  launch_early(axpby_kernel, ew_grid(n), 256, 0, s, a, x, b, y, n);
   TTGB_CHECK_LAUNCH();
 }
 
 void sub(const double* x, const double* y, double* z, int64_t n, cudaStream_t s) {
   if (n <= 0) return;
-  sub_kernel<<<ew_grid(n), 256, 0, s>>>(x, y, z, n);
+  launch_early(sub_kernel, ew_grid(n), 256, 0, s, x, y, z, n);
   TTGB_CHECK_LAUNCH();
 }
 
@@ -287,25 +299,25 @@ void sub_nrm2(const RedWS& ws, const double* x, const double* y, double* z, int6
               cudaStream_t s) {
   int G; int64_t chunk;
   red_launch_dims(ws, n, 1, G, chunk);
-  sub_nrm2_kernel<<<G, RT, 0, s>>>(x, y, z, n, chunk, ws.partial, ws.counter, out);
+  launch_early(sub_nrm2_kernel, G, RT, 0, s, x, y, z, n, chunk, ws.partial, ws.counter, out);
   TTGB_CHECK_LAUNCH();
 }
 
 void scale_dev(double* x, int64_t n, const double* num, const double* den, cudaStream_t s) {
   if (n <= 0) return;
-  scale_dev_kernel<<<ew_grid(n), 256, 0, s>>>(x, n, num, den);
+  launch_early(scale_dev_kernel, ew_grid(n), 256, 0, s, x, n, num, den);
   TTGB_CHECK_LAUNCH();
 }
 
 void scale_copy(const double* x, double a, double* y, int64_t n, cudaStream_t s) {
   if (n <= 0) return;
-  scale_copy_kernel<<<ew_grid(n), 256, 0, s>>>(x, a, y, n);
+  launch_early(scale_copy_kernel, ew_grid(n), 256, 0, s, x, a, y, n);
   TTGB_CHECK_LAUNCH();
 }
 
 void fill(double* x, double v, int64_t n, cudaStream_t s) {
   if (n <= 0) return;
-  fill_kernel<<<ew_grid(n), 256, 0, s>>>(x, v, n);
+  launch_early(fill_kernel, ew_grid(n), 256, 0, s, x, v, n);
   TTGB_CHECK_LAUNCH();
 }
 
@@ -316,20 +328,20 @@ void copy(const double* x, double* y, int64_t n, cudaStream_t s) {
 
 void cast(const double* x, float* y, int64_t n, cudaStream_t s) {
   if (n <= 0) return;
-  cast_kernel<double, float><<<ew_grid(n), 256, 0, s>>>(x, y, n);
+  launch_early(cast_kernel<double, float>, ew_grid(n), 256, 0, s, x, y, n);
   TTGB_CHECK_LAUNCH();
 }
 
 void cast(const float* x, double* y, int64_t n, cudaStream_t s) {
   if (n <= 0) return;
-  cast_kernel<float, double><<<ew_grid(n), 256, 0, s>>>(x, y, n);
+  launch_early(cast_kernel<float, double>, ew_grid(n), 256, 0, s, x, y, n);
   TTGB_CHECK_LAUNCH();
 }
 
 void copy2d(const double* src, int64_t sld, double* dst, int64_t dld, int64_t rows, int64_t cols,
             cudaStream_t s) {
   if (rows <= 0 || cols <= 0) return;
-  copy2d_kernel<<<ew_grid(rows * cols), 256, 0, s>>>(src, sld, dst, dld, rows, cols);
+  launch_early(copy2d_kernel, ew_grid(rows * cols), 256, 0, s, src, sld, dst, dld, rows, cols);
   TTGB_CHECK_LAUNCH();
 }
 
@@ -338,13 +350,14 @@ void transpose(const double* src, int64_t sld, double* dst, int64_t dld, int64_t
   if (rows <= 0 || cols <= 0) return;
   dim3 grid(cdiv(cols, 32), cdiv(rows, 32));
   TTGB_REQUIRE(grid.y < 65536, "transpose too tall");
-  transpose_kernel<<<grid, dim3(32, 8), 0, s>>>(src, sld, dst, dld, rows, cols);
+  launch_early(transpose_kernel, grid, dim3(32, 8), 0, s, src, sld, dst, dld, rows, cols);
   TTGB_CHECK_LAUNCH();
 }
 
 namespace {
 __global__ void scale_rows_cm_kernel(double* X, int64_t ld, int64_t rows, int64_t cols,
                                      const double* S) {
+  stream_wait();
   const int64_t total = rows * cols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -357,7 +370,7 @@ __global__ void scale_rows_cm_kernel(double* X, int64_t ld, int64_t rows, int64_
 void scale_rows_cm(double* X, int64_t ld, int64_t rows, int64_t cols, const double* S,
                    cudaStream_t s) {
   if (rows <= 0 || cols <= 0) return;
-  scale_rows_cm_kernel<<<ew_grid(rows * cols), 256, 0, s>>>(X, ld, rows, cols, S);
+  launch_early(scale_rows_cm_kernel, ew_grid(rows * cols), 256, 0, s, X, ld, rows, cols, S);
   TTGB_CHECK_LAUNCH();
 }
 

@@ -99,10 +99,16 @@ inline void launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
 }
 
 #ifdef __CUDACC__
-// Waits for the kernel before this one, then lets the next one start its blocks.
+// Lets the next kernel of the stream start its blocks, once every block has called it or has ended.
+__device__ __forceinline__ void stream_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Without the release, for kernels of one block that run for long: waiting blocks would keep their place on
+// the other SMs from kernels of other streams.
+__device__ __forceinline__ void stream_wait_only() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void stream_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  stream_wait_only();
+  stream_release();
 }
 #endif
 

@@ -179,6 +179,7 @@ __global__ void __launch_bounds__(NT) contract_kernel(KParams<T> p) {
 // The FP64 -> (hi, lo) split is df_split (df.cuh).
 template <int BM, int BN>
 __global__ void __launch_bounds__(NT) contract_df_kernel(KParams<double> p) {
+  stream_wait();
   constexpr int TM = BM / 16, TN = BN / 16;
   __shared__ float Ah[BK][BM + 1], Al[BK][BM + 1];
   __shared__ float Bh[BK][BN + 1], Bl[BK][BN + 1];
@@ -232,10 +233,10 @@ __global__ void __launch_bounds__(NT) contract_df_kernel(KParams<double> p) {
     const int64_t b_koff = kok ? ax_off(p.bk, k) : 0;
 #pragma unroll
     for (int i = 0; i < BM / ROWS_PER_PASS; ++i)
-      ra[i] = (kok && a_mok[i]) ? __ldg(A + a_moff[i] + a_koff) : 0.0;
+      ra[i] = (kok && a_mok[i]) ? A[a_moff[i] + a_koff] : 0.0;
 #pragma unroll
     for (int i = 0; i < BN / ROWS_PER_PASS; ++i)
-      rb[i] = (kok && b_nok[i]) ? __ldg(B + b_noff[i] + b_koff) : 0.0;
+      rb[i] = (kok && b_nok[i]) ? B[b_noff[i] + b_koff] : 0.0;
   };
   if (kbeg < kend) load_tile(kbeg);
   for (int k0 = kbeg; k0 < kend; k0 += BK) {
@@ -316,6 +317,7 @@ __global__ void __launch_bounds__(NT) contract_df_kernel(KParams<double> p) {
 template <typename T>
 __global__ void scale_output_kernel(T* C, int M, int N, int batch, AxD cm, AxD cn, int64_t c_bs,
                                     T beta) {
+  stream_wait();
   const int64_t total = (int64_t)M * N * batch;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -514,7 +516,7 @@ template <int BM, int BN>
 void launch_emu(const KParams<double>& p, dim3 grid, cudaStream_t stream) {
   using Tile = EmuTile<BM, BN>;
   smem_optin((const void*)contract_emu_kernel<BM, BN>, (int)Tile::kSmem);
-  contract_emu_kernel<BM, BN><<<grid, Tile::kThreads, Tile::kSmem, stream>>>(p);
+  launch_early(contract_emu_kernel<BM, BN>, grid, Tile::kThreads, Tile::kSmem, stream, p);
   TTGB_CHECK_LAUNCH();
 }
 
@@ -534,7 +536,7 @@ void launch_tiles(const ContractDescT<T>& d, KParams<T> p, const TileCfg& t, int
     int64_t total = (int64_t)d.M * d.N * d.batch;
     unsigned g = cdiv(total, 256);
     if (g > 8192) g = 8192;
-    scale_output_kernel<<<g, 256, 0, stream>>>(p.C, p.M, p.N, p.batch, p.cm, p.cn, p.c_bs, p.beta);
+    launch_early(scale_output_kernel<T>, g, 256, 0, stream, p.C, p.M, p.N, p.batch, p.cm, p.cn, p.c_bs, p.beta);
     TTGB_CHECK_LAUNCH();
   }
   if constexpr (std::is_same<T, double>::value) {
@@ -554,9 +556,9 @@ void launch_tiles(const ContractDescT<T>& d, KParams<T> p, const TileCfg& t, int
       return;
     }
     if (t.kind == kDf) {
-      if (bm == 64 && bn == 32) contract_df_kernel<64, 32><<<grid, NT, 0, stream>>>(p);
-      else if (bm == 32 && bn == 64) contract_df_kernel<32, 64><<<grid, NT, 0, stream>>>(p);
-      else contract_df_kernel<32, 32><<<grid, NT, 0, stream>>>(p);
+      if (bm == 64 && bn == 32) launch_early(contract_df_kernel<64, 32>, grid, NT, 0, stream, p);
+      else if (bm == 32 && bn == 64) launch_early(contract_df_kernel<32, 64>, grid, NT, 0, stream, p);
+      else launch_early(contract_df_kernel<32, 32>, grid, NT, 0, stream, p);
     } else if (bm == 16 && bn == 16) launch_early(contract_kernel<T, 16, 16>, grid, NT, 0, stream, p);
     else if (bm == 16 && bn == 32) launch_early(contract_kernel<T, 16, 32>, grid, NT, 0, stream, p);
     else if (bm == 32 && bn == 16) launch_early(contract_kernel<T, 32, 16>, grid, NT, 0, stream, p);
@@ -668,7 +670,7 @@ void launch_contract(const ContractDescT<T>& d, cudaStream_t stream, bool determ
   p.alpha = d.alpha; p.beta = d.beta;
   p.tri = d.tri;
   if (d.K <= 0) {  // empty sum: C = beta * C
-    scale_output_kernel<<<cdiv((int64_t)d.M * d.N * d.batch, 256) > 4096 ? 4096 : cdiv((int64_t)d.M * d.N * d.batch, 256), 256, 0, stream>>>(
+    launch_early(scale_output_kernel<T>, std::min(cdiv((int64_t)d.M * d.N * d.batch, 256), 4096u), 256, 0, stream,
         p.C, p.M, p.N, p.batch, p.cm, p.cn, p.c_bs, p.beta);
     TTGB_CHECK_LAUNCH();
     return;

@@ -95,11 +95,11 @@ struct EmuLoader {
           const double* p = base + off + (int64_t)(k0 + kk) * ak.s0;
 #pragma unroll
           for (int i = 0; i < 4; ++i)
-            if (kk + i < len) v[q][i] = __ldg(p + i * ak.s0);
+            if (kk + i < len) v[q][i] = p[i * ak.s0];
         } else {
 #pragma unroll
           for (int i = 0; i < 4; ++i)
-            if (kk + i < len) v[q][i] = __ldg(base + off + ax_off(ak, k0 + kk + i));
+            if (kk + i < len) v[q][i] = base[off + ax_off(ak, k0 + kk + i)];
         }
       }
 #pragma unroll
@@ -122,6 +122,7 @@ struct EmuTile {
 template <int BM, int BN>
 __global__ void __launch_bounds__(EmuTile<BM, BN>::kThreads, EmuTile<BM, BN>::kMinBlocks)
     contract_emu_kernel(KParams<double> p) {
+  stream_wait();
   using Tile = EmuTile<BM, BN>;
   constexpr int NTH = Tile::kThreads;
   extern __shared__ __align__(16) unsigned char emu_sm[];

@@ -314,10 +314,11 @@ __global__ void __cluster_dims__(kGjCtas, 1, 1) __launch_bounds__(kGjMaxN, 1)
 // LU with partial pivoting on an n x n row-major copy of B, solving for one right-hand side, in one
 // block. Does nothing when *gate is 0 (gate may be null).
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024) lu_solve_kernel(const double* __restrict__ B,
-                                                        const double* __restrict__ b, double* LU,
+__global__ void __launch_bounds__(1024) lu_solve_kernel(const double* B,
+                                                        const double* b, double* LU,
                                                         double* x, int n, int* status,
                                                         const int* gate) {
+  stream_wait_only();
   __shared__ double shv[32];
   __shared__ double piv_inv;
   __shared__ int shi[32];
@@ -410,7 +411,7 @@ void lu_solve(const double* B, int64_t n, const double* rhs, double* x, LinalgWS
     TTGB_CHECK_LAUNCH();
     gate = ws.status + 1;
   }
-  lu_solve_kernel<<<1, 1024, 0, s>>>(B, rhs, ws.e.p + gj, x, (int)n, ws.status, gate);
+  launch_early(lu_solve_kernel, 1, 1024, 0, s, B, rhs, ws.e.p + gj, x, (int)n, ws.status, gate);
   TTGB_CHECK_LAUNCH();
 }
 

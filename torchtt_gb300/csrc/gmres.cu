@@ -92,12 +92,13 @@ struct Layout {   // GmresWS::small
 
 // ||x|| of the cycle's start vector (also ||rhs|| in the first cycle, where r = rhs) and the
 // cycle's start state: H, the rotations and beta cleared, beta[0] = ||r||, the flag words reset.
-__global__ void __launch_bounds__(RT) cycle_start_kernel(const double* __restrict__ x, int64_t n,
+__global__ void __launch_bounds__(RT) cycle_start_kernel(const double* x, int64_t n,
                                                           int64_t chunk, double* partial,
                                                           unsigned* counter, double* scal,
                                                           int first, int iters, double* H,
                                                           double* cs, double* sn, double* beta,
                                                           int* flag) {
+  stream_wait();
   __shared__ double sh[32];
   const int64_t beg = blockIdx.x * chunk, end = min(n, beg + chunk);
   double s = 0.0;
@@ -146,6 +147,7 @@ __device__ __forceinline__ void put_split(const SplitOut& o, int64_t i, double v
 // y = x / den (den device, y = x when den <= 0); y may alias x
 __global__ void scale_by_kernel(const double* x, double* y, int64_t n, const double* den,
                                 SplitOut so) {
+  stream_wait();
   const double d = *den;
   const double f = (d > 0.0) ? 1.0 / d : 1.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
@@ -556,9 +558,10 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
 // per step, the launch took 28-43 us; now 10-13).
 __global__ void __launch_bounds__(RT) cycle_update_kernel(int kk, int iters, const double* H,
                                                            const double* beta,
-                                                           const double* __restrict__ Q,
+                                                           const double* Q,
                                                            int64_t ldq, double* sol, int64_t n,
                                                            int first) {
+  stream_wait();
   __shared__ double ys[kMaxVec];
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
@@ -712,10 +715,10 @@ GmresResult gmres(const LocalOperator& op, const double* rhs, double* sol, int i
       sub(rhs, Q, Q, n, s);
       r = Q;
     }
-    cycle_start_kernel<<<G1, RT, 0, s>>>(r, n, ch1, red.partial, red.counter, scal, cycle == 0 ? 1 : 0,
+    launch_early(cycle_start_kernel, G1, RT, 0, s, r, n, ch1, red.partial, red.counter, scal, cycle == 0 ? 1 : 0,
                                          iters, H, cs, sn, beta, ws.d_flag);
     TTGB_CHECK_LAUNCH();
-    scale_by_kernel<<<elem_grid(n), 256, 0, s>>>(r, Q, n, &scal[kResNorm], so);
+    launch_early(scale_by_kernel, elem_grid(n), 256, 0, s, r, Q, n, &scal[kResNorm], so);
     TTGB_CHECK_LAUNCH();
     const int predicted = predicted_iterations(ws, threshold, iters);
     const int first = predicted > 1 ? predicted - 1 : 1;
@@ -777,7 +780,7 @@ GmresResult gmres(const LocalOperator& op, const double* rhs, double* sol, int i
     res.overrun += (k < iters ? k : iters - 1) - kk;
     res.reorth += flag[kGmresReorth];
     if (op.prof_krylov) op.prof_krylov->aux += 8.0 * (double)n * flag[kGmresReorthVecs];
-    cycle_update_kernel<<<elem_grid(n), RT, 0, s>>>(kk, iters, H, beta, Q, n, sol, n,
+    launch_early(cycle_update_kernel, elem_grid(n), RT, 0, s, kk, iters, H, beta, Q, n, sol, n,
                                                     cycle == 0 ? 1 : 0);
     TTGB_CHECK_LAUNCH();
     res.nit += kk + 1;

@@ -62,6 +62,7 @@ __device__ double block_max_d(double v, double* sh) {
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(512) chol_kernel(double* G, int n, int64_t shift_rows,
                                                    int check_identity, int* status) {
+  stream_wait_only();
   __shared__ double sh[32];
   __shared__ int bad;
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -281,9 +282,10 @@ __device__ void chol_panels(double* A, int n, double floor_d, CholShared& ch) {
       }
 }
 
-__global__ void __launch_bounds__(512) chol_inv_smem_kernel(double* __restrict__ Gin, int n,
+__global__ void __launch_bounds__(512) chol_inv_smem_kernel(double* Gin, int n,
                                                             int64_t shift_rows, int pass, double* Rout,
                                                             double* Riout, int* status, int* done) {
+  stream_wait_only();
   extern __shared__ double A[];
   const int ld = n + 1;
   __shared__ CholShared ch;
@@ -352,7 +354,8 @@ __global__ void __launch_bounds__(512) chol_inv_smem_kernel(double* __restrict__
 }
 
 // Ri = R^{-1} for the upper-triangular row-major R (one thread per column of Ri).
-__global__ void trinv_kernel(const double* __restrict__ R, double* Ri, int n) {
+__global__ void trinv_kernel(const double* R, double* Ri, int n) {
+  stream_wait();
   for (int j = threadIdx.x + blockIdx.x * blockDim.x; j < n; j += blockDim.x * gridDim.x) {
     for (int i = n - 1; i >= 0; --i) {
       double v = (i == j) ? 1.0 : 0.0;
@@ -442,6 +445,7 @@ __device__ __forceinline__ void householder_body(double* W, int m, int n, double
 
 __global__ void __launch_bounds__(512) householder_kernel(double* W, int m, int n, double* Q,
                                                           double* R, double* tau) {
+  stream_wait_only();
   householder_body(W, m, n, Q, R, tau);
 }
 
@@ -450,9 +454,10 @@ __global__ void __launch_bounds__(512) householder_kernel(double* W, int m, int 
 // L2 round trip, which is what bounds the small QRs of the enrichment blocks (m <= 1024, n <= 16).
 constexpr int kHouseholderSmemBytes = 200 * 1024;
 
-__global__ void __launch_bounds__(512, 1) householder_smem_kernel(const double* __restrict__ A,
+__global__ void __launch_bounds__(512, 1) householder_smem_kernel(const double* A,
                                                                int64_t lda, int m, int n,
                                                                double* Qout, double* R) {
+  stream_wait_only();
   extern __shared__ double hs[];
   const int k = min(m, n);
   double* W = hs;
@@ -479,8 +484,9 @@ __global__ void __launch_bounds__(512, 1) householder_smem_kernel(const double* 
 // ---------------------------------------------------------------------------------------------
 constexpr int kCholQrSmallN = 32;
 
-__global__ void __launch_bounds__(512, 1) cholqr_small_kernel(const double* __restrict__ A, int64_t lda,
+__global__ void __launch_bounds__(512, 1) cholqr_small_kernel(const double* A, int64_t lda,
                                                               int m, int n, double* Qout, double* Rout) {
+  stream_wait_only();
   extern __shared__ double hs[];
   const int ldq = m | 1;   // odd pitch of the columns
   double* X = hs;                            // m x n, this pass's input
@@ -825,8 +831,9 @@ __device__ __forceinline__ void jacobi_scale(unsigned top, double& down, double&
 }
 
 // W = R^T scaled by jacobi_scale, *up the factor back. One block.
-__global__ void __launch_bounds__(1024) scaled_transpose_kernel(const double* __restrict__ R, int n, double* W,
+__global__ void __launch_bounds__(1024) scaled_transpose_kernel(const double* R, int n, double* W,
                                                                 double* up) {
+  stream_wait_only();
   __shared__ unsigned top;
   if (threadIdx.x == 0) top = 0u;
   __syncthreads();
@@ -853,8 +860,9 @@ __global__ void __launch_bounds__(1024) scaled_transpose_kernel(const double* __
 // ---------------------------------------------------------------------------------------------
 constexpr int kJacobiWarpMaxN = 16;
 
-__global__ void __launch_bounds__(32) jacobi_warp_kernel(const double* __restrict__ R, int n, double* Un,
+__global__ void __launch_bounds__(32) jacobi_warp_kernel(const double* R, int n, double* Un,
                                                          double* S, double* Vs, int* status) {
+  stream_wait_only();
   constexpr int N = kJacobiWarpMaxN, ld = N + 1;
   __shared__ double W[N * ld], V[N * ld], nrm[N];
   const int lane = threadIdx.x, gid = lane / 4, gl = lane % 4;
@@ -1080,9 +1088,10 @@ constexpr int kJacobiF32MaxN = 224;
 __host__ __device__ constexpr int jacobi_f32_pitch(int epl) { return (8 * epl + 23) / 32 * 32 + 8; }
 
 template <int EPL>
-__global__ void __launch_bounds__(32 * EPL) jacobi_f32_kernel(const double* __restrict__ R, int n, double* X,
+__global__ void __launch_bounds__(32 * EPL) jacobi_f32_kernel(const double* R, int n, double* X,
                                                           double* sig, double* inv_sig, double* scale,
                                                           int* bad) {
+  stream_wait_only();
   constexpr int L = 8, ld = jacobi_f32_pitch(EPL);
   extern __shared__ float wf[];
   __shared__ unsigned top, cmax;
@@ -1200,6 +1209,7 @@ __global__ void __launch_bounds__(32 * EPL) jacobi_f32_kernel(const double* __re
 // E = G - I into G, both triangles, from the lower (column-major) triangle of G. One block. *bad = 1
 // when ||E||_F > 2e-4 (the polar factor below is then not orthonormal to rounding).
 __global__ void __launch_bounds__(1024) polar_error_kernel(double* G, int n, int* bad) {
+  stream_wait_only();
   __shared__ float sums[32];
   float s = 0.f;
   for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
@@ -1221,14 +1231,16 @@ __global__ void __launch_bounds__(1024) polar_error_kernel(double* G, int n, int
 }
 
 // P = I - E / 2 + 3/8 F (column-major n x n)
-__global__ void polar_start_kernel(const double* __restrict__ E, const double* __restrict__ F, double* P,
+__global__ void polar_start_kernel(const double* E, const double* F, double* P,
                                    int n) {
+  stream_wait();
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n * n; t += gridDim.x * blockDim.x)
     P[t] = (t / n == t % n ? 1.0 : 0.0) + fma(0.375, F[t], -0.5 * E[t]);
 }
 
 // X[:, j] *= d[j] (column-major n x n); with T: T[i, j] = X[j, i] d[i] instead
-__global__ void scale_cols_kernel(double* X, const double* __restrict__ d, int n, double* T) {
+__global__ void scale_cols_kernel(double* X, const double* d, int n, double* T) {
+  stream_wait();
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n * n; t += gridDim.x * blockDim.x) {
     const int j = t / n, i = t - j * n;
     const double v = X[t] * d[j];
@@ -1243,6 +1255,7 @@ __global__ void scale_cols_kernel(double* X, const double* __restrict__ d, int n
 __global__ void __launch_bounds__(256) jacobi_grid_round_kernel(double* W, double* V, int n, int nb,
                                                                 int P, int r, double tol,
                                                                 unsigned* count) {
+  stream_wait();
   const int i = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   const int bA = rr_index(i, r, P), bB = rr_index(P - 1 - i, r, P);
@@ -1293,6 +1306,7 @@ __global__ void __launch_bounds__(256) jacobi_grid_round_kernel(double* W, doubl
 }
 
 __global__ void identity_kernel(double* V, int n) {
+  stream_wait();
   const int64_t total = (int64_t)n * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x)
@@ -1301,10 +1315,11 @@ __global__ void identity_kernel(double* V, int n) {
 
 // From the rotated W (column-major n x n) and the rotations V: sigma_j = ||W_j||, descending order;
 // Un[:, rank_j] = W_j / sigma_j, Vs[:, rank_j] = V_j, S[rank_j] = sigma_j *scale. One block.
-__global__ void __launch_bounds__(1024) svd_sort_kernel(const double* __restrict__ W,
-                                                        const double* __restrict__ V, int n,
+__global__ void __launch_bounds__(1024) svd_sort_kernel(const double* W,
+                                                        const double* V, int n,
                                                         double* Un, double* S, double* Vs,
                                                         double* sig, const double* scale) {
+  stream_wait_only();
   __shared__ int rank_sh[1024];
   const int tid = threadIdx.x, nt = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
@@ -1337,8 +1352,9 @@ __global__ void __launch_bounds__(1024) svd_sort_kernel(const double* __restrict
   }
 }
 
-__global__ void gemv_rm_kernel(const double* __restrict__ B, int64_t n, const double* __restrict__ x,
+__global__ void gemv_rm_kernel(const double* B, int64_t n, const double* x,
                                double* y) {
+  stream_wait();
   const int lane = threadIdx.x & 31;
   const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   if (row >= n) return;
@@ -1348,8 +1364,9 @@ __global__ void gemv_rm_kernel(const double* __restrict__ B, int64_t n, const do
   if (lane == 0) y[row] = s;
 }
 
-__global__ void copy_cm_kernel(const double* __restrict__ A, int64_t lda, double* W, int64_t m,
+__global__ void copy_cm_kernel(const double* A, int64_t lda, double* W, int64_t m,
                                int64_t n) {
+  stream_wait();
   const int64_t total = m * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -1364,7 +1381,7 @@ void householder(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, 
   const size_t smem = (size_t)(m * n + m * k + k) * sizeof(double);
   if (smem <= (size_t)kHouseholderSmemBytes) {
     smem_optin((const void*)householder_smem_kernel, kHouseholderSmemBytes);
-    householder_smem_kernel<<<1, 512, smem, s>>>(A, lda, (int)m, (int)n, Q, R);
+    launch_early(householder_smem_kernel, 1, 512, smem, s, A, lda, (int)m, (int)n, Q, R);
     TTGB_CHECK_LAUNCH();
     return;
   }
@@ -1374,9 +1391,9 @@ void householder(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, 
   unsigned g = cdiv(m * n, 256);
   if (g > 4096) g = 4096;
   if (g == 0) g = 1;
-  copy_cm_kernel<<<g, 256, 0, s>>>(A, lda, W, m, n);
+  launch_early(copy_cm_kernel, g, 256, 0, s, A, lda, W, m, n);
   TTGB_CHECK_LAUNCH();
-  householder_kernel<<<1, 512, 0, s>>>(W, (int)m, (int)n, Q, R, tau);
+  launch_early(householder_kernel, 1, 512, 0, s, W, (int)m, (int)n, Q, R, tau);
   TTGB_CHECK_LAUNCH();
 }
 
@@ -1464,7 +1481,7 @@ QRResult qr(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, doubl
   // cost about 30 us a pass, so the line lies where one pass fills that.
   if (n <= kCholQrSmallN && (double)m * n * n <= 3.5e4 && cholqr_small_smem(m, n) <= kHouseholderSmemBytes) {
     smem_optin((const void*)cholqr_small_kernel, kHouseholderSmemBytes);
-    cholqr_small_kernel<<<1, 512, cholqr_small_smem(m, n), s>>>(A, lda, (int)m, (int)n, Q, R);
+    launch_early(cholqr_small_kernel, 1, 512, cholqr_small_smem(m, n), s, A, lda, (int)m, (int)n, Q, R);
     TTGB_CHECK_LAUNCH();
     return res;
   }
@@ -1498,14 +1515,14 @@ QRResult qr(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, doubl
       const size_t smem = (size_t)n * (n + 1) * sizeof(double);
       smem_optin((const void*)chol_inv_smem_kernel,
                  (int)(kCholSmemMax * (kCholSmemMax + 1) * sizeof(double)));
-      chol_inv_smem_kernel<<<1, 512, smem, s>>>(G, (int)n, m, pass, Rp[pass], Ri, ws.status,
+      launch_early(chol_inv_smem_kernel, 1, 512, smem, s, G, (int)n, m, pass, Rp[pass], Ri, ws.status,
                                                 ws.status + 2);
       TTGB_CHECK_LAUNCH();
       if (ws.gram_zero < n * n) ws.gram_zero = n * n;   // the kernel cleared [0, n^2)
     } else {
-      chol_kernel<<<1, 512, 0, s>>>(G, (int)n, pass == 0 ? m : 0, pass == 2 ? 1 : 0, ws.status);
+      launch_early(chol_kernel, 1, 512, 0, s, G, (int)n, pass == 0 ? m : 0, pass == 2 ? 1 : 0, ws.status);
       TTGB_CHECK_LAUNCH();
-      trinv_kernel<<<cdiv(n, 128), 128, 0, s>>>(G, Ri, (int)n);
+      launch_early(trinv_kernel, cdiv(n, 128), 128, 0, s, G, Ri, (int)n);
       TTGB_CHECK_LAUNCH();
       copy(G, Rp[pass], n * n, s);
       ws.gram_zero = 0;   // G now holds R
@@ -1564,7 +1581,7 @@ void jacobi_columns(double* W, double* V, int64_t n, const double* scale, double
     const int nb = (int)std::max<int64_t>(1, (n + 2 * sms - 1) / (2 * sms));
     int P = (int)((n + nb - 1) / nb);
     P += P & 1;
-    identity_kernel<<<cdiv((int64_t)n * n, 256), 256, 0, s>>>(V, (int)n);
+    launch_early(identity_kernel, cdiv((int64_t)n * n, 256), 256, 0, s, V, (int)n);
     TTGB_CHECK_LAUNCH();
     DevBuf<unsigned> cnt(1, s);
     unsigned hcnt = 0;
@@ -1573,7 +1590,7 @@ void jacobi_columns(double* W, double* V, int64_t n, const double* scale, double
     for (; sweep < 60; ++sweep) {
       TTGB_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(unsigned), s));
       for (int r = 0; r < P - 1; ++r) {
-        jacobi_grid_round_kernel<<<P / 2, 256, 0, s>>>(W, V, (int)n, nb, P, r, tol, cnt.p);
+        launch_early(jacobi_grid_round_kernel, P / 2, 256, 0, s, W, V, (int)n, nb, P, r, tol, cnt.p);
         TTGB_CHECK_LAUNCH();
       }
       TTGB_CUDA(cudaMemcpyAsync(&hcnt, cnt.p, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
@@ -1583,7 +1600,7 @@ void jacobi_columns(double* W, double* V, int64_t n, const double* scale, double
     if (sweep >= 60) TTGB_CUDA(cudaMemsetAsync(ws.status, 0x03, 1, s));
   }
   DBuf sig((size_t)n, s);
-  svd_sort_kernel<<<1, 1024, 0, s>>>(W, V, (int)n, Un, S, Vs, sig.p, scale);
+  launch_early(svd_sort_kernel, 1, 1024, 0, s, W, V, (int)n, Un, S, Vs, sig.p, scale);
   TTGB_CHECK_LAUNCH();
 }
 
@@ -1591,7 +1608,7 @@ template <int EPL>
 void launch_jacobi_f32(const double* R, int n, double* X, double* sig, int* bad, cudaStream_t s) {
   const int smem = 8 * EPL * jacobi_f32_pitch(EPL) * (int)sizeof(float);
   smem_optin((const void*)jacobi_f32_kernel<EPL>, smem);
-  jacobi_f32_kernel<EPL><<<1, cdiv((n + 1) / 2 * 8, 32) * 32, smem, s>>>(R, n, X, sig, sig + n, sig + 2 * n,
+  launch_early(jacobi_f32_kernel<EPL>, 1, cdiv((n + 1) / 2 * 8, 32) * 32, smem, s, R, n, X, sig, sig + n, sig + 2 * n,
                                                                            bad);
   TTGB_CHECK_LAUNCH();
 }
@@ -1624,15 +1641,15 @@ bool precondition(const double* R, int64_t n, DBuf& X, DBuf& B, LinalgWS& ws, co
   else launch_jacobi_f32<28>(R, (int)n, X0.p, sig, bad, s);
   // X = X0 (I - E/2 + 3/8 E^2 - 5/16 E^3) with E = X0^T X0 - I: the polar factor to fourth order
   gemm_cm(X0.p, n, X0.p, n, G.p, n, n, n, n, 1.0, 0.0, s, true, false, kTriLowerC);
-  polar_error_kernel<<<1, 1024, 0, s>>>(G.p, (int)n, bad);
+  launch_early(polar_error_kernel, 1, 1024, 0, s, G.p, (int)n, bad);
   TTGB_CHECK_LAUNCH();
   gemm_cm(G.p, n, G.p, n, B.p, n, n, n, n, 1.0, 0.0, s);
-  polar_start_kernel<<<cdiv(n * n, 256), 256, 0, s>>>(G.p, B.p, P.p, (int)n);
+  launch_early(polar_start_kernel, cdiv(n * n, 256), 256, 0, s, G.p, B.p, P.p, (int)n);
   TTGB_CHECK_LAUNCH();
   gemm_cm(B.p, n, G.p, n, P.p, n, n, n, n, -0.3125, 1.0, s);
   gemm_cm(X0.p, n, P.p, n, X.p, n, n, n, n, 1.0, 0.0, s);
   gemm_cm(R, n, X.p, n, B.p, n, n, n, n, 1.0, 0.0, s);
-  scale_cols_kernel<<<cdiv(n * n, 256), 256, 0, s>>>(B.p, inv, (int)n, nullptr);
+  launch_early(scale_cols_kernel, cdiv(n * n, 256), 256, 0, s, B.p, inv, (int)n, nullptr);
   TTGB_CHECK_LAUNCH();
   TTGB_CUDA(cudaMemcpyAsync(ws.h_status, bad, sizeof(int), cudaMemcpyDeviceToHost, s));
   TTGB_CUDA(cudaStreamSynchronize(s));
@@ -1671,7 +1688,7 @@ void svd(const double* A, int64_t lda, int64_t m, int64_t n, double* U, double* 
       const double* sig = X.p + n * n;
       qr(B.p, n, n, n, Q2.p, T.p, ws, red, s);
       ws.c.ensure(3 * n * n + 16, s);
-      scale_cols_kernel<<<cdiv(n * n, 256), 256, 0, s>>>(T.p, sig, (int)n, ws.c.p);
+      launch_early(scale_cols_kernel, cdiv(n * n, 256), 256, 0, s, T.p, sig, (int)n, ws.c.p);
       TTGB_CHECK_LAUNCH();
       jacobi_columns(ws.c.p, ws.c.p + n * n, n, sig + 2 * n, Un.p, S, Vs.p, ws, s);
       gemm_cm(Q2.p, n, Vs.p, n, T.p, n, n, n, n, 1.0, 0.0, s);
@@ -1684,12 +1701,12 @@ void svd(const double* A, int64_t lda, int64_t m, int64_t n, double* U, double* 
   double* Vs = ws.c.p;           // V'
   DBuf Up((size_t)(n * n), s);   // U' (normalised columns of the rotated R^T, sorted)
   if (n < kJacobiWarpMaxN) {
-    jacobi_warp_kernel<<<1, 32, 0, s>>>(Rb.p, (int)n, Up.p, S, Vs, ws.status);
+    launch_early(jacobi_warp_kernel, 1, 32, 0, s, Rb.p, (int)n, Up.p, S, Vs, ws.status);
     TTGB_CHECK_LAUNCH();
   } else {
     double* W = Vs + n * n;      // R^T, rotated in place
     double* scale = W + 2 * n * n;
-    scaled_transpose_kernel<<<1, 1024, 0, s>>>(Rb.p, (int)n, W, scale);
+    launch_early(scaled_transpose_kernel, 1, 1024, 0, s, Rb.p, (int)n, W, scale);
     TTGB_CHECK_LAUNCH();
     jacobi_columns(W, W + n * n, n, scale, Up.p, S, Vs, ws, s);
   }
@@ -1699,7 +1716,7 @@ void svd(const double* A, int64_t lda, int64_t m, int64_t n, double* U, double* 
 
 void gemv(const double* B, int64_t n, const double* x, double* y, cudaStream_t s) {
   if (n <= 0) return;
-  gemv_rm_kernel<<<cdiv(n * 32, 256), 256, 0, s>>>(B, n, x, y);
+  launch_early(gemv_rm_kernel, cdiv(n * 32, 256), 256, 0, s, B, n, x, y);
   TTGB_CHECK_LAUNCH();
 }
 

@@ -121,8 +121,9 @@ __global__ void __launch_bounds__(256) batched_inverse_kernel(double* M, int sz,
 }
 
 // 'c': y[d, m, D] = sum_n J[(d,D), m, n] x[d, n, D]
-__global__ void apply_c_kernel(const double* __restrict__ J, const double* __restrict__ x, double* y,
+__global__ void apply_c_kernel(const double* J, const double* x, double* y,
                                int r, int n, int R) {
+  stream_wait();
   const int64_t total = (int64_t)r * n * R;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -135,8 +136,9 @@ __global__ void apply_c_kernel(const double* __restrict__ J, const double* __res
 }
 
 // 'r': y[d, (m,L)] = sum_{(n,R)} J[d, (m,L), (n,R)] x[d, (n,R)]  (one warp per output)
-__global__ void apply_r_kernel(const double* __restrict__ J, const double* __restrict__ x, double* y,
+__global__ void apply_r_kernel(const double* J, const double* x, double* y,
                                int r, int n, int R) {
+  stream_wait();
   const int64_t sz = (int64_t)n * R;
   const int lane = threadIdx.x & 31;
   const int64_t row = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -191,11 +193,11 @@ void LocalOperator::apply_prec(const double* x, double* y, cudaStream_t s) const
   const LocalOpDims& d = dims;
   if (prec == kCPrec) {
     const int64_t total = d.r * d.n * d.R;
-    apply_c_kernel<<<grid_for(total), 256, 0, s>>>(J, x, y, (int)d.r, (int)d.n, (int)d.R);
+    launch_early(apply_c_kernel, grid_for(total), 256, 0, s, J, x, y, (int)d.r, (int)d.n, (int)d.R);
     TTGB_CHECK_LAUNCH();
   } else if (prec == kRPrec) {
     const int64_t rows = d.r * d.n * d.R;
-    apply_r_kernel<<<cdiv(rows * 32, 256), 256, 0, s>>>(J, x, y, (int)d.r, (int)d.n, (int)d.R);
+    launch_early(apply_r_kernel, cdiv(rows * 32, 256), 256, 0, s, J, x, y, (int)d.r, (int)d.n, (int)d.R);
     TTGB_CHECK_LAUNCH();
   } else {
     copy(x, y, d.r * d.n * d.R, s);

@@ -98,8 +98,9 @@ __device__ __forceinline__ double candidate(const Grouping& g, const double* A, 
 
 // rp (kGroupings arrays of keys + 1 row pointers, one after the other), info: {nonzeros, longest row
 // over all groupings}
-__global__ void __launch_bounds__(kThreads) sparse_count_kernel(const double* __restrict__ A, Groupings gs,
+__global__ void __launch_bounds__(kThreads) sparse_count_kernel(const double* A, Groupings gs,
                                                                 int* rp, unsigned* counter, int64_t* info) {
+  stream_wait();
   __shared__ int longest;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int64_t key = (int64_t)blockIdx.x * (kThreads / 32) + warp;
@@ -148,9 +149,10 @@ __global__ void __launch_bounds__(kThreads) sparse_count_kernel(const double* __
   red::reset_ticket(counter);
 }
 
-__global__ void __launch_bounds__(kThreads) sparse_fill_kernel(const double* __restrict__ A, Grouping g,
-                                                               const int* __restrict__ rp, int* ja, int* jb,
+__global__ void __launch_bounds__(kThreads) sparse_fill_kernel(const double* A, Grouping g,
+                                                               const int* rp, int* ja, int* jb,
                                                                double* val, float* val32) {
+  stream_wait();
   const int lane = threadIdx.x & 31;
   const int64_t key = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   if (key >= g.keys) return;
@@ -205,7 +207,7 @@ void SparseCore::build(const double* A, int64_t s_, int64_t M_, int64_t N_, int6
   unsigned* counter = reinterpret_cast<unsigned*>(row_ptr + keys + kGroupings);
   TTGB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), st));
   int64_t* info = pinned_info();
-  sparse_count_kernel<<<cdiv(keys, kThreads / 32), kThreads, 0, st>>>(A, gs, row_ptr, counter, info);
+  launch_early(sparse_count_kernel, cdiv(keys, kThreads / 32), kThreads, 0, st, A, gs, row_ptr, counter, info);
   TTGB_CHECK_LAUNCH();
   TTGB_CUDA(cudaStreamSynchronize(st));
   const int64_t nnz = info[0];
@@ -224,7 +226,7 @@ void SparseCore::build(const double* A, int64_t s_, int64_t M_, int64_t N_, int6
     rp += c.keys + 1;
     if (!((which >> q) & 1u)) continue;
     c.a = ja; c.b = ja + per; c.val = val; c.val32 = val32;
-    sparse_fill_kernel<<<cdiv(c.keys, kThreads / 32), kThreads, 0, st>>>(A, gs.g[q], c.rp, ja, ja + per, val,
+    launch_early(sparse_fill_kernel, cdiv(c.keys, kThreads / 32), kThreads, 0, st, A, gs.g[q], c.rp, ja, ja + per, val,
                                                                       val32);
     TTGB_CHECK_LAUNCH();
     ja += 2 * per;

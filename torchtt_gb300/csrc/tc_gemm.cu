@@ -187,10 +187,11 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_tma_kernel(const __grid_c
     const CUtensorMap* map = lane == 0 ? &P.a_hi : lane == 1 ? &P.a_lo : lane == 2 ? &P.b_hi : &P.b_lo;
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
   }
-  stream_wait();
+  stream_wait_only();
   const int gate = P.gate != nullptr ? *P.gate : 0;
   asm volatile("tcgen05.fence::before_thread_sync;");
   const int gated = __syncthreads_or(gate);
+  stream_release();   // not before this block has its tensor memory: the next kernel's may ask for some
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_sh;
   if (gated) {
@@ -339,8 +340,9 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_tma_kernel(const __grid_c
   }
 }
 
-__global__ void split_tf32_kernel(const double* __restrict__ x, Gather4 g, int64_t inner,
+__global__ void split_tf32_kernel(const double* x, Gather4 g, int64_t inner,
                                   int64_t out_ld, float* hi, float* lo) {
+  stream_wait();
   const int64_t total = g.e0 * g.e1 * g.e2 * g.e3;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -442,7 +444,7 @@ void split_tf32(const double* x, const Gather4& g, float* hi, float* lo, cudaStr
   unsigned grid = cdiv(total, 256);
   const unsigned cap = 8 * (unsigned)num_sms();
   if (grid > cap) grid = cap;
-  split_tf32_kernel<<<grid, 256, 0, s>>>(x, g, inner, out_ld, hi, lo);
+  launch_early(split_tf32_kernel, grid, 256, 0, s, x, g, inner, out_ld, hi, lo);
   TTGB_CHECK_LAUNCH();
 }
 
