@@ -52,6 +52,7 @@ struct KParams {
   AxD cm, cn;
   int64_t c_bs;
   T alpha, beta;
+  int scale, keep;   // alpha is not 1, beta not 0: comparing in FP64 costs as much as a multiply-add
   int tri;
 };
 
@@ -159,14 +160,68 @@ __global__ void __launch_bounds__(NT) contract_kernel(KParams<T> p) {
       const int n = n0 + tx + 16 * j;
       if (n >= p.N) continue;
       T* c = C + cmo + ax_off(p.cn, n);
-      const T v = p.alpha * acc[i][j];
+      const T v = p.scale ? p.alpha * acc[i][j] : acc[i][j];
       if (p.splitk > 1) {
         atomicAdd(c, v);
       } else {
-        *c = (p.beta == T(0)) ? v : fma(p.beta, *c, v);
+        *c = p.keep ? fma(p.beta, *c, v) : v;
       }
     }
   }
+}
+
+// FP64 in 8 x 8 tiles: the eight warps split a chunk of 32 k in four slices (two warps hold a tile's sums), added at the end. A
+// product of 40 x 240 x 20 has 45 tiles of 16 x 16, whose SMs do 2.2 k clocks of FP64 per 16 k while the
+// other 107 have nothing; in 150 tiles of 8 x 8 the same work takes a quarter of that on every SM.
+__global__ void __launch_bounds__(NT) contract_small_kernel(KParams<double> p) {
+  constexpr int BS = 8, CK = 32, kSlices = 4;
+  __shared__ double As[CK][BS + 1], Bs[CK][BS + 1], part[kSlices - 1][BS * BS];
+  const int tid = threadIdx.x;
+  const int bz = blockIdx.z;
+  const int bidx = bz / p.splitk;
+  const int ks = bz - bidx * p.splitk;
+  const int kbeg = ks * p.kchunk;
+  int kend = min(p.K, kbeg + p.kchunk);
+  const int m0 = blockIdx.y * BS, n0 = blockIdx.x * BS;
+  if (p.tri & kTriUpperB) kend = min(kend, n0 + BS);   // B(k, n) = 0 for k > n
+  const bool skip = (p.tri & kTriLowerC) && m0 + BS <= n0;   // tile strictly above the diagonal
+  // loader: thread (row or column, k) of the chunk
+  const int lk = tid % CK, lr = tid / CK;
+  const bool mok = m0 + lr < p.M, nok = n0 + lr < p.N;
+  const double* A = p.A + (int64_t)bidx * p.a_bs + (mok ? ax_off(p.am, m0 + lr) : 0);
+  const double* B = p.B + (int64_t)bidx * p.b_bs + (nok ? ax_off(p.bn, n0 + lr) : 0);
+  const int slice = tid / (BS * BS), ty = tid / BS % BS, tx = tid % BS;
+  const int m = m0 + ty, n = n0 + tx;
+  const bool own = slice == 0 && m < p.M && n < p.N;
+  double* c = p.C + (int64_t)bidx * p.c_bs + (own ? ax_off(p.cm, m) + ax_off(p.cn, n) : 0);
+  stream_wait();
+  if (skip) return;
+  double ra = 0.0, rb = 0.0, acc = 0.0;
+  const auto load = [&](int k) {
+    const bool kok = k < kend;
+    ra = kok && mok ? A[ax_off(p.ak, k)] : 0.0;
+    rb = kok && nok ? B[ax_off(p.bk, k)] : 0.0;
+  };
+  if (kbeg < kend) load(kbeg + lk);
+  for (int k0 = kbeg; k0 < kend; k0 += CK) {
+    As[lk][lr] = ra;
+    Bs[lk][lr] = rb;
+    __syncthreads();
+    if (k0 + CK < kend) load(k0 + CK + lk);
+    const int k1 = slice * (CK / kSlices);
+    if (k0 + k1 < kend) {   // zeros past the end: a slice without any is left out
+#pragma unroll
+      for (int kk = 0; kk < CK / kSlices; ++kk) acc = fma(As[k1 + kk][ty], Bs[k1 + kk][tx], acc);
+    }
+    __syncthreads();
+  }
+  if (slice > 0) part[slice - 1][tid % (BS * BS)] = acc;
+  __syncthreads();
+  if (!own) return;
+  acc = (acc + part[0][tid]) + (part[1][tid] + part[2][tid]);
+  if (p.scale) acc *= p.alpha;
+  if (p.splitk > 1) atomicAdd(c, acc);
+  else *c = p.keep ? fma(p.beta, *c, acc) : acc;
 }
 
 // The same contraction in double-float arithmetic on the FP32 pipe: every FP64 operand is split
@@ -306,7 +361,7 @@ __global__ void __launch_bounds__(NT) contract_df_kernel(KParams<double> p) {
       double* c = C + cmo + ax_off(p.cn, n);
       const double v = p.alpha * ((double)ch[i][j] + (double)cl[i][j]);
       if (p.splitk > 1) atomicAdd(c, v);
-      else *c = (p.beta == 0.0) ? v : fma(p.beta, *c, v);
+      else *c = p.keep ? fma(p.beta, *c, v) : v;
     }
   }
 }
@@ -370,13 +425,13 @@ constexpr TileCfg kCandidates64[] = {
     {16, 16, 0}, {16, 32, 0}, {32, 16, 0}, {32, 32, 0}, {16, 16, 1}, {32, 32, 1},
     {64, 32, 0, kEmu}, {32, 64, 0, kEmu}, {64, 16, 0, kEmu}, {16, 64, 0, kEmu},
     {64, 32, 1, kEmu}, {32, 64, 1, kEmu}, {64, 16, 1, kEmu}, {16, 64, 1, kEmu},
-    {128, 32, 0, kOz}, {128, 32, 1, kOz}};
+    {128, 32, 0, kOz}, {128, 32, 1, kOz}, {8, 8, 0}};
 // where the caller takes double-float accuracy
 constexpr TileCfg kCandidatesDf[] = {
     {16, 16, 0}, {16, 16, 1}, {32, 32, 0, kDf}, {64, 32, 0, kDf}, {32, 64, 0, kDf},
     {32, 32, 1, kDf}, {64, 32, 1, kDf}, {32, 64, 1, kDf},
     {64, 32, 0, kEmu}, {32, 64, 0, kEmu}, {64, 32, 1, kEmu}, {32, 64, 1, kEmu},
-    {128, 32, 0, kOz}, {128, 32, 1, kOz}};
+    {128, 32, 0, kOz}, {128, 32, 1, kOz}, {8, 8, 0}};
 constexpr TileCfg kCandidates32[] = {{64, 64, 0}, {64, 32, 0}, {32, 64, 0}, {32, 32, 0},
                                      {64, 64, 1}, {64, 32, 1}, {32, 64, 1}, {32, 32, 1}};
 struct CandidateList {
@@ -489,6 +544,7 @@ bool usable(const TileCfg& t, const ContractDescT<T>& d, cudaStream_t stream) {
   if (t.kind == kEmu || t.kind == kOz) {
     if (componentwise(d)) return false;
   }
+  if (t.kind != kOz && cdiv(d.M, t.bm) >= 65536) return false;   // rows of tiles in the grid
   if constexpr (std::is_same<T, double>::value) {
     if (t.kind == kOz) {
       cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -559,7 +615,8 @@ void launch_tiles(const ContractDescT<T>& d, KParams<T> p, const TileCfg& t, int
       if (bm == 64 && bn == 32) launch_early(contract_df_kernel<64, 32>, grid, NT, 0, stream, p);
       else if (bm == 32 && bn == 64) launch_early(contract_df_kernel<32, 64>, grid, NT, 0, stream, p);
       else launch_early(contract_df_kernel<32, 32>, grid, NT, 0, stream, p);
-    } else if (bm == 16 && bn == 16) launch_early(contract_kernel<T, 16, 16>, grid, NT, 0, stream, p);
+    } else if (bm == 8) launch_early(contract_small_kernel, grid, NT, 0, stream, p);
+    else if (bm == 16 && bn == 16) launch_early(contract_kernel<T, 16, 16>, grid, NT, 0, stream, p);
     else if (bm == 16 && bn == 32) launch_early(contract_kernel<T, 16, 32>, grid, NT, 0, stream, p);
     else if (bm == 32 && bn == 16) launch_early(contract_kernel<T, 32, 16>, grid, NT, 0, stream, p);
     else launch_early(contract_kernel<T, 32, 32>, grid, NT, 0, stream, p);
@@ -668,6 +725,7 @@ void launch_contract(const ContractDescT<T>& d, cudaStream_t stream, bool determ
   p.B = d.B; p.bk = to_dev(d.bk, d.K); p.bn = to_dev(d.bn, d.N); p.b_bs = d.b_bs;
   p.C = d.C; p.cm = to_dev(d.cm, d.M); p.cn = to_dev(d.cn, d.N); p.c_bs = d.c_bs;
   p.alpha = d.alpha; p.beta = d.beta;
+  p.scale = d.alpha != T(1); p.keep = d.beta != T(0);
   p.tri = d.tri;
   if (d.K <= 0) {  // empty sum: C = beta * C
     launch_early(scale_output_kernel<T>, std::min(cdiv((int64_t)d.M * d.N * d.batch, 256), 4096u), 256, 0, stream,
@@ -711,7 +769,8 @@ void launch_contract(const ContractDescT<T>& d, cudaStream_t stream, bool determ
       else if (d.M >= d.N) t.bm = 64;
       else t.bn = 64;
     } else if (t.kind == kFma && tiles(32, 32) < target) {
-      t.bm = t.bn = 16;
+      // 8 x 8 where 16 x 16 would leave half of the SMs without a tile
+      t.bm = t.bn = 2 * tiles(16, 16) <= sms ? 8 : 16;
     }
   } else if (tiles(64, 64) < target) {
     if (d.M >= d.N) { t.bm = 64; t.bn = 32; } else { t.bm = 32; t.bn = 64; }

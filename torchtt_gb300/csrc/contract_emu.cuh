@@ -315,9 +315,9 @@ __global__ void __launch_bounds__(EmuTile<BM, BN>::kThreads, EmuTile<BM, BN>::kM
         const int n = n0 + wn + 8 * j + t2 + h;
         if (n >= p.N) continue;
         double* c = C + cmo + ax_off(p.cn, n);
-        const double v = p.alpha == 1.0 ? acc[j][r + h] : p.alpha * acc[j][r + h];
+        const double v = p.scale ? p.alpha * acc[j][r + h] : acc[j][r + h];
         if (p.splitk > 1) atomicAdd(c, v);
-        else *c = (p.beta == 0.0) ? v : fma(p.beta, *c, v);
+        else *c = p.keep ? fma(p.beta, *c, v) : v;
       }
   }
 }
