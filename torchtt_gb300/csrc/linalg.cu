@@ -209,10 +209,13 @@ __device__ void chol_panels(double* A, int n, double floor_d, CholShared& ch) {
           double v = (i == (c & 15)) ? 1.0 : 0.0;   // also the padding of the last panel
           if (c < w && i < w) v = c >= i ? A[(j0 + i) * ld + j0 + c] : A[(j0 + c) * ld + j0 + i];
   #pragma unroll 1
-          for (int j = 0; j < kCholNb; ++j) {
+          for (int j = 0; j < w; ++j) {
             if (i == j) {
               const double d = __shfl_sync(0xffffffffu, v, j);
-              if (!(d > floor_d) || !isfinite(d)) ch.bad = 1;   // the same in every lane
+              // d > floor_d >= 0 and finite, as integers: an FP64 comparison is a round trip to a busy pipe
+              const long long bits = __double_as_longlong(d);
+              if (bits <= __double_as_longlong(floor_d) || bits >= 0x7ff0000000000000ll)
+                ch.bad = 1;   // the same in every lane
               v *= rsqrt_refined(d);
               ch.rowbuf[j & 1][c] = v;
             }
