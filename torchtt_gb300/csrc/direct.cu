@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(1024) lu_solve_kernel(const double* B,
                                                         const double* b, double* LU,
                                                         double* x, int n, int* status,
                                                         const int* gate) {
-  stream_wait_only();
+  stream_wait();
   __shared__ double shv[32];
   __shared__ double piv_inv;
   __shared__ int shi[32];

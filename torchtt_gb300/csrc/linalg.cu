@@ -62,7 +62,7 @@ __device__ double block_max_d(double v, double* sh) {
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(512) chol_kernel(double* G, int n, int64_t shift_rows,
                                                    int check_identity, int* status) {
-  stream_wait_only();
+  stream_wait();
   __shared__ double sh[32];
   __shared__ int bad;
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -288,7 +288,7 @@ __device__ void chol_panels(double* A, int n, double floor_d, CholShared& ch) {
 __global__ void __launch_bounds__(512) chol_inv_smem_kernel(double* Gin, int n,
                                                             int64_t shift_rows, int pass, double* Rout,
                                                             double* Riout, int* status, int* done) {
-  stream_wait_only();
+  stream_wait();
   extern __shared__ double A[];
   const int ld = n + 1;
   __shared__ CholShared ch;
@@ -448,7 +448,7 @@ __device__ __forceinline__ void householder_body(double* W, int m, int n, double
 
 __global__ void __launch_bounds__(512) householder_kernel(double* W, int m, int n, double* Q,
                                                           double* R, double* tau) {
-  stream_wait_only();
+  stream_wait();
   householder_body(W, m, n, Q, R, tau);
 }
 
@@ -460,7 +460,7 @@ constexpr int kHouseholderSmemBytes = 200 * 1024;
 __global__ void __launch_bounds__(512, 1) householder_smem_kernel(const double* A,
                                                                int64_t lda, int m, int n,
                                                                double* Qout, double* R) {
-  stream_wait_only();
+  stream_wait();
   extern __shared__ double hs[];
   const int k = min(m, n);
   double* W = hs;
@@ -489,7 +489,7 @@ constexpr int kCholQrSmallN = 32;
 
 __global__ void __launch_bounds__(512, 1) cholqr_small_kernel(const double* A, int64_t lda,
                                                               int m, int n, double* Qout, double* Rout) {
-  stream_wait_only();
+  stream_wait();
   extern __shared__ double hs[];
   const int ldq = m | 1;   // odd pitch of the columns
   double* X = hs;                            // m x n, this pass's input
@@ -836,7 +836,7 @@ __device__ __forceinline__ void jacobi_scale(unsigned top, double& down, double&
 // W = R^T scaled by jacobi_scale, *up the factor back. One block.
 __global__ void __launch_bounds__(1024) scaled_transpose_kernel(const double* R, int n, double* W,
                                                                 double* up) {
-  stream_wait_only();
+  stream_wait();
   __shared__ unsigned top;
   if (threadIdx.x == 0) top = 0u;
   __syncthreads();
@@ -865,7 +865,7 @@ constexpr int kJacobiWarpMaxN = 16;
 
 __global__ void __launch_bounds__(32) jacobi_warp_kernel(const double* R, int n, double* Un,
                                                          double* S, double* Vs, int* status) {
-  stream_wait_only();
+  stream_wait();
   constexpr int N = kJacobiWarpMaxN, ld = N + 1;
   __shared__ double W[N * ld], V[N * ld], nrm[N];
   const int lane = threadIdx.x, gid = lane / 4, gl = lane % 4;
@@ -1094,7 +1094,7 @@ template <int EPL>
 __global__ void __launch_bounds__(32 * EPL) jacobi_f32_kernel(const double* R, int n, double* X,
                                                           double* sig, double* inv_sig, double* scale,
                                                           int* bad) {
-  stream_wait_only();
+  stream_wait();
   constexpr int L = 8, ld = jacobi_f32_pitch(EPL);
   extern __shared__ float wf[];
   __shared__ unsigned top, cmax;
@@ -1212,7 +1212,7 @@ __global__ void __launch_bounds__(32 * EPL) jacobi_f32_kernel(const double* R, i
 // E = G - I into G, both triangles, from the lower (column-major) triangle of G. One block. *bad = 1
 // when ||E||_F > 2e-4 (the polar factor below is then not orthonormal to rounding).
 __global__ void __launch_bounds__(1024) polar_error_kernel(double* G, int n, int* bad) {
-  stream_wait_only();
+  stream_wait();
   __shared__ float sums[32];
   float s = 0.f;
   for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
@@ -1322,7 +1322,7 @@ __global__ void __launch_bounds__(1024) svd_sort_kernel(const double* W,
                                                         const double* V, int n,
                                                         double* Un, double* S, double* Vs,
                                                         double* sig, const double* scale) {
-  stream_wait_only();
+  stream_wait();
   __shared__ int rank_sh[1024];
   const int tid = threadIdx.x, nt = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;

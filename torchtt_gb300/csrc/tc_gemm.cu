@@ -187,11 +187,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_tma_kernel(const __grid_c
     const CUtensorMap* map = lane == 0 ? &P.a_hi : lane == 1 ? &P.a_lo : lane == 2 ? &P.b_hi : &P.b_lo;
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
   }
-  stream_wait_only();
+  stream_wait();
   const int gate = P.gate != nullptr ? *P.gate : 0;
   asm volatile("tcgen05.fence::before_thread_sync;");
   const int gated = __syncthreads_or(gate);
-  stream_release();   // not before this block has its tensor memory: the next kernel's may ask for some
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_sh;
   if (gated) {
