@@ -442,8 +442,8 @@ __device__ __forceinline__ void givens_step(double* h, const double* rot, int k,
 // b <= orth_tol^2 a (the new vector's component along the basis, |V^T w'| / |w'|, is already below the
 // tolerated loss of orthogonality) also takes mode 0. With a split target, q is also written as
 // the tcgen05 engine's TF32 operand, so the next operator application starts from it without a
-// split launch. In mode 0 the norm is known and an extra block takes the Givens step while the others write; in
-// modes 1 and 2 the last block takes it, after it has corrected the scale where the finished vector's
+// split launch. In mode 0, and in mode 1 without a tolerated loss of orthogonality, the norm is known and an extra
+// block takes the Givens step while the others write; otherwise the last block takes it, after it has corrected the scale where the finished vector's
 // norm is not 1 to rounding. Once the flag is set, later iterations leave H, beta and the flag
 // alone, so iterations queued past the stopping point change nothing the solution uses.
 template <int E, int VP>
@@ -505,6 +505,16 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
       givens_step(hcol, rot, k, iters, hp, H, cs, sn, beta, threshold, scal, flag, 0);
     return;
   }
+  // Without a tolerated loss of orthogonality V is orthonormal to rounding after the second projection, so in
+  // mode 1 the norm is known as well: the finished vector's would be 1 to some 1e-14.
+  const bool known = mode == 1 && orth_tol2 == 0.0;
+  if (extra && known) {
+    if (tid < kv) hcol[tid] += sums[tid];
+    __syncthreads();
+    if (warp == 0)
+      givens_step(hcol, rot, k, iters, hp, H, cs, sn, beta, threshold, scal, flag, kv);
+    return;
+  }
   double ss = 0.0;
   for (int64_t c = beg; c < end; c += 32 * E) {
     const double s = slice_combination<E, VP>(Q, ldq, kv, sums, c, end, sh);
@@ -516,6 +526,7 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
     }
     __syncthreads();
   }
+  if (known) return;
   ss = block_sum(ss, sh);
   if (tid == 0) part_out[blockIdx.x] = ss;
   if (!red::take_last_ticket(counter)) return;
