@@ -610,10 +610,12 @@ def run_gb300(args):
                  "avg_launch_us": 1000 * pf["contract_ms"] / max(1, pf["contract_launches"])}
 
     # the mixed solve's FP64 products (true residuals, interface updates, local right-hand sides)
-    # run in double-float on the FP32 pipe: ~12 FP32 operations per FP64 multiply-add (error-free
-    # product, two-sum, accumulation), so the pipe's share is (flops / 2) * 12 / FP32 peak
+    # have double-float accuracy: by the tuner's choice digit products on the tensor cores, FP64
+    # multiply-adds, or double-float on the FP32 pipe at ~12 FP32 operations per FP64 multiply-add (the
+    # share of that pipe they would take: (flops / 2) * 12 / FP32 peak)
     df_tflops = pm["contract_flops"] / (pm["contract_ms"] * 1e-3) / 1e12 if pm["contract_ms"] > 0 else None
-    df_roof = {"kernel": "contract_df_kernel (double-float FP64 products of the mixed path)",
+    df_roof = {"kernel": "contract_emu_kernel, oz_gemm_kernel, contract_kernel, contract_df_kernel (FP64 products of the "
+                         "mixed path)",
                "achieved": df_tflops, "unit": "TFLOP/s (FP64-equivalent)",
                "fp32_pipe_frac": df_tflops / 2 * 12 / fp32_peak if (df_tflops and fp32_peak) else None,
                "fp32_peak": fp32_peak, "peak_source": "FP32 FMA pipe measured live (ttgb_calibrate_fma)",

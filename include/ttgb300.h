@@ -69,14 +69,15 @@ typedef struct ttgb_amen_params {
   int32_t a_structure;          /* 1 (default): A cores with density < 1/4 (Kronecker-sum
                                    operators) are applied from their nonzeros; 0: always dense */
   int32_t fp64_engine;          /* FP64 products of local matvecs, interfaces and local rhs:
-                                   0 auto (double-float arithmetic on the FP32 pipe on the MIXED
-                                   path when eps >= 1e-9 and A and b fit the FP32 exponent range,
-                                   ~1e-13 relative; native FP64 otherwise), 1 native FP64,
-                                   2 double-float.
-                                   On the MIXED path with double-float products the GEMMs
-                                   of the QR/SVD (CholeskyQR Gram and apply products) run in
-                                   double-float too; the factorisations themselves (Cholesky,
-                                   Jacobi rotations) always run in native FP64. */
+                                   0 auto (double-float accuracy on the MIXED path when
+                                   eps >= 1e-9 and A and b fit the FP32 exponent range, ~1e-13
+                                   relative: double-float arithmetic on the FP32 pipe, or FP64
+                                   kernels where they are faster; FP64 otherwise), 1 FP64,
+                                   2 double-float accuracy.
+                                   On the MIXED path with double-float accuracy the GEMMs
+                                   of the QR/SVD (CholeskyQR Gram and apply products) have it
+                                   too; the factorisations themselves (Cholesky, the Jacobi
+                                   rotations that give the result) always run in FP64. */
   int32_t strict_eps;           /* 0 (default): the reference's tolerance and stopping rule,
                                    which bound the local residuals (its true residual can end a
                                    few times above eps); 1: the sweeps solve, truncate and stop
@@ -227,8 +228,8 @@ int ttgb_local_product(int64_t rl, int64_t s, int64_t r, int64_t m, int64_t n, i
 /* The local product with a low-precision engine (the operator of the mixed path's inner GMRES):
  * FP64 in and out, contraction in TTGB_ENGINE_FP32 (CUDA-core FFMA) or TTGB_ENGINE_TC
  * (tcgen05 tensor cores, 3xTF32 with FP32 accumulation in tensor memory); TTGB_ENGINE_DF is the
- * mixed path's FP64-class engine for its residual products (double-float arithmetic on the FP32
- * pipe, ~1e-13 relative for operands within the FP32 exponent range). Same shapes as
+ * mixed path's FP64-class engine for its residual products (double-float accuracy, ~1e-13 relative
+ * for operands within the FP32 exponent range, or better). Same shapes as
  * ttgb_local_product with one right-hand side. No counterpart in the reference (its only mixed mode
  * is the FP32 GMRES of torchtt/solvers.py:469-496). */
 #define TTGB_ENGINE_FP32 1

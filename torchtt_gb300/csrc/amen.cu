@@ -912,12 +912,11 @@ void AmenRun::z_update_forward(int k, const double* trunc) {
   z_[k] = std::move(zk);
 }
 
-// Engine of the GEMMs of the mixed path's dense linear algebra (the CholeskyQR3 Gram and apply
-// products, U = Q V', the enrichment's block Gram-Schmidt, reconstructions): double-float whenever
-// the mixed path's FP64 products are double-float. Those GEMMs dominate the SM time of a solve on
-// GB300's FP64 pipe; in double-float they keep ~1e-13 of the sum of magnitudes of their terms,
-// Q stays orthogonal to ~1e-13 (CholeskyQR3's third pass), far below the eps >= 1e-9 where the
-// double-float engine is chosen. The Cholesky factorisations, the Jacobi rotations, Gram-Schmidt
+// Engine of the GEMMs of the mixed path's dense linear algebra (the CholeskyQR Gram and apply
+// products, U = Q V', the enrichment's block Gram-Schmidt, reconstructions): double-float accuracy
+// whenever the mixed path's FP64 products have it. They then keep at least ~1e-13 of the sum of
+// magnitudes of their terms, and Q stays orthogonal to ~1e-13 (the last pass), far below the
+// eps >= 1e-9 where that accuracy is chosen. The Cholesky factorisations, the Jacobi rotations, Gram-Schmidt
 // of the Krylov basis and every norm stay native FP64. TTGB_LA_ENGINE=native keeps them native.
 static int linalg_engine(int fp64_products_engine, double eps) {
   static const bool force_native = [] {

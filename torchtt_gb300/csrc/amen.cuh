@@ -30,8 +30,8 @@ struct AmenParams {
   double lowp_floor = 1e-5;    // relative target of one low-precision inner solve (mixed)
   int a_structure = 1;         // 1: apply A cores of density < 1/4 from their nonzeros
   // FP64 contractions of the local products, interfaces and local right-hand sides: 0 auto
-  // (double-float on the mixed path when A and b lie within the FP32 exponent range, native FP64
-  // otherwise), 1 native FP64, 2 double-float. QR/SVD always run in native FP64.
+  // (double-float accuracy on the mixed path when A and b lie within the FP32 exponent range, FP64
+  // otherwise), 1 FP64, 2 double-float accuracy. The factorisations always run in FP64.
   int fp64_engine = 0;
   // 1: the sweeps solve, truncate and stop at eps / 4, so that the true relative residual ends at
   // or below eps (the reference's rule bounds only the local residuals)

@@ -3,8 +3,9 @@
 // Every operand index of the GEMM kernels here may be a pair of tensor indices with their own strides
 // (struct Ax), so the reference's tensordot permutes (cpp/amen_solve.h:17-98) cost no copies.
 // contract_kernel multiplies shared-memory tiles in the operand type (BK = 16, 256 threads, each thread
-// a (BM/16) x (BN/16) register tile); contract_emu_kernel takes the large FP64 products on the tensor
-// cores; contract_df_kernel runs in double-float arithmetic on the FP32 pipe where the caller takes
+// a (BM/16) x (BN/16) register tile), contract_small_kernel FP64 in 8 x 8 tiles; contract_emu_kernel
+// and, from some 3e7 multiply-adds, oz_gemm.cu take the large FP64 products on the tensor cores;
+// contract_df_kernel runs in double-float arithmetic on the FP32 pipe where the caller takes
 // that accuracy. Which kernel, tile shape and split-K (atomic FP64 adds) a launch gets comes from the
 // tile autotuner's record for its shape class, or from an occupancy heuristic.
 #include <climits>
@@ -404,8 +405,8 @@ thread_local int t_fp64_engine = kFp64Native;
 // FP32), power-of-two buckets of M, N, K and the batch, the triangular flags and which operand
 // strides are unit, and the device. The first launch of a class with beta == 0 (the output is
 // overwritten, so running it several times is harmless) and no overlap between C and its inputs
-// times every candidate - the four tile shapes, each with and without split-K - with CUDA events
-// on the caller's stream (best of two runs) and records the fastest; later launches of the class
+// times every candidate of its engine (the lists below) with CUDA events on the caller's stream, the
+// second of two runs in a row, and records the fastest; later launches of the class
 // use the record. Launches that cannot be tuned (beta != 0, aliasing, a capturing stream, a
 // deterministic request) and classes being tuned by another thread use the occupancy heuristic.
 // ---------------------------------------------------------------------------------------------

@@ -169,7 +169,7 @@ __global__ void scale_by_kernel(const double* x, double* y, int64_t n, const dou
 // a warp together (a step halves the number of values as it halves the lanes: 9 adds for 8 vectors
 // instead of 40), and leave the sum over the blocks to the blocks of the next launch, each of which
 // adds the G x nv partial sums for itself, so that no pass ends in one block's serial tail.
-// Measured per launch (n = 4 k to 32 k, kv up to 41): project 2.3-7 us, update 4-16 us, finish 7-15 us;
+// Measured per launch (n = 4 k to 32 k, kv up to 41): project 2.3-7 us, update 4-16 us, finish 7-14 us;
 // with the elements dealt to the warps and the last block adding the partial sums 18, 31 and 13.5 us.
 // ---------------------------------------------------------------------------------------------
 constexpr int kWarps = RT / 32;

@@ -13,7 +13,7 @@ struct LinalgWS {
   DBuf a, b, c, d, e;
   int* status = nullptr;      // device status word of the last factorisation (0 = ok)
   int* h_status = nullptr;    // pinned host mirror
-  // Gram matrices of CholeskyQR3. The shared-memory Cholesky kernel clears the Gram matrix it has
+  // Gram matrices of CholeskyQR. The shared-memory Cholesky kernel clears the Gram matrix it has
   // read, so the next Gram product (split-K, atomic partial sums) starts from zeros without a
   // zeroing launch; the first gram_zero elements are known to be zero.
   DBuf gram;
@@ -25,9 +25,10 @@ struct QRResult {
 };
 
 // Thin QR of the m x n column-major matrix A (lda): Q (m x k, ldq = m), R (k x n, ldr = k),
-// k = min(m, n). A is not modified. Tall matrices use shifted CholeskyQR3 (three Gram/Cholesky
-// passes built on the contraction engine), checked for orthogonality; small, wide or degenerate
-// ones use a single-block Householder QR.
+// k = min(m, n). A is not modified. Tall matrices use CholeskyQR in two passes, or in three after a
+// shifted start (Gram and apply products on the contraction engine, all in one launch for small ones),
+// checked for orthogonality; wide ones take Q from their leading square block above 8 rows. A
+// single-block Householder QR does the rest: fewer rows, breakdowns, more than 1024 columns.
 QRResult qr(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, double* R,
             LinalgWS& ws, const RedWS& red, cudaStream_t s);
 
@@ -38,7 +39,8 @@ void qr_r(const double* A, int64_t lda, int64_t m, int64_t n, double* R, LinalgW
           cudaStream_t s);
 
 // Thin SVD A = U diag(S) Vh of the m x n column-major matrix A (lda): U (m x k, ld m),
-// S (k), Vh (k x n, ld k), k = min(m, n), singular values in descending order.
+// S (k), Vh (k x n, ld k), k = min(m, n), singular values in descending order: one-sided Jacobi in FP64, from 16 to
+// 224 columns after an FP32 start and a second QR.
 // (reference: at::linalg_svd(A, full_matrices=false))
 void svd(const double* A, int64_t lda, int64_t m, int64_t n, double* U, double* S, double* Vh,
          LinalgWS& ws, const RedWS& red, cudaStream_t s);

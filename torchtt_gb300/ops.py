@@ -135,7 +135,7 @@ ENGINE_DF = 3
 def local_product_lowp(Phi_right, Phi_left, coreA, core, engine=ENGINE_TC):
     """The local product with a low-precision engine (FP32 CUDA cores or tcgen05 3xTF32),
     FP64 in and out: the operator of the mixed path's inner GMRES. ``ENGINE_DF`` runs the mixed
-    path's FP64-class products instead (double-float arithmetic on the FP32 pipe)."""
+    path's FP64-class products instead (double-float accuracy or better)."""
     _dev64(Phi_right, Phi_left, coreA, core)
     rl, s, r = Phi_left.shape
     _, m, n, S = coreA.shape
