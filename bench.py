@@ -598,7 +598,9 @@ def run_gb300(args):
            "ms": kms, "launches": pm.get("krylov_launches"),
            "avg_launch_us": 1000 * kms / max(1, pm.get("krylov_launches", 0))}
     kry["frac"] = kry["achieved"] / hbm if kry["achieved"] else None
-    fp64_roof = {"kernel": "contract_kernel<double> (FP64 contraction engine, plain path)",
+    fp64_roof = {"kernel": "contract_kernel<double>, contract_small_kernel, contract_emu_kernel, oz_gemm_kernel (FP64 "
+                           "contraction engine, plain path; large products run on the tensor cores, so that "
+                           "the FP64 pipe's rate is no bound)",
                  "achieved": fp64_tflops, "peak": fp64_peak, "unit": "TFLOP/s",
                  "frac": fp64_tflops / fp64_peak if fp64_tflops else None,
                  "peak_source": "FP64 FMA pipe measured live (ttgb_calibrate_fma)",
