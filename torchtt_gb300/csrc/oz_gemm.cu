@@ -123,7 +123,7 @@ __device__ __forceinline__ bool load_row(double (&v)[PER], const Operand& o, int
   Walk w(o.k, k0);
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
-    v[i] = (ok && k0 + i < K) ? __ldg(base + w.off) : 0.0;
+    v[i] = (ok && k0 + i < K) ? base[w.off] : 0.0;
     w.next(o.k);
   }
 #pragma unroll
@@ -200,7 +200,8 @@ __global__ void __cluster_dims__(kQCtas, 1, 1) __launch_bounds__(kQCols * 8)
 // Digits of P: 32 rows of one chunk per CTA, thread (row, eighth of the chunk). Scale: the row's largest
 // exponent after k's scale kappa(k).
 __global__ void __launch_bounds__(256) oz_digits_p_kernel(Operand p, int K, int kp,
-                                                          const int* __restrict__ kappa, int kappa_z) {
+                                                          const int* kappa, int kappa_z) {
+  stream_wait();
   constexpr int kPer = kOzChunk / 8;
   __shared__ int emax[kPRows], kk[kOzChunk];
   const int chunk = blockIdx.y, z = blockIdx.z, nchunk = gridDim.y;
@@ -402,21 +403,6 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
   __shared__ int abort_sh, issued_sh, consumed_sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  // a special value in what this CTA reads
-  int special = 0;
-  OzTile o;
-  for (int t = blockIdx.x; t < P.tiles; t += gridDim.x) {
-    if (!oz_tile<BN>(P, t, o)) continue;
-    const int pblocks = (P.p.rows + kPRows - 1) / kPRows;
-    const int ch0 = o.kbeg / kOzChunk, ch1 = (o.kend + kOzChunk - 1) / kOzChunk;
-    for (int i = tid; i < (ch1 - ch0) * (kBM / kPRows); i += kThreads) {
-      const int b = o.r0 / kPRows + i % (kBM / kPRows);
-      if (b < pblocks)
-        special |= P.p.special[((int64_t)o.zp * P.nchunk + ch0 + i / (kBM / kPRows)) * pblocks + b];
-    }
-    for (int i = tid; i < (ch1 - ch0) * kQCtas; i += kThreads)
-      special |= P.q.special[(o.zq * P.nchunk + ch0) * kQCtas + i];
-  }
   // the blocks of zeros before Q's first digit
   for (int t = tid; t < kStages * 2 * (kGroup - 1) * BN; t += kThreads) {
     const int blk = t / ((kGroup - 1) * BN), r = t - blk * ((kGroup - 1) * BN);
@@ -437,6 +423,22 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
     abort_sh = 0;
     issued_sh = 0;
     consumed_sh = INT_MAX;
+  }
+  stream_wait();   // for the digits and what an earlier kernel left in C
+  // a special value in what this CTA reads
+  int special = 0;
+  OzTile o;
+  for (int t = blockIdx.x; t < P.tiles; t += gridDim.x) {
+    if (!oz_tile<BN>(P, t, o)) continue;
+    const int pblocks = (P.p.rows + kPRows - 1) / kPRows;
+    const int ch0 = o.kbeg / kOzChunk, ch1 = (o.kend + kOzChunk - 1) / kOzChunk;
+    for (int i = tid; i < (ch1 - ch0) * (kBM / kPRows); i += kThreads) {
+      const int b = o.r0 / kPRows + i % (kBM / kPRows);
+      if (b < pblocks)
+        special |= P.p.special[((int64_t)o.zp * P.nchunk + ch0 + i / (kBM / kPRows)) * pblocks + b];
+    }
+    for (int i = tid; i < (ch1 - ch0) * kQCtas; i += kThreads)
+      special |= P.q.special[(o.zq * P.nchunk + ch0) * kQCtas + i];
   }
   const auto put = [&](double* c, double x) {
     if (P.scale) x *= P.alpha;
@@ -652,7 +654,7 @@ template <int BN>
 void launch_gemm(OzParams& P, int batch, cudaStream_t s) {
   smem_optin((const void*)oz_gemm_kernel<BN>, OzRing<BN>::kSmem);
   P.tiles = (int)(cdiv(P.p.rows, kBM) * cdiv(P.q.rows, BN) * batch * P.splitk);
-  oz_gemm_kernel<BN><<<P.tiles < num_sms() ? P.tiles : num_sms(), kThreads, OzRing<BN>::kSmem, s>>>(P);
+  launch_early(oz_gemm_kernel<BN>, P.tiles < num_sms() ? P.tiles : num_sms(), kThreads, OzRing<BN>::kSmem, s, P);
   TTGB_CHECK_LAUNCH();
 }
 
@@ -717,8 +719,8 @@ void oz_contract(const ContractDesc& d, int splitk, int kchunk, cudaStream_t s) 
   oz_digits_q_kernel<<<dim3((unsigned)(nchunk * kQCtas), (unsigned)P.q.z), kQCols * 8, 0, s>>>(P.q, d.K, kp,
                                                                                                      kappa);
   TTGB_CHECK_LAUNCH();
-  oz_digits_p_kernel<<<dim3((unsigned)pblocks, (unsigned)nchunk, (unsigned)P.p.z), 256, 0, s>>>(P.p, d.K, kp,
-                                                                                                kappa, P.q.z);
+  launch_early(oz_digits_p_kernel, dim3((unsigned)pblocks, (unsigned)nchunk, (unsigned)P.p.z), 256, 0, s, P.p, d.K,
+               kp, kappa, P.q.z);
   TTGB_CHECK_LAUNCH();
   P.K = d.K; P.kp = kp; P.kchunk = splitk > 1 ? kchunk : d.K; P.splitk = splitk; P.nchunk = nchunk;
   P.swap = qa ? 1 : 0;
