@@ -1,0 +1,46 @@
+"""Rules of the kernel sources that no run can show reliably (no compute: read from the files): a kernel
+launched while the kernel before it drains waits for that one, and reads global memory with plain loads."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "torchtt_gb300", "csrc")
+
+
+def _text(path):
+    text = re.sub(r"//[^\n]*", "", open(path).read())
+    return re.sub(r"/\*.*?\*/", "", text, flags=re.S)
+
+
+def _kernels(text):
+    """name -> (signature, body) of the __global__ functions of a source."""
+    out = {}
+    for m in re.finditer(r"__global__", text):
+        brace = text.index("{", m.end())
+        head = text[m.end():brace]
+        name = re.findall(r"(\w+_kernel)\s*\(", head)[-1]
+        depth, i = 1, brace + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[i], 0)
+            i += 1
+        out[name] = (head, text[brace:i])
+    return out
+
+
+def _early_launches():
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
+        text = _text(path)
+        kernels = _kernels(text)
+        for inc in re.findall(r'#include "(\w+\.cuh)"', text):
+            kernels = {**_kernels(_text(os.path.join(CSRC, inc))), **kernels}
+        for name in sorted(set(re.findall(r"launch_early\(\s*(\w+)", text))):
+            yield pytest.param(name, kernels, id="%s-%s" % (os.path.basename(path), name))
+
+
+@pytest.mark.parametrize("name,kernels", list(_early_launches()))
+def test_early_launched_kernels_wait(name, kernels):
+    head, body = kernels[name]
+    assert "stream_wait();" in body
+    assert "__restrict__" not in head and "__ldg(" not in body

@@ -22,6 +22,7 @@ namespace {
 
 __global__ void scale_cols_kernel(double* X, int64_t ld, int64_t rows, int64_t cols,
                                   const double* S) {
+  stream_wait();
   const int64_t total = rows * cols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
        t += (int64_t)gridDim.x * blockDim.x) {
