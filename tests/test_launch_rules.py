@@ -44,3 +44,11 @@ def test_early_launched_kernels_wait(name, kernels):
     head, body = kernels[name]
     assert "stream_wait();" in body
     assert "__restrict__" not in head and "__ldg(" not in body
+
+
+def test_blocks_decide_together_on_a_flag_of_their_own_launch():
+    """The Arnoldi finishing pass writes the stop flag in one of its blocks while others may still be
+    starting, so a block takes one decision from it for all of its threads."""
+    _, body = _kernels(_text(os.path.join(CSRC, "gmres.cu")))["arnoldi_finish_kernel"]
+    reads = [line.strip() for line in body.splitlines() if "flag[" in line]
+    assert reads == ["if (__syncthreads_or(flag[kGmresState] != 0)) return;"]

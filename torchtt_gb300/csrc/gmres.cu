@@ -458,7 +458,10 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
   __shared__ double dec[3];                 // mode, norm, 1 / norm
   __shared__ double fac;
   stream_wait();
-  if (flag[kGmresState] != 0) return;   // queued past the stopping point: nothing changes
+  // Queued past the stopping point, nothing changes. The extra block may set the flag of this very launch
+  // while a block starts late: the block decides once for all its threads, or some of its warps would go
+  // on without the others' sums.
+  if (__syncthreads_or(flag[kGmresState] != 0)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, k = kv - 1;
   const int G = (int)gridDim.x - 1;   // slices; the block after them takes the Givens step in mode 0
   const bool extra = (int)blockIdx.x == G;
@@ -499,8 +502,8 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
       w[i] = v;
       if (so.hi) put_split(so, i, v);
     }
-    // a block that starts after the flag is set leaves its slice of q unscaled: the cycle has ended
-    // then, and its solution does not use q
+    // a block that starts after the flag is set leaves its slice of q as it is: the cycle has ended then,
+    // and its solution does not use q
     if (extra && warp == 0)
       givens_step(hcol, rot, k, iters, hp, H, cs, sn, beta, threshold, scal, flag, 0);
     return;
