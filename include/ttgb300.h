@@ -72,8 +72,9 @@ typedef struct ttgb_amen_params {
                                    0 auto (double-float accuracy on the MIXED path when
                                    eps >= 1e-9 and A and b fit the FP32 exponent range, ~1e-13
                                    relative: double-float arithmetic on the FP32 pipe, or FP64
-                                   kernels where they are faster; FP64 otherwise), 1 FP64,
-                                   2 double-float accuracy.
+                                   kernels where they are faster; FP64 otherwise, large products
+                                   from digits, see ttgb_fp64_multiply_adds), 1 FP64
+                                   multiply-adds, 2 double-float accuracy.
                                    On the MIXED path with double-float accuracy the GEMMs
                                    of the QR/SVD (CholeskyQR Gram and apply products) have it
                                    too; the factorisations themselves (Cholesky, the Jacobi
@@ -297,6 +298,15 @@ int64_t ttgb_launch_count(void);
 /* Measured peak of this GPU's FMA pipe in TFLOP/s (dtype 0: FP64, 1: FP32): independent FMA
    chains on every SM, best of three timed launches (about 50 ms each). */
 int ttgb_calibrate_fma(int32_t dtype, double* tflops);
+
+/* FP64 products of the calling thread (no counterpart in the reference). By default the large ones are
+   computed from digits on the tensor cores: the error is some 1e-16 of the scale of a row of the
+   left operand times the scale of a column of the right one, below that of multiply-adds, but an
+   element whose own terms lie far below both scales keeps fewer digits than multiply-adds give it.
+   mode 1: multiply-adds only, every element within (K + 2) 2^-53 sum |a b|; 0: the default; any
+   other value only queries. Returns the previous state. A solve has the same choice in fp64_engine,
+   also where another thread runs it (ttgb_server_submit). */
+int ttgb_fp64_multiply_adds(int32_t mode);
 
 /* Tile autotuner of the contraction engine (no counterpart in the reference): the first launch of
    each shape class (engine, power-of-two buckets of M, N, K and batch, triangular flags, unit

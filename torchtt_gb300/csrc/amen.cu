@@ -930,6 +930,7 @@ static int linalg_engine(int fp64_products_engine, double eps) {
 }
 
 AmenResult AmenRun::run(const TTView& x0, const TTView& z0) {
+  NoDigitsScope multiply_adds(p_.fp64_engine == 1);   // every contraction of the solve
   init(x0, z0);
   // every contraction issued by this solve's thread outside the scopes of the FP64 products
   Fp64EngineScope la_engine(mixed_ ? linalg_engine(fp64e_, p_.eps) : kFp64Native);

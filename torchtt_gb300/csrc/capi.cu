@@ -519,6 +519,8 @@ int64_t ttgb_launch_count(void) { return launch_count(); }
 
 int ttgb_autotune(int32_t mode) { return set_autotune(mode); }
 
+int ttgb_fp64_multiply_adds(int32_t mode) { return set_no_digits(mode); }
+
 int64_t ttgb_autotune_classes(void) { return autotune_classes(); }
 
 int ttgb_calibrate_fma(int32_t dtype, double* tflops) {

@@ -399,6 +399,7 @@ AxD to_dev(const Ax& a, int extent) {
 }
 
 thread_local int t_fp64_engine = kFp64Native;
+thread_local bool t_no_digits = false;   // set by NoDigitsScope and set_no_digits
 
 // ---------------------------------------------------------------------------------------------
 // Tile autotuner. A launch is described by its shape class: the engine (FP64, double-float,
@@ -538,13 +539,17 @@ bool componentwise(const ContractDescT<T>& d) {
   return (d.tri & kTriUpperB) != 0;
 }
 
-// Whether candidate t may run d: no digit products for componentwise(d), and no workspace for a caller
-// that must not allocate or whose stream is being captured.
+// Whether d may be a digit product.
+template <typename T>
+bool digits_allowed(const ContractDescT<T>& d) {
+  return std::is_same<T, double>::value && !t_no_digits && !componentwise(d);
+}
+
+// Whether candidate t may run d: no workspace for a caller that must not allocate or whose stream is being
+// captured.
 template <typename T>
 bool usable(const TileCfg& t, const ContractDescT<T>& d, cudaStream_t stream) {
-  if (t.kind == kEmu || t.kind == kOz) {
-    if (componentwise(d)) return false;
-  }
+  if ((t.kind == kEmu || t.kind == kOz) && !digits_allowed(d)) return false;
   if (t.kind != kOz && cdiv(d.M, t.bm) >= 65536) return false;   // rows of tiles in the grid
   if constexpr (std::is_same<T, double>::value) {
     if (t.kind == kOz) {
@@ -632,7 +637,8 @@ void launch_tiles(const ContractDescT<T>& d, KParams<T> p, const TileCfg& t, int
 
 template <typename T>
 uint64_t tune_key(const ContractDescT<T>& d) {
-  const int eng = std::is_same<T, float>::value ? 2 : (t_fp64_engine == kFp64DoubleFloat ? 4 : 3);
+  const int eng = std::is_same<T, float>::value ? 2
+                  : (t_fp64_engine == kFp64DoubleFloat ? 4 : 3) + (t_no_digits ? 2 : 0);
   const int units = (d.am.s0 == 1) | ((d.ak.s0 == 1) << 1) | ((d.bk.s0 == 1) << 2) |
                     ((d.bn.s0 == 1) << 3) | ((d.cm.s0 == 1) << 4);
   uint64_t k = (uint64_t)eng;
@@ -754,8 +760,8 @@ void launch_contract(const ContractDescT<T>& d, cudaStream_t stream, bool determ
   TileCfg t{64, 64, 0};
   if (std::is_same<T, double>::value) {
     const double work = (double)d.M * d.N * d.K * d.batch;
-    if (componentwise(d) ? t_fp64_engine == kFp64DoubleFloat : work > 4e6)
-      t.kind = componentwise(d) ? kDf : kEmu;
+    if (!digits_allowed(d)) t.kind = t_fp64_engine == kFp64DoubleFloat ? kDf : kFma;
+    else if (work > 4e6) t.kind = kEmu;
     t.bm = t.bn = 32;
     // 200 x 300 x 100 (6 M): 22 us either way; 60 x 13440 x 60 (48 M): 40 us with digits made per tile, 29 us
     // with digits made beforehand; 176 x 5632 x 88 (87 M): 60 and 31 us
@@ -795,6 +801,15 @@ int64_t autotune_classes() {
 
 NoTuningScope::NoTuningScope() : prev_(t_no_tuning_runs) { t_no_tuning_runs = true; }
 NoTuningScope::~NoTuningScope() { t_no_tuning_runs = prev_; }
+
+NoDigitsScope::NoDigitsScope(bool on) : prev_(t_no_digits) { t_no_digits = t_no_digits || on; }
+NoDigitsScope::~NoDigitsScope() { t_no_digits = prev_; }
+
+int set_no_digits(int mode) {
+  const int prev = t_no_digits ? 1 : 0;
+  if (mode == 0 || mode == 1) t_no_digits = mode == 1;
+  return prev;
+}
 
 Fp64EngineScope::Fp64EngineScope(int engine) : prev_(t_fp64_engine) { t_fp64_engine = engine; }
 Fp64EngineScope::~Fp64EngineScope() { t_fp64_engine = prev_; }

@@ -45,10 +45,13 @@ constexpr int kTriUpperB = 2;
 using ContractDesc = ContractDescT<double>;
 using ContractDescF = ContractDescT<float>;
 
-// Accuracy of the FP64 contractions issued by the calling thread: kFp64Native computes them at least as
-// accurately as FP64 multiply-adds; kFp64DoubleFloat also admits double-float arithmetic on the FP32
-// pipe (~1e-13 relative, for operands within the FP32 exponent range) where it is the faster.
-// Set for a scope with Fp64EngineScope.
+// Accuracy of the FP64 contractions issued by the calling thread. kFp64Native: FP64 multiply-adds or, for the
+// large ones, digit products (contract_emu.cuh, oz_gemm.cu). Those are more accurate than multiply-adds
+// relative to the scale of a row of A times the scale of a column of B (some 1e-16 of it per K chunk), but not
+// element by element: an element whose own terms lie far below both scales keeps fewer digits than
+// multiply-adds give it. NoDigitsScope leaves them out. kFp64DoubleFloat also admits double-float arithmetic on
+// the FP32 pipe (~1e-13 relative, for operands within the FP32 exponent range) where it is the
+// faster. Set for a scope with Fp64EngineScope.
 constexpr int kFp64Native = 0;
 constexpr int kFp64DoubleFloat = 1;
 struct Fp64EngineScope {
@@ -59,6 +62,20 @@ struct Fp64EngineScope {
  private:
   int prev_;
 };
+
+// Within this scope the calling thread's FP64 contractions are multiply-adds (in FP64, or in double-float
+// where that engine is chosen): every element within (K + 2) 2^-53 sum_k |a_ik b_kj|, in FP64.
+struct NoDigitsScope {
+  explicit NoDigitsScope(bool on = true);
+  ~NoDigitsScope();
+  NoDigitsScope(const NoDigitsScope&) = delete;
+  NoDigitsScope& operator=(const NoDigitsScope&) = delete;
+ private:
+  bool prev_;
+};
+// The calling thread's setting outside such scopes: 1 multiply-adds, 0 any engine, other values only
+// query. Returns the previous one.
+int set_no_digits(int mode);
 
 // Within this scope the calling thread's contractions run no tile-tuning measurements (which
 // synchronise the host): a shape class that already has a record uses it, others the heuristic.

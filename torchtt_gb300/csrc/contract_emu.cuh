@@ -11,10 +11,15 @@
 // column j of B once more by Ec = max_k exponent(b_kj) - Fj - kb(k). An element becomes a signed 62-bit integer, cut into 8 balanced 8-bit digits, which BF16 holds
 // exactly. The products of digits p and q with p + q = d (0 is the leading digit) share one FP32
 // accumulator: at most 8 x 64 products of at most 2^14, below 2^24, so every sum is exact. The digits
-// with p + q <= 7 are used; what is left out is below 2^-60 of the largest |a_ik| |b_kj| of a term, and
-// with the two scales folded together that bound holds for rows and columns of any grading. The
-// eight sums are put together as a 64-bit integer and rounded once to FP64 by integer operations;
-// several chunks (and splits) are added in FP64.
+// with p + q <= 7 are used. The eight sums are put together as a 64-bit integer and rounded once to FP64 by
+// integer operations; several chunks (and splits) are added in FP64.
+//
+// Error of an element: per k up to 2^-57 of 2^(Ei + Fj + Ec) is left out (seven products of 2^14 at weight 2^48 for
+// p + q = 8), and the integer is rounded to 2^-55 of it per chunk. The folded scales follow a grading of
+// rows, of columns and of k, but they are the scales of a whole row and column: where an element's own terms lie
+// far below them it keeps fewer digits than multiply-adds give it. For a row (1, e) of A and columns (e, 1) and
+// (1, e) of B, e = 2^-50, every scale is 1 and the element 2 e keeps 6 bits. NoDigitsScope is for callers whom
+// that concerns.
 //
 // Relative error (2-norm) of random products with K = 30 to 130: 4e-17 to 1e-16, FP64 multiply-adds
 // 1.9e-16 to 3.7e-16; graded rows, columns and opposite gradings of both alike. A chunk with an
@@ -137,10 +142,9 @@ __global__ void __launch_bounds__(EmuTile<BM, BN>::kThreads, EmuTile<BM, BN>::kM
   const int bidx = bz / p.splitk;
   const int ks = bz - bidx * p.splitk;
   const int kbeg = ks * p.kchunk;
-  int kend = min(p.K, kbeg + p.kchunk);
+  const int kend = min(p.K, kbeg + p.kchunk);
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   if ((p.tri & kTriLowerC) && m0 + BM <= n0) return;   // tile strictly above the diagonal
-  if (p.tri & kTriUpperB) kend = min(kend, n0 + BN);   // B(k, n) = 0 for k > n
   const double* A = p.A + (int64_t)bidx * p.a_bs;
   const double* B = p.B + (int64_t)bidx * p.b_bs;
 

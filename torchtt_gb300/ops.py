@@ -3,6 +3,7 @@
 Each function mirrors one reference helper (cited) and runs the library's kernel on the current
 CUDA stream. Shapes follow the reference's tensor layouts.
 """
+import contextlib
 import ctypes
 
 import torch
@@ -161,3 +162,17 @@ def autotune(mode=None):
     L = _lib.lib()
     prev = L.ttgb_autotune(-1 if mode is None else int(bool(mode)))
     return bool(prev), int(L.ttgb_autotune_classes())
+
+
+@contextlib.contextmanager
+def fp64_multiply_adds(on=True):
+    """FP64 products of the calling thread inside this context are multiply-adds: each element is within
+    (K + 2) 2^-53 of the sum of its terms' magnitudes. By default large products are computed from digits
+    on the tensor cores, whose error is relative to a row's scale times a column's. A solve inside the context
+    takes them too; ``solve_cores`` and ``Server.submit`` have the same choice in ``fp64_engine="native"``."""
+    L = _lib.lib()
+    before = L.ttgb_fp64_multiply_adds(int(bool(on)))
+    try:
+        yield
+    finally:
+        L.ttgb_fp64_multiply_adds(before)

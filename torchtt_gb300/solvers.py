@@ -124,7 +124,7 @@ def make_params(nswp=22, eps=1e-10, rmax=32768, max_full=500, kickrank=4, kick2=
                 fp64_engine="auto", strict_eps=False):
     """A ``ttgb_amen_params`` structure from keyword arguments (defaults of the reference).
     ``a_structure=False`` forces the dense contraction of the A cores; ``fp64_engine`` is
-    'auto' (double-float FP64 products on the mixed path), 'native' or 'df'; ``strict_eps``
+    'auto' (double-float FP64 products on the mixed path), 'native' (FP64 multiply-adds) or 'df'; ``strict_eps``
     runs the sweeps at eps / 4 so that the true residual ends at or below eps (the reference's
     rule bounds the local residuals only, and its true residual can end a few times above eps)."""
     p = _lib.AmenParams()
