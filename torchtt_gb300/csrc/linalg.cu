@@ -771,14 +771,16 @@ constexpr int kJacobiBlockMaxN = 160;
 // The lanes' EPL elements of the four columns are loaded before anything is stored, so the loads do not
 // wait for the stores. The rotation is recorded in `worst`.
 //
-// A sweep whose rotations had cosines up to c and sines up to t leaves cosines of about n c t: where that
-// is below the tolerance of n 2^-52 the sweep that would only confirm it is not run. (The cosines alone do
-// not tell: within a cluster of equal norms the angles stay large however small the cosines are.)
+// A rotation of (p, q) adds s |q| / |p| times the cosine of (q, r) to the cosine of (p, r). Where |q| is the larger
+// norm, s |q| / |p| is about the cosine of (p, q); within a cluster of equal norms it is s, which stays large
+// however small the cosines are. So a sweep whose rotations had cosines up to c and sines up to t
+// leaves cosines of about n c max(c, t): where that is below the tolerance of n 2^-52 the sweep that would
+// only confirm it is not run. (Stopping by c t left 4e-12 for three rows 1e6 apart in norm.)
 constexpr int kNoRotation = -4096;
 
 struct JacobiWorst {
   int cosine = kNoRotation, sine = kNoRotation;   // exponents of the largest squares
-  __device__ __forceinline__ bool converged() const { return cosine + sine <= -114; }
+  __device__ __forceinline__ bool converged() const { return cosine + max(cosine, sine) <= -114; }
 };
 
 template <int L, int EPL>
