@@ -52,3 +52,16 @@ def test_blocks_decide_together_on_a_flag_of_their_own_launch():
     _, body = _kernels(_text(os.path.join(CSRC, "gmres.cu")))["arnoldi_finish_kernel"]
     reads = [line.strip() for line in body.splitlines() if "flag[" in line]
     assert reads == ["if (__syncthreads_or(flag[kGmresState] != 0)) return;"]
+
+
+def test_the_lane_that_issues_the_mmas_asks_for_their_completion():
+    """A commit covers the MMAs of the executing thread only, so every commit of the digit product stands in
+    the issuing lane's branches, and the barriers are initialised once."""
+    _, body = _kernels(_text(os.path.join(CSRC, "oz_gemm.cu")))["oz_gemm_kernel"]
+    issuer = body[body.index("elect_one()"):body.index("double* turn")]
+    assert body.count("commit(smem") == issuer.count("commit(smem") == 3
+    for i in (m.start() for m in re.finditer(r"commit\(smem", issuer)):
+        before = issuer[:i]
+        branch = before[before.rindex("if (leader) {"):]
+        assert branch.count("{") > branch.count("}")
+    assert "mbar_init" not in body[body.index("stream_wait();"):]

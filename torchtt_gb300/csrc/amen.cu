@@ -15,6 +15,7 @@
 #include "contract.cuh"
 #include "gmres.cuh"
 #include "linalg.cuh"
+#include "oz_gemm.cuh"
 #include "prec.cuh"
 
 namespace ttgb {
@@ -965,6 +966,7 @@ AmenResult AmenRun::run(const TTView& x0, const TTView& z0) {
   }
   res.ranks = rx_;
   TTGB_CUDA(cudaStreamSynchronize(s_));
+  if (take_wait_error()) throw Error(kTimeout, "FP64 product: a bounded wait gave up");
   if (tc_err_) {
     int herr = 0;
     TTGB_CUDA(cudaMemcpy(&herr, tc_err_, sizeof(int), cudaMemcpyDeviceToHost));

@@ -11,6 +11,7 @@
 #include "contract.cuh"
 #include "gmres.cuh"
 #include "linalg.cuh"
+#include "oz_gemm.cuh"
 #include "prec.cuh"
 #include "tc_gemm.cuh"
 #include "tc_local.cuh"
@@ -25,14 +26,22 @@ namespace {
 
 thread_local std::string g_last_error;
 
+// Status of an entry point. A product whose bounded wait gave up (NaN in its result) is reported by the call that
+// made it where that call waits for the GPU, else by a later call of the same thread.
+int finished(int status) {
+  if (!take_wait_error()) return status;
+  g_last_error = "FP64 product: a bounded wait gave up (now or in an earlier call of this thread)";
+  return TTGB_ERR_TIMEOUT;
+}
+
 template <typename F>
 int guarded(F&& f) {
   try {
     f();
-    return TTGB_OK;
+    return finished(TTGB_OK);
   } catch (const Error& e) {
     g_last_error = e.what();
-    return e.status;
+    return finished(e.status);
   } catch (const std::exception& e) {
     g_last_error = e.what();
     return TTGB_ERR_INTERNAL;

@@ -29,12 +29,16 @@
 // of accumulators, took 46 us for the first. What bounds the product is the tensor pipe (a stage 32 columns wide is 770 clocks of
 // MMAs) and what waits and commits add to it, some 250 clocks per stage; the digit kernels are latency.
 //
-// Every wait is bounded: a CTA whose wait gives up drains its copies and MMAs, frees its tensor memory
-// and writes NaN into its tiles. An infinity, a NaN or a subnormal number in an operand is noted by the
+// Every wait is bounded: a CTA whose wait gives up drains its copies and MMAs (again bounded: the lane that issued
+// the MMAs, which alone can ask for their completion, waits for them before it leaves), frees its tensor
+// memory, writes NaN into its tiles and sets the calling thread's error word, which the entry points turn into
+// a timeout. An infinity, a NaN or a subnormal number in an operand is noted by the
 // digit kernels, and the CTAs that would read it compute their tiles with FP64 multiply-adds instead.
 #include <cooperative_groups.h>
 
+#include <atomic>
 #include <climits>
+#include <mutex>
 
 #include "emu_digits.cuh"
 #include "oz_gemm.cuh"
@@ -312,6 +316,7 @@ struct OzParams {
   int tri;
   int tiles;
   int scale, keep;      // alpha is not 1; beta is not 0
+  int* err;             // set when a wait gave up
   double* C;
   Axis cp, cq;          // C's axes along P's and Q's rows
   int64_t c_bs;
@@ -398,7 +403,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
   constexpr int kPeriod = kOzChunk / kBK;                                  // stages between flushes
   extern __shared__ uint8_t smraw[];
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t full[kStages], empty[kStages], accf[2], acce[2];
+  __shared__ __align__(8) uint64_t full[kStages], empty[kStages], accf[2], acce[2], drained;
   __shared__ uint32_t tmem_sh;
   __shared__ int abort_sh, issued_sh, consumed_sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -419,6 +424,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
       mbar_init(smem_u32(&accf[b]), 1);
       mbar_init(smem_u32(&acce[b]), kFlushWarps);
     }
+    mbar_init(smem_u32(&drained), 1);
     asm volatile("fence.mbarrier_init.release.cluster;");
     abort_sh = 0;
     issued_sh = 0;
@@ -545,6 +551,13 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
         __syncwarp();
       }
     }
+    // the MMAs issued and the arrivals of the commits above are complete when the CTA leaves, also after a
+    // wait that gave up
+    if (leader) {
+      commit(smem_u32(&drained));
+      if (!mbar_wait(smem_u32(&drained), 0u)) atomicExch(&abort_sh, 1);
+    }
+    __syncwarp();
   } else {   // ---- flush: the four warps of a TMEM lane quarter take a quarter of the columns each
     const int q = warp & 3;
     const int cb = (warp - 2) / 4 * kPart;
@@ -625,13 +638,12 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (abort_sh) {
-    if (tid == 0) {   // drain (bounded): copies issued but not consumed, then the MMAs
+    if (tid == 0) {   // copies issued but not consumed (bounded; the MMAs are drained)
       const int issued = issued_sh;
       for (int g = consumed_sh; g < issued; ++g)
         mbar_wait(smem_u32(&full[g % kStages]), (uint32_t)((g / kStages) & 1));
-      mbar_init(smem_u32(&accf[0]), 1);
-      commit(smem_u32(&accf[0]));
-      mbar_wait(smem_u32(&accf[0]), 0u);
+      *(volatile int*)P.err = 1;
+      __threadfence_system();
     }
     __syncthreads();
     for (int t = blockIdx.x; t < P.tiles; t += gridDim.x) {
@@ -660,6 +672,8 @@ void launch_gemm(OzParams& P, int batch, cudaStream_t s) {
 
 bool q_is_a(const ContractDesc& d) { return d.M <= d.N; }   // the smaller operand is Q
 
+thread_local int* t_wait_error = nullptr;   // the thread's word, once it has one
+
 // Tile width: the shorter time of the SM with the most tiles. A stage takes about 620 clocks 16 columns wide,
 // 1020 clocks 32 wide.
 int tile_width(int p_rows, int q_rows, int64_t rest) {
@@ -671,6 +685,31 @@ int tile_width(int p_rows, int q_rows, int64_t rest) {
 }
 
 }  // namespace
+
+// One page of pinned words for the process, dealt to its threads: a word outlives its thread, as a kernel may.
+int* wait_error_word() {
+  constexpr unsigned kWords = 1024;
+  static std::once_flag once;
+  static int* page = nullptr;
+  static std::atomic<unsigned> next{0};
+  if (t_wait_error == nullptr) {
+    std::call_once(once, [] {
+      int* p = nullptr;
+      TTGB_CUDA(cudaHostAlloc((void**)&p, kWords * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+      for (unsigned i = 0; i < kWords; ++i) p[i] = 0;
+      page = p;
+    });
+    t_wait_error = page + next.fetch_add(1) % kWords;
+  }
+  return t_wait_error;
+}
+
+bool take_wait_error() {
+  volatile int* w = t_wait_error;
+  if (w == nullptr || *w == 0) return false;
+  *w = 0;
+  return true;
+}
 
 bool oz_takes(const ContractDesc& d) {
   const int small = d.M < d.N ? d.M : d.N, large = d.M < d.N ? d.N : d.M;
@@ -722,6 +761,7 @@ void oz_contract(const ContractDesc& d, int splitk, int kchunk, cudaStream_t s) 
   launch_early(oz_digits_p_kernel, dim3((unsigned)pblocks, (unsigned)nchunk, (unsigned)P.p.z), 256, 0, s, P.p, d.K,
                kp, kappa, P.q.z);
   TTGB_CHECK_LAUNCH();
+  P.err = wait_error_word();
   P.K = d.K; P.kp = kp; P.kchunk = splitk > 1 ? kchunk : d.K; P.splitk = splitk; P.nchunk = nchunk;
   P.swap = qa ? 1 : 0;
   P.tri = d.tri;

@@ -20,4 +20,10 @@ int64_t oz_tiles(const ContractDesc& d);
 // (which already holds beta C), one range writes alpha A B + beta C.
 void oz_contract(const ContractDesc& d, int splitk, int kchunk, cudaStream_t s);
 
+// The calling host thread's error word (pinned): a kernel launched by it sets the word when one of its bounded
+// waits gave up.
+int* wait_error_word();
+// Whether the word was set, which it then no longer is. Covers the kernels that have completed.
+bool take_wait_error();
+
 }  // namespace ttgb

@@ -17,6 +17,7 @@
 
 #include "../../include/ttgb300.h"
 #include "amen.cuh"
+#include "oz_gemm.cuh"
 #include "solution.cuh"
 
 using namespace ttgb;
@@ -110,8 +111,9 @@ struct ttgb_server {
         req->sol = std::move(sol);
         req->status = TTGB_OK;
       } catch (const Error& e) {
-        req->status = e.status;
-        req->error = e.what();
+        const bool gave_up = take_wait_error();   // the cause where a solve failed on the NaN it left
+        req->status = gave_up ? TTGB_ERR_TIMEOUT : e.status;
+        req->error = gave_up ? "FP64 product: a bounded wait gave up" : e.what();
       } catch (const std::exception& e) {
         req->status = TTGB_ERR_INTERNAL;
         req->error = e.what();
