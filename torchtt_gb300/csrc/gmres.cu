@@ -124,7 +124,8 @@ __global__ void __launch_bounds__(RT) cycle_start_kernel(const double* x, int64_
     }
     scal[kResNorm] = nr;
     beta[0] = nr;
-    flag[kGmresState] = (nr > 0.0) ? 0 : 2;   // 2: r == 0, nothing to do (gmres.h:56-65)
+    // 2: r == 0, nothing to do (gmres.h:56-65); 3: not finite
+    flag[kGmresState] = !isfinite(nr) ? 3 : nr > 0.0 ? 0 : 2;
     flag[kGmresBreakdown] = 0;
     flag[kGmresAtIter] = -1;
     flag[kGmresReorth] = 0;
@@ -417,9 +418,10 @@ __device__ __forceinline__ void givens_step(double* h, const double* rot, int k,
     const double err = fabs(b1) * scal[kRhsInv];
     scal[kErr] = err;
     scal[kHn] = hn;
-    const bool breakdown = !(hn > 0.0) || !isfinite(hn);
+    const bool breakdown = !(hn > 0.0);
     int state = (err <= threshold || breakdown) ? 1 : 0;
-    if (!isfinite(err)) state = 3;
+    // a NaN in the column leaves the rotation the identity and err 0
+    if (!isfinite(err) || !isfinite(den2)) state = 3;
     flag[kGmresBreakdown] = breakdown ? 1 : 0;
     if (state != 0) flag[kGmresAtIter] = k;
     if (reorth_vecs > 0) {
@@ -477,7 +479,7 @@ __global__ void __launch_bounds__(RT) arnoldi_finish_kernel(
       if (!(a < 0.5 * ww) || (a > 0.0 && b <= orth_tol2 * a)) {   // NaN: the Givens step reports it
         mode = 0.0;
         inv = a > 0.0 ? rsqrt_full(a) : 1.0;
-        hp = a > 0.0 ? a * inv : sqrt(a);   // sqrt: 0 or NaN
+        hp = a > 0.0 && isfinite(a) ? a * inv : sqrt(a);   // sqrt: 0, infinite or NaN
       } else if (a > 0.0 && a - b >= 0.5 * a) {
         mode = 1.0;
         inv = rsqrt_full(a - b);
