@@ -1037,7 +1037,9 @@ size_t footprint_bound(const TTView& A, const TTView& b, const TTView& x0, const
   const double local = (double)(p.local_iterations + 1) * nloc + 2.0 * nloc * (double)smax +
                        2.0 * nloc * (double)smax /* split copies, 2 x FP32 */ + 6.0 * nloc +
                        6.0 * r * r + 16.0 * nloc;
-  return (size_t)(8.0 * ((double)A.d * per_core + local)) + ((size_t)64 << 20);
+  // digits of the largest operand of one FP64 product at a time
+  const double operand = std::max(nloc * (double)smax, (double)(smax * smax) * (double)(nmax * nmax));
+  return (size_t)(8.0 * ((double)A.d * per_core + local) + oz_workspace_bound(operand)) + ((size_t)64 << 20);
 }
 
 void randn(double* out, int64_t n, uint64_t seed, uint64_t offset, cudaStream_t s) {

@@ -583,9 +583,7 @@ void launch_emu(const KParams<double>& p, dim3 grid, cudaStream_t stream) {
 }
 
 template <typename T>
-void launch_tiles(const ContractDescT<T>& d, KParams<T> p, const TileCfg& t, int splitk,
-                  cudaStream_t stream) {
-  const int bm = t.bm, bn = t.bn;
+void launch_tiles(const ContractDescT<T>& d, KParams<T> p, TileCfg t, int splitk, cudaStream_t stream) {
   int kchunk = d.K;
   if (splitk > 1) {
     const int unit = t.kind == kOz ? kOzChunk : t.kind == kEmu ? kEmuK : BK;
@@ -603,10 +601,11 @@ void launch_tiles(const ContractDescT<T>& d, KParams<T> p, const TileCfg& t, int
   }
   if constexpr (std::is_same<T, double>::value) {
     if (t.kind == kOz) {
-      oz_contract(d, splitk, kchunk, stream);
-      return;
+      if (oz_contract(d, splitk, kchunk, stream)) return;
+      t = d.M >= d.N ? TileCfg{64, 32, 0, kEmu} : TileCfg{32, 64, 0, kEmu};   // digits made per tile
     }
   }
+  const int bm = t.bm, bn = t.bn;
   dim3 grid(cdiv(d.N, bn), cdiv(d.M, bm), (unsigned)(d.batch * splitk));
   TTGB_REQUIRE(grid.y < 65536 && grid.z < 65536, "contraction grid too large");
   if constexpr (std::is_same<T, double>::value) {
@@ -689,6 +688,15 @@ int tuned_choice(const ContractDescT<T>& d, const KParams<T>& p, cudaStream_t st
       if (e[1]) cudaEventDestroy(e[1]);
     }
   } evs;
+  struct Claim {   // a class whose tuning throws is tuned by a later launch
+    uint64_t key;
+    bool kept = false;
+    ~Claim() {
+      if (kept) return;
+      std::unique_lock<std::shared_mutex> g(g_tune_mu);
+      g_tune_table.erase(key);
+    }
+  } claim{key};
   cudaEvent_t* ev = evs.e;
   TTGB_CUDA(cudaEventCreate(&ev[0]));
   TTGB_CUDA(cudaEventCreate(&ev[1]));
@@ -715,6 +723,7 @@ int tuned_choice(const ContractDescT<T>& d, const KParams<T>& p, cudaStream_t st
     std::unique_lock<std::shared_mutex> g(g_tune_mu);
     g_tune_table[key] = best;
     append_record(key, best);
+    claim.kept = true;
   }
   tuned = true;
   return best;

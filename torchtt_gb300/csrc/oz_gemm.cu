@@ -711,10 +711,62 @@ bool take_wait_error() {
   return true;
 }
 
+namespace {
+
+int64_t align256(int64_t bytes) { return (bytes + 255) / 256 * 256; }
+
+// Operands of d, with Q's digits in blocks of q_blk rows.
+void operands(const ContractDesc& d, int q_blk, Operand& p, Operand& q) {
+  const bool qa = q_is_a(d);
+  Operand a, b;
+  a.base = d.A; a.row = axis(d.am, d.M); a.k = axis(d.ak, d.K); a.bs = d.batch > 1 ? d.a_bs : 0; a.rows = d.M;
+  b.base = d.B; b.row = axis(d.bn, d.N); b.k = axis(d.bk, d.K); b.bs = d.batch > 1 ? d.b_bs : 0; b.rows = d.N;
+  p = qa ? b : a;
+  q = qa ? a : b;
+  // Q's scales enter P's digits, so P has digits per batch entry wherever either operand differs
+  q.z = q.bs != 0 ? d.batch : 1;
+  p.z = (p.bs != 0 || q.bs != 0) ? d.batch : 1;
+  p.blk = kBM;
+  q.blk = q_blk;
+}
+
+// Bytes of the parts of a workspace, each aligned.
+struct Workspace {
+  int64_t dp, dq, sp, sq, kap, fp, fq;
+  Workspace(const Operand& p, const Operand& q, int K) {
+    const int64_t nchunk = cdiv(K, kOzChunk), kp = cdiv(K, kBK) * kBK;
+    const auto digits = [&](const Operand& o) {   // rows in whole blocks
+      return align256((int64_t)o.z * cdiv(o.rows, o.blk) * o.blk * kp * kDig * 2);
+    };
+    dp = digits(p);
+    dq = digits(q);
+    sp = align256((int64_t)p.z * nchunk * p.rows * 4);
+    sq = align256((int64_t)q.z * nchunk * q.rows * 4);
+    kap = align256((int64_t)q.z * nchunk * kOzChunk * 4);
+    fp = align256((int64_t)p.z * nchunk * cdiv(p.rows, kPRows) * 4);
+    fq = align256((int64_t)q.z * nchunk * kQCtas * 4);
+  }
+  int64_t total() const { return dp + dq + sp + sq + kap + fp + fq; }
+};
+
+}  // namespace
+
+// The digits take 16 bytes per element of both operands, with rows in whole blocks and k in whole stages. Where
+// that padding is most of it (short rows in many batch entries), the tensor cores would multiply
+// it as well; and what a solve reserves beforehand has to cover the workspace.
 bool oz_takes(const ContractDesc& d) {
   const int small = d.M < d.N ? d.M : d.N, large = d.M < d.N ? d.N : d.M;
-  return small >= 8 && small <= kMaxQ && d.K >= 16 && (d.tri & kTriUpperB) == 0 &&
-         d.batch < 4096 && (int64_t)large * d.K * d.batch < (int64_t(1) << 25);
+  if (small < 8 || small > kMaxQ || d.K < 16 || (d.tri & kTriUpperB) != 0 || d.batch >= 4096 ||
+      (int64_t)large * d.K * d.batch >= (int64_t(1) << 25))
+    return false;
+  Operand p, q;
+  operands(d, 32, p, q);
+  return Workspace(p, q, d.K).total() <= (int64_t)oz_workspace_bound((double)large * d.K * p.z);
+}
+
+double oz_workspace_bound(double elements) {
+  const double bytes = 48.0 * elements + (double)(1 << 22);
+  return bytes < (double)(1 << 29) ? bytes : (double)(1 << 29);
 }
 
 int64_t oz_tiles(const ContractDesc& d) {
@@ -722,38 +774,28 @@ int64_t oz_tiles(const ContractDesc& d) {
   return (int64_t)cdiv(large, kBM) * cdiv(small, 32) * d.batch;
 }
 
-void oz_contract(const ContractDesc& d, int splitk, int kchunk, cudaStream_t s) {
+bool oz_contract(const ContractDesc& d, int splitk, int kchunk, cudaStream_t s) {
   const bool qa = q_is_a(d);
   OzParams P;
-  Operand a, b;
-  a.base = d.A; a.row = axis(d.am, d.M); a.k = axis(d.ak, d.K); a.bs = d.batch > 1 ? d.a_bs : 0; a.rows = d.M;
-  b.base = d.B; b.row = axis(d.bn, d.N); b.k = axis(d.bk, d.K); b.bs = d.batch > 1 ? d.b_bs : 0; b.rows = d.N;
-  P.p = qa ? b : a;
-  P.q = qa ? a : b;
-  // Q's scales enter P's digits, so P has digits per batch entry wherever either operand differs
-  P.q.z = P.q.bs != 0 ? d.batch : 1;
-  P.p.z = (P.p.bs != 0 || P.q.bs != 0) ? d.batch : 1;
+  operands(d, tile_width(qa ? d.N : d.M, qa ? d.M : d.N, (int64_t)d.batch * splitk), P.p, P.q);
   const int nchunk = (int)cdiv(d.K, kOzChunk);
   const int kp = (d.K + kBK - 1) / kBK * kBK;   // whole stages
-  P.p.blk = kBM;
-  P.q.blk = tile_width(P.p.rows, P.q.rows, (int64_t)d.batch * splitk);
   const int pblocks = (int)cdiv(P.p.rows, kPRows);
-  const auto al = [](int64_t bytes) { return (bytes + 255) / 256 * 256; };
-  const auto digits = [&](const Operand& o) {   // rows in whole blocks
-    return al((int64_t)o.z * cdiv(o.rows, o.blk) * o.blk * kp * kDig * 2);
-  };
-  const int64_t dp = digits(P.p), dq = digits(P.q);
-  const int64_t sp = al((int64_t)P.p.z * nchunk * P.p.rows * 4), sq = al((int64_t)P.q.z * nchunk * P.q.rows * 4);
-  const int64_t kap = al((int64_t)P.q.z * nchunk * kOzChunk * 4);
-  const int64_t fp = al((int64_t)P.p.z * nchunk * pblocks * 4), fq = al((int64_t)P.q.z * nchunk * kQCtas * 4);
-  DevBuf<unsigned char> ws((size_t)(dp + dq + sp + sq + kap + fp + fq), s);
+  const Workspace size(P.p, P.q, d.K);
+  DevBuf<unsigned char> ws;
+  ws.s = s;
+  if (cudaMallocAsync((void**)&ws.p, (size_t)size.total(), s) != cudaSuccess) {
+    cudaGetLastError();   // no memory for the digits: the caller has kernels that need none
+    ws.p = nullptr;
+    return false;
+  }
   unsigned char* w = ws.p;
-  P.p.dig = reinterpret_cast<__nv_bfloat16*>(w); w += dp;
-  P.q.dig = reinterpret_cast<__nv_bfloat16*>(w); w += dq;
-  P.p.scale = reinterpret_cast<int*>(w); w += sp;
-  P.q.scale = reinterpret_cast<int*>(w); w += sq;
-  int* kappa = reinterpret_cast<int*>(w); w += kap;
-  P.p.special = reinterpret_cast<int*>(w); w += fp;
+  P.p.dig = reinterpret_cast<__nv_bfloat16*>(w); w += size.dp;
+  P.q.dig = reinterpret_cast<__nv_bfloat16*>(w); w += size.dq;
+  P.p.scale = reinterpret_cast<int*>(w); w += size.sp;
+  P.q.scale = reinterpret_cast<int*>(w); w += size.sq;
+  int* kappa = reinterpret_cast<int*>(w); w += size.kap;
+  P.p.special = reinterpret_cast<int*>(w); w += size.fp;
   P.q.special = reinterpret_cast<int*>(w);
   oz_digits_q_kernel<<<dim3((unsigned)(nchunk * kQCtas), (unsigned)P.q.z), kQCols * 8, 0, s>>>(P.q, d.K, kp,
                                                                                                      kappa);
@@ -774,6 +816,7 @@ void oz_contract(const ContractDesc& d, int splitk, int kchunk, cudaStream_t s) 
   P.scale = d.alpha != 1.0; P.keep = d.beta != 0.0;
   if (P.q.blk == 32) launch_gemm<32>(P, d.batch, s);
   else launch_gemm<16>(P, d.batch, s);
+  return true;
 }
 
 }  // namespace ttgb

@@ -10,6 +10,10 @@ namespace ttgb {
 // Whether oz_contract takes the contraction.
 bool oz_takes(const ContractDesc& d);
 
+// Upper bound of the workspace of an oz_contract that oz_takes, in bytes: elements is the number of elements of
+// its larger operand (of all batch entries that differ).
+double oz_workspace_bound(double elements);
+
 // K units of its split (a split's range is a multiple of this).
 constexpr int kOzChunk = 128;
 
@@ -18,7 +22,8 @@ int64_t oz_tiles(const ContractDesc& d);
 
 // C (+)= alpha A B as launch_tiles' other kernels: splitk ranges of kchunk are added atomically into C
 // (which already holds beta C), one range writes alpha A B + beta C.
-void oz_contract(const ContractDesc& d, int splitk, int kchunk, cudaStream_t s);
+// False, with nothing launched, when there is no memory for the digits.
+bool oz_contract(const ContractDesc& d, int splitk, int kchunk, cudaStream_t s);
 
 // The calling host thread's error word (pinned): a kernel launched by it sets the word when one of its bounded
 // waits gave up.
