@@ -49,7 +49,8 @@ struct GjScratch {
   float T[2][kGjMaxN * kGjNb];        // transform of the panel, one row per matrix row
   float part[2][kGjCtas][kGjMaxN];    // each CTA's share of inverse * residual
   double r[kGjMaxN];                  // residual
-  float amax[kGjCtas], norm1[kGjCtas];
+  unsigned amax[kGjCtas];             // bits of the largest magnitudes
+  float norm1[kGjCtas];
   int piv[kGjMaxN];                   // pivot row of each column
 };
 
@@ -74,6 +75,7 @@ __global__ void __cluster_dims__(kGjCtas, 1, 1) __launch_bounds__(kGjMaxN, 1)
   __shared__ float rf[kGjMaxN];
   __shared__ double sh[32];
   __shared__ float shf[32];
+  __shared__ unsigned tops[32];
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
@@ -84,31 +86,24 @@ __global__ void __cluster_dims__(kGjCtas, 1, 1) __launch_bounds__(kGjMaxN, 1)
   const int ncol = mine * kGjNb;                                             // own columns
   auto column = [&](int c) { return ((c / kGjNb) * kGjCtas + rank) * kGjNb + c % kGjNb; };
 
-  // the largest magnitude sets a power-of-two scale, so that FP32 holds the scaled entries
-  float mx = 0.f;
+  // the largest magnitude sets a power-of-two scale, so that FP32 holds the scaled entries (compared as
+  // integers: a NaN is above every number)
+  unsigned top = 0u;
   for (int t = tid; t < n * ncol; t += nt) {
     const int i = t / ncol, j = column(t % ncol);
-    if (j < n) {
-      const float v = fabsf((float)B[(int64_t)i * n + j]);
-      mx = (v <= mx) ? mx : v;   // a NaN is taken
-    }
+    if (j < n) top = max(top, __float_as_uint(fabsf((float)B[(int64_t)i * n + j])));
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    const float v = __shfl_xor_sync(0xffffffffu, mx, o);
-    mx = (v <= mx) ? mx : v;
-  }
-  if (lane == 0) shf[warp] = mx;
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) tops[warp] = top;
   __syncthreads();
   if (tid == 0) {
-    for (int w = 0; w < nw; ++w) mx = (shf[w] <= mx) ? mx : shf[w];
-    g->amax[rank] = mx;
+    for (int w = 0; w < nw; ++w) top = max(top, tops[w]);
+    g->amax[rank] = top;
   }
   cluster.sync();
-  mx = 0.f;
-  for (int c = 0; c < kGjCtas; ++c) {
-    const float v = __ldcg(&g->amax[c]);
-    mx = (v <= mx) ? mx : v;
-  }
+  top = 0u;
+  for (int c = 0; c < kGjCtas; ++c) top = max(top, __ldcg(&g->amax[c]));
+  const float mx = __uint_as_float(top);
   if (!(mx > 1e-30f) || !(mx < 1e30f)) {   // zero, not finite, or outside the scale's range
     if (rank == 0 && tid == 0) *fail = 1;
     return;   // the same decision in every thread of the cluster
@@ -253,7 +248,8 @@ __global__ void __cluster_dims__(kGjCtas, 1, 1) __launch_bounds__(kGjMaxN, 1)
   double ri = row < n ? b[row] : 0.0;            // residual of row
   double rp = row < n ? b[prow] : 0.0;           // residual of column row's pivot row
   double rn = block_sum_d(fabs(ri), sh);
-  bool ok = isfinite(rn);
+  // b = 0 is solved by x = 0 only if the matrix is regular, which no residual would tell: left to the LU
+  bool ok = isfinite(rn) && rn > 0.0;
   for (int it = 0; ok && rn > 0.0 && it < kGjMaxRefine; ++it) {
     const int ex = (int)((__double_as_longlong(rn) >> 52) & 0x7ff);
     if (ex < 64 || ex > 1982) { ok = false; break; }
@@ -303,7 +299,6 @@ __global__ void __cluster_dims__(kGjCtas, 1, 1) __launch_bounds__(kGjMaxN, 1)
   const double x1 = block_sum_d(row < n ? fabs(xs[row]) : 0.0, sh);
   // the rounding of x alone leaves about eps ||B||_1 ||x||_1
   ok = ok && isfinite(x1) && rn * scale <= 4.0 * 2.220446049250313e-16 * (double)a1 * x1;
-  if (rn == 0.0) ok = true;
   if (rank == 0) {
     if (row < n) x[row] = xs[row];
     if (tid == 0) *fail = ok ? 0 : 1;
