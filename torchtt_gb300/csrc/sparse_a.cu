@@ -221,11 +221,12 @@ void SparseCore::build(const double* A, int64_t s_, int64_t M_, int64_t N_, int6
   int* rp = row_ptr;
   for (int q = 0; q < kGroupings; ++q) {
     SparseCsr& c = *csr[q];
+    c = SparseCsr();
     c.keys = gs.g[q].keys;
-    c.rp = rp;
+    const int* rows = rp;
     rp += c.keys + 1;
-    if (!((which >> q) & 1u)) continue;
-    c.a = ja; c.b = ja + per; c.val = val; c.val32 = val32;
+    if (!((which >> q) & 1u)) continue;   // its rp stays null: a stage refuses it
+    c.rp = rows; c.a = ja; c.b = ja + per; c.val = val; c.val32 = val32;
     launch_early(sparse_fill_kernel, cdiv(c.keys, kThreads / 32), kThreads, 0, st, A, gs.g[q], c.rp, ja, ja + per, val,
                                                                       val32);
     TTGB_CHECK_LAUNCH();
