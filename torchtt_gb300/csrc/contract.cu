@@ -820,6 +820,7 @@ int set_no_digits(int mode) {
   return prev;
 }
 
+int fp64_engine() { return t_fp64_engine; }
 Fp64EngineScope::Fp64EngineScope(int engine) : prev_(t_fp64_engine) { t_fp64_engine = engine; }
 Fp64EngineScope::~Fp64EngineScope() { t_fp64_engine = prev_; }
 

@@ -54,6 +54,7 @@ using ContractDescF = ContractDescT<float>;
 // faster. Set for a scope with Fp64EngineScope.
 constexpr int kFp64Native = 0;
 constexpr int kFp64DoubleFloat = 1;
+int fp64_engine();
 struct Fp64EngineScope {
   explicit Fp64EngineScope(int engine);
   ~Fp64EngineScope();

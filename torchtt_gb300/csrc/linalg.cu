@@ -1466,6 +1466,9 @@ QRResult qr(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, doubl
   QRResult res;
   res.k = m < n ? m : n;
   if (m <= 0 || n <= 0) return res;
+  // Wide and small factors have FP64 products whatever the engine of the calling thread: the bases of the mixed
+  // path's enrichment are orthonormal to rounding.
+  Fp64EngineScope engine(m < n || (m < 1024 && (double)m * n * n < 4e5) ? kFp64Native : fp64_engine());
   if (m < n && m <= kHouseholderMaxRows) {
     householder(A, lda, m, n, Q, R, ws, s);
     return res;
