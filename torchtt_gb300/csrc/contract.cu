@@ -55,7 +55,14 @@ struct KParams {
   T alpha, beta;
   int scale, keep;   // alpha is not 1, beta not 0: comparing in FP64 costs as much as a multiply-add
   int tri;
+  int tall;   // the tiles' rows run along the grid's first dimension, the only one with more than 65535 blocks
 };
+
+// Row and column of the block's tile among the tiles of C.
+template <typename T>
+__device__ __forceinline__ int2 tile_of(const KParams<T>& p) {
+  return p.tall ? make_int2((int)blockIdx.x, (int)blockIdx.y) : make_int2((int)blockIdx.y, (int)blockIdx.x);
+}
 
 constexpr int BK = 16;
 constexpr int NT = 256;
@@ -72,7 +79,8 @@ __global__ void __launch_bounds__(NT) contract_kernel(KParams<T> p) {
   const int ks = bz - bidx * p.splitk;
   const int kbeg = ks * p.kchunk;
   int kend = min(p.K, kbeg + p.kchunk);
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int2 tile = tile_of(p);
+  const int m0 = tile.x * BM, n0 = tile.y * BN;
   if ((p.tri & kTriLowerC) && m0 + BM <= n0) {   // tile strictly above the diagonal
     stream_wait();
     return;
@@ -183,7 +191,8 @@ __global__ void __launch_bounds__(NT) contract_small_kernel(KParams<double> p) {
   const int ks = bz - bidx * p.splitk;
   const int kbeg = ks * p.kchunk;
   int kend = min(p.K, kbeg + p.kchunk);
-  const int m0 = blockIdx.y * BS, n0 = blockIdx.x * BS;
+  const int2 tile = tile_of(p);
+  const int m0 = tile.x * BS, n0 = tile.y * BS;
   if (p.tri & kTriUpperB) kend = min(kend, n0 + BS);   // B(k, n) = 0 for k > n
   const bool skip = (p.tri & kTriLowerC) && m0 + BS <= n0;   // tile strictly above the diagonal
   // loader: thread (row or column, k) of the chunk
@@ -246,7 +255,8 @@ __global__ void __launch_bounds__(NT) contract_df_kernel(KParams<double> p) {
   const int ks = bz - bidx * p.splitk;
   const int kbeg = ks * p.kchunk;
   int kend = min(p.K, kbeg + p.kchunk);
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int2 tile = tile_of(p);
+  const int m0 = tile.x * BM, n0 = tile.y * BN;
   if ((p.tri & kTriLowerC) && m0 + BM <= n0) return;
   if (p.tri & kTriUpperB) kend = min(kend, n0 + BN);
 
@@ -550,7 +560,7 @@ bool digits_allowed(const ContractDescT<T>& d) {
 template <typename T>
 bool usable(const TileCfg& t, const ContractDescT<T>& d, cudaStream_t stream) {
   if ((t.kind == kEmu || t.kind == kOz) && !digits_allowed(d)) return false;
-  if (t.kind != kOz && cdiv(d.M, t.bm) >= 65536) return false;   // rows of tiles in the grid
+  if (t.kind != kOz && std::min(cdiv(d.M, t.bm), cdiv(d.N, t.bn)) >= 65536) return false;   // tiles in the grid
   if constexpr (std::is_same<T, double>::value) {
     if (t.kind == kOz) {
       cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -607,6 +617,8 @@ void launch_tiles(const ContractDescT<T>& d, KParams<T> p, TileCfg t, int splitk
   }
   const int bm = t.bm, bn = t.bn;
   dim3 grid(cdiv(d.N, bn), cdiv(d.M, bm), (unsigned)(d.batch * splitk));
+  p.tall = grid.y >= 65536;
+  if (p.tall) std::swap(grid.x, grid.y);
   TTGB_REQUIRE(grid.y < 65536 && grid.z < 65536, "contraction grid too large");
   if constexpr (std::is_same<T, double>::value) {
     if (t.kind == kEmu) {

@@ -143,7 +143,8 @@ __global__ void __launch_bounds__(EmuTile<BM, BN>::kThreads, EmuTile<BM, BN>::kM
   const int ks = bz - bidx * p.splitk;
   const int kbeg = ks * p.kchunk;
   const int kend = min(p.K, kbeg + p.kchunk);
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int2 tile = tile_of(p);
+  const int m0 = tile.x * BM, n0 = tile.y * BN;
   if ((p.tri & kTriLowerC) && m0 + BM <= n0) return;   // tile strictly above the diagonal
   const double* A = p.A + (int64_t)bidx * p.a_bs;
   const double* B = p.B + (int64_t)bidx * p.b_bs;
