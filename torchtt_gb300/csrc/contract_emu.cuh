@@ -23,8 +23,8 @@
 //
 // Relative error (2-norm) of random products with K = 30 to 130: 4e-17 to 1e-16, FP64 multiply-adds
 // 1.9e-16 to 3.7e-16; graded rows, columns and opposite gradings of both alike. A chunk with an
-// infinity, a NaN or a subnormal number is computed with FP64 multiply-adds, so these go through as
-// before.
+// infinity or a NaN is computed with FP64 multiply-adds, so these go through; subnormal numbers have digits as
+// any others.
 //
 // Measured (M = 322, N = 5024, K = 161): 130 us against 513 us for FP64 multiply-adds in 32 x 32 tiles, which
 // ran at 80% of the FP64 pipe. The tensor pipe is 25% busy; what bounds the kernel is the integer work of
@@ -85,6 +85,14 @@ struct EmuLoader {
     part = tid / ROWS;
     ok = r0 + row < extent;
     off = ok ? ax_off(ax, r0 + row) : 0;
+  }
+  __device__ __forceinline__ bool nonfinite() const {
+    bool r = false;
+#pragma unroll
+    for (int q = 0; q < kQuads; ++q)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) r |= emu_nonfinite(v[q][i]);
+    return r;
   }
   __device__ __forceinline__ int k(int q) const { return (part + q * kPer) * 4; }
   // Loads the chunk of len elements at k0; true when an element is special.
@@ -172,7 +180,8 @@ __global__ void __launch_bounds__(EmuTile<BM, BN>::kThreads, EmuTile<BM, BN>::kM
     for (int i = tid; i < BM; i += NTH) emax_a[par][i] = kEmuZero;
     for (int i = tid; i < BN; i += NTH) { fmax_b[par][i] = kEmuZero; emax_b[par][i] = kEmuZero; }
     // the previous chunk's digits have been read, this chunk's scales are cleared
-    if (__syncthreads_or(special ? 1 : 0)) {   // rare: infinities, NaN or subnormals in the chunk
+    const bool rare = __syncthreads_or(special ? 1 : 0) != 0;   // infinities, NaN or subnormals in the chunk
+    if (rare && __syncthreads_or(la.nonfinite() | lb.nonfinite() ? 1 : 0)) {
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -187,86 +196,91 @@ __global__ void __launch_bounds__(EmuTile<BM, BN>::kThreads, EmuTile<BM, BN>::kM
         }
       continue;
     }
-    int mb = kEmuZero;
+    const auto make_digits = [&](auto sub) {
+      constexpr bool kSub = decltype(sub)::value;
+      int mb = kEmuZero;
 #pragma unroll
-    for (int q = 0; q < lb.kQuads; ++q)
+      for (int q = 0; q < lb.kQuads; ++q)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) mb = max(mb, emu_exponent(lb.v[q][i]));
-    atomicMax(&fmax_b[par][lb.row], mb);
-    __syncthreads();
-    const int F = fmax_b[par][lb.row];
-#pragma unroll
-    for (int q = 0; q < lb.kQuads; ++q) {
-      if (q * lb.kPer * 4 >= len) break;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        constexpr bool kHalf = BN < 32;   // lanes of a half warp share k
-        const int e = emu_exponent(lb.v[q][i]);
-        const int m = __reduce_max_sync(kHalf ? 0xffffu << (lane & 16) : 0xffffffffu,
-                                        e == kEmuZero ? kEmuZero : e - F);
-        if ((lane & (kHalf ? 15 : 31)) == 0) atomicMax(&kmax[par][lb.k(q) + i], m);
-      }
-    }
-    __syncthreads();
-    auto kb = [&](int k, int (&out)[4]) {
-      const int4 m = *reinterpret_cast<const int4*>(&kmax[par][k]);
-      out[0] = m.x; out[1] = m.y; out[2] = m.z; out[3] = m.w;
-    };
-    // a row k of B that is zero (kb = kEmuZero) takes column k of A out of the scale; a zero of A or
-    // B stays more than 2^11 below any other exponent
-    int ma = 2 * kEmuZero;
-    mb = kEmuZero;
-#pragma unroll
-    for (int q = 0; q < la.kQuads; ++q) {
-      if (q * la.kPer * 4 >= len) break;
-      int b[4];
-      kb(la.k(q), b);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) ma = max(ma, emu_exponent(la.v[q][i]) + b[i]);
-    }
-#pragma unroll
-    for (int q = 0; q < lb.kQuads; ++q) {
-      if (q * lb.kPer * 4 >= len) break;
-      int b[4];
-      kb(lb.k(q), b);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int e = emu_exponent(lb.v[q][i]);
-        mb = max(mb, e == kEmuZero ? kEmuZero : e - F - b[i]);
-      }
-    }
-    atomicMax(&emax_a[par][la.row], ma);
-    atomicMax(&emax_b[par][lb.row], mb);
-    __syncthreads();
-    {
-      const int E = emax_a[par][la.row];
-#pragma unroll
-      for (int q = 0; q < la.kQuads; ++q) {
-        if (q * la.kPer * 4 >= len16) break;
-        int b[4];
-        uint2 y[4];
-        kb(la.k(q), b);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          y[i] = fixed_digits(la.v[q][i], emu_exponent(la.v[q][i]) + b[i], E);
-        store_digits(y, As + (size_t)la.row * kEmuPitch + la.k(q), BM);
-      }
-      const int G = emax_b[par][lb.row];
+        for (int i = 0; i < 4; ++i) mb = max(mb, emu_exponent<kSub>(lb.v[q][i]));
+      atomicMax(&fmax_b[par][lb.row], mb);
+      __syncthreads();
+      const int F = fmax_b[par][lb.row];
 #pragma unroll
       for (int q = 0; q < lb.kQuads; ++q) {
-        if (q * lb.kPer * 4 >= len16) break;
+        if (q * lb.kPer * 4 >= len) break;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          constexpr bool kHalf = BN < 32;   // lanes of a half warp share k
+          const int e = emu_exponent<kSub>(lb.v[q][i]);
+          const int m = __reduce_max_sync(kHalf ? 0xffffu << (lane & 16) : 0xffffffffu,
+                                          e == kEmuZero ? kEmuZero : e - F);
+          if ((lane & (kHalf ? 15 : 31)) == 0) atomicMax(&kmax[par][lb.k(q) + i], m);
+        }
+      }
+      __syncthreads();
+      auto kb = [&](int k, int (&out)[4]) {
+        const int4 m = *reinterpret_cast<const int4*>(&kmax[par][k]);
+        out[0] = m.x; out[1] = m.y; out[2] = m.z; out[3] = m.w;
+      };
+      // a row k of B that is zero (kb = kEmuZero) takes column k of A out of the scale; a zero of A or
+      // B stays more than 2^11 below any other exponent
+      int ma = 2 * kEmuZero;
+      mb = kEmuZero;
+#pragma unroll
+      for (int q = 0; q < la.kQuads; ++q) {
+        if (q * la.kPer * 4 >= len) break;
         int b[4];
-        uint2 y[4];
+        kb(la.k(q), b);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ma = max(ma, emu_exponent<kSub>(la.v[q][i]) + b[i]);
+      }
+#pragma unroll
+      for (int q = 0; q < lb.kQuads; ++q) {
+        if (q * lb.kPer * 4 >= len) break;
+        int b[4];
         kb(lb.k(q), b);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int e = emu_exponent(lb.v[q][i]);
-          y[i] = fixed_digits(lb.v[q][i], e == kEmuZero ? kEmuZero : e - F - b[i], G);
+          const int e = emu_exponent<kSub>(lb.v[q][i]);
+          mb = max(mb, e == kEmuZero ? kEmuZero : e - F - b[i]);
         }
-        store_digits(y, Bs + (size_t)lb.row * kEmuPitch + lb.k(q), BN);
       }
-    }
-    __syncthreads();
+      atomicMax(&emax_a[par][la.row], ma);
+      atomicMax(&emax_b[par][lb.row], mb);
+      __syncthreads();
+      {
+        const int E = emax_a[par][la.row];
+#pragma unroll
+        for (int q = 0; q < la.kQuads; ++q) {
+          if (q * la.kPer * 4 >= len16) break;
+          int b[4];
+          uint2 y[4];
+          kb(la.k(q), b);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            y[i] = fixed_digits<kSub>(la.v[q][i], emu_exponent<kSub>(la.v[q][i]) + b[i], E);
+          store_digits(y, As + (size_t)la.row * kEmuPitch + la.k(q), BM);
+        }
+        const int G = emax_b[par][lb.row];
+#pragma unroll
+        for (int q = 0; q < lb.kQuads; ++q) {
+          if (q * lb.kPer * 4 >= len16) break;
+          int b[4];
+          uint2 y[4];
+          kb(lb.k(q), b);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int e = emu_exponent<kSub>(lb.v[q][i]);
+            y[i] = fixed_digits<kSub>(lb.v[q][i], e == kEmuZero ? kEmuZero : e - F - b[i], G);
+          }
+          store_digits(y, Bs + (size_t)lb.row * kEmuPitch + lb.k(q), BN);
+        }
+      }
+      __syncthreads();
+    };
+    if (rare) make_digits(std::true_type());
+    else make_digits(std::false_type());
     if (!work) continue;
     // one n8 half of the warp's tile at a time: its eight accumulators and B digits stay in registers
 #pragma unroll

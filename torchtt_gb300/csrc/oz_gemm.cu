@@ -32,13 +32,14 @@
 // Every wait is bounded: a CTA whose wait gives up drains its copies and MMAs (again bounded: the lane that issued
 // the MMAs, which alone can ask for their completion, waits for them before it leaves), frees its tensor
 // memory, writes NaN into its tiles and sets the calling thread's error word, which the entry points turn into
-// a timeout. An infinity, a NaN or a subnormal number in an operand is noted by the
+// a timeout. An infinity or a NaN in an operand is noted by the
 // digit kernels, and the CTAs that would read it compute their tiles with FP64 multiply-adds instead.
 #include <cooperative_groups.h>
 
 #include <atomic>
 #include <climits>
 #include <mutex>
+#include <type_traits>
 
 #include "emu_digits.cuh"
 #include "oz_gemm.cuh"
@@ -135,6 +136,14 @@ __device__ __forceinline__ bool load_row(double (&v)[PER], const Operand& o, int
   return special;
 }
 
+template <int PER>
+__device__ __forceinline__ bool nonfinite(const double (&v)[PER]) {
+  bool r = false;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) r |= emu_nonfinite(v[i]);
+  return r;
+}
+
 // Digits of Q, one cluster per chunk of 128 k and batch entry: thread (column, eighth of the chunk).
 // Scales: Fj the column's largest exponent, kappa(k) the largest that Fj leaves in row k of Q over all
 // columns (a maximum over the cluster). kappa(k) is 0 where column j has its largest element and never
@@ -155,50 +164,55 @@ __global__ void __cluster_dims__(kQCtas, 1, 1) __launch_bounds__(kQCols * 8)
   if (tid < kQCols) f[tid] = kEmuZero;
   if (tid < kOzChunk) km[tid] = kEmuZero;
   double v[kPer];
-  const bool special = load_row(v, q, z, j, ok, k0, K);
-  const int any = __syncthreads_or(special ? 1 : 0);
+  const bool rare = __syncthreads_or(load_row(v, q, z, j, ok, k0, K) ? 1 : 0) != 0;
+  const int any = rare && __syncthreads_or(nonfinite(v) ? 1 : 0);
   if (tid == 0) q.special[(z * nchunk + chunk) * kQCtas + rank] = any;
-  int mx = kEmuZero;
+  const auto digits = [&](auto sub) {
+    constexpr bool kSub = decltype(sub)::value;
+    int mx = kEmuZero;
 #pragma unroll
-  for (int i = 0; i < kPer; ++i) mx = max(mx, emu_exponent(v[i]));
-  atomicMax(&f[c], mx);
-  __syncthreads();
-  const int F = f[c];
-  int mine = kEmuZero;   // lane i: the maximum of k0 + i over the warp's columns
+    for (int i = 0; i < kPer; ++i) mx = max(mx, emu_exponent<kSub>(v[i]));
+    atomicMax(&f[c], mx);
+    __syncthreads();
+    const int F = f[c];
+    int mine = kEmuZero;   // lane i: the maximum of k0 + i over the warp's columns
 #pragma unroll
-  for (int i = 0; i < kPer; ++i) {
-    const int e = emu_exponent(v[i]);
-    const int m = __reduce_max_sync(0xffffffffu, e == kEmuZero ? kEmuZero : e - F);
-    if (lane == i) mine = m;
-  }
-  if (lane < kPer) atomicMax(&km[part * kPer + lane], mine);
-  cluster.sync();
-  if (tid < kOzChunk) {
-    int m = kEmuZero;
-#pragma unroll
-    for (int r = 0; r < kQCtas; ++r) m = max(m, cluster.map_shared_rank(km, r)[tid]);
-    kall[tid] = m;
-    if (rank == 0) kappa[((int64_t)z * nchunk + chunk) * kOzChunk + tid] = m;
-  }
-  __syncthreads();
-  if (ok) {
-    if (part == 0) q.scale[((int64_t)z * nchunk + chunk) * q.rows + j] = F;
-    const int64_t pitch = (int64_t)q.blk * 8;
-    __nv_bfloat16* p = digit_ptr(q, kp, z, j, k0);
-#pragma unroll
-    for (int o = 0; o < kPer / 8; ++o) {
-      if (k0 >= kp) break;   // kp is a multiple of 16
-      uint2 y[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const double x = v[8 * o + i];
-        const int e = emu_exponent(x);
-        y[i] = fixed_digits(x, e == kEmuZero ? kEmuZero : e - F - kall[part * kPer + 8 * o + i], 0);
-      }
-      put8(y, p + o * kDig * pitch, pitch);
+    for (int i = 0; i < kPer; ++i) {
+      const int e = emu_exponent<kSub>(v[i]);
+      const int m = __reduce_max_sync(0xffffffffu, e == kEmuZero ? kEmuZero : e - F);
+      if (lane == i) mine = m;
     }
-  }
-  cluster.sync();   // no CTA leaves while another may still read its maxima
+    if (lane < kPer) atomicMax(&km[part * kPer + lane], mine);
+    cluster.sync();
+    if (tid < kOzChunk) {
+      int m = kEmuZero;
+#pragma unroll
+      for (int r = 0; r < kQCtas; ++r) m = max(m, cluster.map_shared_rank(km, r)[tid]);
+      kall[tid] = m;
+      if (rank == 0) kappa[((int64_t)z * nchunk + chunk) * kOzChunk + tid] = m;
+    }
+    __syncthreads();
+    if (ok) {
+      if (part == 0) q.scale[((int64_t)z * nchunk + chunk) * q.rows + j] = F;
+      const int64_t pitch = (int64_t)q.blk * 8;
+      __nv_bfloat16* p = digit_ptr(q, kp, z, j, k0);
+#pragma unroll
+      for (int o = 0; o < kPer / 8; ++o) {
+        if (k0 >= kp) break;   // kp is a multiple of 16
+        uint2 y[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const double x = v[8 * o + i];
+          const int e = emu_exponent<kSub>(x);
+          y[i] = fixed_digits<kSub>(x, e == kEmuZero ? kEmuZero : e - F - kall[part * kPer + 8 * o + i], 0);
+        }
+        put8(y, p + o * kDig * pitch, pitch);
+      }
+    }
+    cluster.sync();   // no CTA leaves while another may still read its maxima
+  };
+  if (rare) digits(std::true_type());
+  else digits(std::false_type());
 }
 
 // Digits of P: 32 rows of one chunk per CTA, thread (row, eighth of the chunk). Scale: the row's largest
@@ -217,28 +231,33 @@ __global__ void __launch_bounds__(256) oz_digits_p_kernel(Operand p, int K, int 
   if (tid < kPRows) emax[tid] = kEmuZero;
   if (tid < kOzChunk) kk[tid] = kappa[((int64_t)(kappa_z > 1 ? z : 0) * nchunk + chunk) * kOzChunk + tid];
   double v[kPer];
-  const bool special = load_row(v, p, z, i, ok, k0, K);
-  const int any = __syncthreads_or(special ? 1 : 0);
+  const bool rare = __syncthreads_or(load_row(v, p, z, i, ok, k0, K) ? 1 : 0) != 0;
+  const int any = rare && __syncthreads_or(nonfinite(v) ? 1 : 0);
   if (tid == 0) p.special[((int64_t)z * nchunk + chunk) * gridDim.x + blockIdx.x] = any;
-  int mx = 2 * kEmuZero;
+  const auto digits = [&](auto sub) {
+    constexpr bool kSub = decltype(sub)::value;
+    int mx = 2 * kEmuZero;
 #pragma unroll
-  for (int q = 0; q < kPer; ++q) mx = max(mx, emu_exponent(v[q]) + kk[part * kPer + q]);
-  atomicMax(&emax[c], mx);
-  __syncthreads();
-  if (!ok) return;
-  const int E = emax[c];
-  if (part == 0) p.scale[((int64_t)z * nchunk + chunk) * p.rows + i] = E;
-  const int64_t pitch = (int64_t)p.blk * 8;
-  __nv_bfloat16* d = digit_ptr(p, kp, z, i, k0);
+    for (int q = 0; q < kPer; ++q) mx = max(mx, emu_exponent<kSub>(v[q]) + kk[part * kPer + q]);
+    atomicMax(&emax[c], mx);
+    __syncthreads();
+    if (!ok) return;
+    const int E = emax[c];
+    if (part == 0) p.scale[((int64_t)z * nchunk + chunk) * p.rows + i] = E;
+    const int64_t pitch = (int64_t)p.blk * 8;
+    __nv_bfloat16* d = digit_ptr(p, kp, z, i, k0);
 #pragma unroll
-  for (int o = 0; o < kPer / 8; ++o) {
-    if (k0 >= kp) break;   // kp is a multiple of 16
-    uint2 y[8];
+    for (int o = 0; o < kPer / 8; ++o) {
+      if (k0 >= kp) break;   // kp is a multiple of 16
+      uint2 y[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-      y[q] = fixed_digits(v[8 * o + q], emu_exponent(v[8 * o + q]) + kk[part * kPer + 8 * o + q], E);
-    put8(y, d + o * kDig * pitch, pitch);
-  }
+      for (int q = 0; q < 8; ++q)
+        y[q] = fixed_digits<kSub>(v[8 * o + q], emu_exponent<kSub>(v[8 * o + q]) + kk[part * kPer + 8 * o + q], E);
+      put8(y, d + o * kDig * pitch, pitch);
+    }
+  };
+  if (rare) digits(std::true_type());
+  else digits(std::false_type());
 }
 
 // ---- product ---------------------------------------------------------------------------------------
