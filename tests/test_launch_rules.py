@@ -65,3 +65,11 @@ def test_the_lane_that_issues_the_mmas_asks_for_their_completion():
         branch = before[before.rindex("if (leader) {"):]
         assert branch.count("{") > branch.count("}")
     assert "mbar_init" not in body[body.index("stream_wait();"):]
+
+
+def test_kernels_called_in_place_promise_nothing():
+    """jacobi_columns passes one buffer as the input and the output of the cluster Jacobi."""
+    text = _text(os.path.join(CSRC, "linalg.cu"))
+    launch = re.search(r"jacobi_block_kernel<EPL><<<[^>]*>>>\((\w+), n, (\w+),", text)
+    assert launch.group(1) == launch.group(2)
+    assert "__restrict__" not in _kernels(text)["jacobi_block_kernel"][0]

@@ -932,7 +932,7 @@ __global__ void __launch_bounds__(32) jacobi_warp_kernel(const double* R, int n,
 
 template <int EPL>
 __global__ void __cluster_dims__(kJacobiCluster, 1, 1) __launch_bounds__(256)
-    jacobi_block_kernel(const double* __restrict__ Win, int n, double* Wout, double* Vout, int max_sweeps,
+    jacobi_block_kernel(const double* Win, int n, double* Wout, double* Vout, int max_sweeps,
                         int* status) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   double* sm = reinterpret_cast<double*>(sm_raw);
