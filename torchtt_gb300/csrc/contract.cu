@@ -663,7 +663,8 @@ uint64_t tune_key(const ContractDescT<T>& d) {
   return k;
 }
 
-// Returns the candidate index to use, tuning the class first when this launch may be repeated.
+// Returns the candidate index to use, tuning the class first when this launch may be repeated (a record of a file
+// that names no candidate counts as none).
 // -1: use the heuristic. A tuned launch has already written C (tuned = true).
 template <typename T>
 int tuned_choice(const ContractDescT<T>& d, const KParams<T>& p, cudaStream_t stream,
@@ -680,12 +681,12 @@ int tuned_choice(const ContractDescT<T>& d, const KParams<T>& p, cudaStream_t st
   {
     std::shared_lock<std::shared_mutex> g(g_tune_mu);
     auto it = g_tune_table.find(key);
-    if (it != g_tune_table.end()) return it->second < cand.n ? it->second : -1;
+    if (it != g_tune_table.end() && it->second < cand.n) return it->second;
   }
   {
     std::unique_lock<std::shared_mutex> g(g_tune_mu);
     auto it = g_tune_table.find(key);
-    if (it != g_tune_table.end()) return it->second < cand.n ? it->second : -1;
+    if (it != g_tune_table.end() && it->second < cand.n) return it->second;
     if (t_no_tuning_runs) return -1;   // a caller that must not block: heuristic tile
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)
