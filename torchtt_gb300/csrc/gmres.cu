@@ -6,6 +6,7 @@
 
 #include "gmres.cuh"
 #include "reduce.cuh"
+#include "rsqrt.cuh"
 #include "tc_gemm.cuh"
 
 namespace ttgb {
@@ -62,7 +63,6 @@ namespace {
 
 using red::RT;
 using red::block_sum;
-using red::rsqrt_full;
 constexpr int kMaxVec = 128;   // basis vectors a cycle may hold (RedWS::cap_vec + 1)
 
 // scalar slots after the Hessenberg data in GmresWS::small

@@ -13,6 +13,7 @@
 
 #include "contract.cuh"
 #include "linalg.cuh"
+#include "rsqrt.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -135,13 +136,6 @@ constexpr int kCholNb = 16;
 constexpr double kNearIdentity = 1e-9;   // max |G - I| below which the first-order factor is used
 constexpr double kPivotTol = 1e-11;
 
-// 1 / sqrt(d) for d in the FP32 range: y from FP32, y (1 + e / 2 + 3 e^2 / 8) with e = 1 - d y^2
-__device__ __forceinline__ double rsqrt_refined(double d) {
-  const double y = (double)rsqrtf((float)d);
-  const double e = fma(-d * y, y, 1.0);
-  return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
 // Largest |G - I| and largest diagonal entry of an upper triangle by their high words (upper bounds
 // within 2^-20; 1e300 for an infinity or a NaN), and the trace. FP64 comparisons and block-wide FP64
 // reductions would hold the FP64 pipe for microseconds; these are integer maxima.
@@ -202,87 +196,87 @@ struct CholShared {
 __device__ void chol_panels(double* A, int n, double floor_d, CholShared& ch) {
   const int ld = n + 1;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-      for (int j0 = 0; j0 < n; j0 += kCholNb) {
-        const int w = min(kCholNb, n - j0);
-        {   // [R_JJ | L_JJ^{-1}] of the diagonal block: element (i, c) = (warp, lane)
-          const int i = warp, c = lane;
-          double v = (i == (c & 15)) ? 1.0 : 0.0;   // also the padding of the last panel
-          if (c < w && i < w) v = c >= i ? A[(j0 + i) * ld + j0 + c] : A[(j0 + c) * ld + j0 + i];
-  #pragma unroll 1
-          for (int j = 0; j < w; ++j) {
-            if (i == j) {
-              const double d = __shfl_sync(0xffffffffu, v, j);
-              // d > floor_d >= 0 and finite, as integers: an FP64 comparison is a round trip to a busy pipe
-              const long long bits = __double_as_longlong(d);
-              if (bits <= __double_as_longlong(floor_d) || bits >= 0x7ff0000000000000ll)
-                ch.bad = 1;   // the same in every lane
-              v *= rsqrt_refined(d);
-              ch.rowbuf[j & 1][c] = v;
-            }
-            __syncthreads();
-            if (i > j) v = fma(-ch.rowbuf[j & 1][i], ch.rowbuf[j & 1][c], v);
-          }
-          if (i < w) {
-            if (c < w && c >= i) A[(j0 + i) * ld + j0 + c] = v;
-            if (c >= kCholNb) {
-              const int q = c - kCholNb;
-              ch.Ls[i][q] = v;   // zero above the diagonal
-              if (q < i) A[(j0 + i) * ld + j0 + q] = v;
-              if (q == i) ch.xd[j0 + i] = v;
-            }
-          }
+  for (int j0 = 0; j0 < n; j0 += kCholNb) {
+    const int w = min(kCholNb, n - j0);
+    {   // [R_JJ | L_JJ^{-1}] of the diagonal block: element (i, c) = (warp, lane)
+      const int i = warp, c = lane;
+      double v = (i == (c & 15)) ? 1.0 : 0.0;   // also the padding of the last panel
+      if (c < w && i < w) v = c >= i ? A[(j0 + i) * ld + j0 + c] : A[(j0 + c) * ld + j0 + i];
+#pragma unroll 1
+      for (int j = 0; j < w; ++j) {
+        if (i == j) {
+          const double d = __shfl_sync(0xffffffffu, v, j);
+          // d > floor_d >= 0 and finite, as integers: an FP64 comparison is a round trip to a busy pipe
+          const long long bits = __double_as_longlong(d);
+          if (bits <= __double_as_longlong(floor_d) || bits >= 0x7ff0000000000000ll)
+            ch.bad = 1;   // the same in every lane
+          v *= rsqrt_refined(d);
+          ch.rowbuf[j & 1][c] = v;
         }
         __syncthreads();
-        if (ch.bad) return;
-        {   // the panel's rows of the other columns: L_JJ^{-1} [X | G]
-          const int cols = n - w;
-          constexpr int kPer = kCholNb * kCholSmemMax / 512;
-          double y[kPer];
-  #pragma unroll
-          for (int u = 0; u < kPer; ++u) {
-            const int t = tid + u * 512;
-            double sum = 0.0;
-            if (t < w * cols) {
-              const int i = t / cols, q = t - i * cols;
-              const double* col = A + j0 * ld + (q < j0 ? q : q + w);
-              for (int k = 0; k <= i; ++k) sum = fma(ch.Ls[i][k], col[k * ld], sum);
-            }
-            y[u] = sum;
-          }
-          __syncthreads();
-  #pragma unroll
-          for (int u = 0; u < kPer; ++u) {
-            const int t = tid + u * 512;
-            if (t < w * cols) {
-              const int i = t / cols, q = t - i * cols;
-              A[(j0 + i) * ld + (q < j0 ? q : q + w)] = y[u];
-            }
-          }
-        }
-        __syncthreads();
-        // rows below: columns left of the panel and the panel's own (L^{-1}), and from the diagonal on (G)
-        const int r0 = j0 + w;
-        for (int i = r0 + warp; i < n; i += 16) {
-          double f[kCholNb];
-  #pragma unroll
-          for (int k = 0; k < kCholNb; ++k) f[k] = k < w ? A[(j0 + k) * ld + i] : 0.0;
-          for (int q = lane; q < r0 + (n - i); q += 32) {
-            const int c = q < r0 ? q : q - r0 + i;
-            double v = A[i * ld + c];
-            if (c >= j0 && c < r0) {
-  #pragma unroll
-              for (int k = 0; k < kCholNb; ++k)
-                if (k < w) v = fma(-f[k], ch.Ls[k][c - j0], v);
-            } else {
-  #pragma unroll
-              for (int k = 0; k < kCholNb; ++k)
-                if (k < w) v = fma(-f[k], A[(j0 + k) * ld + c], v);
-            }
-            A[i * ld + c] = v;
-          }
-        }
-        __syncthreads();
+        if (i > j) v = fma(-ch.rowbuf[j & 1][i], ch.rowbuf[j & 1][c], v);
       }
+      if (i < w) {
+        if (c < w && c >= i) A[(j0 + i) * ld + j0 + c] = v;
+        if (c >= kCholNb) {
+          const int q = c - kCholNb;
+          ch.Ls[i][q] = v;   // zero above the diagonal
+          if (q < i) A[(j0 + i) * ld + j0 + q] = v;
+          if (q == i) ch.xd[j0 + i] = v;
+        }
+      }
+    }
+    __syncthreads();
+    if (ch.bad) return;
+    {   // the panel's rows of the other columns: L_JJ^{-1} [X | G]
+      const int cols = n - w;
+      constexpr int kPer = kCholNb * kCholSmemMax / 512;
+      double y[kPer];
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        const int t = tid + u * 512;
+        double sum = 0.0;
+        if (t < w * cols) {
+          const int i = t / cols, q = t - i * cols;
+          const double* col = A + j0 * ld + (q < j0 ? q : q + w);
+          for (int k = 0; k <= i; ++k) sum = fma(ch.Ls[i][k], col[k * ld], sum);
+        }
+        y[u] = sum;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        const int t = tid + u * 512;
+        if (t < w * cols) {
+          const int i = t / cols, q = t - i * cols;
+          A[(j0 + i) * ld + (q < j0 ? q : q + w)] = y[u];
+        }
+      }
+    }
+    __syncthreads();
+    // rows below: columns left of the panel and the panel's own (L^{-1}), and from the diagonal on (G)
+    const int r0 = j0 + w;
+    for (int i = r0 + warp; i < n; i += 16) {
+      double f[kCholNb];
+#pragma unroll
+      for (int k = 0; k < kCholNb; ++k) f[k] = k < w ? A[(j0 + k) * ld + i] : 0.0;
+      for (int q = lane; q < r0 + (n - i); q += 32) {
+        const int c = q < r0 ? q : q - r0 + i;
+        double v = A[i * ld + c];
+        if (c >= j0 && c < r0) {
+#pragma unroll
+          for (int k = 0; k < kCholNb; ++k)
+            if (k < w) v = fma(-f[k], ch.Ls[k][c - j0], v);
+        } else {
+#pragma unroll
+          for (int k = 0; k < kCholNb; ++k)
+            if (k < w) v = fma(-f[k], A[(j0 + k) * ld + c], v);
+        }
+        A[i * ld + c] = v;
+      }
+    }
+    __syncthreads();
+  }
 }
 
 __global__ void __launch_bounds__(512) chol_inv_smem_kernel(double* Gin, int n,
@@ -740,7 +734,7 @@ __device__ __forceinline__ bool jacobi_rotation(double a, double b, double g, do
   c = (double)cf;
   s = (double)(cf * tf);
   const double d = fma(-s, s, fma(-c, c, 1.0));
-  const double f = fma(d, fma(d, 0.375, 0.5), 1.0);
+  const double f = rsqrt_corrected(1.0, d);
   c *= f;
   s *= f;
   return true;

@@ -8,20 +8,6 @@
 namespace ttgb {
 namespace red {
 
-// 1 / sqrt(d) to FP64 accuracy for a normal d > 0 from the FP32 reciprocal square root of its significand:
-// y (1 + e / 2 + 3 e^2 / 8) with e = 1 - m y^2 ~ 1e-7. Five dependent FP64 operations where sqrt and a
-// division take more than twenty, at some 80 cycles of latency each on this GPU.
-__device__ __forceinline__ double rsqrt_full(double d) {
-  const int hi = __double2hiint(d);
-  if (hi < 0x00100000 || hi >= 0x7ff00000) return 1.0 / sqrt(d);   // zero, subnormal, negative, not finite
-  const int e = ((hi >> 20) - 1023) & ~1;
-  const double m = __hiloint2double(hi - (e << 20), __double2loint(d));   // in [1, 4)
-  const double y = (double)rsqrtf((float)m);
-  const double r = fma(-m * y, y, 1.0);
-  const double v = fma(y * r, fma(r, 0.375, 0.5), y);
-  return __hiloint2double(__double2hiint(v) - ((e >> 1) << 20), __double2loint(v));
-}
-
 constexpr int RT = 256;   // threads per reduction block
 
 __device__ __forceinline__ double warp_sum(double v) {
