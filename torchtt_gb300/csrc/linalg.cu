@@ -1449,11 +1449,6 @@ void gemm_cm(const double* A, int64_t lda, const double* B, int64_t ldb, double*
   contract(c, s);
 }
 
-// Rows up to which a wide matrix goes through one Householder sweep. It takes 18 us for 3 x 6 and 51 us for 8 x
-// 12, the leading block's route some 25 us; below the line the sweep stays because the smallest systems (4
-// to 6 modes) follow the recorded trajectories only with its signs of Q.
-constexpr int64_t kHouseholderMaxRows = 8;
-
 QRResult qr(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, double* R,
             LinalgWS& ws, const RedWS& red, cudaStream_t s) {
   (void)red;
@@ -1463,14 +1458,10 @@ QRResult qr(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, doubl
   // Wide and small factors have FP64 products whatever the engine of the calling thread: the bases of the mixed
   // path's enrichment are orthonormal to rounding.
   Fp64EngineScope engine(m < n || (m < 1024 && (double)m * n * n < 4e5) ? kFp64Native : fp64_engine());
-  if (m < n && m <= kHouseholderMaxRows) {
-    householder(A, lda, m, n, Q, R, ws, s);
-    return res;
-  }
   if (m < n) {
     // Wide: a factorisation of the leading m x m block has all of Q, whatever the block's rank; the other
-    // columns of R are products. Against the sweep over the whole matrix: 10 x 15 66 -> 27 us, 16 x 24
-    // 118 -> 30, 32 x 48 307 -> 73, 48 x 64 568 -> 110.
+    // columns of R are products. Against the sweep over the whole matrix: 3 x 6 18 -> 15 us, 5 x 8 31 -> 18, 8 x 12
+    // 51 -> 19, 10 x 15 66 -> 27, 16 x 24 118 -> 30, 32 x 48 307 -> 73, 48 x 64 568 -> 110.
     qr(A, lda, m, m, Q, R, ws, red, s);
     gemm_cm(Q, m, A + m * lda, lda, R + m * m, m, m, n - m, m, 1.0, 0.0, s, true, false);
     return res;

@@ -27,8 +27,8 @@ struct QRResult {
 // Thin QR of the m x n column-major matrix A (lda): Q (m x k, ldq = m), R (k x n, ldr = k),
 // k = min(m, n). A is not modified. Tall matrices use CholeskyQR in two passes, or in three after a
 // shifted start (Gram and apply products on the contraction engine, all in one launch for small ones),
-// checked for orthogonality; wide ones take Q from their leading square block above 8 rows. A
-// single-block Householder QR does the rest: fewer rows, breakdowns, more than 1024 columns.
+// checked for orthogonality; wide ones take Q from their leading square block. A single-block Householder QR does
+// the rest: breakdowns, more than 1024 columns.
 QRResult qr(const double* A, int64_t lda, int64_t m, int64_t n, double* Q, double* R,
             LinalgWS& ws, const RedWS& red, cudaStream_t s);
 
