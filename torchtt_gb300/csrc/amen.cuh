@@ -31,7 +31,8 @@ struct AmenParams {
   int a_structure = 1;         // 1: apply A cores of density < 1/4 from their nonzeros
   // FP64 contractions of the local products, interfaces and local right-hand sides: 0 auto
   // (double-float accuracy on the mixed path when A and b lie within the FP32 exponent range, FP64
-  // otherwise), 1 FP64, 2 double-float accuracy. The factorisations always run in FP64.
+  // otherwise), 1 FP64 multiply-adds (every contraction of the solve), 2 double-float accuracy. The
+  // factorisations run in FP64, that of a direct local solve in FP32 under an FP64 refinement.
   int fp64_engine = 0;
   // 1: the sweeps solve, truncate and stop at eps / 4, so that the true relative residual ends at
   // or below eps (the reference's rule bounds only the local residuals)

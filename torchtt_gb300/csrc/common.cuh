@@ -76,12 +76,13 @@ inline unsigned cdiv(int64_t a, int64_t b) { return (unsigned)((a + b - 1) / b);
 // runtime only when the cached limit for that (kernel, device) is lower.
 void smem_optin(const void* kernel, int bytes);
 
-// Launches whose blocks may start while the kernel before them in the stream still runs (programmatic dependent
-// launch). The solvers' kernels take 2 to 10 us, and from one to the next the GPU spent 1 to 2 us on
-// draining and launching: the d = 5, n = 12 Laplacian solve took 92 ms, 76 ms this way, six served requests
-// 265 and 233 ms. A kernel launched this way calls stream_wait() in every thread before it reads or
-// writes global memory and before it returns: it waits until the kernel before it is complete and its
-// writes are visible. Its global loads are plain ones, not __ldg or loads through const __restrict__ pointers,
+// Launches that do not wait for the kernel before them to be complete (programmatic dependent launch). As no kernel
+// releases its successor early, the blocks start when all blocks of the kernel before have ended: what
+// overlaps is the launch and the flush at the end of that kernel, not its work. The solvers' kernels take 2 to 10
+// us, and from one to the next the GPU spent 1 to 2 us on these: the d = 5, n = 12 Laplacian solve took 92 ms, 76 ms
+// this way, six served requests 265 and 233 ms. A kernel launched this way calls stream_wait() in every thread
+// before it reads or writes global memory and before it returns: it waits until the kernel before it is
+// complete and its writes are visible. Its global loads are plain ones, not __ldg or loads through const __restrict__ pointers,
 // which may assume that nothing is written while the kernel runs.
 template <typename... P, typename... A>
 inline void launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {

@@ -14,8 +14,8 @@
 //           32 (w % 4) .. +31, the rows its lanes own, and one half of the columns) and write the tile
 //           with arbitrary output strides as FP32, FP64 or a new TF32 split.
 // The local products' GEMMs have K chunks to the number of 2 to 10, so a launch is a chain of latencies: set-up, one
-// copy, the MMAs, the stores. Hence the set-up, tensor maps included, runs beside the kernel before, the
-// issuer asks for a stage before it issues the previous one, and the epilogue has eight warps that
+// copy, the MMAs, the stores. Hence the set-up, tensor maps included, comes before the wait for the kernel before to be
+// complete, the issuer asks for a stage before it issues the previous one, and the epilogue has eight warps that
 // walk their columns with one division and store whole rows where C's neighbours lie along N.
 // Averages over the mixed d = 4, n = 32 solve: 6.5 -> 5.75 us (BN = 32), 9.4 -> 6.8 (64), 13.1 -> 9.6 (128).
 // Copies, tensor-core work and the other CTAs' epilogues overlap with no block-wide barrier in the
