@@ -29,17 +29,6 @@ namespace ttgb {
 
 namespace {
 
-struct AxD {  // device copy of Ax with a 32-bit inner extent
-  int e0;
-  int64_t s1, s0;
-};
-
-__device__ __forceinline__ int64_t ax_off(const AxD& a, int i) {
-  int i1 = i / a.e0;
-  int i0 = i - i1 * a.e0;
-  return (int64_t)i1 * a.s1 + (int64_t)i0 * a.s0;
-}
-
 template <typename T>
 struct KParams {
   int M, N, K, batch, splitk, kchunk;
@@ -393,19 +382,6 @@ __global__ void scale_output_kernel(T* C, int M, int N, int batch, AxD cm, AxD c
     T* c = C + (int64_t)b * c_bs + ax_off(cm, m) + ax_off(cn, n);
     *c = (beta == T(0)) ? T(0) : beta * *c;
   }
-}
-
-AxD to_dev(const Ax& a, int extent) {
-  AxD r;
-  if (a.e0 >= extent || a.e0 >= INT_MAX) {
-    r.e0 = INT_MAX;
-    r.s1 = 0;
-  } else {
-    r.e0 = (int)a.e0;
-    r.s1 = a.s1;
-  }
-  r.s0 = a.s0;
-  return r;
 }
 
 thread_local int t_fp64_engine = kFp64Native;

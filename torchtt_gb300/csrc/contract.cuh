@@ -3,6 +3,9 @@
 // (cpp/amen_solve.h:17-98, cpp/matvecs.h:196-212) are folded into addressing instead of copies.
 #pragma once
 
+#include <climits>
+
+#include "axis.cuh"
 #include "common.cuh"
 #include "sparse_a.cuh"
 
@@ -17,6 +20,20 @@ struct Ax {
   static Ax one(int64_t s) { Ax a; a.e0 = int64_t(1) << 40; a.s1 = 0; a.s0 = s; return a; }
   static Ax two(int64_t e0, int64_t s1, int64_t s0) { Ax a; a.e0 = e0; a.s1 = s1; a.s0 = s0; return a; }
 };
+
+// The device form of an index of the given extent.
+inline AxD to_dev(const Ax& a, int extent) {
+  AxD r;
+  if (a.e0 >= extent || a.e0 >= INT_MAX) {
+    r.e0 = INT_MAX;
+    r.s1 = 0;
+  } else {
+    r.e0 = (int)a.e0;
+    r.s1 = a.s1;
+  }
+  r.s0 = a.s0;
+  return r;
+}
 
 // C[b](m, n) = alpha * sum_k A[b](m, k) * B[b](k, n) + beta * C[b](m, n)
 template <typename T>

@@ -16,6 +16,7 @@
 #include <cooperative_groups.h>
 
 #include "linalg.cuh"
+#include "reduce.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -23,20 +24,14 @@ namespace ttgb {
 
 namespace {
 
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 // sum over the block, valid in every thread
 __device__ double block_sum_d(double v, double* sh) {
-  v = warp_sum_d(v);
+  v = red::warp_sum(v);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   __syncthreads();
   if (lane == 0) sh[w] = v;
   __syncthreads();
-  return warp_sum_d(lane < nw ? sh[lane] : 0.0);
+  return red::warp_sum(lane < nw ? sh[lane] : 0.0);
 }
 
 constexpr int kGjCtas = 8;      // cluster size
@@ -281,7 +276,7 @@ __global__ void __cluster_dims__(kGjCtas, 1, 1) __launch_bounds__(kGjMaxN, 1)
       const double* bi = B + (int64_t)i * n;
       double s = 0.0;
       for (int j = lane; j < n; j += 32) s = fma(bi[j], xn[j], s);
-      s = warp_sum_d(s);
+      s = red::warp_sum(s);
       if (lane == 0) g->r[i] = b[i] - s;
     }
     cluster.sync();
@@ -377,7 +372,7 @@ __global__ void __launch_bounds__(1024) lu_solve_kernel(const double* B,
   for (int i = n - 1; i >= 0; --i) {
     double s = 0.0;
     for (int c = i + 1 + tid; c < n; c += nt) s = fma(LU[(int64_t)i * n + c], x[c], s);
-    s = warp_sum_d(s);
+    s = red::warp_sum(s);
     if (lane == 0) shs[warp] = s;
     __syncthreads();
     if (tid == 0) {

@@ -13,6 +13,7 @@
 
 #include "contract.cuh"
 #include "linalg.cuh"
+#include "reduce.cuh"
 #include "rsqrt.cuh"
 
 namespace cg = cooperative_groups;
@@ -23,14 +24,8 @@ namespace {
 
 constexpr double kEps = 2.220446049250313e-16;
 
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 __device__ double block_sum_d(double v, double* sh) {
-  v = warp_sum_d(v);
+  v = red::warp_sum(v);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   __syncthreads();
   if (lane == 0) sh[w] = v;
@@ -168,7 +163,7 @@ __device__ __forceinline__ void gram_stats(const double* g, int n, int pitch, bo
   if (tid < 32) {
     double tr = 0.0;
     for (int i = lane; i < n; i += 32) tr += g[i * pitch + i];
-    tr = warp_sum_d(tr);
+    tr = red::warp_sum(tr);
     if (lane == 0) st->tr = tr;
   }
 }
@@ -403,7 +398,7 @@ __device__ __forceinline__ void householder_body(double* W, int m, int n, double
         const double c0 = cc[j];   // read by every lane before lane 0 updates it
         double w = 0.0;
         for (int i = j + 1 + lane; i < m; i += 32) w = fma(col[i], cc[i], w);
-        w = warp_sum_d(w) + c0;
+        w = red::warp_sum(w) + c0;
         const double tw = tj * w;
         if (lane == 0) cc[j] -= tw;
         for (int i = j + 1 + lane; i < m; i += 32) cc[i] = fma(-tw, col[i], cc[i]);
@@ -431,7 +426,7 @@ __device__ __forceinline__ void householder_body(double* W, int m, int n, double
       const double q0 = qc[j];
       double w = 0.0;
       for (int i = j + 1 + lane; i < m; i += 32) w = fma(col[i], qc[i], w);
-      w = warp_sum_d(w) + q0;
+      w = red::warp_sum(w) + q0;
       const double tw = tj * w;
       if (lane == 0) qc[j] -= tw;
       for (int i = j + 1 + lane; i < m; i += 32) qc[i] = fma(-tw, col[i], qc[i]);
@@ -661,7 +656,7 @@ __global__ void __launch_bounds__(512) householder_r_kernel(double* Wall, int64_
         const double c0 = cc[j];
         double w = 0.0;
         for (int i = j + 1 + lane; i < rows; i += 32) w = fma(col[i], cc[i], w);
-        w = warp_sum_d(w) + c0;
+        w = red::warp_sum(w) + c0;
         const double tw = tj * w;
         if (lane == 0) cc[j] -= tw;
         for (int i = j + 1 + lane; i < rows; i += 32) cc[i] = fma(-tw, col[i], cc[i]);
@@ -973,7 +968,7 @@ __global__ void __cluster_dims__(kJacobiCluster, 1, 1) __launch_bounds__(256)
         const double* w = (c < nb ? WA : WB) + (int64_t)(c % nb) * n;
         double a = 0.0;
         for (int i = lane; i < n; i += 32) a = fma(w[i], w[i], a);
-        a = warp_sum_d(a);
+        a = red::warp_sum(a);
         if (lane == 0) (c < nb ? NA : NB)[c % nb] = a;
       }
       __syncthreads();
@@ -1269,7 +1264,7 @@ __global__ void __launch_bounds__(256) jacobi_grid_round_kernel(double* W, doubl
       const double x = wp[k], y = wq[k];
       a = fma(x, x, a); b = fma(y, y, b); g = fma(x, y, g);
     }
-    a = warp_sum_d(a); b = warp_sum_d(b); g = warp_sum_d(g);
+    a = red::warp_sum(a); b = red::warp_sum(b); g = red::warp_sum(g);
     double c, sn;
     if (!jacobi_rotation(a, b, g, tol, c, sn)) return;
     double* vp = V + (int64_t)p * n;
@@ -1325,7 +1320,7 @@ __global__ void __launch_bounds__(1024) svd_sort_kernel(const double* W,
   for (int j = warp; j < n; j += nw) {
     double a = 0.0;
     for (int i = lane; i < n; i += 32) a = fma(W[(int64_t)j * n + i], W[(int64_t)j * n + i], a);
-    a = warp_sum_d(a);
+    a = red::warp_sum(a);
     if (lane == 0) sig[j] = sqrt(a);
   }
   __syncthreads();
@@ -1359,7 +1354,7 @@ __global__ void gemv_rm_kernel(const double* B, int64_t n, const double* x,
   if (row >= n) return;
   double s = 0.0;
   for (int64_t c = lane; c < n; c += 32) s = fma(B[row * n + c], x[c], s);
-  s = warp_sum_d(s);
+  s = red::warp_sum(s);
   if (lane == 0) y[row] = s;
 }
 

@@ -42,6 +42,7 @@
 #include <type_traits>
 
 #include "emu_digits.cuh"
+#include "mbarrier.cuh"
 #include "oz_gemm.cuh"
 
 namespace cg = cooperative_groups;
@@ -55,45 +56,15 @@ constexpr int kBK = 16;               // k per stage: one tcgen05.mma deep
 constexpr int kDig = kEmuSlices;
 constexpr int kFlushWarps = 16;
 constexpr int kThreads = 32 * (2 + kFlushWarps);
-constexpr int kWaitIters = 1 << 22;
 constexpr int kQCtas = 8;             // cluster that slices one chunk of Q
 constexpr int kQCols = 64;            // columns per CTA of it
 constexpr int kMaxQ = kQCtas * kQCols;
 constexpr int kPRows = 32;            // rows per CTA of the P slicer
 
-struct Axis {
-  int e0;
-  int64_t s1, s0;
-};
-
-Axis axis(const Ax& a, int extent) {
-  Axis r;
-  if (a.e0 >= extent || a.e0 >= INT_MAX) { r.e0 = INT_MAX; r.s1 = 0; }
-  else { r.e0 = (int)a.e0; r.s1 = a.s1; }
-  r.s0 = a.s0;
-  return r;
-}
-
-__device__ __forceinline__ int64_t at(const Axis& a, int i) {
-  const int i1 = i / a.e0;
-  return (int64_t)i1 * a.s1 + (int64_t)(i - i1 * a.e0) * a.s0;
-}
-
-// Offsets of consecutive indexes: one division at the start.
-struct Walk {
-  int64_t off;
-  int i0;
-  __device__ __forceinline__ Walk(const Axis& a, int i) : off(at(a, i)), i0(i % a.e0) {}
-  __device__ __forceinline__ void next(const Axis& a) {
-    off += a.s0;
-    if (++i0 == a.e0) { i0 = 0; off += a.s1 - (int64_t)a.e0 * a.s0; }
-  }
-};
-
-// An operand: element (row, k) of batch entry z at base[z bs + at(row) + at(k)].
+// An operand: element (row, k) of batch entry z at base[z bs + off(row) + off(k)].
 struct Operand {
   const double* base;
-  Axis row, k;
+  AxD row, k;
   int64_t bs;
   int rows, z;          // z: batch entries with digits of their own
   int blk;              // rows of a block
@@ -124,8 +95,8 @@ template <int PER>
 __device__ __forceinline__ bool load_row(double (&v)[PER], const Operand& o, int z, int row, bool ok, int k0,
                                          int K) {
   bool special = false;
-  const double* base = o.base + (int64_t)z * o.bs + (ok ? at(o.row, row) : 0);
-  Walk w(o.k, k0);
+  const double* base = o.base + (int64_t)z * o.bs + (ok ? ax_off(o.row, row) : 0);
+  AxWalk w(o.k, k0);
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
     v[i] = (ok && k0 + i < K) ? base[w.off] : 0.0;
@@ -262,10 +233,6 @@ __global__ void __launch_bounds__(256) oz_digits_p_kernel(Operand p, int K, int 
 
 // ---- product ---------------------------------------------------------------------------------------
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
 // Shared-memory matrix descriptor: K-major, no swizzle, core matrices of 8 rows x 16 bytes; 8-row groups
 // 128 bytes apart, the next 8 k `kstep` bytes on.
 __device__ __forceinline__ uint64_t desc_cores(uint32_t saddr, uint32_t kstep) {
@@ -281,39 +248,8 @@ __device__ __forceinline__ void mma_bf16_ss(uint32_t tmem, uint64_t a, uint64_t 
       "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
 }
 
-__device__ __forceinline__ bool mbar_done(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(done)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  for (int i = 0; i < kWaitIters; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
 __device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
-  return p != 0;
 }
 
 __device__ __forceinline__ void commit(uint32_t bar) {
@@ -337,7 +273,7 @@ struct OzParams {
   int scale, keep;      // alpha is not 1; beta is not 0
   int* err;             // set when a wait gave up
   double* C;
-  Axis cp, cq;          // C's axes along P's and Q's rows
+  AxD cp, cq;          // C's axes along P's and Q's rows
   int64_t c_bs;
   double alpha, beta;
 };
@@ -477,11 +413,11 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
       for (int e = tid; e < kBM * BN; e += kThreads) {
         const int i = o.r0 + e % kBM, j = o.c0 + e / kBM;
         if (i >= P.p.rows || j >= P.q.rows) continue;
-        const double* a = P.p.base + (int64_t)o.z * P.p.bs + at(P.p.row, i);
-        const double* b = P.q.base + (int64_t)o.z * P.q.bs + at(P.q.row, j);
+        const double* a = P.p.base + (int64_t)o.z * P.p.bs + ax_off(P.p.row, i);
+        const double* b = P.q.base + (int64_t)o.z * P.q.bs + ax_off(P.q.row, j);
         double s = 0.0;
-        for (int k = o.kbeg; k < o.kend; ++k) s = fma(a[at(P.p.k, k)], b[at(P.q.k, k)], s);
-        put(P.C + (int64_t)o.z * P.c_bs + at(P.cp, i) + at(P.cq, j), s);
+        for (int k = o.kbeg; k < o.kend; ++k) s = fma(a[ax_off(P.p.k, k)], b[ax_off(P.q.k, k)], s);
+        put(P.C + (int64_t)o.z * P.c_bs + ax_off(P.cp, i) + ax_off(P.cq, j), s);
       }
     }
     return;
@@ -632,8 +568,8 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
         // covers whole sectors
 #pragma unroll
         for (int c = 0; c < kPart; ++c) turn[lane * (kPart + 1) + c] = acc[c];
-        const int64_t cq = at(P.cq, col0 + (lane < kPart ? lane : 0));
-        const int64_t cp = at(P.cp, row_ok ? row : 0);
+        const int64_t cq = ax_off(P.cq, col0 + (lane < kPart ? lane : 0));
+        const int64_t cp = ax_off(P.cp, row_ok ? row : 0);
         __syncwarp();
 #pragma unroll 4
         for (int i = 0; i < kPart; ++i) {
@@ -643,8 +579,8 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
         }
         __syncwarp();
       } else if (row_ok) {
-        C += at(P.cp, row);
-        Walk w(P.cq, col0);
+        C += ax_off(P.cp, row);
+        AxWalk w(P.cq, col0);
 #pragma unroll
         for (int c = 0; c < kPart; ++c) {
           if (col0 + c < P.q.rows) put(C + w.off, acc[c]);
@@ -670,7 +606,7 @@ __global__ void __launch_bounds__(kThreads, 1) oz_gemm_kernel(const __grid_const
       for (int e = tid; e < kBM * BN; e += kThreads) {
         const int i = o.r0 + e % kBM, j = o.c0 + e / kBM;
         if (i < P.p.rows && j < P.q.rows)
-          P.C[(int64_t)o.z * P.c_bs + at(P.cp, i) + at(P.cq, j)] = __longlong_as_double(0x7ff8000000000000ll);
+          P.C[(int64_t)o.z * P.c_bs + ax_off(P.cp, i) + ax_off(P.cq, j)] = __longlong_as_double(0x7ff8000000000000ll);
       }
     }
   }
@@ -738,8 +674,8 @@ int64_t align256(int64_t bytes) { return (bytes + 255) / 256 * 256; }
 void operands(const ContractDesc& d, int q_blk, Operand& p, Operand& q) {
   const bool qa = q_is_a(d);
   Operand a, b;
-  a.base = d.A; a.row = axis(d.am, d.M); a.k = axis(d.ak, d.K); a.bs = d.batch > 1 ? d.a_bs : 0; a.rows = d.M;
-  b.base = d.B; b.row = axis(d.bn, d.N); b.k = axis(d.bk, d.K); b.bs = d.batch > 1 ? d.b_bs : 0; b.rows = d.N;
+  a.base = d.A; a.row = to_dev(d.am, d.M); a.k = to_dev(d.ak, d.K); a.bs = d.batch > 1 ? d.a_bs : 0; a.rows = d.M;
+  b.base = d.B; b.row = to_dev(d.bn, d.N); b.k = to_dev(d.bk, d.K); b.bs = d.batch > 1 ? d.b_bs : 0; b.rows = d.N;
   p = qa ? b : a;
   q = qa ? a : b;
   // Q's scales enter P's digits, so P has digits per batch entry wherever either operand differs
@@ -827,7 +763,7 @@ bool oz_contract(const ContractDesc& d, int splitk, int kchunk, cudaStream_t s) 
   P.swap = qa ? 1 : 0;
   P.tri = d.tri;
   P.C = d.C;
-  const Axis cm = axis(d.cm, d.M), cn = axis(d.cn, d.N);
+  const AxD cm = to_dev(d.cm, d.M), cn = to_dev(d.cn, d.N);
   P.cp = qa ? cn : cm;
   P.cq = qa ? cm : cn;
   P.c_bs = d.c_bs;

@@ -26,6 +26,7 @@
 
 #include <mutex>
 
+#include "mbarrier.cuh"
 #include "tc_gemm.cuh"
 
 namespace ttgb {
@@ -37,12 +38,7 @@ constexpr int kBK = 32;         // TF32 elements per K chunk = one 128-byte swiz
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 32 * (2 + kEpiWarps);   // producer, MMA, epilogue
 constexpr int kMaxStages = 6;
-constexpr int kWaitIters = 1 << 22;
 constexpr int kStageBudget = 200 * 1024;   // shared memory for the operand ring
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
 
 // Shared-memory matrix descriptor (tcgen05): K-major, 128-byte swizzle, 8-row groups 1024 B apart
 // (the layout a TMA load with CU_TENSOR_MAP_SWIZZLE_128B writes for a box of 128-byte rows).
@@ -67,38 +63,6 @@ __device__ __forceinline__ void mma_tf32(uint32_t tmem, uint64_t a, uint64_t b, 
       "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
 }
 
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  for (int i = 0; i < kWaitIters; ++i) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
-// whether the phase is complete, without waiting
-__device__ __forceinline__ bool mbar_done(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(done)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return done != 0;
-}
-
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
-  return p != 0;
-}
-
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
@@ -114,23 +78,6 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
-__device__ __forceinline__ int64_t tc_off(const TcAx& a, int i) {
-  const int i1 = i / a.e0;
-  const int i0 = i - i1 * a.e0;
-  return (int64_t)i1 * a.s1 + (int64_t)i0 * a.s0;
-}
-
-// Offsets of consecutive indexes: one division at the start.
-struct TcWalk {
-  int64_t off;
-  int i0;
-  __device__ __forceinline__ TcWalk(const TcAx& a, int i) : off(tc_off(a, i)), i0(i % a.e0) {}
-  __device__ __forceinline__ void next(const TcAx& a) {
-    off += a.s0;
-    if (++i0 == a.e0) { i0 = 0; off += a.s1 - (int64_t)a.e0 * a.s0; }
-  }
-};
-
 struct TmaParams {
   CUtensorMap a_hi, a_lo, b_hi, b_lo;   // 64-byte aligned inside the kernel parameters
   int M, N, K, stages;
@@ -141,7 +88,7 @@ struct TmaParams {
   double* C64;
   float* C_hi;
   float* C_lo;
-  TcAx cm, cn;
+  AxD cm, cn;
   int64_t c_bs;
   int turn;          // neighbours in C lie along N: the epilogue stores rows of the tile
   const int* gate;   // when non-zero at launch time every CTA returns before any set-up
@@ -273,10 +220,10 @@ __global__ void __launch_bounds__(kThreads, 1) tc_gemm_tma_kernel(const __grid_c
     const int row = m0 + q * 32 + lane;
     const bool live = ok && !*(volatile int*)&abort_sh;
     const bool row_ok = live && row < P.M;
-    const int64_t roff = row_ok ? (int64_t)bz * P.c_bs + tc_off(P.cm, row) : 0;
+    const int64_t roff = row_ok ? (int64_t)bz * P.c_bs + ax_off(P.cm, row) : 0;
     // the warp's 32 x 16 part, turned in the ring, whose copies have all been consumed
     float* part = reinterpret_cast<float*>(ring) + (warp - 2) * (32 * 17);
-    TcWalk w(P.cn, n0 + cb);
+    AxWalk w(P.cn, n0 + cb);
     const auto put = [&](int64_t o, float x) {
       if (P.out == kTcOutF32) {
         P.C32[o] = x;

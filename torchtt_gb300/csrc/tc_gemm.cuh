@@ -12,14 +12,10 @@
 // and the row counts are the true extents (the copy fills zeros beyond them).
 #pragma once
 
+#include "axis.cuh"
 #include "common.cuh"
 
 namespace ttgb {
-
-struct TcAx {         // output index -> offset, i = i1 * e0 + i0
-  int e0 = 1 << 30;
-  int64_t s1 = 0, s0 = 1;
-};
 
 enum TcOut : int { kTcOutF32 = 0, kTcOutF64 = 1, kTcOutSplit = 2 };
 
@@ -36,7 +32,7 @@ struct TcGemm {
   double* C64 = nullptr;          // kTcOutF64
   float* C_hi = nullptr;          // kTcOutSplit
   float* C_lo = nullptr;
-  TcAx cm, cn;
+  AxD cm, cn;                      // C's axes
   int64_t c_bs = 0;
   float alpha = 1.0f;
   const int* gate = nullptr;   // device flag: when non-zero at launch time the GEMM does nothing
