@@ -11,7 +11,7 @@ CODE = """
 import torch
 from torchtt_gb300 import ops
 r = lambda *s: torch.randn(*s, dtype=torch.float64, device="cuda")
-ops.local_product(r(9, 3, 9), r(12, 3, 12), r(3, 20, 20, 3), r(12, 20, 9))
+ops.local_product(r(19, 3, 19), r(22, 3, 22), r(3, 20, 20, 3), r(22, 20, 19))
 torch.cuda.synchronize()
 """
 

@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(NT) contract_small_kernel(KParams<double> p) {
   if (slice > 0) part[slice - 1][tid % (BS * BS)] = acc;
   __syncthreads();
   if (!own) return;
-  acc = (acc + part[0][tid]) + (part[1][tid] + part[2][tid]);
+  acc = ((acc + part[0][tid]) + part[1][tid]) + part[2][tid];   // in the order of k
   if (p.scale) acc *= p.alpha;
   if (p.splitk > 1) atomicAdd(c, acc);
   else *c = p.keep ? fma(p.beta, *c, acc) : acc;
@@ -397,6 +397,10 @@ thread_local bool t_no_digits = false;   // set by NoDigitsScope and set_no_digi
 // use the record. Launches that cannot be tuned (beta != 0, aliasing, a capturing stream, a
 // deterministic request) and classes being tuned by another thread use the occupancy heuristic.
 // ---------------------------------------------------------------------------------------------
+// Multiply-adds up to which a product takes the heuristic tile: it is as fast as the one chosen by time (4x5x6 solve 5.0
+// and 5.1 ms, d = 5, n = 12 Laplacian 57 and 57 ms, 58 us of a small local product both ways), and a choice
+// by time only makes the rounding, and with it the trajectory of a small solve, differ from run to run.
+constexpr double kTuneWork = 1e5;
 enum TileKind : int {
   kFma = 0,   // multiply-adds in the operand type
   kEmu = 1,   // FP64 from BF16 digits on the tensor cores (contract_emu.cuh)
@@ -739,7 +743,8 @@ void launch_contract(const ContractDescT<T>& d, cudaStream_t stream, bool determ
     return;
   }
   const int sms = num_sms();
-  if (!deterministic && autotune_on()) {
+  const double work = (double)d.M * d.N * d.K * d.batch;
+  if (!deterministic && autotune_on() && work > kTuneWork) {
     bool tuned = false;
     const int c = tuned_choice(dz, p, stream, tuned);
     // after tuning, C holds the last candidate's result: the chosen tile runs once more, so the
@@ -757,7 +762,6 @@ void launch_contract(const ContractDescT<T>& d, cudaStream_t stream, bool determ
   const int64_t target = 2 * (int64_t)sms;
   TileCfg t{64, 64, 0};
   if (std::is_same<T, double>::value) {
-    const double work = (double)d.M * d.N * d.K * d.batch;
     if (!digits_allowed(d)) t.kind = t_fp64_engine == kFp64DoubleFloat ? kDf : kFma;
     else if (work > 4e6) t.kind = kEmu;
     t.bm = t.bn = 32;
