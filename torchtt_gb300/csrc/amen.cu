@@ -638,8 +638,9 @@ void AmenRun::forward_step(int k, int swp, bool last, double& max_res) {
   }
   if (p_.verbose && res_old / res_new < damp && res_new > real_tol)
     std::printf("WARNING: residual increase. res_old %g, res_new %g, %g\n", res_old, res_new, real_tol);
-  // the comparisons of the sweep are false for a NaN and would take it as converged
-  if (!std::isfinite(norm_rhs) || (norm_rhs > 0.0 && !(std::isfinite(res_old) && std::isfinite(res_new))))
+  // the comparisons of the sweep are false for a NaN and would take it as converged (an infinite residual is above
+  // every tolerance; b = 0 has no relative residual)
+  if (!std::isfinite(norm_rhs) || (norm_rhs > 0.0 && (std::isnan(res_old) || std::isnan(res_new))))
     throw Error(kNumericalError, "AMEn: non-finite local residual");
   if (res_old > max_res) max_res = res_old;   // amen_solve.h:375
 
