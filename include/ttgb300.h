@@ -300,8 +300,9 @@ int64_t ttgb_launch_count(void);
 int ttgb_calibrate_fma(int32_t dtype, double* tflops);
 
 /* FP64 products of the calling thread (no counterpart in the reference). By default the large ones are
-   computed from digits on the tensor cores: the error is some 1e-16 of the scale of a row of the
-   left operand times the scale of a column of the right one, below that of multiply-adds, but an
+   computed from digits on the tensor cores: beside its rounding an element has an error of up to 2^-57
+   per term of the scale of a row of the left operand times that of a column of the right one, in norm
+   below that of multiply-adds, but an
    element whose own terms lie far below both scales keeps fewer digits than multiply-adds give it.
    mode 1: multiply-adds only, every element within (K + 2) 2^-53 sum |a b|; 0: the default; any
    other value only queries. Returns the previous state. A solve has the same choice in fp64_engine,

@@ -64,7 +64,7 @@ using ContractDescF = ContractDescT<float>;
 
 // Accuracy of the FP64 contractions issued by the calling thread. kFp64Native: FP64 multiply-adds or, for the
 // large ones, digit products (contract_emu.cuh, oz_gemm.cu). Those are more accurate than multiply-adds
-// relative to the scale of a row of A times the scale of a column of B (some 1e-16 of it per K chunk), but not
+// relative to the scale of a row of A times the scale of a column of B (2^-57 of it per k at most), but not
 // element by element: an element whose own terms lie far below both scales keeps fewer digits than
 // multiply-adds give it. NoDigitsScope leaves them out. kFp64DoubleFloat also admits double-float arithmetic on
 // the FP32 pipe (~1e-13 relative, for operands within the FP32 exponent range) where it is the

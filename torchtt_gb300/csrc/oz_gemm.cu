@@ -281,23 +281,22 @@ struct OzParams {
 __noinline__ __device__ double emu_round_any(long long T, int E) { return emu_round(T, E); }
 
 // The value of the eight sums over at most 128 k (weight 2^(8 (14 - d)) each) at scale exponents E, rounded
-// to nearest. The flush is bound by the issue of these instructions, so: sums 0 to 2 are at most 2^22 and
-// become integers by adding 1.5 2^23 (a conversion takes eight issue slots); sums 6 and 7, of which only
-// the bits from 2^5 and 2^13 on reach T, are rounded to multiples of 4 in the same way.
+// to nearest. Sums 0 to 2 are at most 2^22 and become integers by adding 1.5 2^23 (a conversion takes eight
+// issue slots); sum 7 is rounded to a multiple of 4 in the same way, 2^-64 of the scales.
 __device__ __forceinline__ double oz_value(const uint32_t (&D)[8], int E) {
   constexpr unsigned kOne = 0x4b400000u, kFour = 0x4c400000u;   // 1.5 2^23, 1.5 2^25
   const auto f = [&](int d) { return __uint_as_float(D[d]); };
   const auto bits = [&](int d, unsigned magic) { return __float_as_uint(f(d) + __uint_as_float(magic)); };
-  const unsigned w0 = bits(0, kOne) * 256u + bits(1, kOne) - kOne * 257u;
+  const int w0 = (int)(bits(0, kOne) * 256u + bits(1, kOne) - kOne * 257u);
   const int w1 = (int)(bits(2, kOne) * 256u + (unsigned)__float2int_rn(f(3)) - kOne * 256u);
-  const int i4 = __float2int_rn(f(4)), i5 = __float2int_rn(f(5));
-  const int q6 = (int)(bits(6, kFour) - kFour), q7 = (int)(bits(7, kFour) - kFour);
-  // sums 0 to 3 are below 2^43.1 in units of 2^88; T is in units of 2^69
-  const int low = i5 * 8 + ((q6 + (q7 >> 8) + 4) >> 3);
-  long long T = (long long)w1 * (1 << 19) + low;
-  T += (long long)i4 * 2048;
-  T += (long long)((unsigned long long)(w0 * 8u) << 32);
-  E -= 2099;
+  const int i4 = __float2int_rn(f(4)), i5 = __float2int_rn(f(5)), i6 = __float2int_rn(f(6));
+  const int q7 = (int)(bits(7, kFour) - kFour);   // sum 7 in fours
+  // sums 4 to 7 in units of 2^58, sums 0 to 3 (below 2^43.1) in units of 2^88
+  const long long low = (long long)i4 * (1 << 22) + ((long long)i5 * (1 << 14) + (long long)(i6 * 64 + q7));
+  const long long high = (long long)w0 * 65536 + w1 + (low >> 30);
+  int sh;
+  const long long T = join_words<30>(high, (unsigned)low & 0x3fffffffu, sh);
+  E += sh - 2110;   // T 2^(58 + sh) 2^(E - 2168)
   const unsigned long long m = (unsigned long long)(T < 0 ? -T : T);
   unsigned mh = (unsigned)(m >> 32), ml = (unsigned)m;
   int ef = E + 1023 + 63;
