@@ -67,8 +67,12 @@ __device__ __forceinline__ double emu_value(const float (&D)[8], int E) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) w[i] = __float2int_rn(D[2 * i]) * 256 + __float2int_rn(D[2 * i + 1]);
   const long long H = (long long)w[0] * 65536 + w[1], L = (long long)w[2] * 65536 + w[3];
-  int sh;   // |H| < 2^42.1, in units of 2^88; L in units of 2^56
-  const long long T = join_words<32>(H + (L >> 32), (unsigned)L, sh);
+  // H in units of 2^88, |H| < 2^42.1, L in units of 2^56: as T 2^sh to 62 bits or all there are, so that what an
+  // element has far below the scales of its row and column stays in T
+  const long long hi = H + (L >> 32);
+  const int sh = max(0, 34 - __clzll(hi < 0 ? ~hi : hi));
+  const unsigned long long lo = ((unsigned long long)(unsigned)L + ((1u << sh) >> 1)) >> sh;
+  const long long T = (long long)(((unsigned long long)hi << (32 - sh)) + lo);
   return emu_round(T, E - 2112 + sh);   // T 2^(56 + sh) 2^(E - 2168)
 }
 

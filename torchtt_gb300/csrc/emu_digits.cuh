@@ -73,16 +73,6 @@ __device__ __forceinline__ void digits4(const uint2 (&y)[4], unsigned (&v)[kEmuS
   }
 }
 
-// hi 2^BITS + lo (0 <= lo < 2^BITS, |hi| below 2^(BITS + 31)) as T 2^sh to 62 bits or more: what an element has far
-// below the scale of its row and column stays in T.
-template <int BITS>
-__device__ __forceinline__ long long join_words(long long hi, unsigned lo, int& sh) {
-  const int bits = 64 - __clzll(hi < 0 ? ~hi : hi);
-  sh = max(0, bits - (62 - BITS));
-  const unsigned long long low = ((unsigned long long)lo + ((1u << sh) >> 1)) >> sh;
-  return (long long)(((unsigned long long)hi << (BITS - sh)) + low);
-}
-
 // T 2^E rounded to nearest even (E below -17000: of a row or column of zeros, whose digits mean nothing).
 __device__ __forceinline__ double emu_round(long long T, int E) {
   if (T == 0 || E < -17000) return 0.0;

@@ -294,24 +294,29 @@ __device__ __forceinline__ double oz_value(const uint32_t (&D)[8], int E) {
   // sums 4 to 7 in units of 2^58, sums 0 to 3 (below 2^43.1) in units of 2^88
   const long long low = (long long)i4 * (1 << 22) + ((long long)i5 * (1 << 14) + (long long)(i6 * 64 + q7));
   const long long high = (long long)w0 * 65536 + w1 + (low >> 30);
-  int sh;
-  const long long T = join_words<30>(high, (unsigned)low & 0x3fffffffu, sh);
-  E += sh - 2110;   // T 2^(58 + sh) 2^(E - 2168)
-  const unsigned long long m = (unsigned long long)(T < 0 ? -T : T);
-  unsigned mh = (unsigned)(m >> 32), ml = (unsigned)m;
-  int ef = E + 1023 + 63;
-  if (mh == 0u) { mh = ml; ml = 0u; ef -= 32; }
-  if (mh == 0u) return 0.0;
-  const int lz = __clz((int)mh);
+  // their sum in 96 bits, its magnitude, and the leading 64 bits of that
+  unsigned v0 = ((unsigned)low & 0x3fffffffu) | (unsigned)high << 30, v1 = (unsigned)(high >> 2);
+  unsigned v2 = (unsigned)(high >> 34);
+  const unsigned sign = (unsigned)((int)v2 >> 31);
+  v0 ^= sign; v1 ^= sign; v2 ^= sign;
+  asm("{\n\tadd.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.u32 %2, %2, 0;\n\t}\n"
+      : "+r"(v0), "+r"(v1), "+r"(v2) : "r"(sign & 1u));
+  int ef = E - 2110 + 1023 + 95;   // units of 2^58 at 2^(E - 2168)
+  if (v2 == 0u) { v2 = v1; v1 = v0; v0 = 0u; ef -= 32; }
+  if (v2 == 0u) { v2 = v1; v1 = 0u; ef -= 32; }
+  if (v2 == 0u) return 0.0;
+  const int lz = __clz((int)v2);
   ef -= lz;
-  mh = __funnelshift_l(ml, mh, lz);
-  ml <<= lz;
-  if ((unsigned)(ef - 1) >= 2045u) return emu_round_any(T, E);
+  const unsigned mh = __funnelshift_l(v1, v2, lz), ml = __funnelshift_l(v0, v1, lz);
+  if ((unsigned)(ef - 1) >= 2045u) {
+    const long long T = (long long)(((unsigned long long)mh << 32 | ml) >> 2);
+    return emu_round_any(sign != 0u ? -T : T, ef - 1023 - 61);
+  }
   // 53 bits, the leading one adding itself to the exponent; a carry out of them does the same
   const unsigned long long frac = ((unsigned long long)(mh >> 11) << 32 | __funnelshift_r(ml, mh, 11)) +
                                   ((ml >> 10) & 1u);
   const unsigned hi = (unsigned)(frac >> 32) + ((unsigned)(ef - 1) << 20);
-  return __hiloint2double((int)(hi | ((unsigned)(T >> 32) & 0x80000000u)), (int)(unsigned)frac);
+  return __hiloint2double((int)(hi | (sign & 0x80000000u)), (int)(unsigned)frac);
 }
 
 template <int BN>
